@@ -13,8 +13,9 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
-SOURCES = ["runtime.cc", "loader.cc", "vmprog.cc", "static_sum.cu"]
-KERNEL = "vm_kernel.cu"      # compiled once per entry of csrc/variants.h
+SOURCES = ["runtime.cc", "loader.cc", "replan.cc", "vmprog.cc", "static_sum.cu"]
+KERNEL = "vm_kernel.cu"      # compiled once per entry of csrc/variants.h,
+PLAN_KERNEL = "plan_kernel.cu"   # except the entries named plan*, which are this one's
 OUT = os.path.join(HERE, "libb2vm.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -38,7 +39,7 @@ def variants():
     text = open(os.path.join(CSRC, "variants.h")).read()
     fam = {m.group(1): 1 << int(m.group(2))
            for m in re.finditer(r"(kFam\w+) = 1u << (\d+)", open(os.path.join(CSRC, "format.h")).read())}
-    fam["kFamAll"] = 0xFFFFFFFF
+    fam["kFamWire"] = 0x1FF
     macros = {m.group(1): m.group(2) for m in re.finditer(r"#define (B2_FAMS_\w+) \((.*?)\)\n", text)}
 
     def mask(expr: str) -> int:
@@ -69,9 +70,16 @@ def build(force: bool = False, verbose: bool = False) -> str:
     heads = _headers()
     units = [(os.path.join(CSRC, s), os.path.join(OBJ, os.path.splitext(s)[0] + ".o"), ()) for s in SOURCES]
     for name, mask in variants():
-        units.append((os.path.join(CSRC, KERNEL), os.path.join(OBJ, f"vm_kernel_{name}.o"),
+        src = PLAN_KERNEL if name.startswith("plan") else KERNEL
+        units.append((os.path.join(CSRC, src), os.path.join(OBJ, f"vm_kernel_{name}.o"),
                       (f"-DB2_VARIANT={name}", f"-DB2_FAMILIES={mask:#x}u")))
-    jobs = [u for u in units if force or _newer(u[1], [u[0], *heads])]
+    plan_only = ("plan_format.h", "replan.h", "ops_fuse.cuh", "ops_rowpipe.cuh", "ops_pairs.cuh")
+
+    def deps(u):
+        if u[0].endswith(KERNEL):       # the wire builds do not include the planned ops
+            return [u[0], *(h for h in heads if os.path.basename(h) not in plan_only)]
+        return [u[0], *heads]
+    jobs = [u for u in units if force or _newer(u[1], deps(u))]
     if jobs:
         with concurrent.futures.ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 1)) as ex:
             logs = list(ex.map(lambda j: _compile(nvcc, j[0], j[1], verbose, j[2]), jobs))

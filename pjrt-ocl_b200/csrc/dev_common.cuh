@@ -24,6 +24,12 @@ namespace b2 {
 constexpr int kSmemRed = 0;          // 64 x 16 B reduction scratch
 constexpr int kSmemPtrs = 512;       // 8 resolved pointers (MAP_REGION inputs)
 constexpr int kSmemFlag = 576;       // grid-barrier outcome, broadcast from thread 0
+// (plan_kernel.cu, which has no elementwise chain cache)
+constexpr uint32_t kSmemNextTask = 592;                      // the task about to run,
+constexpr uint32_t kSmemNextPc = kSmemNextTask + 96;         // the entry it was staged for,
+constexpr uint32_t kSmemNextDesc = kSmemNextPc + 4;          // and the descriptor (word offset) that kSmemDesc holds
+constexpr uint32_t kSmemEntries = 2048, kSmemEntriesMax = 128;   // the lane's first entries
+constexpr uint32_t kSmemDesc = 6144, kSmemDescMax = 2048;
 constexpr int kSmemChain = 1024;     // decoded elementwise chain (EwOp[kChainMax])
 constexpr int kSmemSys = 8192;
 constexpr int kChainMax = 8;
@@ -40,6 +46,21 @@ struct Lane {
 __device__ __forceinline__ uint8_t *resolve(const KParams &P, BufRef r) {
   return (r & kPortBit) ? static_cast<uint8_t *>(P.io.p[r & (kMaxIoPorts - 1)])
                         : reinterpret_cast<uint8_t *>(static_cast<uintptr_t>(r));
+}
+
+// The descriptor of a planned op in shared memory: already there when the interpreter staged it while it waited, else
+// copied by all threads. All threads call; the lane's previous task may still be reading the shared memory.
+__device__ __forceinline__ const uint8_t *planned_desc(const Lane &L, const DTask &t) {
+  volatile uint32_t *have = reinterpret_cast<volatile uint32_t *>(L.smem + kSmemNextDesc);
+  __syncthreads();
+  if (*have != t.desc) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(L.P->desc + t.desc);
+    for (uint32_t i = L.tid; i < t.desc_bytes / 16u; i += L.nthr) reinterpret_cast<uint4 *>(L.smem + kSmemDesc)[i] = src[i];
+    __syncthreads();
+    if (L.tid == 0) *have = t.desc;
+    __syncthreads();
+  }
+  return L.smem + kSmemDesc;
 }
 
 // Record the first device-side error and raise the abort flag every wait polls.

@@ -34,7 +34,10 @@ enum TileOp : uint32_t {
   kTopMax = kTopScatterIndex,
   // Not on the wire: the loader's own row op for a recognised RMS-norm idiom over bf16 rows (convert, square, row sum,
   // per-row scalar region, two broadcast multiplies, convert back), see rms_rows_tiles.
-  kTopRmsRows = 32
+  kTopRmsRows = 32,
+  // Not on the wire either: what the re-planner (replan.h) makes of groups of tile ops.
+  kTopFuseRows = 33,   // a row-local pipeline: loads, row norms, elementwise steps, row and full reductions, stores
+  kTopPairs = 34       // all-pairs sums w_ij (x_j - x_i), w_ij = m_j (|x_j - x_i|^2 s + t)^-1.5, and the short elementwise tail on them
 };
 
 // Tile-op families: the unit in which code is compiled into a build of the
@@ -50,7 +53,10 @@ enum Family : uint32_t {
   kFamIndex = 1u << 7,   // RED_WINDOW, GATHER_INDEX, SCATTER_INDEX, CONV
   kFamShort = 1u << 8,   // short-run paths of the families above: RED_SEG over segments of 2..8 elements, elementwise
                          // views and gathers whose source runs are shorter than 16 bytes, pow with constant exponents
-  kFamAll = 0xFFFFFFFFu
+  // the re-planner's own ops (no wire program names them)
+  kFamFuse = 1u << 9,    // FuseRows
+  kFamPairs = 1u << 10,  // Pairs
+  kFamWire = 0x1FFu      // every family a wire program can name
 };
 B2_HOST_DEVICE inline uint32_t family_of(uint32_t tile_op) {
   switch (tile_op) {
@@ -61,6 +67,8 @@ B2_HOST_DEVICE inline uint32_t family_of(uint32_t tile_op) {
     case kTopMapRegion: return kFamRegion;
     case kTopMma: return kFamMma;
     case kTopFlashAttn: return kFamFlash;
+    case kTopFuseRows: return kFamFuse;
+    case kTopPairs: return kFamPairs;
     default: return kFamIndex;
   }
 }
@@ -155,9 +163,9 @@ enum TaskFlags : uint32_t {
 constexpr uint32_t kMaxWorkSlots = 6;
 struct RedScratch {
   uint32_t arrived;
-  uint32_t pad[3];
+  uint32_t pad[3];                    // arrival counters of the full sums that fused ops carry (one per op of a phase); at rest 0
   uint32_t work[2 * kMaxWorkSlots];   // {next unit, lanes done} per dynamically distributed task; at rest 0
-  unsigned long long total[1];        // [n_lanes] lane totals, then [n_lanes] carry words (kRowCarrySum; at rest 0)
+  unsigned long long total[1];        // [n_lanes] lane totals, [n_lanes] carry words (kRowCarrySum; at rest 0), 3 x [n_lanes] {total, took part} of fused ops
 };
 
 struct DTask {
@@ -166,7 +174,8 @@ struct DTask {
   uint32_t p[8];        // p0..p7 as in the wire task (buffer ids already resolved elsewhere)
   uint32_t desc;        // word offset into the descriptor pool (op specific), 0 = none
   uint32_t cdt;         // dtype of ptr[3] where it matters (epilogue residual)
-  uint32_t pad[2];
+  uint32_t desc_bytes;  // planned ops: size of the descriptor (the op reads it from shared memory)
+  uint32_t pad;
 };
 static_assert(sizeof(DTask) == 96, "DTask layout");
 
@@ -180,15 +189,17 @@ struct DEntry {
 };
 static_assert(sizeof(DEntry) == 32, "DEntry layout");
 
+// What a lane reads first: its span of the entries, the first entry and that entry's task.
+struct DHead { VmLane span; DEntry entry; DTask task; };
+static_assert(sizeof(DHead) == 144, "DHead layout");
+
 enum StatusCode : uint32_t { kStOk = 0, kStBarrierTimeout = 1, kStStackOverflow = 2, kStBadOp = 3, kStTensorTimeout = 4 };
 
 // Barrier + status block in device memory (one per loaded program).
 struct DSync {
-  uint32_t arrive;       // arrival counter
-  uint32_t pad;
-  uint32_t gen;          // barrier generation   } one aligned 8-byte word: a waiting lane polls
-  uint32_t abort;        // set by the first lane } both with a single load
-                         // whose wait ran out
+  uint32_t arrive;       // arrivals so far, over all launches: n_lanes per barrier, so a multiple of n_lanes at rest
+  uint32_t abort;        // set by the first lane whose wait ran out
+  uint32_t pad[2];
   uint32_t status[4];    // code, lane, where, detail (first writer wins)
   unsigned long long barriers;   // lane 0
   unsigned long long device_ns;  // lane 0
@@ -198,7 +209,6 @@ struct DSync {
   unsigned long long phase_ns[64];
 };
 constexpr uint32_t kPhaseSlots = 64;
-static_assert(offsetof(DSync, gen) % 8 == 0 && offsetof(DSync, abort) == offsetof(DSync, gen) + 4, "gen and abort are polled as one 8-byte word");
 
 // ---- per-op descriptors the loader writes into the descriptor pool -------------
 // Descriptor the loader writes for GATHER / SCATTER / DYN_* tasks.
@@ -306,6 +316,7 @@ struct KParams {
   const DTask *tasks;
   const DEntry *entries;
   const VmLane *lanes;
+  const DHead *heads;       // one per lane (programs the re-planner made)
   const int32_t *aux;       // the program's aux pool, unmodified
   const uint64_t *desc;     // loader-built descriptor pool (views, pointers, ...)
   DSync *sync;

@@ -1,5 +1,8 @@
 // Builds the device tables for one program. See loader.h.
 #include "loader.h"
+#include "plan_format.h"
+
+#include "replan.h"
 
 #include <algorithm>
 #include <cstdlib>
@@ -48,6 +51,13 @@ bool Wide(uint32_t dt) { return dt == kI64 || dt == kF64; }
 // Buffer ids a task reads from memory (for the dead-store proof).
 void TaskReads(const VmProgram &p, const VmTask &t, std::vector<uint32_t> *r) {
   const uint32_t op = t.tile_op & 0xFFu;
+  if (IsPlannedOp(op)) {
+    const int32_t *rd, *wr, *pay;
+    int n_rd, n_wr;
+    PlannedLists(p, t, &rd, &n_rd, &wr, &n_wr, &pay);
+    for (int k = 0; k < n_rd; ++k) r->push_back(static_cast<uint32_t>(rd[k]));
+    return;
+  }
   switch (op) {
     case kTopEw:
       if (EwReadsA(t.p0)) r->push_back(t.a);
@@ -94,6 +104,15 @@ void TaskReads(const VmProgram &p, const VmTask &t, std::vector<uint32_t> *r) {
   }
 }
 
+// Buffer ids a task writes.
+void TaskWrites(const VmProgram &p, const VmTask &t, std::vector<uint32_t> *w) {
+  if (!IsPlannedOp(t.tile_op & 0xFFu)) { w->push_back(t.dst); return; }
+  const int32_t *rd, *wr, *pay;
+  int n_rd, n_wr;
+  PlannedLists(p, t, &rd, &n_rd, &wr, &n_wr, &pay);
+  for (int k = 0; k < n_wr; ++k) w->push_back(static_cast<uint32_t>(wr[k]));
+}
+
 bool ViewFromAux(const VmProgram &p, uint32_t aux_off, DView *v, std::string *err) {
   if (aux_off >= p.aux.size()) { *err = "view descriptor out of the aux pool"; return false; }
   const int32_t rank = p.aux[aux_off];
@@ -129,6 +148,59 @@ bool ViewInsideBuffer(const VmProgram &p, uint32_t aux_off, uint32_t buf, uint32
   if (AccessInside(&p.aux[aux_off + 1], &p.aux[aux_off + 1 + rank], rank, p.aux[aux_off + 1 + 2 * rank], 0, n)) return true;
   *err = "operand view reaches outside buffer " + std::to_string(buf) + " (" + std::to_string(n) + " elements)";
   return false;
+}
+
+// Is a fused step list one of the row pipelines of ops_rowpipe.cuh? Every tensor in one storage type; between the stages
+// of 16-bit rows either every value is rounded or none.
+void MatchPipe(const DFuStep *st, uint32_t n, bool whole_rows, DPipe *out) {
+  std::memset(out, 0, sizeof(*out));
+  uint32_t i = 0;
+  if (!whole_rows || n < 2 || st[0].code != kFuLoadX) return;
+  DPipe p;
+  std::memset(&p, 0, sizeof(p));
+  p.dt = st[0].dt;
+  p.flags = kRpOn;
+  p.x = st[0].ptr;
+  const bool half = p.dt != kF32;
+  int rounded = 0, plain = 0;              // stages followed / not followed by a rounding
+  i = 1;
+  auto quant = [&] {
+    if (!half) return;
+    if (i < n && st[i].code == kFuQuant && st[i].dt == p.dt) { ++i; ++rounded; } else { ++plain; }
+  };
+  auto at = [&](uint32_t k, uint32_t code) { return k < n && st[k].code == code; };
+  if (at(i, kFuLoadY) && st[i].dt == p.dt && at(i + 1, kFuAdd)) {
+    p.flags |= kRpRes;
+    p.y = st[i].ptr;
+    i += 2;
+    if (half) { if (!at(i, kFuQuant)) return; ++i; }
+    if (at(i, kFuStore) && st[i].dt == p.dt) p.mid = st[i++].ptr;
+  }
+  if (at(i, kFuLayerNorm)) {
+    p.flags |= kRpLn;
+    p.eps = st[i++].s;
+    quant();
+  } else if (at(i, kFuRedSumSq) && st[i].reg == 0 && at(i + 1, kFuSAffine) && at(i + 2, kFuSRsqrt) && at(i + 3, kFuMulS) && st[i + 3].reg == 0) {
+    p.flags |= kRpRms;
+    p.s = st[i + 1].s;
+    p.t = st[i + 1].t;
+    i += 4;
+    quant();
+  }
+  if (at(i, kFuRowVecY) && st[i].dt == p.dt && at(i + 1, kFuMul)) { p.flags |= kRpMul; p.mul = st[i].ptr; i += 2; quant(); }
+  if (at(i, kFuRowVecY) && st[i].dt == p.dt && at(i + 1, kFuAdd)) { p.flags |= kRpAdd; p.add = st[i].ptr; i += 2; quant(); }
+  if (at(i, kFuGelu)) { p.flags |= kRpGelu; ++i; quant(); }
+  if (at(i, kFuSoftmax)) { p.flags |= kRpSoftmax; ++i; quant(); }
+  if (at(i, kFuCarrySum)) { p.flags |= kRpCarry; ++i; }
+  if (at(i, kFuStore) && st[i].dt == p.dt) p.out = st[i++].ptr;
+  if (at(i, kFuCarrySum) && !(p.flags & kRpCarry)) { p.flags |= kRpCarry; ++i; }
+  if (i != n || (p.flags & (kRpLn | kRpRms | kRpSoftmax)) == 0u) return;
+  if (half) {
+    // rounded after every stage, or (the RMS norm on f32 intermediates) only at the end
+    if (plain == 0) p.flags |= kRpQ;
+    else if (!(rounded == 1 && plain >= 1 && (p.flags & (kRpLn | kRpSoftmax)) == 0u)) return;
+  }
+  *out = p;
 }
 
 // Is the view, read over the row-major flat index of a [n0, n1, n2] tensor, affine
@@ -687,7 +759,11 @@ bool RebalancePhases(const VmProgram &p, VmProgram *q, uint32_t *n_done, uint32_
 }
 
 static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, DeviceTables *out, std::string *err,
-                                 bool *unimplemented);
+                                 bool *unimplemented, bool planned = false);
+
+bool BuildPlannedTables(const VmProgram &p, uint64_t arena_base, DeviceTables *out, std::string *err, bool *unimplemented) {
+  return BuildDeviceTablesFor(p, arena_base, out, err, unimplemented, true);
+}
 
 bool BuildDeviceTables(const VmProgram &p, uint64_t arena_base, DeviceTables *out, std::string *err,
                        bool *unimplemented) {
@@ -701,10 +777,11 @@ bool BuildDeviceTables(const VmProgram &p, uint64_t arena_base, DeviceTables *ou
 }
 
 static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, DeviceTables *out, std::string *err,
-                                 bool *unimplemented) {
+                                 bool *unimplemented, bool planned) {
   *unimplemented = false;
   Ctx c{p, arena_base, {}, out};
   out->desc.assign(1, 0);
+  if (planned) out->families = 0;      // its builds hold its own ops and no others
 
   // ---- zero-copy I/O ports (runtime.cc:798-821): a buffer that is only an input
   // or only an output, is not a constant, and is among the first kMaxIoPorts such.
@@ -718,7 +795,11 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
   // A result buffer that no task ever writes (a pass-through of arena-resident
   // data) has to come out of the arena.
   std::set<uint32_t> written;
-  for (const VmTask &t : p.tasks) written.insert(t.dst);
+  for (const VmTask &t : p.tasks) {
+    std::vector<uint32_t> w;
+    TaskWrites(p, t, &w);
+    written.insert(w.begin(), w.end());
+  }
   auto times_in = [](const std::vector<uint32_t> &v, uint32_t id) { return std::count(v.begin(), v.end(), id); };
   auto assign_port = [&](uint32_t id) -> int {
     if (in_ids.count(id) && out_ids.count(id) &&
@@ -1142,6 +1223,77 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         d.desc = c.PushDesc(k);
         break;
       }
+      case kTopFuseRows: {
+        if (!planned) return fail_unimpl("tile op " + std::to_string(d.op) + " is not implemented by this backend");
+        const int32_t *rd, *wr, *x;
+        int n_rd, n_wr;
+        PlannedLists(p, t, &rd, &n_rd, &wr, &n_wr, &x);
+        std::vector<uint64_t> words((sizeof(DFuse) + sizeof(DFuStep) * static_cast<size_t>(x[2])) / 8, 0);
+        DFuse *f = reinterpret_cast<DFuse *>(words.data());
+        f->rows = static_cast<uint32_t>(x[0]);
+        f->cols = static_cast<uint32_t>(x[1]);
+        f->n_steps = static_cast<uint32_t>(x[2]);
+        f->total = x[3] ? c.Ref(static_cast<uint32_t>(x[3] - 1)) : 0;
+        f->n_owner_lanes = static_cast<uint32_t>(x[5]);
+        f->n_elems = static_cast<uint32_t>(x[6]);
+        DFuStep *fs = reinterpret_cast<DFuStep *>(f + 1);
+        bool vec = x[4] != 0;
+        for (int32_t k = 0; k < x[2]; ++k) {
+          const int32_t *w = x + 7 + 6 * k;
+          DFuStep &st = fs[k];
+          st.code = static_cast<uint32_t>(w[0]);
+          st.dt = static_cast<uint32_t>(w[1]);
+          std::memcpy(&st.s, &w[2], 4);
+          std::memcpy(&st.t, &w[3], 4);
+          st.reg = static_cast<uint32_t>(w[5]);
+          st.slot = kFuNoSlot;
+          if (w[4]) {
+            st.ptr = c.Ref(static_cast<uint32_t>(w[4] - 1));
+            vec = vec && c.Aligned16(static_cast<uint32_t>(w[4] - 1));
+          }
+        }
+        f->vec = vec ? 1u : 0u;
+        MatchPipe(fs, static_cast<uint32_t>(x[2]), f->n_elems == static_cast<uint64_t>(f->rows) * f->cols, &f->pipe);
+        if (f->total) out->needs_scratch = true;
+        d.desc = static_cast<uint32_t>(out->desc.size());
+        if (d.desc % 2) { out->desc.push_back(0); ++d.desc; }              // 16-byte copies
+        if (words.size() % 2) words.push_back(0);
+        out->desc.insert(out->desc.end(), words.begin(), words.end());
+        d.desc_bytes = static_cast<uint32_t>(words.size() * 8);
+        break;
+      }
+      case kTopPairs: {
+        if (!planned) return fail_unimpl("tile op " + std::to_string(d.op) + " is not implemented by this backend");
+        const int32_t *rd, *wr, *x;
+        int n_rd, n_wr;
+        PlannedLists(p, t, &rd, &n_rd, &wr, &n_wr, &x);
+        DPairs pr;
+        std::memset(&pr, 0, sizeof(pr));
+        pr.n = static_cast<uint32_t>(x[0]);
+        std::memcpy(&pr.s, &x[1], 4);
+        std::memcpy(&pr.t, &x[2], 4);
+        pr.pos = c.Ref(static_cast<uint32_t>(x[3]));
+        pr.mass = c.Ref(static_cast<uint32_t>(x[4]));
+        pr.out = c.Ref(static_cast<uint32_t>(x[5]));
+        pr.n_tail = static_cast<uint32_t>(x[6]);
+        for (uint32_t k = 0; k < pr.n_tail; ++k) {
+          const int32_t *w = x + 7 + 8 * k;
+          DPairTail &tl = pr.tail[k];
+          tl.sub = static_cast<uint32_t>(w[0]);
+          tl.a_src = static_cast<uint32_t>(w[1]);
+          tl.b_src = static_cast<uint32_t>(w[2]);
+          std::memcpy(&tl.s, &w[3], 4);
+          std::memcpy(&tl.t, &w[4], 4);
+          tl.dst = c.Ref(static_cast<uint32_t>(w[5]));
+          tl.a = c.Ref(static_cast<uint32_t>(w[6]));
+          tl.b = c.Ref(static_cast<uint32_t>(w[7]));
+        }
+        if (out->desc.size() % 2) out->desc.push_back(0);
+        d.desc = c.PushDesc(pr);
+        if (out->desc.size() % 2) out->desc.push_back(0);
+        d.desc_bytes = static_cast<uint32_t>((sizeof(pr) + 15) / 16 * 16);
+        break;
+      }
       default:
         return fail_unimpl("tile op " + std::to_string(d.op) + " is not implemented by this backend");
     }
@@ -1311,7 +1463,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
   // before and read by nothing else: the reduction streams the 16-bit source instead (half the bytes) and the
   // convert's phase does nothing. Straight-line programs only (phases counted by barriers in the root walk).
   std::vector<int> half_src(p.tasks.size(), -1);
-  bool straight_line = true;
+  bool straight_line = !planned;       // the re-planner has made its own fusions of this kind
   for (const VmEntry &e : p.entries)
     if (e.task == kEntWhile || e.task == kEntIf || e.task == kEntFor) straight_line = false;
   std::vector<int> phase_lo(p.tasks.size(), 1 << 30), phase_hi(p.tasks.size(), -1);

@@ -72,6 +72,9 @@ struct DeviceTables {
 bool BuildDeviceTables(const VmProgram &p, uint64_t arena_base, DeviceTables *out, std::string *err,
                        bool *unimplemented);
 
+// The same for a program the re-planner made (replan.h): its own ops are known, its cut and its phases stand.
+bool BuildPlannedTables(const VmProgram &p, uint64_t arena_base, DeviceTables *out, std::string *err, bool *unimplemented);
+
 // Collapse {dims, strides, off} to at most kViewDims dims; exposed for unit tests.
 bool CollapseView(const int32_t *dims, const int32_t *strides, int rank, int64_t off, DView *out);
 

@@ -1,0 +1,78 @@
+// Descriptors of the re-planner's own ops (replan.h), shared by the loader and plan_kernel.cu.
+#ifndef B2VM_PLAN_FORMAT_H_
+#define B2VM_PLAN_FORMAT_H_
+
+#include "format.h"
+
+namespace b2 {
+
+// ---- steps of a fused op ---------------------------------------------------------------
+//
+// A fused op carries one value X per element through a list of steps; Y holds a second operand. Values are f32
+// in registers whatever the storage type (bf16 and f16 are exact in f32; kFuQuant rounds to the type a value
+// would have been stored with). The same list format drives the row pipelines and the matmul epilogues.
+enum FuCode : uint32_t {
+  kFuLoadX = 0, kFuLoadY,          // dense operand (the op's own element index)
+  kFuRowVecY,                      // one value per column
+  kFuColVecY,                      // one value per row
+  kFuScalarY,                      // one value
+  kFuStore,                        // X to a dense result
+  kFuQuant, kFuQuantY,             // round to dt
+  kFuMovYX,                        // Y = X
+  kFuAdd, kFuMul, kFuSub, kFuRSub, kFuDiv, kFuRDiv, kFuMax, kFuMin,   // X = X op Y (R: Y op X)
+  kFuAddS, kFuMulS, kFuSubS, kFuDivS,                                 // X = X op the row scalar `reg`
+  kFuAffine, kFuGelu, kFuGeluGrad, kFuExp, kFuTanh, kFuNeg, kFuSqrt, kFuRsqrt, kFuLog, kFuAbs,   // on X
+  kFuAffineY, kFuGeluGradY,        // on Y
+  kFuRedSum, kFuRedSumSq, kFuRedMax,   // row reduction of X into row scalar `reg`
+  kFuSAffine, kFuSRsqrt,           // on row scalar `reg`
+  kFuLayerNorm, kFuSoftmax,        // whole-row normalisations of X (s = eps)
+  kFuIAdd, kFuISub, kFuIRSub, kFuIMul, kFuIAnd, kFuIOr, kFuIXor, kFuIMax, kFuIMin, kFuUMax, kFuUMin,   // X, Y as 32-bit integers
+  kFuINot, kFuINeg,
+  kFuCarrySum, kFuCarrySumSq,      // add every X (or its square) to the op's full sum
+  kFuEnd
+};
+constexpr int kFuMaxSteps = 40;
+constexpr int kFuScalars = 2;      // row scalars
+struct DFuStep {
+  uint32_t code, dt;
+  float s, t;
+  BufRef ptr;
+  uint32_t reg, slot;              // row scalar; staging slot of a dense load / row vector (kFuNoSlot: none)
+};
+constexpr uint32_t kFuNoSlot = 0xFFFFFFFFu;
+static_assert(sizeof(DFuStep) == 32, "DFuStep layout");
+// A step list that is one of the common row pipelines (ops_rowpipe.cuh), its stages in this order.
+enum PipeFlags : uint32_t {
+  kRpOn = 1u, kRpRes = 2u, kRpLn = 4u, kRpRms = 8u, kRpMul = 16u, kRpAdd = 32u, kRpGelu = 64u, kRpSoftmax = 128u, kRpCarry = 256u,
+  kRpQ = 512u                      // round to the storage type after every stage (else only the result)
+};
+struct DPipe {
+  uint32_t flags, dt;
+  float eps, s, t;
+  uint32_t pad;
+  BufRef x, y, mul, add, mid, out;
+};
+// Header of a fused-rows task's descriptor; the steps follow.
+struct DFuse {
+  uint32_t rows, cols, n_steps;
+  uint32_t vec;                    // cols % 4 == 0: 4 consecutive elements per thread and group
+  BufRef total;                    // where the full sum goes (kFuCarry*), 0 = none
+  uint32_t n_owner_lanes;          // lanes that take part in the full sum
+  DPipe pipe;                      // flags != 0: the rows run as this pipeline
+  uint32_t n_elems;                // rows x cols, or less where the last "row" of a flat list of elements is short
+  uint32_t pad;
+};
+static_assert(sizeof(DFuse) % 8 == 0, "steps follow");
+// All-pairs task: the tail is a list of elementwise ops over the n x 3 result, run by the lane on its own rows.
+constexpr int kPairTailMax = 24;
+// a_src / b_src: 0 = the buffer, 1 = the pair sum itself, 2 + k = what tail op k made
+struct DPairTail { uint32_t sub, a_src, b_src, pad; float s, t; BufRef dst, a, b; };
+struct DPairs {
+  uint32_t n, n_tail;
+  float s, t;                      // the affine on the squared distance
+  BufRef pos, mass, out;
+  DPairTail tail[kPairTailMax];
+};
+
+}  // namespace b2
+#endif

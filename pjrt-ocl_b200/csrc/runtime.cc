@@ -24,6 +24,7 @@
 #include "../../include/b2vm.h"
 #include "format.h"
 #include "loader.h"
+#include "replan.h"
 #include "variants.h"
 #include "vmprog.h"
 
@@ -161,6 +162,7 @@ struct b2_loaded {
   b2::DTask *d_tasks = nullptr;
   b2::DEntry *d_entries = nullptr;
   b2::VmLane *d_lanes = nullptr;
+  b2::DHead *d_heads = nullptr;
   int32_t *d_aux = nullptr;
   uint64_t *d_desc = nullptr;
   b2::DTmap *d_tmaps = nullptr;          // tensor maps of the tensor-core matmul operands
@@ -173,6 +175,8 @@ struct b2_loaded {
   uint8_t *d_scratch = nullptr; // lane totals of re-cut full reductions (RedScratch), when the program has one
   size_t scratch_bytes = 0;
   int variant = b2::kNumVariants - 1;   // which build of the megakernel runs this program
+  bool is_planned = false;               // prog is the re-planner's
+  b2::ReplanStats plan;
   uint64_t launches = 0;
   bool sync_dirty = true;       // the device sync block must be cleared before the next launch
   uint64_t wait_budget_ns = 2000000000ull;
@@ -234,6 +238,7 @@ b2_status Enqueue(b2_loaded *lp, const b2::IoTable &io, cudaStream_t stream, std
   kp.tasks = lp->d_tasks;
   kp.entries = lp->d_entries;
   kp.lanes = lp->d_lanes;
+  kp.heads = lp->d_heads;
   kp.aux = lp->d_aux;
   kp.desc = lp->d_desc;
   kp.sync = lp->d_sync;
@@ -461,21 +466,39 @@ b2_status b2_program_load(b2_runtime *rt, b2_program *prog, b2_loaded **out, cha
   }
   auto lp = std::make_unique<b2_loaded>();
   lp->rt = rt;
-  cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&lp->arena), std::max<uint64_t>(p.arena_bytes, 256));
+  std::string m;
+  bool unimpl = false;
+  // The smallest build of the megakernel that holds every tile-op family a set of tables uses, or -1.
+  auto build_for = [](const b2::DeviceTables &t) {
+    for (int v = 0; v < b2::kNumVariants; ++v)
+      if ((t.families & ~b2::kVariants[v].families) == 0u) return v;
+    return -1;
+  };
+  // Re-planned for this device where that fuses anything (replan.h). The program is checked as it came first: the
+  // re-planner relies on every index the tables' builder refuses to be in range.
+  b2::VmProgram planned;
+  if (p.n_lanes * 2 >= static_cast<uint32_t>(rt->prop.multiProcessorCount)) {
+    b2::DeviceTables check;
+    if (!b2::BuildDeviceTables(p, 0, &check, &m, &unimpl)) {
+      SetErr(err, err_cap, "load: " + m);
+      return unimpl ? B2_UNIMPLEMENTED : B2_INVALID_ARGUMENT;
+    }
+    b2::DeviceTables fits;
+    lp->is_planned = b2::Replan(p, static_cast<uint32_t>(rt->max_lanes), &planned, &lp->plan) &&
+                     b2::BuildPlannedTables(planned, 0, &fits, &m, &unimpl) && build_for(fits) >= 0;
+  }
+  const b2::VmProgram &use = lp->is_planned ? planned : p;
+  cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&lp->arena), std::max<uint64_t>(use.arena_bytes, 256));
   if (e != cudaSuccess) {
-    SetErr(err, err_cap, CudaMsg("arena allocation", e) + " for " + std::to_string(p.arena_bytes) + " bytes");
+    SetErr(err, err_cap, CudaMsg("arena allocation", e) + " for " + std::to_string(use.arena_bytes) + " bytes");
     cudaGetLastError();
     return B2_RESOURCE_EXHAUSTED;
   }
-  std::string m;
-  bool unimpl = false;
-  if (!b2::BuildDeviceTables(p, reinterpret_cast<uint64_t>(lp->arena), &lp->tab, &m, &unimpl)) {
+  if (!(lp->is_planned ? b2::BuildPlannedTables : b2::BuildDeviceTables)(use, reinterpret_cast<uint64_t>(lp->arena), &lp->tab, &m, &unimpl)) {
     SetErr(err, err_cap, "load: " + m);
     return unimpl ? B2_UNIMPLEMENTED : B2_INVALID_ARGUMENT;
   }
-  // The smallest build of the megakernel that holds every tile-op family the program uses.
-  for (int v = 0; v < b2::kNumVariants; ++v)
-    if ((lp->tab.families & ~b2::kVariants[v].families) == 0u) { lp->variant = v; break; }
+  lp->variant = std::max(0, build_for(lp->tab));
   if (const char *force = std::getenv("B2VM_VARIANT")) {   // measurement aid: run on a named (larger) build
     for (int v = 0; v < b2::kNumVariants; ++v)
       if (!std::strcmp(force, b2::kVariants[v].name) && (lp->tab.families & ~b2::kVariants[v].families) == 0u) lp->variant = v;
@@ -510,15 +533,24 @@ b2_status b2_program_load(b2_runtime *rt, b2_program *prog, b2_loaded **out, cha
     }
     i += group;
   }
-  std::vector<int32_t> aux = p.aux;
+  std::vector<int32_t> aux = use.aux;
+  std::vector<b2::DHead> heads(lp->tab.lanes.size());
+  for (size_t l = 0; l < heads.size(); ++l) {
+    std::memset(&heads[l], 0, sizeof(heads[l]));
+    heads[l].span = lp->tab.lanes[l];
+    heads[l].entry.task = b2::kEntNop;
+    if (!heads[l].span.count) continue;
+    heads[l].entry = lp->tab.entries[heads[l].span.off];
+    if (heads[l].entry.task < lp->tab.tasks.size()) heads[l].task = lp->tab.tasks[heads[l].entry.task];
+  }
   lp->tables_bytes = TableBytes(lp->h_tmaps.size() * sizeof(lp->h_tmaps[0])) + TableBytes(lp->tab.tasks.size() * sizeof(lp->tab.tasks[0])) +
-                     TableBytes(lp->tab.entries.size() * sizeof(lp->tab.entries[0])) + TableBytes(lp->tab.lanes.size() * sizeof(lp->tab.lanes[0])) +
+                     TableBytes(lp->tab.entries.size() * sizeof(lp->tab.entries[0])) + TableBytes(heads.size() * sizeof(heads[0])) + TableBytes(lp->tab.lanes.size() * sizeof(lp->tab.lanes[0])) +
                      TableBytes(aux.size() * sizeof(aux[0])) + TableBytes(lp->tab.desc.size() * sizeof(lp->tab.desc[0]));
   size_t toff = 0;
   if ((e = cudaMalloc(reinterpret_cast<void **>(&lp->d_tables), lp->tables_bytes)) != cudaSuccess ||
       (e = Carve(lp->d_tables, &toff, &lp->d_tmaps, lp->h_tmaps)) != cudaSuccess || (e = Carve(lp->d_tables, &toff, &lp->d_tasks, lp->tab.tasks)) != cudaSuccess ||
       (e = Carve(lp->d_tables, &toff, &lp->d_entries, lp->tab.entries)) != cudaSuccess ||
-      (e = Carve(lp->d_tables, &toff, &lp->d_lanes, lp->tab.lanes)) != cudaSuccess || (e = Carve(lp->d_tables, &toff, &lp->d_aux, aux)) != cudaSuccess ||
+      (e = Carve(lp->d_tables, &toff, &lp->d_lanes, lp->tab.lanes)) != cudaSuccess || (e = Carve(lp->d_tables, &toff, &lp->d_heads, heads)) != cudaSuccess || (e = Carve(lp->d_tables, &toff, &lp->d_aux, aux)) != cudaSuccess ||
       (e = Carve(lp->d_tables, &toff, &lp->d_desc, lp->tab.desc)) != cudaSuccess ||
       (e = cudaMalloc(reinterpret_cast<void **>(&lp->d_sync), sizeof(b2::DSync))) != cudaSuccess ||
       (e = cudaMallocHost(reinterpret_cast<void **>(&lp->h_sync), sizeof(b2::DSync))) != cudaSuccess) {
@@ -528,7 +560,7 @@ b2_status b2_program_load(b2_runtime *rt, b2_program *prog, b2_loaded **out, cha
   }
   std::memset(lp->h_sync, 0, sizeof(b2::DSync));
   if (lp->tab.needs_scratch) {
-    lp->scratch_bytes = sizeof(b2::RedScratch) + sizeof(unsigned long long) * 2u * p.n_lanes;   // zero = rest state of every counter
+    lp->scratch_bytes = sizeof(b2::RedScratch) + sizeof(unsigned long long) * 5u * use.n_lanes;   // zero = rest state of every counter
     if ((e = cudaMalloc(reinterpret_cast<void **>(&lp->d_scratch), lp->scratch_bytes)) != cudaSuccess ||
         (e = cudaMemset(lp->d_scratch, 0, lp->scratch_bytes)) != cudaSuccess) {
       SetErr(err, err_cap, CudaMsg("reduction scratch allocation", e));
@@ -536,12 +568,12 @@ b2_status b2_program_load(b2_runtime *rt, b2_program *prog, b2_loaded **out, cha
       return B2_RESOURCE_EXHAUSTED;
     }
   }
-  for (const auto &k : p.consts) {  // constants are uploaded once (runtime.cc:1064-1072)
+  for (const auto &k : use.consts) {  // constants are uploaded once (runtime.cc:1064-1072)
     if (k.data.empty()) continue;
-    e = cudaMemcpy(lp->arena + p.buffers[k.buffer].offset, k.data.data(), k.data.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpy(lp->arena + use.buffers[k.buffer].offset, k.data.data(), k.data.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { SetErr(err, err_cap, CudaMsg("constant upload", e)); return B2_INTERNAL; }
   }
-  lp->prog = std::move(prog->prog);
+  lp->prog = lp->is_planned ? std::move(planned) : std::move(prog->prog);
   delete prog;
   *out = lp.release();
   return B2_OK;
@@ -583,6 +615,11 @@ uint64_t b2_loaded_stat(const b2_loaded *lp, int which) {
     case 19: return lp->tab.n_rms_rows;
     case 20: return lp->tab.n_empty_phases_dropped;
     case 13: return static_cast<uint64_t>(std::count_if(lp->tab.inout_result.begin(), lp->tab.inout_result.end(), [](int o) { return o >= 0; }));
+    case 21: return lp->is_planned ? 1 : 0;
+    case 22: return lp->plan.fused_rows;
+    case 23: return lp->plan.pairs;
+    case 24: return lp->plan.absorbed;
+    case 25: return lp->plan.phases;
     default: return 0;
   }
 }

@@ -7,8 +7,9 @@
 // pjrt_plugin/kernels/vm_main.cl:19-27); here the mask selects what is shipped.
 //
 // B2_VARIANT_LIST(X) expands X(name, family mask) in order of preference
-// (smallest first; the last one holds everything). The build script reads the
-// same list to compile one object per entry.
+// (smallest first; `all` holds every family a wire program can name; the ones after
+// it hold the re-planner's own ops and run on plan_kernel.cu). The build script
+// reads the same list to compile one object per entry.
 #ifndef B2VM_VARIANTS_H_
 #define B2VM_VARIANTS_H_
 
@@ -20,6 +21,8 @@
   X(shortrun, B2_FAMS_STREAM | b2::kFamShort)            \
   X(matmul, B2_FAMS_STREAM | b2::kFamMma)                \
   X(attn, B2_FAMS_STREAM | b2::kFamMma | b2::kFamFlash)  \
-  X(all, b2::kFamAll)
+  X(all, b2::kFamWire)                                   \
+  X(plan_rows, b2::kFamFuse)                             \
+  X(plan_pairs, b2::kFamFuse | b2::kFamPairs)
 
 #endif

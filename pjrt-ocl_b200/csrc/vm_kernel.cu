@@ -5,8 +5,8 @@
 // python/pjrt_ocl/vmreader.py:655-773).
 //
 // Differences from the reference that the bytecode cannot see:
-//  - the grid barrier is one release-add plus an acquire-polled generation word
-//    (vm_common.cl:284-300 uses the same two words), every wait is bounded: when
+//  - the grid barrier is one release-add on a counter that every lane polls
+//    (vm_common.cl:284-300: a counter and a generation word), every wait is bounded: when
 //    the budget runs out the lane records {code, lane, barrier index}, raises an
 //    abort flag all other waits poll, and every lane leaves the kernel normally;
 //  - consecutive lane-local elementwise entries run as one fused pass (ops_ew.cuh);
@@ -28,6 +28,7 @@
 #include <cstring>
 #define B2_SHORT B2_HAS(0x100u)   // kFamShort
 #include "dev_common.cuh"
+#include "grid_barrier.cuh"
 #include "ops_ew.cuh"
 #include "ops_ew_steps.cuh"
 #if B2_HAS(0x20u)   // kFamMma
@@ -61,53 +62,6 @@ static_assert(kFamMove == 0x02u && kFamRed == 0x04u && kFamRows == 0x08u && kFam
 constexpr int kVmThreads = 512;   // threads per lane: the one instantiation the library carries
 struct Frame { uint32_t pc, end, widx, phase; };  // phase: 0 while-cond, 1 while-body, 2 if, FOR: trips left
 constexpr uint32_t kRoot = 0xFFFFFFFFu;
-
-// Grid-wide barrier over the n_lanes co-resident CTAs. Returns false when the
-// wait was abandoned (budget exhausted here or abort raised by another lane).
-// `gen` is the generation this lane expects (thread 0's copy, read once at kernel
-// entry: every lane passes every barrier, so it advances by one per call).
-// Ordering: the CTA barrier makes the lane's stores visible to thread 0, whose
-// acq_rel arrival publishes them (release is cumulative); the last arriver's release
-// on `gen` and the waiters' acquire loads of it carry them to every other lane, and
-// the closing CTA barrier to that lane's other threads.
-__device__ __forceinline__ bool grid_barrier(const Lane &L, uint32_t barrier_index, unsigned long long t_start, uint32_t &gen) {
-  const KParams &P = *L.P;
-  volatile uint32_t &ok_flag = *reinterpret_cast<volatile uint32_t *>(L.smem + kSmemFlag);
-  __syncthreads();
-  if (L.tid == 0) {
-    bool ok = true;
-    DSync *s = P.sync;
-    if (P.lane_ts && barrier_index < kPhaseSlots) P.lane_ts[L.lane * kLaneTsSlots + 2u + barrier_index] = globaltimer_ns();
-    const uint32_t prev = atom_add_acq_rel_gpu(&s->arrive, 1u);
-    if (prev == P.n_lanes - 1u) {
-      st_relaxed_gpu(&s->arrive, 0u);
-      red_release_gpu_add(&s->gen, 1u);
-      if (ld_relaxed_gpu(&s->abort)) ok = false;
-    } else {
-      const unsigned long long t0 = globaltimer_ns();
-      uint32_t spins = 0;
-      for (;;) {
-        const unsigned long long v = ld_acquire_gpu_u64(&s->gen);      // {gen, abort}
-        if (static_cast<uint32_t>(v >> 32)) { ok = false; break; }
-        if (static_cast<uint32_t>(v) != gen) break;
-        if (++spins > 32u) {
-          nanosleep_ns(64);
-          if ((spins & 255u) == 0u && globaltimer_ns() - t0 > P.wait_budget_ns) {
-            set_status(P, kStBarrierTimeout, L.lane, barrier_index, 0u);
-            ok = false;
-            break;
-          }
-        }
-      }
-    }
-    ++gen;
-    // when the phase ended for everybody: the barrier's release as lane 0 sees it
-    if (L.lane == 0 && barrier_index < kPhaseSlots) s->phase_ns[barrier_index] = globaltimer_ns() - t_start;
-    ok_flag = ok ? 1u : 0u;
-  }
-  __syncthreads();
-  return ok_flag != 0u;
-}
 
 template <int NT>
 __device__ __forceinline__ void exec_entry(const Lane &L, const DEntry &en) {
@@ -181,7 +135,8 @@ __global__ void __launch_bounds__(NT, 1) B2_VM_KERNEL(const __grid_constant__ KP
   int sp = 0;
   st[0].pc = 0; st[0].end = span.root_len; st[0].widx = kRoot; st[0].phase = 0;
   uint32_t barrier_i = 0;
-  uint32_t gen = L.tid == 0 ? ld_relaxed_gpu(&P.sync->gen) : 0u;   // thread 0's copy of the barrier generation
+  uint32_t target = 0;   // thread 0: the barrier's arrival counter once the last passed barrier was complete
+  const auto nothing = [] {};
   bool pub = false;   // a tile entry ran since the last barrier (vm_main.cl:82-100)
   bool alive = true;
 
@@ -195,7 +150,7 @@ __global__ void __launch_bounds__(NT, 1) B2_VM_KERNEL(const __grid_constant__ KP
         st[sp].pc++;
         continue;
       }
-      alive = grid_barrier(L, barrier_i++, t_start, gen);
+      alive = grid_barrier(L, barrier_i++, t_start, target, nothing);
       pub = false;
       if (!alive) break;
       if (w.task == kEntFor) {                   // one iteration done
@@ -213,7 +168,7 @@ __global__ void __launch_bounds__(NT, 1) B2_VM_KERNEL(const __grid_constant__ KP
     const uint32_t epc = f.pc;
     const DEntry en = stream[epc];
     if (en.task == kEntBarrier) {
-      alive = grid_barrier(L, barrier_i++, t_start, gen);
+      alive = grid_barrier(L, barrier_i++, t_start, target, nothing);
       pub = false;
       f.pc++;
       continue;
