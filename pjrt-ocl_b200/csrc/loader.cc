@@ -150,6 +150,19 @@ bool ViewInsideBuffer(const VmProgram &p, uint32_t aux_off, uint32_t buf, uint32
   return false;
 }
 
+// Binary ops of a chain load, (load, op) x 1..3, store over 4-byte elements (ops_flatpipe.cuh), or 0.
+uint32_t FlatOps(const DFuStep *st, uint32_t n) {
+  if (n < 4 || n > 8 || n % 2 || st[0].code != kFuLoadX || st[n - 1].code != kFuStore) return 0;
+  for (uint32_t i = 0; i < n; ++i) {
+    const bool mem = i == 0 || i == n - 1 || i % 2 == 1;
+    if (mem && st[i].dt != kF32) return 0;
+    if (i > 0 && i < n - 1 && i % 2 == 1 && st[i].code != kFuLoadY) return 0;
+    const uint32_t k = st[i].code;
+    if (!mem && !(k == kFuAdd || k == kFuMul || k == kFuSub || k == kFuRSub || k == kFuMax || k == kFuMin || (k >= kFuIAdd && k <= kFuUMin))) return 0;
+  }
+  return (n - 2) / 2;
+}
+
 // Is a fused step list one of the row pipelines of ops_rowpipe.cuh? Every tensor in one storage type; between the stages
 // of 16-bit rows either every value is rounded or none.
 void MatchPipe(const DFuStep *st, uint32_t n, bool whole_rows, DPipe *out) {
@@ -1254,6 +1267,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         }
         f->vec = vec ? 1u : 0u;
         MatchPipe(fs, static_cast<uint32_t>(x[2]), f->n_elems == static_cast<uint64_t>(f->rows) * f->cols, &f->pipe);
+        f->flat = f->vec && f->cols == 4096u ? FlatOps(fs, static_cast<uint32_t>(x[2])) : 0u;
         if (f->total) out->needs_scratch = true;
         d.desc = static_cast<uint32_t>(out->desc.size());
         if (d.desc % 2) { out->desc.push_back(0); ++d.desc; }              // 16-byte copies

@@ -402,9 +402,12 @@ static __device__ __noinline__ float fuse_rows_run(uint32_t tid, uint32_t nthr, 
 
 static __device__ __noinline__ void row_pipe_tiles(const Lane &L, const DTask &t, const DFuse &f, uint32_t tile_lo, uint32_t tile_hi);
 
+static __device__ __noinline__ void flat_pipe_tiles(const Lane &L, const DFuse &f, uint32_t tile_lo, uint32_t tile_hi);
+
 static __device__ __noinline__ void fuse_rows_tiles(const Lane &L, const DTask &t, uint32_t tile_lo, uint32_t tile_hi) {
   const KParams &P = *L.P;
   const DFuse &f = *reinterpret_cast<const DFuse *>(planned_desc(L, t));
+  if (f.flat) { flat_pipe_tiles(L, f, tile_lo, tile_hi); return; }
   if (f.pipe.flags) { row_pipe_tiles(L, t, f, tile_lo, tile_hi); return; }
   const DFuStep *ws = reinterpret_cast<const DFuStep *>(&f + 1);
   const uint32_t cols = f.cols, hi = min(tile_hi, f.rows), n = f.n_steps;
@@ -474,5 +477,6 @@ static __device__ __noinline__ void fuse_rows_tiles(const Lane &L, const DTask &
 
 }  // namespace b2
 
+#include "ops_flatpipe.cuh"
 #include "ops_rowpipe.cuh"
 #endif

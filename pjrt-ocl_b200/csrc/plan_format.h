@@ -60,7 +60,7 @@ struct DFuse {
   uint32_t n_owner_lanes;          // lanes that take part in the full sum
   DPipe pipe;                      // flags != 0: the rows run as this pipeline
   uint32_t n_elems;                // rows x cols, or less where the last "row" of a flat list of elements is short
-  uint32_t pad;
+  uint32_t flat;                   // > 0: a straight chain of so many binary ops on 4-byte elements (ops_flatpipe.cuh)
 };
 static_assert(sizeof(DFuse) % 8 == 0, "steps follow");
 // All-pairs task: the tail is a list of elementwise ops over the n x 3 result, run by the lane on its own rows.

@@ -1021,7 +1021,7 @@ bool Planner::FuseFlat(int seed) {
   if (!c.Close(&writes, true) || writes.empty()) return false;
   if (R == 1) {
     // pieces of one "row": long enough for wide accesses, short enough that every lane has several
-    C = n >= 2ull * L_ * 4096 ? 4096 : n >= 4ull * L_ * 1024 ? 1024 : 256;
+    C = n >= static_cast<uint64_t>(L_) * 4096 ? 4096 : n >= 4ull * L_ * 1024 ? 1024 : 256;
     R = (n + C - 1) / C;
   }
   return AddPlanned(RowsNode(c, start, writes, R, C, n), c.members) >= 0;
