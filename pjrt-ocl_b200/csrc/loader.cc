@@ -771,6 +771,19 @@ bool RebalancePhases(const VmProgram &p, VmProgram *q, uint32_t *n_done, uint32_
   return true;
 }
 
+bool MmaOperandLayout(const VmProgram &p, const VmTask &t, MmaLayout *o) {
+  const int64_t M = t.p0, N = t.p1, K = t.p2;
+  if ((t.p3 ? t.p3 : 1u) != 1u || M <= 0 || N <= 0 || K <= 0) return false;
+  int64_t sa[3] = {0, K, 1}, sb[3] = {0, N, 1}, gs;
+  o->a_off = o->b_off = 0;
+  std::string err;
+  DView va, vb;
+  const int64_t na[3] = {1, M, K}, nb[3] = {1, K, N};
+  if (t.p4 && (!ViewFromAux(p, t.p4 - 1, &va, &err) || !AffineOverAxes(va, na, sa, &o->a_off))) return false;
+  if (t.p5 && (!ViewFromAux(p, t.p5 - 1, &vb, &err) || !AffineOverAxes(vb, nb, sb, &o->b_off))) return false;
+  return TcOperand(M, K, 0, sa[1], sa[2], o->a_off, &o->amn, &o->a_ld, &gs) && TcOperand(N, K, 0, sb[2], sb[1], o->b_off, &o->bmn, &o->b_ld, &gs);
+}
+
 static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, DeviceTables *out, std::string *err,
                                  bool *unimplemented, bool planned = false);
 
@@ -1274,6 +1287,58 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         if (words.size() % 2) words.push_back(0);
         out->desc.insert(out->desc.end(), words.begin(), words.end());
         d.desc_bytes = static_cast<uint32_t>(words.size() * 8);
+        break;
+      }
+      case kTopGemm: {
+        if (!planned) return fail_unimpl("tile op " + std::to_string(d.op) + " is not implemented by this backend");
+        const int32_t *rd, *wr, *x;
+        int n_rd, n_wr;
+        PlannedLists(p, t, &rd, &n_rd, &wr, &n_wr, &x);
+        std::vector<uint64_t> words(sizeof(DGemm) / 8, 0);
+        DGemm *g = reinterpret_cast<DGemm *>(words.data());
+        g->n_prob = static_cast<uint32_t>(x[0]);
+        g->total = x[1] ? c.Ref(static_cast<uint32_t>(x[1] - 1)) : 0;
+        g->n_owner_lanes = static_cast<uint32_t>(x[2]);
+        if (g->total) out->needs_scratch = true;
+        for (uint32_t k = 0; k < g->n_prob; ++k) {
+          const int32_t *w = x + 3 + kGemmWords * k;
+          DGemmProb &q = g->prob[k];
+          q.M = w[0]; q.N = w[1]; q.K = w[2]; q.halves = w[3]; q.bn = w[4];
+          q.amn = w[5]; q.bmn = w[6]; q.adt = w[7];
+          q.first = g->tiles;
+          q.tm = (q.M + 128u * q.halves - 1u) / (128u * q.halves);
+          q.tn = (q.N + q.bn - 1u) / q.bn;
+          g->tiles += q.tm * q.tn;
+          q.epi = w[14]; q.qdt = w[15]; q.rdt = w[16];
+          std::memcpy(&q.s0, &w[17], 4); std::memcpy(&q.s1, &w[18], 4); std::memcpy(&q.gg, &w[19], 4);
+          q.res = w[20] ? c.Ref(static_cast<uint32_t>(w[20] - 1)) : 0;
+          q.out0 = w[21] ? c.Ref(static_cast<uint32_t>(w[21] - 1)) : 0; q.dt0 = w[22];
+          q.out1 = w[23] ? c.Ref(static_cast<uint32_t>(w[23] - 1)) : 0; q.dt1 = w[24];
+          q.tmap = static_cast<int32_t>(out->tmaps.size());
+          for (int side = 0; side < 2; ++side) {
+            TmapSpec sp;
+            std::memset(&sp, 0, sizeof(sp));
+            const bool mn = side ? q.bmn != 0 : q.amn != 0;
+            const uint64_t rows = side ? q.N : q.M;
+            const int64_t ld = w[10 + side];
+            sp.base = c.Ref(static_cast<uint32_t>(w[8 + side])); sp.off = w[12 + side]; sp.dtype = q.adt; sp.rank = 3;
+            sp.dims[0] = mn ? rows : q.K; sp.dims[1] = mn ? q.K : rows; sp.dims[2] = 1;
+            sp.strides[0] = ld; sp.strides[1] = ld * static_cast<int64_t>(sp.dims[1]);
+            sp.box[0] = 64u; sp.box[1] = 64u; sp.box[2] = 1u;
+            sp.owner_is_flash = kTmapPlanned2;
+            sp.valid = true;
+            out->tmaps.push_back(sp);
+          }
+          ++out->n_mma;
+          ++out->n_mma_tc;
+          out->mma_flops += 2ull * q.M * q.N * q.K;
+        }
+        const size_t bytes = (offsetof(DGemm, prob) + g->n_prob * sizeof(DGemmProb) + 15) / 16 * 16;
+        if (out->desc.size() % 2) out->desc.push_back(0);
+        d.desc = static_cast<uint32_t>(out->desc.size());
+        words.resize((bytes + 7) / 8, 0);
+        out->desc.insert(out->desc.end(), words.begin(), words.end());
+        d.desc_bytes = static_cast<uint32_t>(bytes);
         break;
       }
       case kTopPairs: {

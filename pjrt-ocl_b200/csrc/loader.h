@@ -29,9 +29,11 @@ struct TmapSpec {
   int64_t strides[3];     // elements, of dims[1..]; must be positive multiples of 8
   uint32_t box[4];
   uint32_t desc_word;     // where the owning DMma / DFlash sits in the descriptor pool (to clear its tmap on failure)
-  uint32_t owner_is_flash;
+  uint32_t owner_is_flash;   // 0: two maps of a matmul; 1: three of an attention task; kTmapPlanned*: of a planned op
   bool valid;             // false: known at load to be indescribable (e.g. a batch-broadcast operand)
 };
+
+constexpr uint32_t kTmapPlanned2 = 2, kTmapPlanned3 = 3;   // ... in groups of two / three
 
 struct DeviceTables {
   std::vector<DTask> tasks;
@@ -74,6 +76,11 @@ bool BuildDeviceTables(const VmProgram &p, uint64_t arena_base, DeviceTables *ou
 
 // The same for a program the re-planner made (replan.h): its own ops are known, its cut and its phases stand.
 bool BuildPlannedTables(const VmProgram &p, uint64_t arena_base, DeviceTables *out, std::string *err, bool *unimplemented);
+
+// How a 16-bit matmul task's operands lie, for the tensor cores (batch of one): unit stride along k, or along the rows /
+// columns (`mn`), leading dimension and offset in elements. False where they cannot be fed directly.
+struct MmaLayout { bool amn, bmn; int64_t a_ld, b_ld, a_off, b_off; };
+bool MmaOperandLayout(const VmProgram &p, const VmTask &t, MmaLayout *out);
 
 // Collapse {dims, strides, off} to at most kViewDims dims; exposed for unit tests.
 bool CollapseView(const int32_t *dims, const int32_t *strides, int rank, int64_t off, DView *out);

@@ -48,12 +48,12 @@ __device__ __forceinline__ float rsqrt_nr(float x) {
 }
 
 // d/dz of tanh-GELU with the micro-ops, roundings and tanh of the region it replaces.
-__device__ __forceinline__ float gelu_grad(float z) {
+__device__ __forceinline__ float gelu_grad(float z, float c) {      // c = 3 x 0.7978845608 x 0.044715 as the program rounds it
   const float z2 = __fmul_rn(z, z);
   const float w = __fadd_rn(z, __fmul_rn(__fmul_rn(z2, z), 0.044715f));
   const float th = fast_tanh(__fmul_rn(w, 0.7978845608f));
   const float sech2 = __fadd_rn(-__fmul_rn(th, th), 1.0f);
-  const float du = __fadd_rn(__fmul_rn(z2, static_cast<float>(3.0 * 0.7978845608 * 0.044715)), 0.7978845608f);
+  const float du = __fadd_rn(__fmul_rn(z2, c), 0.7978845608f);
   const float a = __fadd_rn(__fmul_rn(th, 0.5f), 0.5f);
   const float b = __fmul_rn(__fmul_rn(z, 0.5f), __fmul_rn(sech2, du));
   return __fadd_rn(a, b);
@@ -310,8 +310,8 @@ static __device__ __noinline__ float fuse_rows_run(uint32_t tid, uint32_t nthr, 
         case kFuAffine: { const float s = st.s, t = st.t; B2_FU_ALL(X[g][e] = affine2(X[g][e], s, t)) break; }
         case kFuAffineY: { const float s = st.s, t = st.t; B2_FU_ALL(Y[g][e] = affine2(Y[g][e], s, t)) break; }
         case kFuGelu: B2_FU_ALL(X[g][e] = gelu_tanh(X[g][e])) break;
-        case kFuGeluGrad: B2_FU_ALL(X[g][e] = gelu_grad(X[g][e])) break;
-        case kFuGeluGradY: B2_FU_ALL(Y[g][e] = gelu_grad(Y[g][e])) break;
+        case kFuGeluGrad: B2_FU_ALL(X[g][e] = gelu_grad(X[g][e], st.s)) break;
+        case kFuGeluGradY: B2_FU_ALL(Y[g][e] = gelu_grad(Y[g][e], st.s)) break;
         case kFuExp: if constexpr (RARE) { B2_FU_ALL(X[g][e] = expf(X[g][e])) } break;
         case kFuTanh: if constexpr (RARE) { B2_FU_ALL(X[g][e] = tanhf(X[g][e])) } break;
         case kFuNeg: B2_FU_ALL(X[g][e] = -X[g][e]) break;

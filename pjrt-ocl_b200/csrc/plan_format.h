@@ -74,5 +74,36 @@ struct DPairs {
   DPairTail tail[kPairTailMax];
 };
 
+// ---- matmuls ------------------------------------------------------------------------------
+// What happens to an accumulated element, in this order.
+enum GemmEpi_ : uint32_t {
+  kGeQuant0 = 1u,          // round to the product's own 16-bit type (and, with out0, store it)
+  kGeGelu = 2u,
+  kGeScale0 = 4u,          // times s0
+  kGeMaxS = 8u,            // max with s1
+  kGeRes = 16u,            // with the residual's element:
+  kGeResAdd = 0u << 8, kGeResSub = 1u << 8, kGeResRSub = 2u << 8, kGeResMul = 3u << 8, kGeResGeluGrad = 4u << 8, kGeResMask = 7u << 8,
+  kGeCarrySq = 32u,        // add its square to the task's full sum
+  kGeScale1 = 64u          // times s1
+};
+struct DGemmProb {
+  uint32_t first, tm, tn;          // number of its first tile; tile grid
+  uint32_t halves, bn;             // a tile is halves x 128 rows by bn columns
+  uint32_t M, N, K;
+  uint32_t amn, bmn;               // operand's unit stride runs along its rows / columns instead of k
+  uint32_t adt, dt0, dt1;
+  int32_t tmap;
+  uint32_t epi, qdt, rdt;
+  float s0, s1, gg;                // gg: the GELU derivative's free constant
+  BufRef res, out0, out1;
+};
+constexpr int kGemmMaxProbs = 6;
+struct DGemm {
+  uint32_t n_prob, tiles;
+  BufRef total;
+  uint32_t n_owner_lanes, pad;
+  DGemmProb prob[kGemmMaxProbs];
+};
+
 }  // namespace b2
 #endif

@@ -24,9 +24,12 @@
 #if B2_HAS(0x400u)  // kFamPairs
 #include "ops_pairs.cuh"
 #endif
+#if B2_HAS(0x800u)  // kFamGemm
+#include "ops_gemm.cuh"
+#endif
 
 namespace b2 {
-static_assert(kFamFuse == 0x200u && kFamPairs == 0x400u, "the literals in the #if lines above");
+static_assert(kFamFuse == 0x200u && kFamPairs == 0x400u && kFamGemm == 0x800u, "the literals in the #if lines above");
 
 constexpr int kVmThreads = 512;
 constexpr uint32_t kNoPc = 0xFFFFFFFFu;
@@ -136,6 +139,9 @@ __global__ void __launch_bounds__(kVmThreads, 1) B2_PLAN_KERNEL(const __grid_con
 #endif
 #if B2_HAS(0x400u)
         case kTopPairs: pairs_tiles(L, t, en.tile_lo, en.tile_hi); break;
+#endif
+#if B2_HAS(0x800u)
+        case kTopGemm: gemm_tiles(L, t, en.tile_lo, en.tile_hi); break;
 #endif
         default:
           if (L.tid == 0) set_status(P, kStBadOp, L.lane, en.task, t.op);

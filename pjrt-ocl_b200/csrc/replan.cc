@@ -14,7 +14,7 @@
 
 namespace b2 {
 
-bool IsPlannedOp(uint32_t op) { return op == kTopFuseRows || op == kTopPairs; }
+bool IsPlannedOp(uint32_t op) { return op >= kTopFuseRows && op <= kTopPlanLast; }
 
 void PlannedLists(const VmProgram &p, const VmTask &t, const int32_t **reads, int *n_reads, const int32_t **writes, int *n_writes,
                   const int32_t **payload) {
@@ -47,6 +47,7 @@ struct Node {
   std::vector<uint32_t> rd, wr;
   std::vector<int32_t> payload;
   int carry_slot = -1;       // full sum counter it uses
+  bool by_slot = false;      // entries name {lane slot, slots} instead of a tile range (matmuls)
   size_t owner_word = 0;     // payload word that takes the number of owner lanes (carry_slot >= 0)
 };
 
@@ -98,6 +99,9 @@ class Planner {
 
   struct Chain;
   bool FusePairs(int seed);
+  bool FuseGemm(int seed);
+  bool GemmEpilogue(const Chain &c, uint32_t dst, std::vector<int32_t> *w) const;
+  void GroupGemms(std::vector<int> *live, std::map<std::pair<int, int>, std::vector<int>> *phases, std::vector<std::vector<int>> *of);
   bool FuseRows(int seed);
   bool FuseFlat(int seed);
   Node RowsNode(const Chain &c, uint32_t start, const std::vector<uint32_t> &writes, uint64_t R, uint64_t C, uint64_t n) const;
@@ -517,7 +521,8 @@ struct Planner::Chain {
   std::map<uint32_t, uint32_t> scalars;  // [R] buffer -> row scalar register
   int total = -1;                        // buffer of the full sum, if any
   uint32_t cur = 0;
-  int n_norms = 0, n_work = 0;
+  int n_norms = 0, n_work = 0, n_through = 0;
+  int limit = 1 << 30;                   // elementwise tasks to go through at most
 
   Chain(Planner &p, uint64_t r, uint64_t c, bool rw) : P(p), R(r), C(c), rows(rw) {}
 
@@ -861,10 +866,11 @@ struct Planner::Chain {
       });
       bool moved = false;
       for (int i : cand) {
-        if (!Open(i) || P.n_[i].region != region || steps.size() + 8 > kFuMaxSteps) continue;
+        if (!Open(i) || P.n_[i].region != region || steps.size() + 8 > kFuMaxSteps || n_through >= limit) continue;
         if (!Norm(i) && !Through(i)) continue;
         cur = P.n_[i].t.dst;
         ++n_work;
+        ++n_through;
         moved = true;
         break;
       }
@@ -919,6 +925,196 @@ struct Planner::Chain {
     return steps.size() <= static_cast<size_t>(kFuMaxSteps);
   }
 };
+
+// A chain's steps as the store epilogue of the product that makes `dst`: fills words 14 .. 24 of its payload.
+bool Planner::GemmEpilogue(const Chain &c, uint32_t dst, std::vector<int32_t> *w) const {
+  const auto &st = c.steps;
+  const bool half = Half(Dt(dst));
+  uint32_t flags = 0, rdt = 0, dt0 = 0, dt1 = 0;
+  float s0 = 0, s1 = 0, gg = 0;
+  int64_t res = -1, out0 = -1, out1 = -1;
+  size_t i = 0;
+  const size_t n = st.size();
+  auto at = [&](size_t k, uint32_t code) { return k < n && st[k].code == code; };
+  auto plain_scale = [&](size_t k) { return at(k, kFuAffine) && st[k].t == 0.0f; };
+  if (n > 1 && half) flags |= kGeQuant0;
+  if (at(0, kFuStore) && n > 1) { out0 = st[0].id; dt0 = st[0].dt; i = 1; }
+  bool rounded = true;                // the value in hand is as the program would have stored it
+  auto quant = [&](uint32_t dt) { if (at(i, kFuQuant)) { if (st[i].dt != dt) return false; ++i; rounded = true; } return true; };
+  uint32_t last_dt = Dt(dst);
+  if (at(i, kFuGelu)) { flags |= kGeGelu; ++i; rounded = !half; if (!quant(last_dt)) return false; if (i + 1 < n) return false; }
+  if (plain_scale(i) && (at(i + 1, kFuLoadY))) { flags |= kGeScale0; s0 = st[i].s; ++i; if (at(i, kFuQuant)) return false; }
+  if (at(i, kFuScalarY) && at(i + 1, kFuMax)) {
+    bool known = false;
+    for (const auto &k : p_.consts)
+      if (k.buffer == static_cast<uint32_t>(st[i].id) && st[i].dt == kF32 && k.data.size() >= 4 && !written_.count(k.buffer)) {
+        uint32_t u;
+        std::memcpy(&u, k.data.data(), 4);
+        s1 = BitsF(u);
+        known = true;
+      }
+    if (!known) return false;
+    flags |= kGeMaxS;
+    i += 2;
+    if (at(i, kFuQuant)) ++i;
+  }
+  if (at(i, kFuLoadY)) {
+    res = st[i].id;
+    rdt = st[i].dt;
+    ++i;
+    flags |= kGeRes;
+    if (at(i, kFuGeluGradY)) { gg = st[i].s; ++i; if (!at(i, kFuMul)) return false; flags |= kGeResGeluGrad; ++i; }
+    else if (at(i, kFuAdd)) { flags |= kGeResAdd; ++i; }
+    else if (at(i, kFuSub)) { flags |= kGeResSub; ++i; }
+    else if (at(i, kFuRSub)) { flags |= kGeResRSub; ++i; }
+    else if (at(i, kFuMul)) { flags |= kGeResMul; ++i; }
+    else return false;
+    if (at(i, kFuCarrySumSq)) { flags |= kGeCarrySq; ++i; }
+    if (plain_scale(i) && !(flags & kGeMaxS)) { flags |= kGeScale1; s1 = st[i].s; ++i; }
+    if (at(i, kFuQuant)) ++i;
+  }
+  if (!(i + 1 == n && at(i, kFuStore))) return false;
+  out1 = st[i].id;
+  dt1 = st[i].dt;
+  (void)rounded;
+  *w = {static_cast<int32_t>(flags), static_cast<int32_t>(Dt(dst)), static_cast<int32_t>(rdt), FBits(s0), FBits(s1), FBits(gg),
+        static_cast<int32_t>(res + 1), static_cast<int32_t>(out0 + 1), static_cast<int32_t>(dt0), static_cast<int32_t>(out1 + 1), static_cast<int32_t>(dt1)};
+  return true;
+}
+
+// A 16-bit matmul and the elementwise tasks on its result that a store epilogue can do.
+bool Planner::FuseGemm(int seed) {
+  const Node &sd = n_[seed];
+  const VmTask t = sd.t;
+  if (!Half(sd.adt) || !IsFloatDt(sd.dt) || Dt(t.a) != sd.adt || Dt(t.b) != sd.adt || Dt(t.dst) != sd.dt) return false;
+  MmaLayout lay;
+  if (!MmaOperandLayout(p_, t, &lay)) return false;
+  for (int64_t v : {lay.a_ld, lay.b_ld, lay.a_off, lay.b_off}) if (v > 0x7fffffff) return false;
+  // as many of the tasks that follow as the epilogue has room for: all that the chain takes, then ever fewer
+  for (int limit = 1 << 30; limit >= 0;) {
+    Chain c(*this, t.p0, t.p1, false);
+    c.Take(seed);
+    c.limit = limit;
+    std::vector<int32_t> epi;
+    std::vector<uint32_t> writes;
+    if (t.p6) {
+      // its own store epilogue: GELU, or a residual sum, on the accumulator
+      const int32_t *e = &p_.aux[t.p6 - 1];
+      if (e[0] != 1) return false;
+      uint32_t flags;
+      int64_t res = -1;
+      if (e[1] == static_cast<int32_t>(kGelu)) flags = kGeGelu;
+      else if (e[1] == static_cast<int32_t>(kAdd) && e[2] == 1 && IsFloatDt(Dt(t.p7))) { flags = kGeRes | kGeResAdd; res = t.p7; c.reads.push_back(t.p7); }
+      else return false;
+      epi = {static_cast<int32_t>(flags), static_cast<int32_t>(Dt(t.dst)), res >= 0 ? static_cast<int32_t>(Dt(t.p7)) : 0, 0, 0, 0, static_cast<int32_t>(res + 1), 0, 0,
+             static_cast<int32_t>(t.dst + 1), static_cast<int32_t>(Dt(t.dst))};
+      writes = {t.dst};
+    } else {
+      c.Follow(t.dst, sd.region);
+      limit = std::min(limit, c.n_through) - 1;
+      c.Trim();
+      if (!c.Close(&writes, false) || writes.empty() || !GemmEpilogue(c, t.dst, &epi)) continue;
+    }
+    Node nd;
+    nd.op = kTopGemm;
+    nd.dt = sd.dt; nd.adt = sd.adt;
+    nd.t = VmTask{};
+    nd.t.dst = writes[0];
+    nd.t.a = t.a; nd.t.b = t.b;
+    nd.rd = c.reads;
+    nd.rd.push_back(t.a);
+    nd.rd.push_back(t.b);
+    nd.wr = writes;
+    nd.tiles = 1;
+    nd.by_slot = true;
+    nd.carry_slot = c.total >= 0 ? 0 : -1;
+    nd.owner_word = 2;
+    nd.payload = {1, c.total + 1, 0, static_cast<int32_t>(t.p0), static_cast<int32_t>(t.p1), static_cast<int32_t>(t.p2), 0, 0, lay.amn ? 1 : 0, lay.bmn ? 1 : 0,
+                  static_cast<int32_t>(sd.adt), static_cast<int32_t>(t.a), static_cast<int32_t>(t.b), static_cast<int32_t>(lay.a_ld), static_cast<int32_t>(lay.b_ld),
+                  static_cast<int32_t>(lay.a_off), static_cast<int32_t>(lay.b_off)};
+    nd.payload.insert(nd.payload.end(), epi.begin(), epi.end());
+    if (AddPlanned(nd, c.members) >= 0) return true;
+    if (t.p6) return false;
+  }
+  return false;
+}
+
+// Matmuls of one phase become one task (deepest first), and every product gets its tile shape. A lane's time for a tile is
+// the larger of its tensor cycles (2 per column and half, per 64 k) and what it pulls through L2 (~36 bytes per cycle and SM: what
+// 128 x 256 tiles were measured to get), plus the part of the epilogue that nothing hides.
+void Planner::GroupGemms(std::vector<int> *live, std::map<std::pair<int, int>, std::vector<int>> *phases, std::vector<std::vector<int>> *of) {
+  for (auto &kv : *phases) {
+    std::vector<int> gs, rest;
+    for (int u : kv.second) (n_[u].op == kTopGemm && n_[u].planned ? gs : rest).push_back(u);
+    if (gs.empty()) continue;
+    std::sort(gs.begin(), gs.end(), [&](int a, int b) { return n_[a].payload[5] > n_[b].payload[5]; });
+    std::vector<int> heads;
+    for (int g : gs) {
+      int into = -1;
+      for (int h : heads)
+        if (n_[h].payload[0] < kGemmMaxProbs && !(n_[h].carry_slot >= 0 && n_[g].carry_slot >= 0)) { into = h; break; }
+      if (into < 0) { heads.push_back(g); continue; }
+      Node &h = n_[into];
+      const Node &x = n_[g];
+      h.payload[0] += 1;
+      if (x.carry_slot >= 0) { h.payload[1] = x.payload[1]; h.carry_slot = 0; }
+      h.payload.insert(h.payload.end(), x.payload.begin() + 3, x.payload.end());
+      h.rd.insert(h.rd.end(), x.rd.begin(), x.rd.end());
+      h.wr.insert(h.wr.end(), x.wr.begin(), x.wr.end());
+      live->erase(std::find(live->begin(), live->end(), g));
+      for (int &r : rep_) if (r == g) r = into;
+      (*of)[g].clear();
+    }
+    for (int h : heads) {
+      Node &nd = n_[h];
+      const int np = nd.payload[0];
+      static const int shapes[6][2] = {{2, 256}, {1, 256}, {2, 128}, {1, 128}, {2, 64}, {1, 64}};
+      auto tile_cost = [&](int p, int s) {
+        const int32_t *w = &nd.payload[3 + kGemmWords * p];
+        const double kb = (w[2] + 63) / 64, hv = shapes[s][0], bn = std::min<double>(shapes[s][1], (w[1] + 15) / 16 * 16);
+        const double rows = std::min<double>(hv * 128, (w[0] + 127) / 128 * 128);
+        const double tensor = 2.0 * bn * rows / 128, l2 = (rows + bn) * 128 / 36.0;
+        return kb * std::max(tensor, l2) + (hv == 2 && bn > 128 ? 1500 : 900) + (hv * bn) * 1.0;
+      };
+      auto tiles = [&](int p, int s) {
+        const int32_t *w = &nd.payload[3 + kGemmWords * p];
+        return static_cast<double>((w[0] + 128 * shapes[s][0] - 1) / (128 * shapes[s][0])) * ((w[1] + shapes[s][1] - 1) / shapes[s][1]);
+      };
+      std::vector<int> best(np, 0);
+      double best_t = 1e300;
+      const int combos = np == 1 ? 6 : np == 2 ? 36 : np == 3 ? 216 : 6;
+      for (int k = 0; k < combos; ++k) {
+        std::vector<int> sh(np);
+        for (int p = 0, q = k; p < np; ++p) { sh[p] = np <= 3 ? q % 6 : k; if (np <= 3) q /= 6; }
+        // the lanes' loads when tiles are dealt out in order
+        double load_max = 0, at = 0;
+        std::vector<double> load(L_, 0.0);
+        uint64_t next = 0;
+        for (int p = 0; p < np; ++p) {
+          const double T = tiles(p, sh[p]), c = tile_cost(p, sh[p]);
+          const uint64_t n = static_cast<uint64_t>(T), whole = n / L_, left = n % L_;
+          for (uint32_t l = 0; l < L_; ++l) load[l] += c * static_cast<double>(whole);
+          for (uint64_t i = 0; i < left; ++i) load[(next + i) % L_] += c;
+          next += n;
+          at += c;
+        }
+        for (double x : load) load_max = std::max(load_max, x);
+        if (load_max < best_t) { best_t = load_max; best = sh; }
+      }
+      uint64_t total = 0;
+      for (int p = 0; p < np; ++p) {
+        int32_t *w = &nd.payload[3 + kGemmWords * p];
+        w[3] = shapes[best[p]][0];
+        w[4] = shapes[best[p]][1];
+        total += static_cast<uint64_t>(tiles(p, best[p]));
+      }
+      nd.tiles = static_cast<uint32_t>(std::min<uint64_t>(total, 0x7fffffffu));
+      nd.cost = best_t * L_ / std::max<double>(1.0, static_cast<double>(total)) / 6000.0;      // a 4096-element tile of work ~ 6000 cycles
+      rest.push_back(h);
+    }
+    kv.second = rest;
+  }
+}
 
 // A row pipeline around a row norm or a row reduction: back along the elementwise tasks that lead to it, then forward.
 bool Planner::FuseRows(int seed) {
@@ -1088,6 +1284,7 @@ bool Planner::Assemble(VmProgram *q, ReplanStats *st) {
   }
   std::map<std::pair<int, int>, std::vector<int>> phases;        // (region, level) -> units
   for (int i : live) if (unit[i] == i) phases[{n_[i].region, level[i]}].push_back(i);
+  GroupGemms(&live, &phases, &of);
 
   // ---- the program ----
   *q = p_;
@@ -1176,6 +1373,22 @@ bool Planner::Assemble(VmProgram *q, ReplanStats *st) {
         at += c * static_cast<double>(T);
       }
       uint32_t owners = 0;
+      if (n_[us[k]].by_slot) {
+        // a share of the lanes, each with a slot number (alone in the phase: all of them, as many as there are tiles)
+        std::vector<uint32_t> mine;
+        for (uint32_t l = 0; l < L_; ++l)
+          if (us.size() == 1 ? l < T : cut[k][l].second > cut[k][l].first) mine.push_back(l);
+        owners = static_cast<uint32_t>(mine.size());
+        for (uint32_t i = 0; i < owners; ++i) {
+          VmEntry e = blank;
+          e.task = task_of[us[k]];
+          e.tile_lo = i;
+          e.tile_hi = owners;
+          stream[mine[i]].push_back(e);
+        }
+        if (n_[us[k]].carry_slot >= 0) q->aux[payload_at[us[k]] + n_[us[k]].owner_word] = static_cast<int32_t>(owners);
+        continue;
+      }
       for (uint32_t l = 0; l < L_; ++l) {
         if (cut[k][l].second <= cut[k][l].first) continue;
         ++owners;
@@ -1267,6 +1480,8 @@ bool Planner::Run(VmProgram *q, ReplanStats *st) {
   if (!Extract()) return false;
   for (int i = 0; i < n_orig_; ++i)
     if (Free(i) && n_[i].op == kTopRedStrided && FusePairs(i)) ++st->pairs;
+  for (int i = 0; i < n_orig_; ++i)
+    if (Free(i) && n_[i].op == kTopMma && FuseGemm(i)) ++st->gemms;
   for (int i = 0; i < n_orig_; ++i)
     if (Free(i) && (n_[i].op == kTopLayernormSeg || n_[i].op == kTopSoftmaxSeg || n_[i].op == kTopRedSeg) && FuseRows(i)) ++st->fused_rows;
   for (int i = 0; i < n_orig_; ++i)

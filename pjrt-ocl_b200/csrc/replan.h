@@ -22,6 +22,7 @@ namespace b2 {
 struct ReplanStats {
   uint32_t fused_rows = 0;   // row pipelines
   uint32_t pairs = 0;        // all-pairs evaluations
+  uint32_t gemms = 0;        // matmuls with what followed them as store epilogue
   uint32_t absorbed = 0;     // tasks of the program that no longer exist
   uint32_t phases = 0;       // barrier phases of the new plan (root and loop body)
 };
@@ -32,6 +33,10 @@ bool Replan(const VmProgram &p, uint32_t device_lanes, VmProgram *q, ReplanStats
 bool IsPlannedOp(uint32_t tile_op);
 void PlannedLists(const VmProgram &p, const VmTask &t, const int32_t **reads, int *n_reads, const int32_t **writes, int *n_writes,
                   const int32_t **payload);
+
+// Words per product in a kTopGemm payload {n, total + 1, owner lanes, products}: M N K halves bn amn bmn adt a b a_ld b_ld a_off b_off
+// epi qdt rdt s0 s1 gg res+1 out0+1 dt0 out1+1 dt1.
+constexpr int kGemmWords = 25;
 
 }  // namespace b2
 #endif

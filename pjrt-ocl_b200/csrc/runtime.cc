@@ -510,7 +510,8 @@ b2_status b2_program_load(b2_runtime *rt, b2_program *prog, b2_loaded **out, cha
   lp->tmap_base.assign(lp->tab.tmaps.size(), nullptr);
   lp->tmap_off.assign(lp->tab.tmaps.size(), 0);
   for (size_t i = 0; i < lp->tab.tmaps.size();) {
-    const size_t group = lp->tab.tmaps[i].owner_is_flash ? 3 : 2;   // Q K V, or A B
+    const uint32_t owner = lp->tab.tmaps[i].owner_is_flash;
+    const size_t group = owner == 1 || owner == b2::kTmapPlanned3 ? 3 : 2;   // Q K V, or A B
     bool ok = i + group <= lp->tab.tmaps.size();
     for (size_t j = i; ok && j < i + group; ++j) {
       const b2::TmapSpec &sp = lp->tab.tmaps[j];
@@ -519,10 +520,14 @@ b2_status b2_program_load(b2_runtime *rt, b2_program *prog, b2_loaded **out, cha
       ok = ok && EncodeTmap(sp, base, &lp->h_tmaps[j]);
       lp->tmap_base[j] = port ? nullptr : base;
     }
+    if (!ok && owner >= b2::kTmapPlanned2) {       // the planner only takes operands a map can describe
+      SetErr(err, err_cap, "load: the driver refused a matmul operand's tensor map");
+      return B2_INTERNAL;
+    }
     if (!ok) {
       // the task keeps its other path: per-thread copies (matmul) or the CUDA-core kernel (attention)
       uint64_t *dw = &lp->tab.desc[lp->tab.tmaps[i].desc_word];
-      if (lp->tab.tmaps[i].owner_is_flash) {
+      if (owner) {
         b2::DFlash *f = reinterpret_cast<b2::DFlash *>(dw);
         f->tmap = -1;
         f->tc_mode = 0;

@@ -23,6 +23,7 @@
   X(attn, B2_FAMS_STREAM | b2::kFamMma | b2::kFamFlash)  \
   X(all, b2::kFamWire)                                   \
   X(plan_rows, b2::kFamFuse)                             \
-  X(plan_pairs, b2::kFamFuse | b2::kFamPairs)
+  X(plan_pairs, b2::kFamFuse | b2::kFamPairs)            \
+  X(plan_gemm, b2::kFamFuse | b2::kFamGemm)
 
 #endif
