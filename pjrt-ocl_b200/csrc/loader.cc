@@ -1322,9 +1322,17 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
             const uint64_t rows = side ? q.N : q.M;
             const int64_t ld = w[10 + side];
             sp.base = c.Ref(static_cast<uint32_t>(w[8 + side])); sp.off = w[12 + side]; sp.dtype = q.adt; sp.rank = 3;
+            const uint32_t tile_rows = side ? q.bn : 128u * q.halves;
             sp.dims[0] = mn ? rows : q.K; sp.dims[1] = mn ? q.K : rows; sp.dims[2] = 1;
             sp.strides[0] = ld; sp.strides[1] = ld * static_cast<int64_t>(sp.dims[1]);
-            sp.box[0] = 64u; sp.box[1] = 64u; sp.box[2] = 1u;
+            sp.box[0] = 64u; sp.box[1] = mn ? 64u : tile_rows; sp.box[2] = 1u;
+            if (mn && rows % 64 == 0) {          // [row block][k][64 rows]: one box holds a stage's blocks
+              sp.dims[0] = 64; sp.dims[1] = q.K; sp.dims[2] = rows / 64;
+              sp.strides[0] = ld; sp.strides[1] = 64;
+              sp.box[1] = 64u; sp.box[2] = tile_rows / 64u;
+            } else if (mn) {
+              (side ? q.bmn : q.amn) = kGmMnSingle;
+            }
             sp.owner_is_flash = kTmapPlanned2;
             sp.valid = true;
             out->tmaps.push_back(sp);

@@ -1,9 +1,10 @@
 // Matmuls of re-planned programs on the tensor cores (kTopGemm): bf16 / f16 operands, f32 accumulation in tensor memory,
 // one or several products per task, and what followed the product elementwise as its store epilogue.
 //
-// Bound: what the tiles pull through L2. A 128 x 256 tile per CTA (ops_mma_tc.cuh) moves 48 KB per 512 tensor cycles,
-// ~26 TB/s over the chip at full rate against ~10 it gets: 830 TFLOP/s at 4096 cubed. A 256 x 256 tile (two 128-row
-// halves that share the B block; both 256-column halves of tensor memory) moves 64 KB per 1024 cycles, a third less.
+// Bound: the tensor pipe, under the power cap. What stood in its way in the tile op of the wire programs (ops_mma_tc.cuh,
+// 830 TFLOP/s at 4096 cubed) is the issue of copies: one thread starts a TMA box every ~270 cycles whatever its size, and
+// a 128 x 256 tile took up to six per 512 tensor cycles. Here a stage is two boxes (32 KB each at most) and feeds 1024.
+// A 256 x 256 tile is two 128-row halves that share the B block and fill all of tensor memory.
 //
 // Roles: warp 0 feeds the stages (3 x 64 KB: A 256 x 64 k, B 256 x 64 k, each as 64 x 64 TMA boxes of 8 KB in the
 // 128-byte swizzle, either operand k-contiguous or row / column-contiguous); warp 1 issues tcgen05.mma, the whole warp in
@@ -217,24 +218,25 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
       for (uint32_t tile = slot; ok && gemm_tile(G, tile, q); tile += n_slots) {
         const DGemmProb &pr = G.prob[q.prob];
         const DTmap *ta = P.tmaps + pr.tmap, *tb = ta + 1;
-        const uint32_t nkb = (pr.K + 63u) / 64u, a_boxes = 2u * q.halves, b_boxes = (q.n_inst + 63u) / 64u;
-        const uint32_t bytes = (a_boxes + b_boxes) * kGemmBox;
+        const uint32_t nkb = (pr.K + 63u) / 64u, a_rows = 128u * pr.halves;
+        const uint32_t bytes = (a_rows + pr.bn) * 128u;
+        const int32_t r0 = static_cast<int32_t>(q.r0), c0 = static_cast<int32_t>(q.c0);
+        // An operand's part of a stage is one box; one whose rows are the unit-stride axis comes as 64-row blocks (a box over
+        // the blocks), or block by block where they do not divide the axis.
+        auto fetch = [&](uint32_t dst, const DTmap *tm, uint32_t mode, uint32_t rows, int32_t r, int32_t k0, uint64_t *bar) {
+          if (mode == kGmK) tma_load_3d(dst, tm, k0, r, 0, bar);
+          else if (mode == kGmMnBlocks) tma_load_3d(dst, tm, 0, k0, r / 64, bar);
+          else
+            for (uint32_t i = 0; i < rows / 64u; ++i) tma_load_3d(dst + i * kGemmBox, tm, r + static_cast<int32_t>(64u * i), k0, 0, bar);
+        };
         for (uint32_t kb = 0; kb < nkb; ++kb, ++it) {
           const uint32_t s = it % kGemmStages;
           if (!tc_wait(&S->empty[s], ((it / kGemmStages) & 1u) ^ 1u, failed, budget)) { ok = false; break; }
           mbar_arrive_tx(&S->full[s], bytes);
-          const uint32_t sa = stage0 + s * kGemmStageBytes, sb = sa + kGemmBOff;
-          const int32_t k0 = static_cast<int32_t>(kb * 64u), r0 = static_cast<int32_t>(q.r0), c0 = static_cast<int32_t>(q.c0);
-          for (uint32_t b = 0; b < a_boxes; ++b) {
-            const int32_t r = r0 + static_cast<int32_t>(64u * b);
-            if (pr.amn) tma_load_3d(sa + b * kGemmBox, ta, r, k0, 0, &S->full[s]);
-            else tma_load_3d(sa + b * kGemmBox, ta, k0, r, 0, &S->full[s]);
-          }
-          for (uint32_t b = 0; b < b_boxes; ++b) {
-            const int32_t c = c0 + static_cast<int32_t>(64u * b);
-            if (pr.bmn) tma_load_3d(sb + b * kGemmBox, tb, c, k0, 0, &S->full[s]);
-            else tma_load_3d(sb + b * kGemmBox, tb, k0, c, 0, &S->full[s]);
-          }
+          const uint32_t sa = stage0 + s * kGemmStageBytes;
+          const int32_t k0 = static_cast<int32_t>(kb * 64u);
+          fetch(sa, ta, pr.amn, a_rows, r0, k0, &S->full[s]);
+          fetch(sa + kGemmBOff, tb, pr.bmn, pr.bn, c0, k0, &S->full[s]);
         }
       }
     }

@@ -86,11 +86,13 @@ enum GemmEpi_ : uint32_t {
   kGeCarrySq = 32u,        // add its square to the task's full sum
   kGeScale1 = 64u          // times s1
 };
+// unit stride along k; along the rows / columns (MN), fetched as a box of 64-row blocks or block by block
+enum GemmOperand : uint32_t { kGmK = 0, kGmMnBlocks = 1, kGmMnSingle = 2 };
 struct DGemmProb {
   uint32_t first, tm, tn;          // number of its first tile; tile grid
   uint32_t halves, bn;             // a tile is halves x 128 rows by bn columns
   uint32_t M, N, K;
-  uint32_t amn, bmn;               // operand's unit stride runs along its rows / columns instead of k
+  uint32_t amn, bmn;               // how an operand lies and is fetched (kGm*)
   uint32_t adt, dt0, dt1;
   int32_t tmap;
   uint32_t epi, qdt, rdt;
