@@ -47,16 +47,14 @@ __device__ __forceinline__ float rsqrt_nr(float x) {
   return x > 1.0e-37f && x < 1.0e37f ? fmaf(0.5f * r, e, r) : r;
 }
 
-// d/dz of tanh-GELU with the micro-ops, roundings and tanh of the region it replaces.
-__device__ __forceinline__ float gelu_grad(float z, float c) {      // c = 3 x 0.7978845608 x 0.044715 as the program rounds it
-  const float z2 = __fmul_rn(z, z);
-  const float w = __fadd_rn(z, __fmul_rn(__fmul_rn(z2, z), 0.044715f));
-  const float th = fast_tanh(__fmul_rn(w, 0.7978845608f));
-  const float sech2 = __fadd_rn(-__fmul_rn(th, th), 1.0f);
-  const float du = __fadd_rn(__fmul_rn(z2, c), 0.7978845608f);
-  const float a = __fadd_rn(__fmul_rn(th, 0.5f), 0.5f);
-  const float b = __fmul_rn(__fmul_rn(z, 0.5f), __fmul_rn(sech2, du));
-  return __fadd_rn(a, b);
+// d/dz of tanh-GELU, 0.5 (1 + t) + 0.5 z (1 - t^2) u' with t = tanh(u), u = k (z + 0.044715 z^3), u' = k + c z^2: with
+// e = exp(2u) and r = 1 / (1 + e) that is 0.5 (1 + t) = e r and 1 - t^2 = 4 e r^2, so e r (1 + 2 z r u'): one exponential
+// and one reciprocal, no cancellation. c = 3 x 0.7978845608 x 0.044715 as the program rounds it.
+__device__ __forceinline__ float gelu_grad(float z, float c) {
+  const float z2 = z * z;
+  const float a = fminf(z * fmaf(z2, 2.3022082f * 0.044715f, 2.3022082f), 100.0f);      // 2 u log2(e)
+  const float e = fast_ex2(a), r = fast_rcp(1.0f + e);
+  return (e * r) * fmaf(2.0f * z * r, fmaf(z2, c, 0.7978845608f), 1.0f);
 }
 
 // Reduce two values over the T threads of a row group (a warp, or whole warps). `slot` = 64 floats of the group: the two

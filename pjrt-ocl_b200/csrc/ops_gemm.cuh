@@ -28,7 +28,7 @@ namespace b2 {
 constexpr int kGemmStages = 3;
 constexpr uint32_t kGemmStageBytes = 65536, kGemmBOff = 32768, kGemmBox = 8192;
 constexpr uint32_t kGemmEpiWarps = 12, kGemmEpiFirst = 4;
-constexpr uint32_t kGemmSlab = 32u * 17u * 4u;             // staging of one epilogue warp: 32 rows x 16 words, pitch 17
+constexpr uint32_t kGemmSlab = 32u * 64u;                  // staging of one epilogue warp: 32 rows x 64 bytes, 64-byte swizzle
 constexpr uint32_t kGemmGroup = 8;
 
 struct GemmShared {
@@ -75,29 +75,23 @@ __device__ __forceinline__ void gemm_quant(float (&v)[32], uint32_t dt) {
     for (int j = 0; j < 32; ++j) v[j] = f16_bits_to_f32(f32_to_f16_bits(v[j]));
   }
 }
-// columns c .. c + 7 of the residual's row
-__device__ __forceinline__ void gemm_res8(const uint8_t *row, uint32_t dt, uint32_t c, uint32_t left, bool vec, float (&y)[8]) {
-  if (vec && left >= 8u) {
-    if (dt == kF32) {
-      const float4 a = *reinterpret_cast<const float4 *>(row + static_cast<size_t>(c) * 4u), b = *reinterpret_cast<const float4 *>(row + static_cast<size_t>(c) * 4u + 16u);
-      y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w; y[4] = b.x; y[5] = b.y; y[6] = b.z; y[7] = b.w;
-    } else {
-      const uint4 u = *reinterpret_cast<const uint4 *>(row + static_cast<size_t>(c) * 2u);
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (dt == kBF16) { y[2 * k] = __uint_as_float(w[k] << 16); y[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u); }
-        else { y[2 * k] = f16_bits_to_f32(w[k] & 0xffffu); y[2 * k + 1] = f16_bits_to_f32(w[k] >> 16); }
-      }
-    }
-    return;
-  }
+// eight residual elements from memory (ragged edge, or f32) ...
+__device__ __forceinline__ void gemm_res8(const uint8_t *row, uint32_t dt, uint32_t c, uint32_t left, float (&y)[8]) {
 #pragma unroll
   for (uint32_t k = 0; k < 8u; ++k) y[k] = k < left ? loadf(row, dt, static_cast<int64_t>(c) + k) : 0.0f;
 }
+// ... or out of a prefetched 16-byte word
+__device__ __forceinline__ void gemm_unpack8(const uint4 u, uint32_t dt, float (&y)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (dt == kBF16) { y[2 * k] = __uint_as_float(w[k] << 16); y[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u); }
+    else { y[2 * k] = f16_bits_to_f32(w[k] & 0xffffu); y[2 * k + 1] = f16_bits_to_f32(w[k] >> 16); }
+  }
+}
 
-__device__ __forceinline__ void gemm_epilogue(const GemmEpi &E, float (&v)[32], const uint8_t *res_row, uint32_t c, uint32_t left, bool vec_res,
-                                              bool row_ok, float &csum) {
+__device__ __forceinline__ void gemm_epilogue(const GemmEpi &E, float (&v)[32], const uint8_t *res_row, const uint4 (&pre)[4], bool have_pre, uint32_t c,
+                                              uint32_t left, bool row_ok, float &csum) {
   if (E.flags & kGeGelu) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = gelu_tanh(v[j]);
@@ -115,7 +109,8 @@ __device__ __forceinline__ void gemm_epilogue(const GemmEpi &E, float (&v)[32], 
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       float y[8];
-      if (row_ok) gemm_res8(res_row, E.rdt, c + 8u * b, left > 8u * b ? left - 8u * b : 0u, vec_res, y);
+      if (have_pre) gemm_unpack8(pre[b], E.rdt, y);
+      else if (row_ok) gemm_res8(res_row, E.rdt, c + 8u * b, left > 8u * b ? left - 8u * b : 0u, y);
       else {
 #pragma unroll
         for (int k = 0; k < 8; ++k) y[k] = 0.0f;
@@ -151,31 +146,44 @@ __device__ __forceinline__ void gemm_epilogue(const GemmEpi &E, float (&v)[32], 
   }
 }
 
-// A warp's 32 x 32 block to dst, through its staging slab so that the global stores are whole 64-byte row pieces.
+// A warp's 32 x 32 block to its place. Each thread holds 32 columns of one row; stored like that, a warp instruction would
+// touch 32 rows with 16 bytes each. Through the warp's slab (4 16-byte shared writes and reads per thread and pass, free of
+// bank conflicts by the swizzle) it leaves as whole 64-byte row pieces, 8 rows per instruction. (The store unit out of
+// the slab instead: the wait for the slab's previous box costs as much as it saves.)
 __device__ __forceinline__ void gemm_store(uint8_t *dst, uint32_t dt, uint32_t N, uint32_t r_first, uint32_t M, uint32_t c, uint32_t left, bool vec,
-                                           uint32_t *stg, uint32_t lane, const float (&v)[32]) {
+                                           uint32_t stg, uint32_t lane, const float (&v)[32]) {
+  if (left == 0u) return;
   const uint32_t esz = dt == kF32 ? 4u : 2u;
-  if (vec && left >= 32u) {
+  if (vec && left == 32u) {
+    const uint32_t row = stg + lane * 64u, sw = (lane >> 1) & 3u, r8 = lane >> 2, ch = lane & 3u;
 #pragma unroll
-    for (uint32_t h = 0; h < 2u; ++h) {          // f32: two 16-column halves; 2-byte types: one pass
+    for (uint32_t h = 0; h < 2u; ++h) {                    // 16 columns of f32 fill the 64 bytes
       if (h == 1u && esz == 2u) break;
       __syncwarp();
-      if (esz == 4u) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) stg[lane * 17u + j] = __float_as_uint(h ? v[16 + j] : v[j]);
-      } else {
+      for (uint32_t k = 0; k < 4u; ++k) {
+        uint32_t w[4];
+        if (esz == 4u) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-          stg[lane * 17u + j] = dt == kBF16 ? cvt_bf16x2(v[2 * j + 1], v[2 * j]) : (f32_to_f16_bits(v[2 * j]) | (f32_to_f16_bits(v[2 * j + 1]) << 16));
+          for (uint32_t e = 0; e < 4u; ++e) w[e] = __float_as_uint(h ? v[16 + 4 * k + e] : v[4 * k + e]);
+        } else {
+#pragma unroll
+          for (uint32_t e = 0; e < 4u; ++e) {
+            const float lo = v[8 * k + 2 * e], hi = v[8 * k + 2 * e + 1];
+            w[e] = dt == kBF16 ? cvt_bf16x2(hi, lo) : (f32_to_f16_bits(lo) | (f32_to_f16_bits(hi) << 16));
+          }
+        }
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(row + ((k ^ sw) << 4)), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
       }
       __syncwarp();
+      uint8_t *out = dst + (static_cast<size_t>(r_first + r8) * N + c) * esz + h * 64u + ch * 16u;
+      const size_t step = static_cast<size_t>(8u) * N * esz;
 #pragma unroll
-      for (uint32_t pass = 0; pass < 4u; ++pass) {
-        const uint32_t row = pass * 8u + (lane >> 2), ch = lane & 3u, rr = r_first + row;
-        if (rr < M) {
-          const uint32_t *sp = stg + row * 17u + ch * 4u;
-          stg_v4(dst + (static_cast<size_t>(rr) * N + c) * esz + h * 64u + ch * 16u, make_uint4(sp[0], sp[1], sp[2], sp[3]));
-        }
+      for (uint32_t p = 0; p < 4u; ++p) {
+        const uint32_t rr = 8u * p + r8;
+        uint4 w;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(stg + rr * 64u + ((ch ^ ((rr >> 1) & 3u)) << 4)) : "memory");
+        if (r_first + rr < M) stg_v4(out + p * step, w);
       }
     }
     return;
@@ -212,6 +220,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
   if (w == 0u) {
     // ---------------- producer ----------------
     if (lane == 0u) {
+      fence_proxy_async_global();        // operands written by the previous phase's ordinary stores
       uint32_t it = 0;
       bool ok = true;
       GemmTile q;
@@ -305,7 +314,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
   } else if (w >= kGemmEpiFirst) {
     // ---------------- epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. + 31; three warps share a quarter's column chunks ----------------
     const uint32_t ew = w - kGemmEpiFirst, quarter = w & 3u, third = ew >> 2;
-    uint32_t *stg = reinterpret_cast<uint32_t *>(sm + (stage0 - smem_addr(sm)) + kGemmStages * kGemmStageBytes + ew * kGemmSlab);
+    const uint32_t stg = stage0 + kGemmStages * kGemmStageBytes + ew * kGemmSlab;
     uint32_t n = 0;
     bool ok = true;
     GemmTile q;
@@ -316,27 +325,42 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
       E.res = (pr.epi & kGeRes) ? resolve(P, pr.res) : nullptr;
       uint8_t *out0 = pr.out0 ? resolve(P, pr.out0) : nullptr, *out1 = pr.out1 ? resolve(P, pr.out1) : nullptr;
       const uint32_t M = pr.M, N = pr.N;
-      const bool vec = (N & 7u) == 0u;             // 16-byte pieces of a row start on 16-byte boundaries
+      const bool vec = (N & 7u) == 0u;                                    // 16-byte pieces of a row start on 16-byte boundaries
+      const bool pre_ok = E.res && E.rdt != kF32 && vec;       // residual by 16-byte words, a chunk ahead
       for (uint32_t h = 0; ok && h < q.halves; ++h, ++n) {
         const uint32_t sl = n & 1u;
-        if (!tc_wait_warp(&S->acc_full[sl], (n >> 1) & 1u, failed, budget, 32u)) { ok = false; break; }
-        tc_fence_after_sync();
         const uint32_t rf = q.r0 + 128u * h + 32u * quarter, r = rf + lane;
         const bool row_ok = r < M;
         const uint8_t *res_row = E.res ? E.res + static_cast<size_t>(min(r, M - 1u)) * N * (E.rdt == kF32 ? 4u : 2u) : nullptr;
+        uint4 nxt[4];
+        auto prefetch = [&](uint32_t col) {
+          const uint32_t c = q.c0 + col;
+#pragma unroll
+          for (uint32_t k = 0; k < 4u; ++k)
+            nxt[k] = row_ok && c + 8u * k < N ? ldg_v4(res_row + static_cast<size_t>(c + 8u * k) * 2u) : make_uint4(0u, 0u, 0u, 0u);
+        };
+        if (pre_ok && 32u * third < q.n_inst) prefetch(32u * third);
+        if (!tc_wait_warp(&S->acc_full[sl], (n >> 1) & 1u, failed, budget, 32u)) { ok = false; break; }
+        tc_fence_after_sync();
 #pragma unroll 1
         for (uint32_t col = 32u * third; col < q.n_inst; col += 96u) {
           uint32_t raw[32];
           __syncwarp();
           tc_ld32(tmem + ((32u * quarter) << 16) + sl * 256u + col, raw);
+          uint4 cur[4];
+          if (pre_ok) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) cur[k] = nxt[k];
+            if (col + 96u < q.n_inst) prefetch(col + 96u);
+          }
           tc_wait_ld();
-          const uint32_t c = q.c0 + col, left = c < N ? N - c : 0u;
+          const uint32_t c = q.c0 + col, left = c < N ? min(32u, N - c) : 0u;
           float v[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
           if (E.flags & kGeQuant0) gemm_quant(v, E.qdt);
           if (out0) gemm_store(out0, pr.dt0, N, rf, M, c, left, vec, stg, lane, v);
-          gemm_epilogue(E, v, res_row, c, left, vec, row_ok, csum);
+          gemm_epilogue(E, v, res_row, cur, pre_ok, c, left, row_ok, csum);
           if (out1) gemm_store(out1, pr.dt1, N, rf, M, c, left, vec, stg, lane, v);
         }
         tc_fence_before_sync();

@@ -12,7 +12,7 @@
 namespace b2 {
 
 struct RowPipe {            // resolved, in shared memory
-  uint32_t flags, cols, n_rows, stage_off, mul_off, add_off;   // *_off: staged vectors (byte offset), kFuNoSlot = read from memory
+  uint32_t flags, cols, n_buf, stage_off, mul_off, add_off;   // n_buf: row buffers per thread, 2 or 4; *_off: staged vectors (byte offset), kFuNoSlot = read from memory
   float eps, s, t;
   uint32_t pad;
   const uint8_t *x, *y, *mul, *add;
@@ -85,7 +85,7 @@ static __device__ __noinline__ float row_pipe_run(uint32_t tid, uint32_t nthr, u
   const uint32_t nv = VEC ? (cols > gl * 4u ? (cols - gl * 4u + 4u * T - 1u) / (4u * T) : 0u) : (cols > gl ? (cols - gl + T - 1u) / T : 0u);
   const uint32_t c0 = VEC ? gl * 4u : gl, cstep = VEC ? 4u * T : T;      // column of (group 0 | element 0), and from one to the next
   const float inv_n = 1.0f / static_cast<float>(cols);
-  // staging of the next row: [2 buffers][x, y][G][threads] words of 4 elements
+  // staging of the rows ahead: [n_buf][x, y][G][threads] words of 4 elements
   constexpr uint32_t W = 4u * ESZ;
   const uint32_t nsrc = (fl & kRpRes) ? 2u : 1u;
   uint8_t *stage = sm + A.stage_off + tid * W;
@@ -106,7 +106,6 @@ static __device__ __noinline__ float row_pipe_run(uint32_t tid, uint32_t nthr, u
         }
         d += G * gstride;
       }
-      cp_async_commit();
     } else {
       const uint8_t *q = A.x + static_cast<size_t>(row) * cols * ESZ;
       for (uint32_t b = gl * 128u; b < cols * ESZ; b += T * 128u) prefetch_l2(q + b);
@@ -121,12 +120,19 @@ static __device__ __noinline__ float row_pipe_run(uint32_t tid, uint32_t nthr, u
 #define B2_RP_IN(g, e) (static_cast<uint32_t>(VEC ? (g) : 4 * (g) + (e)) < nv)
   auto add_f = [](float a, float c) { return a + c; };
   float csum = 0.0f;
+  const uint32_t ahead = VEC ? A.n_buf - 1u : 1u;       // rows under way beyond the current one (one commit group per row)
   uint32_t buf = 0, row = lo + gi;
-  if (row < hi) start(row, 0u);
+  for (uint32_t k = 0; k < ahead; ++k) {
+    if (row + k * ng < hi) start(row + k * ng, k);
+    cp_async_commit();
+  }
   for (; row < hi; row += ng) {
     float X[G][4];
-    if (VEC) cp_async_wait<0>();
-    if (row + ng < hi) start(row + ng, buf ^ 1u);
+    if (VEC) {
+      if (ahead == 3u) cp_async_wait<2>(); else cp_async_wait<0>();
+    }
+    if (row + ahead * ng < hi) start(row + ahead * ng, VEC ? (buf + ahead) & ahead : 0u);
+    cp_async_commit();
     const size_t base = static_cast<size_t>(row) * cols * ESZ;
     // a second operand over the row: staged, or straight from memory
     auto dense = [&](const uint8_t *p, uint32_t k, int g, float (&v)[4]) {
@@ -218,7 +224,7 @@ static __device__ __noinline__ float row_pipe_run(uint32_t tid, uint32_t nthr, u
       csum += (a[0] + a[1]) + (a[2] + a[3]);
     }
     if (A.out) store(A.out);
-    buf ^= 1u;
+    if (VEC) buf = (buf + 1u) & ahead;
   }
 #undef B2_RP_IN
 #undef B2_RP_E
@@ -239,7 +245,7 @@ static __device__ __noinline__ void row_pipe_tiles(const Lane &L, const DTask &t
   const uint32_t per = (cols + 4u * T - 1u) / (4u * T);
   const uint32_t G = per <= 1u ? 1u : per <= 2u ? 2u : per <= 4u ? 4u : 8u;
   const uint32_t vbytes = (cols * esz + 15u) & ~15u;
-  const uint32_t stage_bytes = f.vec ? 2u * ((p.flags & kRpRes) ? 2u : 1u) * G * L.nthr * 4u * esz : 0u;
+  const uint32_t buf_bytes = f.vec ? ((p.flags & kRpRes) ? 2u : 1u) * G * L.nthr * 4u * esz : 0u, stage_bytes = 2u * buf_bytes;
   const uint32_t nvec = ((p.flags & kRpMul) ? 1u : 0u) + ((p.flags & kRpAdd) ? 1u : 0u);
   const bool keep = hi - tile_lo > 1u && kFuseData + nvec * vbytes + stage_bytes <= L.smem_bytes;     // column vectors in shared memory
   const uint8_t *mul = p.mul ? resolve(P, p.mul) : nullptr, *add = p.add ? resolve(P, p.add) : nullptr;
@@ -257,7 +263,7 @@ static __device__ __noinline__ void row_pipe_tiles(const Lane &L, const DTask &t
     off += vbytes;
   }
   if (L.tid == 0) {
-    A->flags = p.flags; A->cols = cols; A->n_rows = f.rows; A->stage_off = (off + 15u) & ~15u; A->mul_off = offs[0]; A->add_off = offs[1];
+    A->flags = p.flags; A->cols = cols; A->n_buf = ((off + 15u) & ~15u) + 4u * buf_bytes <= L.smem_bytes ? 4u : 2u; A->stage_off = (off + 15u) & ~15u; A->mul_off = offs[0]; A->add_off = offs[1];
     A->eps = p.eps; A->s = p.s; A->t = p.t;
     A->x = resolve(P, p.x); A->y = p.y ? resolve(P, p.y) : nullptr;
     A->mul = mul; A->add = add;

@@ -27,9 +27,16 @@
 #if B2_HAS(0x800u)  // kFamGemm
 #include "ops_gemm.cuh"
 #endif
+#if B2_HAS(0x40u)   // kFamFlash: the wire programs' attention
+#include "ops_flash_tc.cuh"
+#include "ops_flash.cuh"
+#endif
+#if B2_HAS(0x02u)   // kFamMove: and their moves
+#include "ops_move.cuh"
+#endif
 
 namespace b2 {
-static_assert(kFamFuse == 0x200u && kFamPairs == 0x400u && kFamGemm == 0x800u, "the literals in the #if lines above");
+static_assert(kFamFuse == 0x200u && kFamPairs == 0x400u && kFamGemm == 0x800u && kFamFlash == 0x40u && kFamMove == 0x02u, "the literals in the #if lines above");
 
 constexpr int kVmThreads = 512;
 constexpr uint32_t kNoPc = 0xFFFFFFFFu;
@@ -142,6 +149,17 @@ __global__ void __launch_bounds__(kVmThreads, 1) B2_PLAN_KERNEL(const __grid_con
 #endif
 #if B2_HAS(0x800u)
         case kTopGemm: gemm_tiles(L, t, en.tile_lo, en.tile_hi); break;
+#endif
+#if B2_HAS(0x40u)
+        case kTopFlashAttn: {
+          const DFlash &df = *reinterpret_cast<const DFlash *>(P.desc + t.desc);
+          if (!(df.tc_mode && flash_tc_tiles(L, t, en.tile_lo, en.tile_hi))) flash_simt_tiles(L, t, en.tile_lo, en.tile_hi);
+          break;
+        }
+#endif
+#if B2_HAS(0x02u)
+        case kTopGather: case kTopDynGather: move_tiles(L, t, en.tile_lo, en.tile_hi, false); break;
+        case kTopScatter: case kTopDynScatter: move_tiles(L, t, en.tile_lo, en.tile_hi, true); break;
 #endif
         default:
           if (L.tid == 0) set_status(P, kStBadOp, L.lane, en.task, t.op);

@@ -148,6 +148,8 @@ __device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const void *tmap,
       ::"r"(smem_dst), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_addr(bar))
       : "memory");
 }
+// Generic-proxy writes to global memory made visible here are ordered before this thread's later asynchronous-proxy reads.
+__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 // One arrival that also announces `bytes` of transactions (issued before or after it).
 __device__ __forceinline__ void mbar_arrive_tx(uint64_t *bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");

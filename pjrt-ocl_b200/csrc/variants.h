@@ -24,6 +24,7 @@
   X(all, b2::kFamWire)                                   \
   X(plan_rows, b2::kFamFuse)                             \
   X(plan_pairs, b2::kFamFuse | b2::kFamPairs)            \
-  X(plan_gemm, b2::kFamFuse | b2::kFamGemm)
+  X(plan_gemm, b2::kFamFuse | b2::kFamGemm)              \
+  X(plan_attn, b2::kFamFuse | b2::kFamGemm | b2::kFamFlash | b2::kFamMove)
 
 #endif
