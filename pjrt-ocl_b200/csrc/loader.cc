@@ -784,6 +784,45 @@ bool MmaOperandLayout(const VmProgram &p, const VmTask &t, MmaLayout *o) {
   return TcOperand(M, K, 0, sa[1], sa[2], o->a_off, &o->amn, &o->a_ld, &gs) && TcOperand(N, K, 0, sb[2], sb[1], o->b_off, &o->bmn, &o->b_ld, &gs);
 }
 
+// One operand of a CUDA-core product: rows x K (A) or K x rows (B), dense or through a view in which an element's place is the sum
+// of a row's and a k's part.
+static bool SgOperand(const VmProgram &p, uint32_t field, uint64_t rows, uint64_t K, bool is_b, bool aligned, DSgOperand *o) {
+  std::memset(o, 0, sizeof(*o));
+  o->row_major = is_b ? 0u : 1u;
+  o->inner = static_cast<uint32_t>(is_b ? rows : K);
+  const int64_t n[3] = {1, static_cast<int64_t>(is_b ? K : rows), static_cast<int64_t>(is_b ? rows : K)};
+  int64_t st[3] = {0, n[2], 1}, off = 0;
+  if (rows * K >= (1ull << 32)) return false;
+  if (field) {
+    std::string err;
+    if (!ViewFromAux(p, field - 1, &o->v, &err)) return false;
+    if (!AffineOverAxes(o->v, n, st, &off)) {
+      // whole dims on either side of the boundary between the two axes
+      int64_t in = 1;
+      int k = o->v.rank;
+      while (k > 0 && in < n[2]) in *= o->v.dim[--k];
+      if (in != n[2]) return false;
+      o->viewed = 1;
+      o->k_fast = o->v.stride[o->v.rank - 1] == 1 ? !is_b : is_b;
+      return true;
+    }
+  }
+  const int64_t rs = is_b ? st[2] : st[1], ks = is_b ? st[1] : st[2], most = off + rs * static_cast<int64_t>(rows - 1) + ks * static_cast<int64_t>(K - 1);
+  if (off < 0 || rs < 0 || ks < 0 || most >= (1ll << 32)) return false;
+  o->off = static_cast<uint32_t>(off);
+  o->rs = static_cast<uint32_t>(rs);
+  o->ks = static_cast<uint32_t>(ks);
+  o->k_fast = ks == 1;
+  if (aligned && ks == 1 && rs % 4 == 0 && off % 4 == 0 && K % 4 == 0) o->mode = kSgVecK;
+  else if (aligned && rs == 1 && ks % 4 == 0 && off % 4 == 0 && rows % 4 == 0) o->mode = kSgVecR;
+  return true;
+}
+
+bool SgOperandsFit(const VmProgram &p, const VmTask &t) {
+  DSgOperand o;
+  return SgOperand(p, t.p4, t.p0, t.p2, false, false, &o) && SgOperand(p, t.p5, t.p1, t.p2, true, false, &o);
+}
+
 static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, DeviceTables *out, std::string *err,
                                  bool *unimplemented, bool planned = false);
 
@@ -1347,6 +1386,37 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         words.resize((bytes + 7) / 8, 0);
         out->desc.insert(out->desc.end(), words.begin(), words.end());
         d.desc_bytes = static_cast<uint32_t>(bytes);
+        break;
+      }
+      case kTopSgemm: {
+        if (!planned) return fail_unimpl("tile op " + std::to_string(d.op) + " is not implemented by this backend");
+        const int32_t *rd, *wr, *w;
+        int n_rd, n_wr;
+        PlannedLists(p, t, &rd, &n_rd, &wr, &n_wr, &w);
+        DSgemm g;
+        std::memset(&g, 0, sizeof(g));
+        g.shape = w[0];
+        g.total = w[1] ? c.Ref(static_cast<uint32_t>(w[1] - 1)) : 0;
+        g.n_owner_lanes = w[2];
+        if (g.total) out->needs_scratch = true;
+        g.M = w[3]; g.N = w[4]; g.K = w[5]; g.adt = w[6];
+        const uint32_t ab = static_cast<uint32_t>(w[7]), bb = static_cast<uint32_t>(w[8]);
+        if (!SgOperand(p, w[9], g.M, g.K, false, c.Aligned16(ab), &g.a) || !SgOperand(p, w[10], g.N, g.K, true, c.Aligned16(bb), &g.b))
+          return fail_unimpl("product's operand layout");
+        g.a.ptr = c.Ref(ab);
+        g.b.ptr = c.Ref(bb);
+        w += 11;
+        g.epi = w[0]; g.qdt = w[1]; g.rdt = w[2];
+        std::memcpy(&g.s0, &w[3], 4); std::memcpy(&g.s1, &w[4], 4); std::memcpy(&g.gg, &w[5], 4);
+        g.res = w[6] ? c.Ref(static_cast<uint32_t>(w[6] - 1)) : 0;
+        g.out0 = w[7] ? c.Ref(static_cast<uint32_t>(w[7] - 1)) : 0; g.dt0 = w[8];
+        g.out1 = w[9] ? c.Ref(static_cast<uint32_t>(w[9] - 1)) : 0; g.dt1 = w[10];
+        ++out->n_mma;
+        out->mma_flops += 2ull * g.M * g.N * g.K;
+        if (out->desc.size() % 2) out->desc.push_back(0);
+        d.desc = c.PushDesc(g);
+        if (out->desc.size() % 2) out->desc.push_back(0);
+        d.desc_bytes = static_cast<uint32_t>((sizeof(g) + 15) / 16 * 16);
         break;
       }
       case kTopPairs: {

@@ -81,6 +81,8 @@ bool BuildPlannedTables(const VmProgram &p, uint64_t arena_base, DeviceTables *o
 // columns (`mn`), leading dimension and offset in elements. False where they cannot be fed directly.
 struct MmaLayout { bool amn, bmn; int64_t a_ld, b_ld, a_off, b_off; };
 bool MmaOperandLayout(const VmProgram &p, const VmTask &t, MmaLayout *out);
+// Can the CUDA-core product of re-planned programs (ops_sgemm.cuh) address this matmul's operands?
+bool SgOperandsFit(const VmProgram &p, const VmTask &t);
 
 // Collapse {dims, strides, off} to at most kViewDims dims; exposed for unit tests.
 bool CollapseView(const int32_t *dims, const int32_t *strides, int rank, int64_t off, DView *out);

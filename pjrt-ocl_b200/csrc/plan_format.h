@@ -107,5 +107,24 @@ struct DGemm {
   DGemmProb prob[kGemmMaxProbs];
 };
 
+// Products on the CUDA cores. An operand's element (row or column r, k) sits at row part(r) + k part(k).
+enum SgMode : uint32_t { kSgScalar = 0, kSgVecK = 1, kSgVecR = 2 };
+struct DSgOperand {
+  BufRef ptr;
+  uint32_t mode, k_fast;           // scalar loads: neighbouring threads take neighbouring k (else neighbouring rows)
+  uint32_t off, rs, ks;            // elements, where no view is needed
+  uint32_t viewed, row_major, inner;   // view over [rows, k] (row_major) or [k, rows], `inner` = its second extent
+  DView v;
+};
+struct DSgemm {
+  uint32_t M, N, K, adt;
+  uint32_t shape, epi, qdt, rdt;
+  float s0, s1, gg;
+  uint32_t n_owner_lanes;
+  BufRef res, out0, out1, total;
+  uint32_t dt0, dt1;
+  DSgOperand a, b;
+};
+
 }  // namespace b2
 #endif

@@ -100,6 +100,7 @@ class Planner {
   struct Chain;
   bool FusePairs(int seed);
   bool FuseGemm(int seed);
+  void SgShape(uint64_t M, uint64_t N, uint64_t K, uint32_t lanes, int *shape, uint32_t *tiles, double *cost) const;
   bool GemmEpilogue(const Chain &c, uint32_t dst, std::vector<int32_t> *w) const;
   void GroupGemms(std::vector<int> *live, std::map<std::pair<int, int>, std::vector<int>> *phases, std::vector<std::vector<int>> *of);
   bool FuseRows(int seed);
@@ -982,14 +983,17 @@ bool Planner::GemmEpilogue(const Chain &c, uint32_t dst, std::vector<int32_t> *w
   return true;
 }
 
-// A 16-bit matmul and the elementwise tasks on its result that a store epilogue can do.
+// A matmul and the elementwise tasks on its result that a store epilogue can do: on the tensor cores where both operands are
+// 16-bit and lie as TMA can fetch them, else on the CUDA cores.
 bool Planner::FuseGemm(int seed) {
   const Node &sd = n_[seed];
   const VmTask t = sd.t;
-  if (!Half(sd.adt) || !IsFloatDt(sd.dt) || Dt(t.a) != sd.adt || Dt(t.b) != sd.adt || Dt(t.dst) != sd.dt) return false;
-  MmaLayout lay;
-  if (!MmaOperandLayout(p_, t, &lay)) return false;
-  for (int64_t v : {lay.a_ld, lay.b_ld, lay.a_off, lay.b_off}) if (v > 0x7fffffff) return false;
+  if (!IsFloatDt(sd.adt) || !IsFloatDt(sd.dt) || Dt(t.a) != sd.adt || Dt(t.b) != sd.adt || Dt(t.dst) != sd.dt) return false;
+  if ((t.p3 ? t.p3 : 1u) != 1u || !t.p0 || !t.p1 || !t.p2) return false;
+  MmaLayout lay{};
+  bool tensor = Half(sd.adt) && MmaOperandLayout(p_, t, &lay);
+  for (int64_t v : {lay.a_ld, lay.b_ld, lay.a_off, lay.b_off}) tensor = tensor && v <= 0x7fffffff;
+  if (!tensor && !SgOperandsFit(p_, t)) return false;
   // as many of the tasks that follow as the epilogue has room for: all that the chain takes, then ever fewer
   for (int limit = 1 << 30; limit >= 0;) {
     Chain c(*this, t.p0, t.p1, false);
@@ -1016,7 +1020,7 @@ bool Planner::FuseGemm(int seed) {
       if (!c.Close(&writes, false) || writes.empty() || !GemmEpilogue(c, t.dst, &epi)) continue;
     }
     Node nd;
-    nd.op = kTopGemm;
+    nd.op = tensor ? kTopGemm : kTopSgemm;
     nd.dt = sd.dt; nd.adt = sd.adt;
     nd.t = VmTask{};
     nd.t.dst = writes[0];
@@ -1029,14 +1033,38 @@ bool Planner::FuseGemm(int seed) {
     nd.by_slot = true;
     nd.carry_slot = c.total >= 0 ? 0 : -1;
     nd.owner_word = 2;
-    nd.payload = {1, c.total + 1, 0, static_cast<int32_t>(t.p0), static_cast<int32_t>(t.p1), static_cast<int32_t>(t.p2), 0, 0, lay.amn ? 1 : 0, lay.bmn ? 1 : 0,
-                  static_cast<int32_t>(sd.adt), static_cast<int32_t>(t.a), static_cast<int32_t>(t.b), static_cast<int32_t>(lay.a_ld), static_cast<int32_t>(lay.b_ld),
-                  static_cast<int32_t>(lay.a_off), static_cast<int32_t>(lay.b_off)};
+    auto I = [](auto v) { return static_cast<int32_t>(v); };
+    if (tensor) {
+      nd.payload = {1, c.total + 1, 0, I(t.p0), I(t.p1), I(t.p2), 0, 0, lay.amn ? 1 : 0, lay.bmn ? 1 : 0,
+                    I(sd.adt), I(t.a), I(t.b), I(lay.a_ld), I(lay.b_ld), I(lay.a_off), I(lay.b_off)};
+    } else {
+      int shape = 0;
+      SgShape(t.p0, t.p1, t.p2, L_, &shape, &nd.tiles, &nd.cost);
+      nd.payload = {shape, c.total + 1, 0, I(t.p0), I(t.p1), I(t.p2), I(sd.adt), I(t.a), I(t.b), I(t.p4), I(t.p5)};
+    }
     nd.payload.insert(nd.payload.end(), epi.begin(), epi.end());
     if (AddPlanned(nd, c.members) >= 0) return true;
     if (t.p6) return false;
   }
   return false;
+}
+
+// Tile shape of a CUDA-core product: the one with the least time for the busiest lane. A tile's time is its FMAs at the share of
+// the issue rate that the shape's shared-memory reads leave, or the latency of its blocks' loads (16 k each, one ahead,
+// the CTA's slices taking turns), plus set-up, the slices' sums and stores.
+void Planner::SgShape(uint64_t M, uint64_t N, uint64_t K, uint32_t lanes, int *shape, uint32_t *tiles, double *cost) const {
+  struct S { uint32_t tm, tn, slices; double rate; };
+  static const S shapes[5] = {{128, 64, 2, 0.75}, {64, 64, 2, 0.6}, {64, 32, 4, 0.6}, {32, 32, 8, 0.6}, {16, 16, 8, 0.3}};
+  double best = 1e300;
+  for (int i = 0; i < 5; ++i) {
+    const S &s = shapes[i];
+    const uint64_t T = ((M + s.tm - 1) / s.tm) * ((N + s.tn - 1) / s.tn);
+    if (T > 0x7fffffffu) continue;
+    const double blocks = std::ceil(static_cast<double>((K + 15) / 16) / s.slices);
+    const double tile = std::max(static_cast<double>(K) * s.tm * s.tn / (128.0 * s.rate), blocks * 700.0) + 1500.0 + s.tm * s.tn * 0.15;
+    const double time = tile * static_cast<double>((T + lanes - 1) / lanes);
+    if (time < best) { best = time; *shape = i; *tiles = static_cast<uint32_t>(T); *cost = tile / 6000.0; }
+  }
 }
 
 // Matmuls of one phase become one task (deepest first), and every product gets its tile shape. A lane's time for a tile is
@@ -1046,6 +1074,15 @@ void Planner::GroupGemms(std::vector<int> *live, std::map<std::pair<int, int>, s
   for (auto &kv : *phases) {
     std::vector<int> gs, rest;
     for (int u : kv.second) (n_[u].op == kTopGemm && n_[u].planned ? gs : rest).push_back(u);
+    // CUDA-core products side by side share the lanes by cost
+    double sg_all = 0;
+    for (int u : rest) if (n_[u].op == kTopSgemm) sg_all += n_[u].cost * n_[u].tiles;
+    for (int u : rest) {
+      Node &x = n_[u];
+      if (x.op != kTopSgemm) continue;
+      const double share = x.cost * x.tiles / sg_all;
+      SgShape(x.payload[3], x.payload[4], x.payload[5], std::max(1u, static_cast<uint32_t>(L_ * share + 0.5)), &x.payload[0], &x.tiles, &x.cost);
+    }
     if (gs.empty()) continue;
     std::sort(gs.begin(), gs.end(), [&](int a, int b) { return n_[a].payload[5] > n_[b].payload[5]; });
     std::vector<int> heads;

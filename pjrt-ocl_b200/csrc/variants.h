@@ -25,6 +25,7 @@
   X(plan_rows, b2::kFamFuse)                             \
   X(plan_pairs, b2::kFamFuse | b2::kFamPairs)            \
   X(plan_gemm, b2::kFamFuse | b2::kFamGemm)              \
-  X(plan_attn, b2::kFamFuse | b2::kFamGemm | b2::kFamFlash | b2::kFamMove)
+  X(plan_sgemm, b2::kFamFuse | b2::kFamSgemm)            \
+  X(plan_attn, b2::kFamFuse | b2::kFamGemm | b2::kFamSgemm | b2::kFamFlash | b2::kFamMove)
 
 #endif
