@@ -786,7 +786,7 @@ bool MmaOperandLayout(const VmProgram &p, const VmTask &t, MmaLayout *o) {
 
 // One operand of a CUDA-core product: rows x K (A) or K x rows (B), dense or through a view in which an element's place is the sum
 // of a row's and a k's part.
-static bool SgOperand(const VmProgram &p, uint32_t field, uint64_t rows, uint64_t K, bool is_b, bool aligned, DSgOperand *o) {
+static bool SgOperand(const VmProgram &p, uint32_t field, uint64_t rows, uint64_t K, bool is_b, bool four, DSgOperand *o) {
   std::memset(o, 0, sizeof(*o));
   o->row_major = is_b ? 0u : 1u;
   o->inner = static_cast<uint32_t>(is_b ? rows : K);
@@ -813,8 +813,7 @@ static bool SgOperand(const VmProgram &p, uint32_t field, uint64_t rows, uint64_
   o->rs = static_cast<uint32_t>(rs);
   o->ks = static_cast<uint32_t>(ks);
   o->k_fast = ks == 1;
-  if (aligned && ks == 1 && rs % 4 == 0 && off % 4 == 0 && K % 4 == 0) o->mode = kSgVecK;
-  else if (aligned && rs == 1 && ks % 4 == 0 && off % 4 == 0 && rows % 4 == 0) o->mode = kSgVecR;
+  if (four && rs == 1 && ks % 4 == 0 && off % 4 == 0 && rows % 4 == 0) o->mode = kSgVecR;
   return true;
 }
 
@@ -1401,7 +1400,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         if (g.total) out->needs_scratch = true;
         g.M = w[3]; g.N = w[4]; g.K = w[5]; g.adt = w[6];
         const uint32_t ab = static_cast<uint32_t>(w[7]), bb = static_cast<uint32_t>(w[8]);
-        if (!SgOperand(p, w[9], g.M, g.K, false, c.Aligned16(ab), &g.a) || !SgOperand(p, w[10], g.N, g.K, true, c.Aligned16(bb), &g.b))
+        if (!SgOperand(p, w[9], g.M, g.K, false, g.adt == kF32 && c.Aligned16(ab), &g.a) || !SgOperand(p, w[10], g.N, g.K, true, g.adt == kF32 && c.Aligned16(bb), &g.b))
           return fail_unimpl("product's operand layout");
         g.a.ptr = c.Ref(ab);
         g.b.ptr = c.Ref(bb);

@@ -7,10 +7,9 @@
 // through a gather view over that flat index; with `causal` the T queries are the
 // last T positions of the C-long window (key c is masked when c > m + C - T).
 //
-// One warp per query row: a lane owns one key of the current 32-key chunk for the
-// score, and output columns lane, lane+32, ... for the PV accumulation; masked
-// chunks are never visited. Takes every float dtype and every view; the
-// tensor-core path (ops_flash_tc.cuh) takes the large 2-byte-float cases.
+// Takes every float dtype and every view (flash_rows_tiles); decode-shaped work of one query row per head splits the keys
+// over the lane's warps instead; the tensor-core path (ops_flash_tc.cuh) takes the large 2-byte-float cases. Masked chunks
+// are never visited.
 #ifndef B2VM_OPS_FLASH_CUH_
 #define B2VM_OPS_FLASH_CUH_
 
@@ -310,6 +309,118 @@ static __device__ __noinline__ void flash_decode_ring(const Lane &L, const DTask
   __syncthreads();
 }
 
+// Many query rows, any float type, any views: two rows of one head per warp (32 rows a pass of the lane), and the keys in chunks
+// of 64 that the lane loads once for all of them: K as [d][key], V as [key][d], f32 in shared memory. A thread owns two
+// keys of the chunk for the scores and DJ columns for the output; q and p are read as fours along d and the keys.
+// Bound: shared-memory reads (2.5 per 4 FMAs). A warp per row with every element of K and V fetched through its view by each
+// row's warp took 606 us where this takes 25 (f32, 32 heads x 128 x 128 x 64).
+template <int DJ>
+static __device__ __noinline__ void flash_rows_tiles(const Lane &L, const DTask &t, const DFlash &df, const int32_t *x, uint32_t tile_lo, int64_t hi) {
+  constexpr int HDP = DJ * 32, KC = 64, KP = KC + 1;
+  const KParams &P = *L.P;
+  const int64_t T = x[1], C = x[2], hd = x[3];
+  const float scale = __int_as_float(x[4]);
+  const bool causal = x[5] != 0;
+  uint8_t *out = resolve(P, t.ptr[0]);
+  const uint8_t *Q = resolve(P, t.ptr[1]), *Kp = resolve(P, t.ptr[2]), *V = resolve(P, t.ptr[3]);
+  const uint32_t adt = t.adt, w = L.tid / kWarp, l = L.tid % kWarp, nw = L.nthr / kWarp;
+  float *ks = reinterpret_cast<float *>(L.smem + kSmemSys);      // [HDP][KP]
+  float *vs = ks + HDP * KP;                                     // [KC][HDP]
+  float *qs = vs + KC * HDP + w * 2 * HDP;                       // the warp's two rows
+  float *ps = vs + KC * HDP + nw * 2 * HDP + w * 2 * KC;
+  for (int64_t seg = tile_lo; seg < hi;) {
+    const int64_t g = seg / T, m0 = seg % T;
+    const int64_t rows = min(min(static_cast<int64_t>(2u * nw), T - m0), hi - seg);
+    const int64_t last = causal ? min(C, m0 + rows - 1 + (C - T) + 1) : C;
+    const int64_t m[2] = {m0 + 2 * w, m0 + 2 * w + 1};
+    int64_t c_end[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const bool on = 2 * static_cast<int64_t>(w) + r < rows;
+      c_end[r] = !on ? 0 : causal ? min(C, m[r] + (C - T) + 1) : C;
+      __syncwarp();
+      for (int64_t d = l; d < HDP; d += kWarp) {
+        const int64_t qi = (g * T + m[r]) * hd + d;
+        qs[r * HDP + d] = on && d < hd ? loadf(Q, adt, df.has_q ? view_index(df.vq, static_cast<uint32_t>(qi)) : qi) : 0.0f;
+      }
+    }
+    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f}, o[2][DJ];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int j = 0; j < DJ; ++j) o[r][j] = 0.0f;
+    for (int64_t c0 = 0; c0 < last; c0 += KC) {
+      const uint32_t nk = static_cast<uint32_t>(min(static_cast<int64_t>(KC), C - c0));
+      __syncthreads();
+      // neighbouring threads along d, but for a plain K ([d][key]) along the keys
+#pragma unroll 4
+      for (uint32_t i = L.tid; i < static_cast<uint32_t>(HDP * KC); i += L.nthr) {
+        const uint32_t d = df.has_k ? i % HDP : i / KC, c = df.has_k ? i / HDP : i % KC;
+        const int64_t ki = (g * hd + d) * C + c0 + c;
+        ks[d * KP + c] = d < hd && c < nk ? loadf(Kp, adt, df.has_k ? view_index(df.vk, static_cast<uint32_t>(ki)) : ki) : 0.0f;
+      }
+#pragma unroll 4
+      for (uint32_t i = L.tid; i < static_cast<uint32_t>(HDP * KC); i += L.nthr) {
+        const uint32_t d = i % HDP, c = i / HDP;
+        const int64_t vi = (g * C + c0 + c) * hd + d;
+        vs[c * HDP + d] = d < hd && c < nk ? loadf(V, adt, df.has_v ? view_index(df.vv, static_cast<uint32_t>(vi)) : vi) : 0.0f;
+      }
+      __syncthreads();
+      if (c0 >= c_end[0] && c0 >= c_end[1]) continue;
+      float s[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+#pragma unroll 4
+      for (int d = 0; d < HDP; d += 4) {
+        const float4 qa = *reinterpret_cast<const float4 *>(qs + d), qb = *reinterpret_cast<const float4 *>(qs + HDP + d);
+        const float a4[4] = {qa.x, qa.y, qa.z, qa.w}, b4[4] = {qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float k0 = ks[(d + e) * KP + l], k1 = ks[(d + e) * KP + l + 32];
+          s[0][0] = fmaf(a4[e], k0, s[0][0]); s[0][1] = fmaf(a4[e], k1, s[0][1]);
+          s[1][0] = fmaf(b4[e], k0, s[1][0]); s[1][1] = fmaf(b4[e], k1, s[1][1]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const bool v0 = c0 + l < c_end[r], v1 = c0 + l + 32 < c_end[r];
+        const float s0 = v0 ? s[r][0] * scale : -INFINITY, s1 = v1 ? s[r][1] * scale : -INFINITY;
+        const float m_new = fmaxf(m_run[r], warp_reduce(fmaxf(s0, s1), [](float a, float b) { return fmaxf(a, b); }));
+        const float alpha = m_run[r] == -INFINITY ? 0.0f : expf(m_run[r] - m_new);
+        const float p0 = v0 ? expf(s0 - m_new) : 0.0f, p1 = v1 ? expf(s1 - m_new) : 0.0f;
+        l_run[r] = l_run[r] * alpha + warp_reduce(p0 + p1, [](float a, float b) { return a + b; });
+        m_run[r] = m_new;
+        ps[r * KC + l] = p0;
+        ps[r * KC + l + 32] = p1;
+#pragma unroll
+        for (int j = 0; j < DJ; ++j) o[r][j] *= alpha;
+      }
+      __syncwarp();
+#pragma unroll 2
+      for (int c = 0; c < KC; c += 4) {
+        const float4 pa = *reinterpret_cast<const float4 *>(ps + c), pb = *reinterpret_cast<const float4 *>(ps + KC + c);
+        const float a4[4] = {pa.x, pa.y, pa.z, pa.w}, b4[4] = {pb.x, pb.y, pb.z, pb.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int j = 0; j < DJ; ++j) {
+            const float v = vs[(c + e) * HDP + l + 32 * j];
+            o[0][j] = fmaf(a4[e], v, o[0][j]);
+            o[1][j] = fmaf(b4[e], v, o[1][j]);
+          }
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int j = 0; j < DJ; ++j) {
+        const int64_t d = l + j * kWarp;
+        if (d < hd && 2 * static_cast<int64_t>(w) + r < rows) storef(out, t.dt, (g * T + m[r]) * hd + d, __fdiv_rn(o[r][j], l_run[r]));
+      }
+    seg += rows;
+  }
+  __syncthreads();
+}
+
 static __device__ __noinline__ void flash_simt_tiles(const Lane &L, const DTask &t, uint32_t tile_lo, uint32_t tile_hi) {
   const KParams &P = *L.P;
   const int32_t *x = P.aux + t.p[3];
@@ -323,7 +434,6 @@ static __device__ __noinline__ void flash_simt_tiles(const Lane &L, const DTask 
   const uint8_t *V = resolve(P, t.ptr[3]);
   const uint32_t adt = t.adt, dt = t.dt;
   const uint32_t w = L.tid / kWarp, l = L.tid % kWarp, nw = L.nthr / kWarp;
-  float *qs = reinterpret_cast<float *>(L.smem + kSmemSys) + static_cast<size_t>(w) * kFlashMaxHd;
   const int64_t hi = min(static_cast<int64_t>(tile_hi), H * T);
   __syncthreads();  // workspace handover from the previous op
   if (df.dec_mode && df.dk_c == hd && df.dv_c == hd && L.nthr == 512u &&
@@ -429,59 +539,9 @@ static __device__ __noinline__ void flash_simt_tiles(const Lane &L, const DTask 
     __syncthreads();
     return;
   }
-  for (int64_t tile = tile_lo + w; tile < hi; tile += nw) {
-    const int64_t g = tile / T, m = tile % T;
-    const int64_t qpos = m + (C - T);
-    const int64_t c_end = causal ? min(C, qpos + 1) : C;
-    __syncwarp();
-    for (int64_t d = l; d < hd; d += kWarp) {
-      const int64_t qi = (g * T + m) * hd + d;
-      qs[d] = loadf(Q, adt, df.has_q ? view_index(df.vq, static_cast<uint32_t>(qi)) : qi);
-    }
-    __syncwarp();
-    float m_run = -INFINITY, l_run = 0.0f;
-    float o[kFlashMaxHd / kWarp];
-#pragma unroll
-    for (int j = 0; j < kFlashMaxHd / kWarp; ++j) o[j] = 0.0f;
-    for (int64_t c0 = 0; c0 < c_end; c0 += kWarp) {
-      const int64_t c = c0 + l;
-      float s = -INFINITY;
-      if (c < c_end) {
-        float acc = 0.0f;
-        for (int64_t d = 0; d < hd; ++d) {
-          const int64_t ki = (g * hd + d) * C + c;
-          acc = fmaf(qs[d], loadf(Kp, adt, df.has_k ? view_index(df.vk, static_cast<uint32_t>(ki)) : ki), acc);
-        }
-        s = acc * scale;
-      }
-      const float cmax = warp_reduce(s, [](float a, float b) { return fmaxf(a, b); });
-      const float m_new = fmaxf(m_run, cmax);
-      const float alpha = (m_run == -INFINITY) ? 0.0f : expf(m_run - m_new);
-      const float p = (c < c_end) ? expf(s - m_new) : 0.0f;
-      const float psum = warp_reduce(p, [](float a, float b) { return a + b; });
-      l_run = l_run * alpha + psum;
-      m_run = m_new;
-#pragma unroll
-      for (int j = 0; j < kFlashMaxHd / kWarp; ++j) o[j] *= alpha;
-      const int64_t cn = min(static_cast<int64_t>(kWarp), c_end - c0);
-      for (int64_t cc = 0; cc < cn; ++cc) {
-        const float pc = __shfl_sync(0xffffffffu, p, static_cast<int>(cc));
-#pragma unroll
-        for (int j = 0; j < kFlashMaxHd / kWarp; ++j) {
-          const int64_t d = l + j * kWarp;
-          if (d < hd) {
-            const int64_t vi = (g * C + c0 + cc) * hd + d;
-            o[j] = fmaf(pc, loadf(V, adt, df.has_v ? view_index(df.vv, static_cast<uint32_t>(vi)) : vi), o[j]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kFlashMaxHd / kWarp; ++j) {
-      const int64_t d = l + j * kWarp;
-      if (d < hd) storef(out, dt, (g * T + m) * hd + d, __fdiv_rn(o[j], l_run));
-    }
-  }
+  if (hd <= 64) flash_rows_tiles<2>(L, t, df, x, tile_lo, hi);
+  else if (hd <= 128) flash_rows_tiles<4>(L, t, df, x, tile_lo, hi);
+  else flash_rows_tiles<8>(L, t, df, x, tile_lo, hi);
 }
 
 }  // namespace b2

@@ -107,12 +107,13 @@ struct DGemm {
   DGemmProb prob[kGemmMaxProbs];
 };
 
-// Products on the CUDA cores. An operand's element (row or column r, k) sits at row part(r) + k part(k).
-enum SgMode : uint32_t { kSgScalar = 0, kSgVecK = 1, kSgVecR = 2 };
+// Products on the CUDA cores. An operand's element (row or column r, k) sits at off + r rs + k ks (elements), or
+// through a view where an axis is not affine: at a row's part + a k's part.
+enum SgMode : uint32_t { kSgScalar = 0, kSgVecR = 1 };     // element by element; f32, fours of neighbouring rows
 struct DSgOperand {
   BufRef ptr;
-  uint32_t mode, k_fast;           // scalar loads: neighbouring threads take neighbouring k (else neighbouring rows)
-  uint32_t off, rs, ks;            // elements, where no view is needed
+  uint32_t mode, k_fast;           // element by element: neighbouring threads take neighbouring k (else neighbouring rows)
+  uint32_t off, rs, ks;
   uint32_t viewed, row_major, inner;   // view over [rows, k] (row_major) or [k, rows], `inner` = its second extent
   DView v;
 };

@@ -1054,7 +1054,7 @@ bool Planner::FuseGemm(int seed) {
 // the CTA's slices taking turns), plus set-up, the slices' sums and stores.
 void Planner::SgShape(uint64_t M, uint64_t N, uint64_t K, uint32_t lanes, int *shape, uint32_t *tiles, double *cost) const {
   struct S { uint32_t tm, tn, slices; double rate; };
-  static const S shapes[5] = {{128, 64, 2, 0.75}, {64, 64, 2, 0.6}, {64, 32, 4, 0.6}, {32, 32, 8, 0.6}, {16, 16, 8, 0.3}};
+  static const S shapes[5] = {{128, 64, 4, 0.75}, {64, 64, 8, 0.75}, {64, 32, 8, 0.6}, {32, 32, 8, 0.45}, {16, 16, 8, 0.2}};
   double best = 1e300;
   for (int i = 0; i < 5; ++i) {
     const S &s = shapes[i];
