@@ -73,7 +73,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         src = PLAN_KERNEL if name.startswith("plan") else KERNEL
         units.append((os.path.join(CSRC, src), os.path.join(OBJ, f"vm_kernel_{name}.o"),
                       (f"-DB2_VARIANT={name}", f"-DB2_FAMILIES={mask:#x}u")))
-    plan_only = ("plan_format.h", "replan.h", "ops_fuse.cuh", "ops_rowpipe.cuh", "ops_pairs.cuh", "ops_flatpipe.cuh", "ops_gemm.cuh", "ops_sgemm.cuh")
+    plan_only = ("plan_format.h", "replan.h", "ops_fuse.cuh", "ops_rowpipe.cuh", "ops_pairs.cuh", "ops_flatpipe.cuh", "ops_gemm.cuh", "ops_sgemm.cuh", "ops_skinny.cuh")
 
     def deps(u):
         if u[0].endswith(KERNEL):       # the wire builds do not include the planned ops

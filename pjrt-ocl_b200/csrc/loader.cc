@@ -165,7 +165,7 @@ uint32_t FlatOps(const DFuStep *st, uint32_t n) {
 
 // Is a fused step list one of the row pipelines of ops_rowpipe.cuh? Every tensor in one storage type; between the stages
 // of 16-bit rows either every value is rounded or none.
-void MatchPipe(const DFuStep *st, uint32_t n, bool whole_rows, DPipe *out) {
+void MatchPipe(const DFuStep *st, uint32_t n, bool whole_rows, bool one_row, DPipe *out) {
   std::memset(out, 0, sizeof(*out));
   uint32_t i = 0;
   if (!whole_rows || n < 2 || st[0].code != kFuLoadX) return;
@@ -200,8 +200,9 @@ void MatchPipe(const DFuStep *st, uint32_t n, bool whole_rows, DPipe *out) {
     i += 4;
     quant();
   }
-  if (at(i, kFuRowVecY) && st[i].dt == p.dt && at(i + 1, kFuMul)) { p.flags |= kRpMul; p.mul = st[i].ptr; i += 2; quant(); }
-  if (at(i, kFuRowVecY) && st[i].dt == p.dt && at(i + 1, kFuAdd)) { p.flags |= kRpAdd; p.add = st[i].ptr; i += 2; quant(); }
+  auto row_vec = [&](uint32_t k) { return at(k, kFuRowVecY) || (one_row && at(k, kFuLoadY)); };
+  if (row_vec(i) && st[i].dt == p.dt && at(i + 1, kFuMul)) { p.flags |= kRpMul; p.mul = st[i].ptr; i += 2; quant(); }
+  if (row_vec(i) && st[i].dt == p.dt && at(i + 1, kFuAdd)) { p.flags |= kRpAdd; p.add = st[i].ptr; i += 2; quant(); }
   if (at(i, kFuGelu)) { p.flags |= kRpGelu; ++i; quant(); }
   if (at(i, kFuSoftmax)) { p.flags |= kRpSoftmax; ++i; quant(); }
   if (at(i, kFuCarrySum)) { p.flags |= kRpCarry; ++i; }
@@ -1317,7 +1318,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
           }
         }
         f->vec = vec ? 1u : 0u;
-        MatchPipe(fs, static_cast<uint32_t>(x[2]), f->n_elems == static_cast<uint64_t>(f->rows) * f->cols, &f->pipe);
+        MatchPipe(fs, static_cast<uint32_t>(x[2]), f->n_elems == static_cast<uint64_t>(f->rows) * f->cols, f->rows == 1, &f->pipe);
         f->flat = f->vec && f->cols == 4096u ? FlatOps(fs, static_cast<uint32_t>(x[2])) : 0u;
         if (f->total) out->needs_scratch = true;
         d.desc = static_cast<uint32_t>(out->desc.size());
@@ -1387,7 +1388,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         d.desc_bytes = static_cast<uint32_t>(bytes);
         break;
       }
-      case kTopSgemm: {
+      case kTopSgemm: case kTopSkinny: {
         if (!planned) return fail_unimpl("tile op " + std::to_string(d.op) + " is not implemented by this backend");
         const int32_t *rd, *wr, *w;
         int n_rd, n_wr;
@@ -1411,6 +1412,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         g.out0 = w[7] ? c.Ref(static_cast<uint32_t>(w[7] - 1)) : 0; g.dt0 = w[8];
         g.out1 = w[9] ? c.Ref(static_cast<uint32_t>(w[9] - 1)) : 0; g.dt1 = w[10];
         ++out->n_mma;
+        if (d.op == kTopSkinny) ++out->n_mma_tc;
         out->mma_flops += 2ull * g.M * g.N * g.K;
         if (out->desc.size() % 2) out->desc.push_back(0);
         d.desc = c.PushDesc(g);

@@ -1,0 +1,145 @@
+// Products with at most 32 rows (a decode step) of re-planned programs (kTopSkinny): bf16 / f16 operands, f32
+// accumulation, the store epilogue of ops_sgemm.cuh.
+//
+// Bound: reading the weights once; at these sizes that is latency. On 128-row tensor-core tiles such a product had N / 64
+// lanes at work, each walking all of K alone (a phase of 32 x 1024 by 1024 x 4096: 20 us, now 11; 32 x 4096 by 4096 x 1024:
+// 38 us, now 17; 1 x 512 by 512 x 512: 12-14 us, now 7).
+// Here a tile is all rows by 8, 16 or 32 columns, so that every lane has its own piece of the weights, and the lane's 16 warps
+// split K: warp w takes every 16th group of 32 k, through a ring of its own in shared memory (16-byte asynchronous copies,
+// several groups ahead, no barrier among the warps), multiplies with mma.m16n8k16 (the tensor pipe is not what bounds it, and a tcgen05
+// tile has 128 rows), and the warps' sums meet in shared memory in warp order.
+// Ring block: A as rows of 64 bytes with their 16-byte pieces swizzled; B, columns contiguous: planes of 8 columns, 16 bytes per k;
+// B, k contiguous: like A. ldmatrix reads each without bank conflicts.
+#ifndef B2VM_OPS_SKINNY_CUH_
+#define B2VM_OPS_SKINNY_CUH_
+
+#include "ops_sgemm.cuh"
+
+namespace b2 {
+
+constexpr uint32_t kSkWarps = 16, kSkRing = 12800;        // bytes of a warp's ring
+
+template <int MT, int NB>
+static __device__ __noinline__ void skinny_run(const Lane &L, const DSgemm &g, uint32_t slot, uint32_t n_slots, float &csum) {
+  constexpr uint32_t kA = 1024u * MT, kB = 512u * NB, kBlock = kA + kB, kDepth = kSkRing / kBlock > 8u ? 8u : kSkRing / kBlock;
+  constexpr uint32_t ROWS = 16u * MT, COLS = 8u * NB;
+  static_assert(kDepth >= 2u && kSkWarps * ROWS * COLS * 4u <= kSkWarps * kSkRing, "a block ahead; the sums fit over the rings");
+  const KParams &P = *L.P;
+  const uint8_t *A = resolve(P, g.a.ptr) + static_cast<size_t>(g.a.off) * 2u, *B = resolve(P, g.b.ptr) + static_cast<size_t>(g.b.off) * 2u;
+  const uint8_t *res = (g.epi & kGeRes) ? resolve(P, g.res) : nullptr;
+  uint8_t *out0 = g.out0 ? resolve(P, g.out0) : nullptr, *out1 = g.out1 ? resolve(P, g.out1) : nullptr;
+  const uint32_t M = g.M, N = g.N, K = g.K, w = L.tid / kWarp, l = L.tid % kWarp;
+  const size_t lda = static_cast<size_t>(g.a.rs) * 2u;
+  const bool b_k = g.b.ks == 1u, bf = g.adt == kBF16;
+  const size_t ldb = static_cast<size_t>(b_k ? g.b.rs : g.b.ks) * 2u;
+  const uint32_t ring = smem_addr(L.smem + kSmemSys) + w * kSkRing;
+  float *part = reinterpret_cast<float *>(L.smem + kSmemSys);
+  const uint32_t groups = (K + 31u) / 32u, mine = groups > w ? (groups - w + kSkWarps - 1u) / kSkWarps : 0u;
+  const uint32_t tiles = (N + COLS - 1u) / COLS;
+  for (uint32_t tile = slot; tile < tiles; tile += n_slots) {
+    const uint32_t c0 = tile * COLS;
+    __syncthreads();
+    auto copy = [&](uint32_t i) {
+      if (i < mine) {
+        const uint32_t k0 = (w + i * kSkWarps) * 32u, d = ring + (i % kDepth) * kBlock;
+#pragma unroll
+        for (uint32_t q = 0; q < 2u * MT; ++q) {             // rows x four 16-byte pieces
+          const uint32_t e = l + 32u * q, r = e >> 2, p = e & 3u, k = k0 + 8u * p;
+          const bool in = r < M && k < K;
+          cp_async_16_zfill(d + r * 64u + ((p ^ ((r >> 1) & 3u)) << 4), in ? A + r * lda + k * 2u : A, in ? 16u : 0u);
+        }
+        if (b_k) {
+#pragma unroll
+          for (uint32_t q = 0; q < static_cast<uint32_t>(NB); ++q) {
+            const uint32_t e = l + 32u * q, r = e >> 2, p = e & 3u, k = k0 + 8u * p;
+            const bool in = c0 + r < N && k < K;
+            cp_async_16_zfill(d + kA + r * 64u + ((p ^ ((r >> 1) & 3u)) << 4), in ? B + (c0 + r) * ldb + k * 2u : B, in ? 16u : 0u);
+          }
+        } else {
+#pragma unroll
+          for (uint32_t q = 0; q < static_cast<uint32_t>(NB); ++q) {
+            const uint32_t e = l + 32u * q, kk = e / NB, nb = e % NB;
+            const bool in = c0 + 8u * nb < N && k0 + kk < K;
+            cp_async_16_zfill(d + kA + nb * 512u + kk * 16u, in ? B + (k0 + kk) * ldb + (c0 + 8u * nb) * 2u : B, in ? 16u : 0u);
+          }
+        }
+      }
+      cp_async_commit();
+    };
+    float acc[MT][NB][4];
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int n = 0; n < NB; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.0f;
+    for (uint32_t i = 0; i + 1u < kDepth; ++i) copy(i);
+#pragma unroll 1
+    for (uint32_t i = 0; i < mine; ++i) {
+      cp_async_wait<kDepth - 2>();
+      __syncwarp();                        // the other threads' copies of block i, and their reads of the block before it
+      copy(i + kDepth - 1u);
+      const uint32_t d = ring + (i % kDepth) * kBlock;
+      uint32_t b[NB][4];
+#pragma unroll
+      for (int n = 0; n < NB; ++n) {
+        const uint32_t r = 8u * n + (l & 7u), p = l >> 3;
+        if (b_k) ldmatrix_x4(b[n], d + kA + r * 64u + ((p ^ ((r >> 1) & 3u)) << 4));
+        else ldmatrix_x4_trans(b[n], d + kA + n * 512u + l * 16u);
+      }
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+#pragma unroll
+        for (uint32_t j = 0; j < 2u; ++j) {
+          const uint32_t r = 16u * m + (l & 15u), p = 2u * j + (l >> 4);
+          uint32_t a[4];
+          ldmatrix_x4(a, d + r * 64u + ((p ^ ((r >> 1) & 3u)) << 4));
+#pragma unroll
+          for (int n = 0; n < NB; ++n) {
+            if (bf) mma_bf16_16816(acc[m][n], a, b[n][2 * j], b[n][2 * j + 1]);
+            else mma_f16_16816(acc[m][n], a, b[n][2 * j], b[n][2 * j + 1]);
+          }
+        }
+      }
+    }
+    cp_async_wait_all();
+    __syncthreads();                       // the rings are done with: the sums go over them
+    float *mp = part + w * (ROWS * COLS);
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int n = 0; n < NB; ++n) {
+        float *dp = mp + (16 * m + (l >> 2)) * COLS + 8 * n + 2 * (l & 3u);
+        *reinterpret_cast<float2 *>(dp) = make_float2(acc[m][n][0], acc[m][n][1]);
+        *reinterpret_cast<float2 *>(dp + 8 * COLS) = make_float2(acc[m][n][2], acc[m][n][3]);
+      }
+    __syncthreads();
+    const uint32_t live = min(groups, kSkWarps);
+    for (uint32_t e = L.tid; e < ROWS * COLS; e += 512u) {
+      const uint32_t r = e / COLS, c = c0 + e % COLS;
+      if (r >= M || c >= N) continue;
+      float v = part[e];
+      for (uint32_t s = 1; s < live; ++s) v += part[s * (ROWS * COLS) + e];
+      if (out0) storef(out0, g.dt0, static_cast<int64_t>(r) * N + c, g.dt0 == kF32 ? v : quantize(v, g.qdt));
+      v = sg_epilogue(g, res, v, r, c, csum);
+      if (out1) storef(out1, g.dt1, static_cast<int64_t>(r) * N + c, v);
+    }
+  }
+}
+
+static __device__ __noinline__ void skinny_tiles(const Lane &L, const DTask &t, uint32_t slot, uint32_t n_slots) {
+  const DSgemm &g = *reinterpret_cast<const DSgemm *>(planned_desc(L, t));
+  float csum = 0.0f;
+  switch (g.shape) {           // 16-row blocks (1, 2) x 8-column blocks (1, 2, 4)
+    case 0: skinny_run<1, 1>(L, g, slot, n_slots, csum); break;
+    case 1: skinny_run<1, 2>(L, g, slot, n_slots, csum); break;
+    case 2: skinny_run<1, 4>(L, g, slot, n_slots, csum); break;
+    case 3: skinny_run<2, 1>(L, g, slot, n_slots, csum); break;
+    case 4: skinny_run<2, 2>(L, g, slot, n_slots, csum); break;
+    default: skinny_run<2, 4>(L, g, slot, n_slots, csum); break;
+  }
+  if (g.total) fuse_full_sum(L, csum, reinterpret_cast<float *>(resolve(*L.P, g.total)), t.p[3], g.n_owner_lanes);
+}
+
+}  // namespace b2
+#endif

@@ -30,6 +30,9 @@
 #if B2_HAS(0x2000u) // kFamSgemm
 #include "ops_sgemm.cuh"
 #endif
+#if B2_HAS(0x4000u) // kFamSkinny
+#include "ops_skinny.cuh"
+#endif
 #if B2_HAS(0x40u)   // kFamFlash: the wire programs' attention
 #include "ops_flash_tc.cuh"
 #include "ops_flash.cuh"
@@ -39,7 +42,7 @@
 #endif
 
 namespace b2 {
-static_assert(kFamFuse == 0x200u && kFamPairs == 0x400u && kFamGemm == 0x800u && kFamSgemm == 0x2000u && kFamFlash == 0x40u && kFamMove == 0x02u, "the literals in the #if lines above");
+static_assert(kFamFuse == 0x200u && kFamPairs == 0x400u && kFamGemm == 0x800u && kFamSgemm == 0x2000u && kFamSkinny == 0x4000u && kFamFlash == 0x40u && kFamMove == 0x02u, "the literals in the #if lines above");
 
 constexpr int kVmThreads = 512;
 constexpr uint32_t kNoPc = 0xFFFFFFFFu;
@@ -155,6 +158,9 @@ __global__ void __launch_bounds__(kVmThreads, 1) B2_PLAN_KERNEL(const __grid_con
 #endif
 #if B2_HAS(0x2000u)
         case kTopSgemm: sgemm_tiles(L, t, en.tile_lo, en.tile_hi); break;
+#endif
+#if B2_HAS(0x4000u)
+        case kTopSkinny: skinny_tiles(L, t, en.tile_lo, en.tile_hi); break;
 #endif
 #if B2_HAS(0x40u)
         case kTopFlashAttn: {

@@ -100,7 +100,7 @@ class Planner {
   struct Chain;
   bool FusePairs(int seed);
   bool FuseGemm(int seed);
-  void SgShape(uint64_t M, uint64_t N, uint64_t K, uint32_t lanes, int *shape, uint32_t *tiles, double *cost) const;
+  void SgShape(uint32_t op, uint64_t M, uint64_t N, uint64_t K, uint32_t lanes, int *shape, uint32_t *tiles, double *cost) const;
   bool GemmEpilogue(const Chain &c, uint32_t dst, std::vector<int32_t> *w) const;
   void GroupGemms(std::vector<int> *live, std::map<std::pair<int, int>, std::vector<int>> *phases, std::vector<std::vector<int>> *of);
   bool FuseRows(int seed);
@@ -826,7 +826,8 @@ struct Planner::Chain {
         const uint32_t other = a_cur ? nd.t.b : nd.t.a, field = a_cur ? nd.t.p3 : nd.t.p2;
         auto it = scalars.find(other);
         if (it != scalars.end()) {
-          if (ViewKind(field) != kColVec || code_s == kFuEnd) return undo();
+          const Kind kind = ViewKind(field);       // (of one row, a value per row is a scalar)
+          if (!(kind == kColVec || (R == 1 && kind == kScalar)) || code_s == kFuEnd) return undo();
           Emit(code_s, -1, 0, 0, 0, it->second);
         } else {
           if (!LoadY(other, field, i)) return undo();
@@ -994,6 +995,10 @@ bool Planner::FuseGemm(int seed) {
   bool tensor = Half(sd.adt) && MmaOperandLayout(p_, t, &lay);
   for (int64_t v : {lay.a_ld, lay.b_ld, lay.a_off, lay.b_off}) tensor = tensor && v <= 0x7fffffff;
   if (!tensor && !SgOperandsFit(p_, t)) return false;
+  // Up to 32 rows: every lane a few columns (ops_skinny.cuh). Above that re-reading the rows for every lane's columns costs more
+  // than 128-row tiles leave idle (a 64-row training step: 132 us against 111).
+  const bool skinny = tensor && t.p0 <= 32 && !lay.amn && t.p2 % 8 == 0 && t.p1 >= 8 && (!lay.bmn || t.p1 % 8 == 0) &&
+                      static_cast<uint64_t>(t.p1) * t.p2 < (1ull << 31) && SgOperandsFit(p_, t);
   // as many of the tasks that follow as the epilogue has room for: all that the chain takes, then ever fewer
   for (int limit = 1 << 30; limit >= 0;) {
     Chain c(*this, t.p0, t.p1, false);
@@ -1020,7 +1025,7 @@ bool Planner::FuseGemm(int seed) {
       if (!c.Close(&writes, false) || writes.empty() || !GemmEpilogue(c, t.dst, &epi)) continue;
     }
     Node nd;
-    nd.op = tensor ? kTopGemm : kTopSgemm;
+    nd.op = skinny ? kTopSkinny : tensor ? kTopGemm : kTopSgemm;
     nd.dt = sd.dt; nd.adt = sd.adt;
     nd.t = VmTask{};
     nd.t.dst = writes[0];
@@ -1034,12 +1039,12 @@ bool Planner::FuseGemm(int seed) {
     nd.carry_slot = c.total >= 0 ? 0 : -1;
     nd.owner_word = 2;
     auto I = [](auto v) { return static_cast<int32_t>(v); };
-    if (tensor) {
+    if (tensor && !skinny) {
       nd.payload = {1, c.total + 1, 0, I(t.p0), I(t.p1), I(t.p2), 0, 0, lay.amn ? 1 : 0, lay.bmn ? 1 : 0,
                     I(sd.adt), I(t.a), I(t.b), I(lay.a_ld), I(lay.b_ld), I(lay.a_off), I(lay.b_off)};
     } else {
       int shape = 0;
-      SgShape(t.p0, t.p1, t.p2, L_, &shape, &nd.tiles, &nd.cost);
+      SgShape(nd.op, t.p0, t.p1, t.p2, L_, &shape, &nd.tiles, &nd.cost);
       nd.payload = {shape, c.total + 1, 0, I(t.p0), I(t.p1), I(t.p2), I(sd.adt), I(t.a), I(t.b), I(t.p4), I(t.p5)};
     }
     nd.payload.insert(nd.payload.end(), epi.begin(), epi.end());
@@ -1052,10 +1057,22 @@ bool Planner::FuseGemm(int seed) {
 // Tile shape of a CUDA-core product: the one with the least time for the busiest lane. A tile's time is its FMAs at the share of
 // the issue rate that the shape's shared-memory reads leave, or the latency of its blocks' loads (16 k each, one ahead,
 // the CTA's slices taking turns), plus set-up, the slices' sums and stores.
-void Planner::SgShape(uint64_t M, uint64_t N, uint64_t K, uint32_t lanes, int *shape, uint32_t *tiles, double *cost) const {
+void Planner::SgShape(uint32_t op, uint64_t M, uint64_t N, uint64_t K, uint32_t lanes, int *shape, uint32_t *tiles, double *cost) const {
   struct S { uint32_t tm, tn, slices; double rate; };
   static const S shapes[5] = {{128, 64, 4, 0.75}, {64, 64, 8, 0.75}, {64, 32, 8, 0.6}, {32, 32, 8, 0.45}, {16, 16, 8, 0.2}};
   double best = 1e300;
+  if (op == kTopSkinny) {
+    // a tile's time: the bytes of its rows and columns at what a lane draws from L2 (~40 a cycle), and what every tile has to
+    // wait for once (a first load, the warps' sums, the stores)
+    const int mt = M <= 16 ? 0 : 1;
+    for (int nb = 0; nb < 3; ++nb) {
+      const uint64_t cols = 8ull << nb, T = (N + cols - 1) / cols;
+      const double tile = 3000.0 + static_cast<double>(K) * 2.0 * static_cast<double>((16u << mt) + cols) / 40.0;
+      const double time = tile * static_cast<double>((T + lanes - 1) / lanes);
+      if (time < best) { best = time; *shape = 3 * mt + nb; *tiles = static_cast<uint32_t>(T); *cost = tile / 6000.0; }
+    }
+    return;
+  }
   for (int i = 0; i < 5; ++i) {
     const S &s = shapes[i];
     const uint64_t T = ((M + s.tm - 1) / s.tm) * ((N + s.tn - 1) / s.tn);
@@ -1074,14 +1091,14 @@ void Planner::GroupGemms(std::vector<int> *live, std::map<std::pair<int, int>, s
   for (auto &kv : *phases) {
     std::vector<int> gs, rest;
     for (int u : kv.second) (n_[u].op == kTopGemm && n_[u].planned ? gs : rest).push_back(u);
-    // CUDA-core products side by side share the lanes by cost
+    // CUDA-core and skinny products side by side share the lanes by cost
     double sg_all = 0;
-    for (int u : rest) if (n_[u].op == kTopSgemm) sg_all += n_[u].cost * n_[u].tiles;
+    for (int u : rest) if (n_[u].op == kTopSgemm || n_[u].op == kTopSkinny) sg_all += n_[u].cost * n_[u].tiles;
     for (int u : rest) {
       Node &x = n_[u];
-      if (x.op != kTopSgemm) continue;
+      if (x.op != kTopSgemm && x.op != kTopSkinny) continue;
       const double share = x.cost * x.tiles / sg_all;
-      SgShape(x.payload[3], x.payload[4], x.payload[5], std::max(1u, static_cast<uint32_t>(L_ * share + 0.5)), &x.payload[0], &x.tiles, &x.cost);
+      SgShape(x.op, x.payload[3], x.payload[4], x.payload[5], std::max(1u, static_cast<uint32_t>(L_ * share + 0.5)), &x.payload[0], &x.tiles, &x.cost);
     }
     if (gs.empty()) continue;
     std::sort(gs.begin(), gs.end(), [&](int a, int b) { return n_[a].payload[5] > n_[b].payload[5]; });

@@ -24,8 +24,8 @@
   X(all, b2::kFamWire)                                   \
   X(plan_rows, b2::kFamFuse)                             \
   X(plan_pairs, b2::kFamFuse | b2::kFamPairs)            \
-  X(plan_gemm, b2::kFamFuse | b2::kFamGemm)              \
+  X(plan_gemm, b2::kFamFuse | b2::kFamGemm | b2::kFamSkinny) \
   X(plan_sgemm, b2::kFamFuse | b2::kFamSgemm)            \
-  X(plan_attn, b2::kFamFuse | b2::kFamGemm | b2::kFamSgemm | b2::kFamFlash | b2::kFamMove)
+  X(plan_attn, b2::kFamFuse | b2::kFamGemm | b2::kFamSgemm | b2::kFamSkinny | b2::kFamFlash | b2::kFamMove)
 
 #endif
