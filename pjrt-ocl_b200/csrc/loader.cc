@@ -1411,6 +1411,11 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         g.res = w[6] ? c.Ref(static_cast<uint32_t>(w[6] - 1)) : 0;
         g.out0 = w[7] ? c.Ref(static_cast<uint32_t>(w[7] - 1)) : 0; g.dt0 = w[8];
         g.out1 = w[9] ? c.Ref(static_cast<uint32_t>(w[9] - 1)) : 0; g.dt1 = w[10];
+        if (d.op == kTopSkinny && w[11]) {
+          g.gamma = c.Ref(static_cast<uint32_t>(w[11] - 1));
+          std::memcpy(&g.ns, &w[12], 4);
+          std::memcpy(&g.nt, &w[13], 4);
+        }
         ++out->n_mma;
         if (d.op == kTopSkinny) ++out->n_mma_tc;
         out->mma_flops += 2ull * g.M * g.N * g.K;

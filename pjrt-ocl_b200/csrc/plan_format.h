@@ -125,6 +125,9 @@ struct DSgemm {
   BufRef res, out0, out1, total;
   uint32_t dt0, dt1;
   DSgOperand a, b;
+  // kTopSkinny: A is the RMS norm of the rows at a.ptr: x rsqrt(ns sum x^2 + nt) gamma (0: A as it is)
+  BufRef gamma;
+  float ns, nt;
 };
 
 }  // namespace b2

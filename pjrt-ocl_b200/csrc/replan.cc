@@ -103,6 +103,7 @@ class Planner {
   void SgShape(uint32_t op, uint64_t M, uint64_t N, uint64_t K, uint32_t lanes, int *shape, uint32_t *tiles, double *cost) const;
   bool GemmEpilogue(const Chain &c, uint32_t dst, std::vector<int32_t> *w) const;
   void GroupGemms(std::vector<int> *live, std::map<std::pair<int, int>, std::vector<int>> *phases, std::vector<std::vector<int>> *of);
+  void NormIntoProducts(std::vector<int> *live, std::vector<std::set<int>> *pred);
   bool FuseRows(int seed);
   bool FuseFlat(int seed);
   Node RowsNode(const Chain &c, uint32_t start, const std::vector<uint32_t> &writes, uint64_t R, uint64_t C, uint64_t n) const;
@@ -1048,6 +1049,7 @@ bool Planner::FuseGemm(int seed) {
       nd.payload = {shape, c.total + 1, 0, I(t.p0), I(t.p1), I(t.p2), I(sd.adt), I(t.a), I(t.b), I(t.p4), I(t.p5)};
     }
     nd.payload.insert(nd.payload.end(), epi.begin(), epi.end());
+    if (skinny) nd.payload.insert(nd.payload.end(), {0, 0, 0});       // gamma + 1, ns, nt: NormIntoProducts
     if (AddPlanned(nd, c.members) >= 0) return true;
     if (t.p6) return false;
   }
@@ -1277,6 +1279,50 @@ bool Planner::FuseFlat(int seed) {
   return AddPlanned(RowsNode(c, start, writes, R, C, n), c.members) >= 0;
 }
 
+// The RMS norm of a few rows that only skinny products read: every lane norms the rows for itself while its weights are on
+// their way, instead of in a phase of its own (which is 8 us of latency in a decode step).
+void Planner::NormIntoProducts(std::vector<int> *live, std::vector<std::set<int>> *pred) {
+  for (size_t k = 0; k < live->size();) {
+    const int r = (*live)[k];
+    const Node &nd = n_[r];
+    ++k;
+    if (!nd.planned || nd.op != kTopFuseRows || nd.wr.size() != 1 || nd.payload[0] > 32 || nd.payload[1] > 1024 || nd.payload[1] % 32 != 0 || nd.payload[2] != 9) continue;
+    const int32_t *st = &nd.payload[7];
+    auto code = [&](int i) { return static_cast<uint32_t>(st[6 * i]); };
+    const uint32_t dt = static_cast<uint32_t>(st[1]), h = nd.wr[0];
+    if (!Half(dt) || code(0) != kFuLoadX || code(1) != kFuRedSumSq || code(2) != kFuSAffine || code(3) != kFuSRsqrt || code(4) != kFuMulS ||
+        !(code(5) == kFuRowVecY || (code(5) == kFuLoadY && nd.payload[0] == 1)) || code(6) != kFuMul || code(7) != kFuQuant || code(8) != kFuStore ||
+        static_cast<uint32_t>(st[6 * 5 + 1]) != dt || static_cast<uint32_t>(st[6 * 8 + 1]) != dt || Pinned(h))
+      continue;
+    std::vector<int> users;
+    bool ok = true;
+    for (int u : *live)
+      if (u != r && (*pred)[u].count(r)) {
+        users.push_back(u);
+        const Node &s = n_[u];
+        ok = ok && s.planned && s.op == kTopSkinny && s.region == nd.region && s.payload[3] == nd.payload[0] && s.payload[5] == nd.payload[1] &&
+             s.payload[7] == static_cast<int32_t>(h) && s.payload[8] != static_cast<int32_t>(h) && s.payload[9] == 0 && s.payload[17] != static_cast<int32_t>(h + 1) &&
+             s.payload[22] == 0;
+      }
+    if (!ok || users.empty()) continue;
+    const int32_t x = st[4] - 1, gamma = st[6 * 5 + 4] - 1;
+    for (int u : users) {
+      Node &s = n_[u];
+      s.payload[7] = x;
+      s.payload[22] = gamma + 1;
+      s.payload[23] = st[6 * 2 + 2];
+      s.payload[24] = st[6 * 2 + 3];
+      s.t.a = static_cast<uint32_t>(x);
+      s.rd.erase(std::remove(s.rd.begin(), s.rd.end(), h), s.rd.end());
+      s.rd.push_back(static_cast<uint32_t>(x));
+      s.rd.push_back(static_cast<uint32_t>(gamma));
+      (*pred)[u].erase(r);
+      (*pred)[u].insert((*pred)[r].begin(), (*pred)[r].end());
+    }
+    live->erase(live->begin() + static_cast<long>(--k));
+  }
+}
+
 // Phases by data dependence, lanes by cost, buffers by liveness.
 bool Planner::Assemble(VmProgram *q, ReplanStats *st) {
   const int N = static_cast<int>(n_.size());
@@ -1286,6 +1332,7 @@ bool Planner::Assemble(VmProgram *q, ReplanStats *st) {
   std::vector<std::set<int>> pred(N);
   for (int i = 0; i < n_orig_; ++i)
     for (int j : pred_[i]) if (rep_[j] != rep_[i]) pred[rep_[i]].insert(rep_[j]);
+  NormIntoProducts(&live, &pred);
   std::vector<int> unit(N);
   for (int i : live) unit[i] = i;
   std::vector<std::vector<int>> of(N);
