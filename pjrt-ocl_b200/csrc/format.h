@@ -277,7 +277,7 @@ struct DFlash {        // loader-built
   // program's scratch (heaviest first) instead of keeping their static ranges.
   uint32_t work_slot;             // index of the {next, done} pair in the scratch, or kNoWorkSlot
   uint32_t n_owner_lanes;
-  // Few query rows per head (a decode step) with 16-bit K and V whose head_dim axis is the
+  // Few query rows per head (a decode step) with float K and V whose head_dim axis is the
   // unit-stride one: element (g, key, d) of K at dk_off + g * dk_g + key * dk_c + d (V alike),
   // every term a multiple of 8 elements, so a key's row is read with 16-byte loads.
   uint32_t dec_mode;

@@ -1156,7 +1156,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         }
         // Decode-shaped tasks (few query rows, CUDA-core path): K and V rows by 16-byte loads when
         // head_dim is their unit-stride axis. K arrives as [H, hd, C] (a view of a [H, C, hd] cache).
-        if (!f.tc_mode && (d.adt == kBF16 || d.adt == kF16) && !qv && (x[3] == 64 || x[3] == 128) && x[1] <= 8 &&
+        if (!f.tc_mode && (d.adt == kBF16 || d.adt == kF16 || d.adt == kF32) && !qv && (x[3] == 64 || x[3] == 128) && x[1] <= 8 &&
             x[0] > 0 && x[2] > 0 && c.Aligned16(t.a) && c.Aligned16(t.b) && c.Aligned16(t.p0)) {
           const int64_t H = x[0], C = x[2], hd = x[3];
           const int64_t nk[3] = {H, hd, C}, nv[3] = {H, C, hd};
@@ -1416,6 +1416,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
           std::memcpy(&g.ns, &w[12], 4);
           std::memcpy(&g.nt, &w[13], 4);
         }
+        if (d.op == kTopSkinny && w[14]) g.move = out->tasks[w[14] - 1].desc;
         ++out->n_mma;
         if (d.op == kTopSkinny) ++out->n_mma_tc;
         out->mma_flops += 2ull * g.M * g.N * g.K;

@@ -13,6 +13,8 @@
 #ifndef B2VM_OPS_FLASH_CUH_
 #define B2VM_OPS_FLASH_CUH_
 
+#include <type_traits>
+
 #include "dev_common.cuh"
 #include "ops_ew.cuh"
 
@@ -22,34 +24,49 @@ namespace b2 {
 constexpr int kFlashMaxHd = 256;
 
 // Decode-shaped tasks (DFlash::dec_mode): every (head, query row) tile is worked on by the whole
-// lane. LPK = hd / 8 threads share one key: each holds 8 consecutive d of q (pre-scaled by
+// lane. (f32 takes two words per 8 d; through the views element by element 32 heads x 500
+// keys took 103 us.) LPK = hd / 8 threads share one key: each holds 8 consecutive d of q (pre-scaled by
 // scale * log2 e) and reads the same 8 d of the key's K row and V row as one 16-byte load
 // each. A warp covers 32 / LPK keys per load and 8 loads per operand and trip (16 loads in
 // flight per thread); the lane's warps take trips round-robin, keep their own running (max, sum,
 // accumulator) in the base-2 domain, and are merged through shared memory.
-template <int HD, bool BF>
+template <int HD, int DT>
 static __device__ __noinline__ void flash_decode_tiles(const Lane &L, const DTask &t, const DFlash &df, uint32_t tile_lo,
                                                           int64_t hi, int64_t T, int64_t C, float scale, bool causal) {
   constexpr int LPK = HD / 8;              // threads per key
   constexpr int KPL = 32 / LPK;            // keys per warp-wide load
-  constexpr int U = 8;                     // loads in flight per operand
+  constexpr bool F32 = DT == kF32;
+  constexpr int U = F32 ? 4 : 8;           // keys in flight per thread
+  constexpr int W = F32 ? 2 : 1;           // 16-byte words of 8 elements
+  constexpr uint32_t ESZ = F32 ? 4u : 2u;
   constexpr int KPT = KPL * U;             // keys per warp trip
   const KParams &P = *L.P;
   uint8_t *out = resolve(P, t.ptr[0]);
-  const uint16_t *Q = reinterpret_cast<const uint16_t *>(resolve(P, t.ptr[1]));
-  const uint16_t *K = reinterpret_cast<const uint16_t *>(resolve(P, t.ptr[2])) + df.dk_off;
-  const uint16_t *V = reinterpret_cast<const uint16_t *>(resolve(P, t.ptr[3])) + df.dv_off;
-  constexpr bool bf = BF;
+  const uint8_t *Q = resolve(P, t.ptr[1]), *K = resolve(P, t.ptr[2]) + df.dk_off * ESZ, *V = resolve(P, t.ptr[3]) + df.dv_off * ESZ;
   const uint32_t w = L.tid / kWarp, l = L.tid % kWarp, nw = L.nthr / kWarp;
   const uint32_t part = l % LPK, sub = l / LPK;
   float *ml = reinterpret_cast<float *>(L.smem + kSmemSys);                          // [nw][2]
   float *os = ml + 2 * 32;                                                           // [nw][HD]
-  auto unpack8 = [&](const uint4 &v, float (&f)[8]) {
-    const uint32_t wd[4] = {v.x, v.y, v.z, v.w};
+  struct Oct { uint4 v[W]; };
+  auto get = [&](const uint8_t *p, int64_t i) {
+    Oct o;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      f[2 * i] = bf ? __uint_as_float(wd[i] << 16) : f16_bits_to_f32(wd[i] & 0xffffu);
-      f[2 * i + 1] = bf ? __uint_as_float(wd[i] & 0xffff0000u) : f16_bits_to_f32(wd[i] >> 16);
+    for (int k = 0; k < W; ++k) o.v[k] = ldg_v4(p + i * ESZ + 16 * k);
+    return o;
+  };
+  auto unpack8 = [&](const Oct &o, float (&f)[8]) {
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const uint32_t wd[4] = {o.v[k].x, o.v[k].y, o.v[k].z, o.v[k].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if constexpr (F32) {
+          f[4 * k + i] = __uint_as_float(wd[i]);
+        } else {
+          f[2 * i] = DT == kBF16 ? __uint_as_float(wd[i] << 16) : f16_bits_to_f32(wd[i] & 0xffffu);
+          f[2 * i + 1] = DT == kBF16 ? __uint_as_float(wd[i] & 0xffff0000u) : f16_bits_to_f32(wd[i] >> 16);
+        }
+      }
     }
   };
   const float sl2 = scale * 1.4426950408889634f;
@@ -57,26 +74,27 @@ static __device__ __noinline__ void flash_decode_tiles(const Lane &L, const DTas
     const int64_t g = tile / T, m = tile % T;
     const int64_t c_end = causal ? min(C, m + (C - T) + 1) : C;
     float q[8];
-    unpack8(ldg_v4(Q + (g * T + m) * HD + part * 8), q);
+    unpack8(get(Q, (g * T + m) * HD + part * 8), q);
 #pragma unroll
     for (int i = 0; i < 8; ++i) q[i] *= sl2;
-    const uint16_t *Kg = K + g * df.dk_g + part * 8, *Vg = V + g * df.dv_g + part * 8;
+    const uint8_t *Kg = K + (g * df.dk_g + part * 8) * ESZ, *Vg = V + (g * df.dv_g + part * 8) * ESZ;
     float m_run = -INFINITY, l_run = 0.0f, o[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) o[i] = 0.0f;
-    auto load = [&](uint4 (&kk)[U], uint4 (&vv)[U], int64_t c0) {
+    const Oct none = {};
+    auto load = [&](Oct (&kk)[U], Oct (&vv)[U], int64_t c0) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int64_t key = c0 + u * KPL + sub;
-        kk[u] = key < c_end ? ldg_v4(Kg + key * df.dk_c) : make_uint4(0u, 0u, 0u, 0u);
+        kk[u] = key < c_end ? get(Kg, key * df.dk_c) : none;
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int64_t key = c0 + u * KPL + sub;
-        vv[u] = key < c_end ? ldg_v4(Vg + key * df.dv_c) : make_uint4(0u, 0u, 0u, 0u);
+        vv[u] = key < c_end ? get(Vg, key * df.dv_c) : none;
       }
     };
-    auto compute = [&](const uint4 (&kk)[U], const uint4 (&vv)[U], int64_t c0) {
+    auto compute = [&](const Oct (&kk)[U], const Oct (&vv)[U], int64_t c0) {
       float sc[U], cmax = -INFINITY;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -109,7 +127,7 @@ static __device__ __noinline__ void flash_decode_tiles(const Lane &L, const DTas
       }
     };
     for (int64_t c0 = static_cast<int64_t>(KPT) * w; c0 < c_end; c0 += static_cast<int64_t>(KPT) * nw) {
-      uint4 kk[U], vv[U];
+      Oct kk[U], vv[U];
       load(kk, vv, c0);
       compute(kk, vv, c0);
     }
@@ -436,7 +454,7 @@ static __device__ __noinline__ void flash_simt_tiles(const Lane &L, const DTask 
   const uint32_t w = L.tid / kWarp, l = L.tid % kWarp, nw = L.nthr / kWarp;
   const int64_t hi = min(static_cast<int64_t>(tile_hi), H * T);
   __syncthreads();  // workspace handover from the previous op
-  if (df.dec_mode && df.dk_c == hd && df.dv_c == hd && L.nthr == 512u &&
+  if (df.dec_mode && adt != kF32 && df.dk_c == hd && df.dv_c == hd && L.nthr == 512u &&
       L.smem_bytes >= kSmemSys + 256u + 4u * 32u * static_cast<uint32_t>(hd) + 192u + 3u * 2u * (L.nthr / kWarp) * 4u * (256u / static_cast<uint32_t>(hd)) * static_cast<uint32_t>(hd) * 2u) {
     // contiguous K / V rows: the ring of bulk copies
     if (hd == 64 && adt == kBF16) flash_decode_ring<64, true>(L, t, df, tile_lo, hi, T, C, scale, causal);
@@ -446,10 +464,14 @@ static __device__ __noinline__ void flash_simt_tiles(const Lane &L, const DTask 
     return;
   }
   if (df.dec_mode) {
-    if (hd == 64 && adt == kBF16) flash_decode_tiles<64, true>(L, t, df, tile_lo, hi, T, C, scale, causal);
-    else if (hd == 64) flash_decode_tiles<64, false>(L, t, df, tile_lo, hi, T, C, scale, causal);
-    else if (adt == kBF16) flash_decode_tiles<128, true>(L, t, df, tile_lo, hi, T, C, scale, causal);
-    else flash_decode_tiles<128, false>(L, t, df, tile_lo, hi, T, C, scale, causal);
+    auto run = [&](auto hd_c) {
+      constexpr int HD = decltype(hd_c)::value;
+      if (adt == kF32) flash_decode_tiles<HD, kF32>(L, t, df, tile_lo, hi, T, C, scale, causal);
+      else if (adt == kBF16) flash_decode_tiles<HD, kBF16>(L, t, df, tile_lo, hi, T, C, scale, causal);
+      else flash_decode_tiles<HD, kF16>(L, t, df, tile_lo, hi, T, C, scale, causal);
+    };
+    if (hd == 64) run(std::integral_constant<int, 64>{});
+    else run(std::integral_constant<int, 128>{});
     return;
   }
   if ((hi - static_cast<int64_t>(tile_lo)) * 2 <= static_cast<int64_t>(nw) && hd <= 128) {

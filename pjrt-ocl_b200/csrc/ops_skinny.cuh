@@ -9,11 +9,13 @@
 // several groups ahead, no barrier among the warps), multiplies with mma.m16n8k16 (the tensor pipe is not what bounds it, and a tcgen05
 // tile has 128 rows), and the warps' sums meet in shared memory in warp order.
 // Rows that are an RMS norm's result are normed by every lane for itself, under the first weights' flight.
+// A dynamic slice update that was all a product was for (a cache row) is its store's address.
 // Ring block: A as rows of 64 bytes with their 16-byte pieces swizzled; B, columns contiguous: planes of 8 columns, 16 bytes per k;
 // B, k contiguous: like A. ldmatrix reads each without bank conflicts.
 #ifndef B2VM_OPS_SKINNY_CUH_
 #define B2VM_OPS_SKINNY_CUH_
 
+#include "ops_move.cuh"
 #include "ops_sgemm.cuh"
 
 namespace b2 {
@@ -175,6 +177,8 @@ static __device__ __noinline__ void skinny_run(const Lane &L, const DSgemm &g, u
       }
     __syncthreads();
     const uint32_t live = min(groups, kSkWarps);
+    const DMove *mv = g.move ? reinterpret_cast<const DMove *>(P.desc + g.move) : nullptr;
+    const int64_t at = mv ? dyn_base(P, *mv) : 0;
     for (uint32_t e = L.tid; e < ROWS * COLS; e += 512u) {
       const uint32_t r = e / COLS, c = c0 + e % COLS;
       if (r >= M || c >= N) continue;
@@ -182,7 +186,7 @@ static __device__ __noinline__ void skinny_run(const Lane &L, const DSgemm &g, u
       for (uint32_t s = 1; s < live; ++s) v += part[s * (ROWS * COLS) + e];
       if (out0) storef(out0, g.dt0, static_cast<int64_t>(r) * N + c, g.dt0 == kF32 ? v : quantize(v, g.qdt));
       v = sg_epilogue(g, res, v, r, c, csum);
-      if (out1) storef(out1, g.dt1, static_cast<int64_t>(r) * N + c, v);
+      if (out1) storef(out1, g.dt1, mv ? at + view_index(mv->view, r * N + c) : static_cast<int64_t>(r) * N + c, v);
     }
   }
 }

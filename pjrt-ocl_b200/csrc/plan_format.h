@@ -128,6 +128,7 @@ struct DSgemm {
   // kTopSkinny: A is the RMS norm of the rows at a.ptr: x rsqrt(ns sum x^2 + nt) gamma (0: A as it is)
   BufRef gamma;
   float ns, nt;
+  uint32_t move, pad;      // kTopSkinny: out1 is written through this dynamic slice (desc index of its DMove; 0: dense)
 };
 
 }  // namespace b2

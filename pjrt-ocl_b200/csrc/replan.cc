@@ -1049,7 +1049,23 @@ bool Planner::FuseGemm(int seed) {
       nd.payload = {shape, c.total + 1, 0, I(t.p0), I(t.p1), I(t.p2), I(sd.adt), I(t.a), I(t.b), I(t.p4), I(t.p5)};
     }
     nd.payload.insert(nd.payload.end(), epi.begin(), epi.end());
-    if (skinny) nd.payload.insert(nd.payload.end(), {0, 0, 0});       // gamma + 1, ns, nt: NormIntoProducts
+    if (skinny) {
+      nd.payload.insert(nd.payload.end(), {0, 0, 0, 0});       // gamma + 1, ns, nt: NormIntoProducts; update + 1 (a node here, a task in the program)
+      // a dynamic slice update of nothing but this result takes the store
+      const int u = writes.size() == 1 && writes[0] == static_cast<uint32_t>(epi[9] - 1) && Uses(writes[0]).size() == 1 && !Pinned(writes[0]) ? Uses(writes[0])[0] : -1;
+      if (u >= 0 && Free(u) && n_[u].op == kTopDynScatter && n_[u].t.a == writes[0] && n_[u].dt == Dt(writes[0]) && n_[u].t.p1 == t.p0 * t.p1 &&
+          n_[u].region == sd.region) {
+        Node with = nd;
+        with.payload[20] = static_cast<int32_t>(n_[u].t.dst + 1);
+        with.payload[25] = u + 1;
+        with.t.dst = n_[u].t.dst;
+        with.wr = {n_[u].t.dst};
+        for (uint32_t b : n_[u].rd) if (b != writes[0]) with.rd.push_back(b);
+        std::vector<int> members = c.members;
+        members.push_back(u);
+        if (AddPlanned(with, members) >= 0) return true;
+      }
+    }
     if (AddPlanned(nd, c.members) >= 0) return true;
     if (t.p6) return false;
   }
@@ -1400,6 +1416,12 @@ bool Planner::Assemble(VmProgram *q, ReplanStats *st) {
       for (int i : of[u])
         if (n_[i].carry_slot >= 0) { if (slot >= 3) return false; n_[i].carry_slot = slot++; }
   }
+  // the updates that products store through: tasks that no entry names, for their descriptors
+  for (int i : live)
+    if (n_[i].op == kTopSkinny && n_[i].payload[25]) {
+      q->tasks.push_back(n_[n_[i].payload[25] - 1].t);
+      n_[i].payload[25] = static_cast<int32_t>(q->tasks.size());
+    }
   for (int i : live) {
     VmTask t = n_[i].t;
     if (n_[i].planned) {
