@@ -213,6 +213,7 @@ static __device__ __noinline__ void sgemm_run(const Lane &L, const DSgemm &g, ui
         }
         cp_async_commit();
       };
+#pragma unroll 1
       for (uint32_t i = 0; i < ST - 1; ++i) copy(i);
 #pragma unroll 1
       for (uint32_t i = 0; i < mine; ++i) {
@@ -251,6 +252,7 @@ static __device__ __noinline__ void sgemm_run(const Lane &L, const DSgemm &g, ui
         unpack_f32x2(acc[i][j], d[0], d[TN]);
       }
     __syncthreads();
+#pragma unroll 1
     for (uint32_t e = L.tid; e < TM * TN; e += 512u) {
       const uint32_t r = r0 + e / TN, c = c0 + e % TN;
       if (r >= M || c >= N) continue;

@@ -38,6 +38,7 @@ static __device__ __noinline__ void skinny_norm(const Lane &L, const DSgemm &g, 
   const uint32_t w = L.tid / kWarp, l = L.tid % kWarp, K = g.K, dt = g.adt;
   const uint8_t *x = resolve(P, g.a.ptr), *gam = resolve(P, g.gamma);
   uint8_t *dst = L.smem + kSmemSys + kSkWarps * kSkNormRing;
+#pragma unroll 1
   for (uint32_t r = w; r < rows; r += kSkWarps) {
     uint4 v[4];
     float ss = 0.0f, f[8];
@@ -91,6 +92,7 @@ static __device__ __noinline__ void skinny_run(const Lane &L, const DSgemm &g, u
   const uint32_t groups = (K + 31u) / 32u, mine = groups > w ? (groups - w + kSkWarps - 1u) / kSkWarps : 0u;
   const uint32_t tiles = (N + COLS - 1u) / COLS;
   bool first = true;
+  const DMove *mv = g.move ? reinterpret_cast<const DMove *>(P.desc + g.move) : nullptr;
   for (uint32_t tile = slot; tile < tiles; tile += n_slots) {
     const uint32_t c0 = tile * COLS;
     __syncthreads();
@@ -130,7 +132,10 @@ static __device__ __noinline__ void skinny_run(const Lane &L, const DSgemm &g, u
       for (int n = 0; n < NB; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.0f;
+    // (not unrolled, here and below: a phase runs this code once, and fetching it is much of its time)
+#pragma unroll 1
     for (uint32_t i = 0; i + 1u < kDepth; ++i) copy(i);
+    const int64_t at = mv ? dyn_base(P, *mv) : 0;          // (its loads too under the weights' flight)
     if (NORM && first) {
       skinny_norm(L, g, ROWS);
       __syncthreads();
@@ -177,12 +182,12 @@ static __device__ __noinline__ void skinny_run(const Lane &L, const DSgemm &g, u
       }
     __syncthreads();
     const uint32_t live = min(groups, kSkWarps);
-    const DMove *mv = g.move ? reinterpret_cast<const DMove *>(P.desc + g.move) : nullptr;
-    const int64_t at = mv ? dyn_base(P, *mv) : 0;
+#pragma unroll 1
     for (uint32_t e = L.tid; e < ROWS * COLS; e += 512u) {
       const uint32_t r = e / COLS, c = c0 + e % COLS;
       if (r >= M || c >= N) continue;
       float v = part[e];
+#pragma unroll 4
       for (uint32_t s = 1; s < live; ++s) v += part[s * (ROWS * COLS) + e];
       if (out0) storef(out0, g.dt0, static_cast<int64_t>(r) * N + c, g.dt0 == kF32 ? v : quantize(v, g.qdt));
       v = sg_epilogue(g, res, v, r, c, csum);

@@ -1,0 +1,109 @@
+"""Re-planned programs against a float64 reference, at the sizes where their kernels' tiles, splits and remainders meet."""
+from __future__ import annotations
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+
+def _gelu(x):
+    return torch.nn.functional.gelu(x, approximate="tanh")
+
+
+def _rms(x, g):
+    return x * torch.rsqrt((x * x).mean(1, keepdim=True) + 1e-6) * g
+
+
+def _reference(c, args):
+    a = [x.double() if x.is_floating_point() else x for x in args]
+    k, h = c["kind"], c.get("heads")
+    sdpa = torch.nn.functional.scaled_dot_product_attention
+    if k == "relu_matmul":
+        return [(a[0] @ a[1]).clamp(min=0)]
+    if k == "dot":
+        return [a[0] @ (a[1].T if c["transposed"] else a[1])]
+    if k == "norm_chain":
+        y = (a[0] - a[0].mean(1, keepdim=True)) / torch.sqrt(a[0].var(1, unbiased=False, keepdim=True) + 1e-5)
+        s = torch.softmax(_gelu(y * a[1] + a[2]), 1)
+        return [s, s.sum()]
+    if k == "int_chain":
+        return [torch.maximum((a[0] + a[1]) ^ a[2], a[3])]
+    if k == "mlp":
+        ws = [w.clone().requires_grad_() for w in a[2:5]]
+        loss = ((_gelu(_gelu(a[0] @ ws[0]) @ ws[1]) @ ws[2] - a[1]) ** 2).mean()
+        loss.backward()
+        return [loss.detach()] + [w.detach() - 1e-3 * w.grad for w in ws]
+    if k == "block":
+        g1, x, wq, wk, wv, wo, g2, w1, w2 = a
+        b, s = c["batch"], c["seq"]
+        y = _rms(x, g1)
+        q, kk, v = ((y @ w).view(b, s, h, 64).transpose(1, 2) for w in (wq, wk, wv))
+        x1 = x + sdpa(q, kk, v, is_causal=True).transpose(1, 2).reshape(x.shape) @ wo
+        return [x1 + _gelu(_rms(x1, g2) @ w1) @ w2]
+    if k == "decode":
+        g1, x, kc, vc, _, wq, wk, wv, wo, g2, w1, w2 = a
+        n = c["batch"] * h
+        y, kc, vc = _rms(x, g1), kc.clone(), vc.clone()
+        kc[:, -1], vc[:, -1] = (y @ wk).view(n, 64), (y @ wv).view(n, 64)
+        x1 = x + sdpa((y @ wq).view(n, 1, 64), kc, vc).view(c["batch"], -1) @ wo
+        return [x1 + _gelu(_rms(x1, g2) @ w1) @ w2, kc, vc]
+    p, v, m = a
+    dt = 1e-3
+
+    def acc(p):
+        d = p[None] - p[:, None]
+        return (d * ((d * d).sum(2) + 1e-4).pow(-1.5).mul(m[None])[..., None]).sum(1)
+    for _ in range(c["steps"]):
+        a1 = acc(p); v2 = v + dt / 2 * a1
+        a2 = acc(p + dt / 2 * v); v3 = v + dt / 2 * a2
+        a3 = acc(p + dt / 2 * v2); v4 = v + dt * a3
+        a4 = acc(p + dt * v3)
+        p, v = p + dt / 6 * (v + 2 * v2 + 2 * v3 + v4), v + dt / 6 * (a1 + 2 * a2 + 2 * a3 + a4)
+    return [p, v]
+
+
+def _case(kind, **kw):
+    return pytest.param(dict(kind=kind, **kw), id="-".join([kind, *(str(v) for v in kw.values())]))
+
+
+@pytest.mark.parametrize("c", [
+    # CUDA-core products: one tile, ragged edges, K of one block / not a multiple of a block, every tile shape
+    *(_case("dot", m=m, k=k, n=n, dtype="f32", transposed=t) for m, k, n, t in
+      [(1, 1, 1, False), (17, 33, 15, True), (130, 100, 66, False), (512, 16, 384, True), (700, 250, 516, False), (1024, 64, 1024, True)]),
+    _case("relu_matmul", m=129, k=31, n=65, dtype="f32", call="device"),
+    # ... of 16-bit operands that TMA cannot fetch
+    _case("dot", m=65, k=77, n=131, dtype="bf16", transposed=False), _case("dot", m=200, k=45, n=99, dtype="f16", transposed=True),
+    # tensor-core products: both tile heights, every width, K below and across a stage
+    *(_case("dot", m=m, k=k, n=n, dtype=dt, transposed=t) for m, k, n, dt, t in
+      [(33, 8, 8, "bf16", False), (129, 72, 136, "f16", True), (256, 64, 264, "bf16", True), (1000, 200, 2048, "bf16", False), (2304, 320, 4104, "bf16", True)]),
+    # few rows: one and two row blocks, column blocks of every width, K of less than a group per warp
+    *(_case("dot", m=m, k=k, n=n, dtype=dt, transposed=t) for m, k, n, dt, t in
+      [(1, 8, 8, "bf16", False), (16, 40, 72, "f16", True), (17, 1032, 1000, "bf16", False), (32, 512, 4096, "bf16", True), (32, 2048, 2408, "f16", False)]),
+    # row pipelines and flat chains
+    *(_case("norm_chain", rows=r, cols=n, dtype=dt) for r, n, dt in
+      [(1, 128, "f32"), (149, 130, "bf16"), (64, 1023, "f16"), (300, 2048, "bf16"), (33, 4096, "f32")]),
+    _case("int_chain", rows=1, cols=131), _case("int_chain", rows=601, cols=1025), _case("int_chain", rows=2048, cols=512),
+    # store epilogues: GELU, its derivative, the update step, the loss sum
+    _case("mlp", batch=72, d0=64, d1=136, d2=264, d3=72, dtype="bf16"), _case("mlp", batch=67, d0=33, d1=50, d2=21, d3=40, dtype="f32"),
+    # attention between products; a decode step with its cache rows stored by the products
+    _case("block", batch=2, seq=65, heads=4, dtype="bf16"), _case("block", batch=1, seq=77, heads=4, dtype="f32"), _case("block", batch=1, seq=300, heads=2, dtype="f32"),
+    _case("decode", batch=1, cache=64, heads=4, dtype="bf16"), _case("decode", batch=17, cache=301, heads=8, dtype="f16"), _case("decode", batch=3, cache=70, heads=4, dtype="f32"),
+    _case("nbody", bodies=257, steps=2),
+])
+def test_planned_program(c):
+    import perf.cases as cases
+    state = cases.prepare(c, 5)
+    args = [x.clone() for x in state["args"]]
+    for _ in range(2):                            # the second run finds what the first one left behind
+        outs = cases.run(state)
+    torch.cuda.synchronize()
+    assert state["lp"].Status()["code"] == 0 and state["lp"].stat("replanned") == 1
+    tol = cases.tolerance(c)
+    for got, want in zip(outs, _reference(c, args)):
+        if tol == "exact":
+            assert torch.equal(got, want)
+            continue
+        got, want = got.double(), want.double()
+        assert torch.isfinite(got).all() and float((got - want).norm()) <= tol["rel"] * float(want.norm()) + 1e-30
