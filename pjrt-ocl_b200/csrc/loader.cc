@@ -1319,7 +1319,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         }
         f->vec = vec ? 1u : 0u;
         MatchPipe(fs, static_cast<uint32_t>(x[2]), f->n_elems == static_cast<uint64_t>(f->rows) * f->cols, f->rows == 1, &f->pipe);
-        f->flat = f->vec && f->cols == 4096u ? FlatOps(fs, static_cast<uint32_t>(x[2])) : 0u;
+        f->flat = f->vec && f->cols % 4u == 0u && f->cols <= 4096u ? FlatOps(fs, static_cast<uint32_t>(x[2])) : 0u;
         if (f->total) out->needs_scratch = true;
         d.desc = static_cast<uint32_t>(out->desc.size());
         if (d.desc % 2) { out->desc.push_back(0); ++d.desc; }              // 16-byte copies

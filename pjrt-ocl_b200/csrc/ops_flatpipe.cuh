@@ -1,16 +1,15 @@
 // Flat elementwise chains of 4-byte elements with one to three binary ops, X = load; X = X op load, ...; store, as
 // straight-line code (kTopFuseRows with DFuse::flat set): what config 2's integer chain is. A thread owns two groups of 4
-// consecutive elements of a 4096-element piece; all operands of the next piece are under way as asynchronous copies
+// consecutive elements of a piece (up to 4096 elements; fewer where the whole list would not reach every lane); all operands of the next piece are under way as asynchronous copies
 // into the thread's own staging words while the current one is worked on (64 KB per SM in flight with four operands).
-// Bound: HBM. i32 max((a + b) ^ c, d), 8192 x 4096: 141 us as an interpreted chain, 115 us so (5.8 TB/s).
+// Bound: HBM. i32 max((a + b) ^ c, d), 8192 x 4096: 141 us as an interpreted chain, 115 us so (5.8 TB/s);
+// 1135 x 128 14.1 -> 10.0 us (one piece a lane).
 #ifndef B2VM_OPS_FLATPIPE_CUH_
 #define B2VM_OPS_FLATPIPE_CUH_
 
 #include "ops_fuse.cuh"
 
 namespace b2 {
-
-constexpr uint32_t kFlatPiece = 4096;           // 512 threads x 2 groups x 4 elements
 
 __device__ __forceinline__ void flat_op(uint32_t code, uint32_t (&x)[8], const uint32_t (&y)[8]) {
 #define B2_FLAT_I(C, EXPR) case C: _Pragma("unroll") for (int i = 0; i < 8; ++i) { const uint32_t a = x[i], b = y[i]; x[i] = (EXPR); } break;
@@ -52,15 +51,16 @@ static __device__ __noinline__ void flat_run(const Lane &L, const DFuse &f, uint
   uint8_t *dst = resolve(P, st[1 + 2 * NB].ptr);
   const uint32_t sb = smem_addr(L.smem + kFuseData) + L.tid * 16u;
   constexpr uint32_t kGroup = 512u * 16u, kBuf = (NB + 1) * 2u * kGroup;
-  const uint32_t n = f.n_elems;
+  const uint32_t piece_n = f.cols;         // <= 4096: 512 threads x 2 groups x 4 elements
+  const uint32_t n0 = L.tid * 4u < piece_n ? f.n_elems : 0u, n1 = L.tid * 4u + 2048u < piece_n ? f.n_elems : 0u;      // where this thread's groups end
   auto start = [&](uint32_t piece, uint32_t buf) {
-    const uint32_t e0 = piece * kFlatPiece + L.tid * 4u;
+    const uint32_t e0 = piece * piece_n + L.tid * 4u;
 #pragma unroll
     for (int k = 0; k <= NB; ++k)
 #pragma unroll
       for (uint32_t g = 0; g < 2u; ++g) {
         const uint32_t e = e0 + g * 2048u;
-        if (e < n) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sb + buf * kBuf + (k * 2u + g) * kGroup), "l"(src[k] + static_cast<size_t>(e) * 4u) : "memory");
+        if (e < (g ? n1 : n0)) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sb + buf * kBuf + (k * 2u + g) * kGroup), "l"(src[k] + static_cast<size_t>(e) * 4u) : "memory");
       }
     cp_async_commit();
   };
@@ -78,9 +78,9 @@ static __device__ __noinline__ void flat_run(const Lane &L, const DFuse &f, uint
     take(x, 0);
 #pragma unroll
     for (int k = 0; k < NB; ++k) { take(y, k + 1); flat_op(code[k], x, y); }
-    const uint32_t e = piece * kFlatPiece + L.tid * 4u;
-    if (e < n) stg_v4(dst + static_cast<size_t>(e) * 4u, make_uint4(x[0], x[1], x[2], x[3]));
-    if (e + 2048u < n) stg_v4(dst + static_cast<size_t>(e + 2048u) * 4u, make_uint4(x[4], x[5], x[6], x[7]));
+    const uint32_t e = piece * piece_n + L.tid * 4u;
+    if (e < n0) stg_v4(dst + static_cast<size_t>(e) * 4u, make_uint4(x[0], x[1], x[2], x[3]));
+    if (e + 2048u < n1) stg_v4(dst + static_cast<size_t>(e + 2048u) * 4u, make_uint4(x[4], x[5], x[6], x[7]));
     buf ^= 1u;
   }
   cp_async_wait_all();

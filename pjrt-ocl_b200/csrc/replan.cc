@@ -1288,8 +1288,8 @@ bool Planner::FuseFlat(int seed) {
   std::vector<uint32_t> writes;
   if (!c.Close(&writes, true) || writes.empty()) return false;
   if (R == 1) {
-    // pieces of one "row": long enough for wide accesses, short enough that every lane has several
-    C = n >= static_cast<uint64_t>(L_) * 4096 ? 4096 : n >= 4ull * L_ * 1024 ? 1024 : 256;
+    // pieces of one "row": one for every lane, as long as that takes, up to what its threads hold
+    for (C = 256; C < 4096 && C * L_ < n;) C *= 2;
     R = (n + C - 1) / C;
   }
   return AddPlanned(RowsNode(c, start, writes, R, C, n), c.members) >= 0;
