@@ -39,7 +39,6 @@ enum TileOp : uint32_t {
   kTopFuseRows = 33,   // a row-local pipeline: loads, row norms, elementwise steps, row and full reductions, stores
   kTopPairs = 34,      // all-pairs sums w_ij (x_j - x_i), w_ij = m_j (|x_j - x_i|^2 s + t)^-1.5, and the short elementwise tail on them
   kTopGemm = 35,       // one or several tensor-core products with their store epilogues
-  kTopFlashPlan = 36,  // attention with the head merge in its store
   kTopSgemm = 37,      // products of f32 operands
   kTopSkinny = 38,     // products with few rows (a decode step)
   kTopPlanLast = 63
@@ -62,7 +61,6 @@ enum Family : uint32_t {
   kFamFuse = 1u << 9,    // FuseRows
   kFamPairs = 1u << 10,  // Pairs
   kFamGemm = 1u << 11,
-  kFamFlashPlan = 1u << 12,
   kFamSgemm = 1u << 13,
   kFamSkinny = 1u << 14,
   kFamWire = 0x1FFu      // every family a wire program can name
@@ -79,7 +77,6 @@ B2_HOST_DEVICE inline uint32_t family_of(uint32_t tile_op) {
     case kTopFuseRows: return kFamFuse;
     case kTopPairs: return kFamPairs;
     case kTopGemm: return kFamGemm;
-    case kTopFlashPlan: return kFamFlashPlan;
     case kTopSgemm: return kFamSgemm;
     case kTopSkinny: return kFamSkinny;
     default: return kFamIndex;
