@@ -1319,6 +1319,9 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         }
         f->vec = vec ? 1u : 0u;
         MatchPipe(fs, static_cast<uint32_t>(x[2]), f->n_elems == static_cast<uint64_t>(f->rows) * f->cols, f->rows == 1, &f->pipe);
+        // two buffers of staged rows have to fit (more rows on a lane than it has threads: the most groups a row can take)
+        if (f->pipe.flags && 2u * pipe_shape(f->pipe.flags, static_cast<uint32_t>(DtypeSize(f->pipe.dt)), vec, f->cols, 512u, 512u).buf_bytes > kPlanStageBytes)
+          std::memset(&f->pipe, 0, sizeof(f->pipe));
         f->flat = f->vec && f->cols % 4u == 0u && f->cols <= 4096u ? FlatOps(fs, static_cast<uint32_t>(x[2])) : 0u;
         if (f->total) out->needs_scratch = true;
         d.desc = static_cast<uint32_t>(out->desc.size());

@@ -28,6 +28,7 @@ constexpr uint32_t kFuseSteps = kSmemSys;                                   // r
 constexpr uint32_t kFuseSlots = kFuseSteps + kFuMaxSteps * 32u;             // group reduction slots: 8 groups x 64 floats (warps alone need none)
 constexpr uint32_t kFuseData = kFuseSlots + 8u * 64u * 4u;                  // staged vectors and rows
 static_assert(kFuseData % 128u == 0u, "staging is 128-byte aligned");
+static_assert(kFuseData + 128u <= kLaneSmemBytes - kPlanStageBytes, "what the loader counts on (plan_format.h)");
 
 struct FuStep { uint32_t code, dt; float s, t; uint8_t *ptr; uint32_t reg, slot; };
 static_assert(sizeof(FuStep) == 32, "same size as on the wire");

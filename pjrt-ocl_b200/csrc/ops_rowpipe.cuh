@@ -303,13 +303,9 @@ static __device__ __noinline__ void row_pipe_tiles(const Lane &L, const DTask &t
     else rms_rows<kF16>(L, p, cols, tile_lo, hi);
     return;
   }
-  // Threads per row: up to 8 groups of 4 elements each (only X lives in registers), more threads when rows are few.
-  uint32_t T = 32u;
-  while (T < 512u && (cols > T * 32u || (hi - tile_lo) * T * 2u <= L.nthr)) T *= 2u;
-  const uint32_t per = (cols + 4u * T - 1u) / (4u * T);
-  const uint32_t G = per <= 1u ? 1u : per <= 2u ? 2u : per <= 4u ? 4u : 8u;
+  const PipeShape sh = pipe_shape(p.flags, esz, f.vec != 0u, cols, hi - tile_lo, L.nthr);
+  const uint32_t T = sh.T, G = sh.G, buf_bytes = sh.buf_bytes, stage_bytes = 2u * buf_bytes;      // (two buffers fit: the loader saw to it)
   const uint32_t vbytes = (cols * esz + 15u) & ~15u;
-  const uint32_t buf_bytes = f.vec ? ((p.flags & kRpRes) ? 2u : 1u) * G * L.nthr * 4u * esz : 0u, stage_bytes = 2u * buf_bytes;
   const uint32_t nvec = ((p.flags & kRpMul) ? 1u : 0u) + ((p.flags & kRpAdd) ? 1u : 0u);
   const bool keep = hi - tile_lo > 1u && kFuseData + nvec * vbytes + stage_bytes <= L.smem_bytes;     // column vectors in shared memory
   const uint8_t *mul = p.mul ? resolve(P, p.mul) : nullptr, *add = p.add ? resolve(P, p.add) : nullptr;

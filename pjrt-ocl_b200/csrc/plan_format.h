@@ -46,6 +46,24 @@ enum PipeFlags : uint32_t {
   kRpOn = 1u, kRpRes = 2u, kRpLn = 4u, kRpRms = 8u, kRpMul = 16u, kRpAdd = 32u, kRpGelu = 64u, kRpSoftmax = 128u, kRpCarry = 256u,
   kRpQ = 512u                      // round to the storage type after every stage (else only the result)
 };
+// Dynamic shared memory of a lane on every device this is built for, and what of it a planned op may stage data in
+// (ops_fuse.cuh checks what the interpreter and the step lists take in front).
+constexpr uint32_t kLaneSmemBytes = 226u * 1024u, kPlanStageBytes = kLaneSmemBytes - 12u * 1024u;
+// How a row pipeline lies over the threads of a lane with `rows` rows: T threads per row, G groups of 4 elements per thread
+// (only X lives in registers: up to 8), more threads when rows are few. f32 rows with a residual are staged twice: 8 groups
+// of those would be two buffers of 128 KB, so they take 4, and past 8192 columns (512 threads x 16) no row pipeline at all.
+struct PipeShape { uint32_t T, G, buf_bytes; };      // buf_bytes: one row of every group, staged
+B2_HOST_DEVICE inline PipeShape pipe_shape(uint32_t flags, uint32_t esz, bool vec, uint32_t cols, uint32_t rows, uint32_t nthr) {
+  const bool two = (flags & kRpRes) != 0u;
+  const uint32_t most = two && esz == 4u ? 16u : 32u;
+  PipeShape s;
+  s.T = 32u;
+  while (s.T < 512u && (cols > s.T * most || rows * s.T * 2u <= nthr)) s.T *= 2u;
+  const uint32_t per = (cols + 4u * s.T - 1u) / (4u * s.T);
+  s.G = per <= 1u ? 1u : per <= 2u ? 2u : per <= 4u ? 4u : 8u;
+  s.buf_bytes = vec ? (two ? 2u : 1u) * s.G * nthr * 4u * esz : 0u;
+  return s;
+}
 struct DPipe {
   uint32_t flags, dt;
   float eps, s, t;

@@ -3,6 +3,8 @@ from __future__ import annotations
 
 import pytest
 
+import plan_programs as progs
+
 torch = pytest.importorskip("torch")
 
 pytestmark = pytest.mark.gpu
@@ -107,3 +109,47 @@ def test_planned_program(c):
             continue
         got, want = got.double(), want.double()
         assert torch.isfinite(got).all() and float((got - want).norm()) <= tol["rel"] * float(want.norm()) + 1e-30
+
+
+def _load(asm):
+    import perf.cases as cases
+    s = cases._runtime()
+    return s, s["vm"].LoadedProgram.Load(s["rt"], s["vm"].VmProgram.Parse(asm.blob()))
+
+
+def _execute(asm, args, runs=2):
+    """The results of the program on these arguments (the last of `runs` runs: a later one finds what the first left behind)."""
+    import perf.cases as cases
+    s, lp = _load(asm)
+    outs = [torch.empty(asm.dims[b], dtype=cases._TORCH[asm.bufs[b][1]], device="cuda") for b in asm.outputs]
+    torch.cuda.synchronize()
+    for _ in range(runs):
+        lp.ExecuteDeviceAsync([a.data_ptr() for a in args], [o.data_ptr() for o in outs], s["stream"].cuda_stream)
+    assert lp.Status()["code"] == 0
+    return lp, outs
+
+
+def _normal(shape, dtype, seed, scale=1.0, shift=0.0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(shape, generator=gen, device="cuda") * scale + shift).to(dtype)
+
+
+@pytest.mark.parametrize("rows, cols, dtype", [
+    (4096, 1024, "f32"), (4096, 4096, "f32"), (150, 516, "f32"), (2000, 8192, "f32"), (700, 8196, "f32"), (4096, 4096, "bf16"), (700, 16384, "bf16")])
+def test_residual_and_layer_norm(rows, cols, dtype):
+    """Two staged operands per row: at the widths where the thread groups change, past the widest that is staged, and
+    with enough rows on a lane that every buffer is used. Bound: a sum of squares is chains of at most 64 terms and a
+    tree of 10, 74 x 2^-24 relative, half of that through the root, and the element's own few roundings (16-bit: half a
+    step of 2^-8 per stored value, three of them, and the first changes what is normed)."""
+    dt = getattr(torch, {"f32": "float32", "bf16": "bfloat16"}[dtype])
+    x, y = _normal((rows, cols), dt, 1), _normal((rows, cols), dt, 2)
+    g, b = _normal((cols,), dt, 3, 0.1, 1.0), _normal((cols,), dt, 4, 0.1)
+    lp, (out,) = _execute(progs.residual_norm(rows, cols, dtype), [x, y, g, b])
+    assert lp.stat("replanned") == 1
+    s = (x + y).double()
+    n = (s - s.mean(1, keepdim=True)) / torch.sqrt(s.var(1, unbiased=False, keepdim=True) + 1e-5)
+    if dtype != "f32":
+        n = n.to(dt).double()
+    want = n * g.double() + b.double()
+    tol = 4e-6 if dtype == "f32" else 2.0 ** -7
+    assert bool(((out.double() - want).abs() <= tol * (1.0 + n.abs())).all())

@@ -1,0 +1,40 @@
+"""What the re-planner makes of a program, on the host: the planner and the table builder alone, without a device."""
+from __future__ import annotations
+
+import json
+import os
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+import plan_programs as progs
+
+CSRC = os.path.join(ROOT, "pjrt-ocl_b200", "csrc")
+FUSE_ROWS = 33
+RES, LN, MUL, ADD = 2, 4, 16, 32           # row pipeline stages (plan_format.h)
+
+
+@pytest.fixture(scope="session")
+def plan(tmp_path_factory):
+    """blob -> the plan's facts."""
+    d = tmp_path_factory.mktemp("plan")
+    exe = str(d / "plan_probe")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I" + CSRC, os.path.join(ROOT, "tests", "adapter", "plan_probe.cc"),
+                    *(os.path.join(CSRC, f) for f in ("vmprog.cc", "loader.cc", "replan.cc")), "-o", exe], check=True)
+
+    def run(blob, lanes=148):
+        (d / "blob").write_bytes(blob)
+        r = subprocess.run([exe, str(d / "blob"), str(lanes)], capture_output=True, text=True)
+        assert r.returncode == 0, r.stderr
+        return json.loads(r.stdout)
+    return run
+
+
+@pytest.mark.parametrize("rows, cols", [(149, 516), (8192, 1024), (4096, 4096), (16384, 768), (2000, 8192), (700, 8196), (300, 16384), (40, 16384)])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_staged_rows_of_a_pipeline_fit_the_shared_memory(plan, rows, cols, dtype):
+    (t,) = [t for t in plan(progs.residual_norm(rows, cols, dtype).blob())["tasks"] if t["op"] == FUSE_ROWS]
+    assert t["stage"] <= t["room"]
+    # f32 rows past 512 threads x 16 elements leave the row pipelines; the others are still on them
+    assert (t["pipe"] & (RES | LN | MUL | ADD)) == (0 if dtype == "f32" and cols > 8192 else RES | LN | MUL | ADD)
