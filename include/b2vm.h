@@ -166,6 +166,9 @@ uint64_t b2_loaded_launch_count(const b2_loaded *lp);
 uint64_t b2_loaded_stat(const b2_loaded *lp, int which);
 /* Per-wait budget of device-side bounded waits, in nanoseconds (default 2e9). */
 void b2_loaded_set_wait_budget_ns(b2_loaded *lp, uint64_t ns);
+/* What the grid barrier's arrival counter (32 bits, wrapping) stands at before the next launch: results do not
+ * depend on it. For tests, which reach the wrap with it. Waits for the last launch. */
+b2_status b2_loaded_preset_arrivals(b2_loaded *lp, uint32_t count, char *err, size_t err_cap);
 /* The time, in ns since kernel entry, at which each of the first grid barriers of
  * the last execute released (every lane had arrived, seen from lane 0) (what the reference prints under
  * PJRT_OCL_PHASE_TS, runtime.cc:2196-2240). Writes at most `cap` values and

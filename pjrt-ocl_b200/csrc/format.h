@@ -207,7 +207,7 @@ enum StatusCode : uint32_t { kStOk = 0, kStBarrierTimeout = 1, kStStackOverflow 
 
 // Barrier + status block in device memory (one per loaded program).
 struct DSync {
-  uint32_t arrive;       // arrivals so far, over all launches: n_lanes per barrier, so a multiple of n_lanes at rest
+  uint32_t arrive;       // arrivals so far, over all launches, modulo 2^32
   uint32_t abort;        // set by the first lane whose wait ran out
   uint32_t pad[2];
   uint32_t status[4];    // code, lane, where, detail (first writer wins)
@@ -217,6 +217,8 @@ struct DSync {
   // kPhaseSlots grid barriers: per-phase wall time, as the reference's
   // per-barrier timestamps (vm_common.cl:258-282) give it.
   unsigned long long phase_ns[64];
+  uint32_t base;         // what `arrive` stood at when the last launch ended: where the next one counts from
+  uint32_t pad2;
 };
 constexpr uint32_t kPhaseSlots = 64;
 

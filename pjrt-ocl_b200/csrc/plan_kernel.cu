@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(kVmThreads, 1) B2_PLAN_KERNEL(const __grid_con
   const unsigned long long t_start = globaltimer_ns();
   if (P.lane_ts && L.tid == 0) P.lane_ts[L.lane * kLaneTsSlots] = t_start;
   uint32_t *next_pc = reinterpret_cast<uint32_t *>(smem + kSmemNextPc);
+  uint32_t target = L.tid == 0 ? grid_barrier_base(P) : 0u;
   {
     const uint32_t *h = reinterpret_cast<const uint32_t *>(P.heads + L.lane);
     const uint32_t w = L.tid < sizeof(DHead) / 4u ? h[L.tid] : 0u;
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(kVmThreads, 1) B2_PLAN_KERNEL(const __grid_con
   };
 
   uint32_t pc = 0, end = span.root_len, trips = 0, body = 0, ret = 0;   // trips: passes of the loop left, 0 outside it
-  uint32_t barrier_i = 0, target = 0;
+  uint32_t barrier_i = 0;
   for (;;) {
     uint32_t then = kNoPc;            // a barrier is due; the entry after it
     bool bar = false;
@@ -182,6 +183,7 @@ __global__ void __launch_bounds__(kVmThreads, 1) B2_PLAN_KERNEL(const __grid_con
   }
   if (P.lane_ts && L.tid == 0) P.lane_ts[L.lane * kLaneTsSlots + 1u] = globaltimer_ns();
   if (L.lane == 0 && L.tid == 0) {
+    grid_barrier_done(P, barrier_i, target);
     P.sync->barriers = barrier_i;
     P.sync->device_ns = globaltimer_ns() - t_start;
   }

@@ -629,6 +629,22 @@ uint64_t b2_loaded_stat(const b2_loaded *lp, int which) {
   }
 }
 void b2_loaded_set_wait_budget_ns(b2_loaded *lp, uint64_t ns) { lp->wait_budget_ns = ns; }
+b2_status b2_loaded_preset_arrivals(b2_loaded *lp, uint32_t count, char *err, size_t err_cap) {
+  if (!lp) return B2_INVALID_ARGUMENT;
+  std::lock_guard<std::mutex> g(lp->rt->mu);
+  lp->rt->Bind();
+  cudaError_t e = cudaStreamSynchronize(lp->last_stream ? lp->last_stream : lp->rt->stream);
+  if (e == cudaSuccess && lp->sync_dirty) {
+    if (lp->d_scratch) e = cudaMemset(lp->d_scratch, 0, lp->scratch_bytes);
+    if (e == cudaSuccess) e = cudaMemset(lp->d_sync, 0, sizeof(b2::DSync));
+    lp->sync_dirty = e != cudaSuccess;
+  }
+  for (uint32_t *word : {&lp->d_sync->arrive, &lp->d_sync->base})
+    if (e == cudaSuccess) e = cudaMemcpy(word, &count, sizeof(count), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) { SetErr(err, err_cap, CudaMsg("barrier preset", e)); lp->sync_dirty = true; return B2_INTERNAL; }
+  return B2_OK;
+}
 size_t b2_loaded_phase_ns(const b2_loaded *lp, uint64_t *out, size_t cap) {
   if (!lp || !out) return 0;
   std::lock_guard<std::mutex> g(lp->rt->mu);

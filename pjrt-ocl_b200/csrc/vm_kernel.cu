@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(NT, 1) B2_VM_KERNEL(const __grid_constant__ KP
   int sp = 0;
   st[0].pc = 0; st[0].end = span.root_len; st[0].widx = kRoot; st[0].phase = 0;
   uint32_t barrier_i = 0;
-  uint32_t target = 0;   // thread 0: the barrier's arrival counter once the last passed barrier was complete
+  uint32_t target = L.tid == 0 ? grid_barrier_base(P) : 0u;   // thread 0: the barrier's arrival counter once the last passed barrier was complete
   const auto nothing = [] {};
   bool pub = false;   // a tile entry ran since the last barrier (vm_main.cl:82-100)
   bool alive = true;
@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(NT, 1) B2_VM_KERNEL(const __grid_constant__ KP
   }
   if (P.lane_ts && L.tid == 0) P.lane_ts[L.lane * kLaneTsSlots + 1u] = globaltimer_ns();
   if (L.lane == 0 && L.tid == 0) {
+    grid_barrier_done(P, barrier_i, target);
     P.sync->barriers = barrier_i;
     P.sync->device_ns = globaltimer_ns() - t_start;
   }

@@ -98,6 +98,7 @@ EXPORTS = [
     "b2_loaded_status", "b2_loaded_launch_count", "b2_loaded_set_wait_budget_ns",
     "b2_loaded_phase_ns", "b2_loaded_stat", "b2_sum_f32_static", "b2_sum_f32_static_max_elems",
     "b2_loaded_lane_timing", "b2_loaded_lane_times", "b2_loaded_in_out_result",
+    "b2_loaded_preset_arrivals",
 ]
 
 
@@ -146,6 +147,7 @@ def lib():
         "b2_loaded_lane_timing": (ctypes.c_int, [vp, ctypes.c_int, cp, sz]),
         "b2_loaded_lane_times": (sz, [vp, ctypes.POINTER(ctypes.c_uint64), sz]),
         "b2_loaded_in_out_result": (ctypes.c_int, [vp, ctypes.c_uint32]),
+        "b2_loaded_preset_arrivals": (ctypes.c_int, [vp, ctypes.c_uint32, cp, sz]),
         "b2_sum_f32_static": (ctypes.c_int, [ctypes.c_int, vp, ctypes.c_uint64, vp, vp, cp, sz]),
         "b2_sum_f32_static_max_elems": (ctypes.c_uint64, []),
     }
@@ -425,6 +427,11 @@ class LoadedProgram:
 
     def set_wait_budget_ns(self, ns: int) -> None:
         lib().b2_loaded_set_wait_budget_ns(self._h, ns)
+
+    def preset_arrivals(self, count: int) -> None:
+        """Where the (wrapping) arrival counter of the grid barrier stands before the next launch."""
+        err = _errbuf()
+        _check(lib().b2_loaded_preset_arrivals(self._h, count & 0xFFFFFFFF, err, _ERRCAP), err)
 
     def close(self):
         if self._h:

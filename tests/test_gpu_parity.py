@@ -332,3 +332,31 @@ def test_bounded_barrier_wait_reports_deadline_and_context_survives(rt):
     blob, args, expected = K.kat_a_two_level()
     out = vm.LoadedProgram.Load(rt, vm.VmProgram.Parse(blob)).Execute(args)
     np.testing.assert_array_equal(out[0], expected[0])
+
+
+@pytest.mark.parametrize("name, planned", [("c5_block_f32_small", False), ("for_loop_carries", False), ("while_loop_data_dependent", False), (None, True)])
+def test_arrival_counter_wraps(rt, name, planned):
+    """The grid barrier's arrival counter is 32 bits wide and no lane count but a power of two divides 2^32: results just below
+    the wrap, across it and after it are those of a fresh program, in the wire kernels (loops among them) and in a re-planned one."""
+    vm = package()
+    if planned:
+        import perf.cases as cases
+        rng = np.random.default_rng(3)
+        c = {"kind": "nbody", "bodies": 300, "steps": 3}
+        blob = cases._BUILD["nbody"](c).blob()
+        args = [rng.uniform(-1, 1, (300, 3)).astype(np.float32), rng.normal(size=(300, 3)).astype(np.float32), rng.uniform(0.5, 1.5, 300).astype(np.float32)]
+    else:
+        g = Golden(name)
+        blob, args = g.blob, g.args
+    lp = vm.LoadedProgram.Load(rt, vm.VmProgram.Parse(blob))
+    assert lp.stat("replanned") == (1 if planned else 0)
+    want = [o.copy() for o in lp.Execute(args)]
+    n, per_run = lp.prog.n_lanes, lp.Status()["barriers"]
+    assert per_run >= 2
+    # wraps at every arrival of the first barrier, inside a later one, and exactly between two
+    for start in [*(-k for k in range(1, n + 1, max(1, n // 5))), -n, -n - 1, -n * per_run, -n * (per_run - 1) - n // 2, 0]:
+        lp.preset_arrivals(start)
+        for _ in range(3):
+            for a, b in zip(_raw(lp.Execute(args)), _raw(want)):
+                np.testing.assert_array_equal(a, b)
+            assert lp.Status()["code"] == 0
