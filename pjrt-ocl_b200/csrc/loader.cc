@@ -803,6 +803,13 @@ static bool SgOperand(const VmProgram &p, uint32_t field, uint64_t rows, uint64_
       int k = o->v.rank;
       while (k > 0 && in < n[2]) in *= o->v.dim[--k];
       if (in != n[2]) return false;
+      // the kernel adds a row's and a k's part as unsigned numbers: no reversed axis (the wire's matmul takes those)
+      int64_t most = o->v.off;
+      for (int d = 0; d < o->v.rank; ++d) {
+        if (o->v.stride[d] < 0) return false;
+        most += static_cast<int64_t>(o->v.stride[d]) * (static_cast<int64_t>(o->v.dim[d]) - 1);
+      }
+      if (o->v.off < 0 || most >= (1ll << 32)) return false;
       o->viewed = 1;
       o->k_fast = o->v.stride[o->v.rank - 1] == 1 ? !is_b : is_b;
       return true;

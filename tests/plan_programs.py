@@ -17,3 +17,17 @@ def residual_norm(rows, cols, dtype):
     out = p.chain((cases._MUL, (out, gamma), dtype, 0, by_col), (cases._ADD, (-1, beta), dtype, 0, by_col))
     p.output(out, (rows, cols))
     return p
+
+
+def viewed_product(M, K, N, dtype, dims, strides, off, elems):
+    """a @ w, where a is read from a buffer of `elems` elements through a view."""
+    p = cases._Assembler(148)
+    a, w = p.input((elems,), dtype), p.input((K, N), dtype)
+    out = p.matmul(a, w, M, N, K, dtype, va=p.view(dims, strides, off))
+    p.output(out, (M, N))
+    return p
+
+
+# a of 16 x 64 out of 1024 elements, as (2, 8, 64): blocks of eight rows, each block's rows last to first / first to last
+REVERSED = (16, 64, 24, "f32", (2, 8, 64), (512, -64, 1), 448, 1024)
+BLOCKED = (16, 64, 24, "f32", (8, 2, 64), (64, 512, 1), 0, 1024)

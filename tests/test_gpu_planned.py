@@ -153,3 +153,16 @@ def test_residual_and_layer_norm(rows, cols, dtype):
     want = n * g.double() + b.double()
     tol = 4e-6 if dtype == "f32" else 2.0 ** -7
     assert bool(((out.double() - want).abs() <= tol * (1.0 + n.abs())).all())
+
+
+@pytest.mark.parametrize("spec", [progs.REVERSED, progs.BLOCKED], ids=["reversed", "blocked"])
+def test_product_through_an_operand_view(spec):
+    """A view that is affine on neither side of a plain matrix; with a reversed axis the program keeps its own matmul."""
+    M, K, N, dtype, dims, strides, off, elems = spec
+    a, w = _normal((elems,), torch.float32, 1), _normal((K, N), torch.float32, 2)
+    lp, (out,) = _execute(progs.viewed_product(*spec), [a, w])
+    assert lp.stat("replanned") == (0 if min(strides) < 0 else 1)
+    idx = sum(torch.arange(d).view([-1 if i == k else 1 for i in range(len(dims))]) * s for k, (d, s) in enumerate(zip(dims, strides))) + off
+    ref = a.double()[idx.reshape(M, K).cuda()]
+    # K products and sums of f32: K x 2^-24 of the sum of magnitudes
+    assert bool(((out.double() - ref @ w.double()).abs() <= K * 2.0 ** -24 * (ref.abs() @ w.double().abs())).all())

@@ -11,7 +11,7 @@ from conftest import ROOT
 import plan_programs as progs
 
 CSRC = os.path.join(ROOT, "pjrt-ocl_b200", "csrc")
-FUSE_ROWS = 33
+FUSE_ROWS, GEMM, SGEMM, SKINNY, MMA = 33, 35, 37, 38, 1
 RES, LN, MUL, ADD = 2, 4, 16, 32           # row pipeline stages (plan_format.h)
 
 
@@ -38,3 +38,13 @@ def test_staged_rows_of_a_pipeline_fit_the_shared_memory(plan, rows, cols, dtype
     assert t["stage"] <= t["room"]
     # f32 rows past 512 threads x 16 elements leave the row pipelines; the others are still on them
     assert (t["pipe"] & (RES | LN | MUL | ADD)) == (0 if dtype == "f32" and cols > 8192 else RES | LN | MUL | ADD)
+
+
+def test_reversed_operand_views_stay_off_the_cuda_core_product(plan):
+    """Its offsets are unsigned: a part of a place that is negative would be read 2^32 elements too far."""
+    ok = plan(progs.viewed_product(*progs.BLOCKED).blob())
+    assert [t["viewed"] for t in ok["tasks"] if t["op"] == SGEMM] == [[1, 0]]
+    assert not [t for t in plan(progs.viewed_product(*progs.REVERSED).blob())["tasks"] if t["op"] in (SGEMM, SKINNY)]
+    # reversed along k, beside a plain second axis; and a plain reversed k
+    for dims, strides, off in (((2, 8, 64), (512, 64, -1), 63), ((2, 8, 2, 32), (512, 64, -32, 1), 32), ((16, 64), (64, -1), 63)):
+        assert not [t for t in plan(progs.viewed_product(16, 64, 24, "f32", dims, strides, off, 1024).blob())["tasks"] if t["op"] in (SGEMM, SKINNY)]
