@@ -940,12 +940,18 @@ bool Planner::GemmEpilogue(const Chain &c, uint32_t dst, std::vector<int32_t> *w
   const size_t n = st.size();
   auto at = [&](size_t k, uint32_t code) { return k < n && st[k].code == code; };
   auto plain_scale = [&](size_t k) { return at(k, kFuAffine) && st[k].t == 0.0f; };
-  if (n > 1 && half) flags |= kGeQuant0;
+  // The epilogue works on the accumulator and the last store rounds: a 16-bit product that goes on, or leaves in another type,
+  // is rounded first; any later value that the program holds in 16 bits may only be the last, and leave in that type.
+  if (half && !(n == 1 && at(0, kFuStore) && st[0].dt == Dt(dst))) flags |= kGeQuant0;
   if (at(0, kFuStore) && n > 1) { out0 = st[0].id; dt0 = st[0].dt; i = 1; }
-  bool rounded = true;                // the value in hand is as the program would have stored it
-  auto quant = [&](uint32_t dt) { if (at(i, kFuQuant)) { if (st[i].dt != dt) return false; ++i; rounded = true; } return true; };
-  uint32_t last_dt = Dt(dst);
-  if (at(i, kFuGelu)) { flags |= kGeGelu; ++i; rounded = !half; if (!quant(last_dt)) return false; if (i + 1 < n) return false; }
+  int64_t rounded = -1;               // the type that the value in hand has yet to be rounded to
+  auto quant = [&] { if (at(i, kFuQuant)) rounded = st[i++].dt; };
+  if (at(i, kFuGelu)) {
+    flags |= kGeGelu;
+    ++i;
+    quant();
+    if ((rounded >= 0 && rounded != static_cast<int64_t>(Dt(dst))) || i + 1 < n) return false;
+  }
   if (plain_scale(i) && (at(i + 1, kFuLoadY))) { flags |= kGeScale0; s0 = st[i].s; ++i; if (at(i, kFuQuant)) return false; }
   if (at(i, kFuScalarY) && at(i + 1, kFuMax)) {
     bool known = false;
@@ -959,9 +965,10 @@ bool Planner::GemmEpilogue(const Chain &c, uint32_t dst, std::vector<int32_t> *w
     if (!known) return false;
     flags |= kGeMaxS;
     i += 2;
-    if (at(i, kFuQuant)) ++i;
+    quant();
   }
   if (at(i, kFuLoadY)) {
+    if (rounded >= 0) return false;
     res = st[i].id;
     rdt = st[i].dt;
     ++i;
@@ -974,12 +981,11 @@ bool Planner::GemmEpilogue(const Chain &c, uint32_t dst, std::vector<int32_t> *w
     else return false;
     if (at(i, kFuCarrySumSq)) { flags |= kGeCarrySq; ++i; }
     if (plain_scale(i) && !(flags & kGeMaxS)) { flags |= kGeScale1; s1 = st[i].s; ++i; }
-    if (at(i, kFuQuant)) ++i;
+    quant();
   }
-  if (!(i + 1 == n && at(i, kFuStore))) return false;
+  if (!(i + 1 == n && at(i, kFuStore)) || (rounded >= 0 && rounded != static_cast<int64_t>(st[i].dt))) return false;
   out1 = st[i].id;
   dt1 = st[i].dt;
-  (void)rounded;
   *w = {static_cast<int32_t>(flags), static_cast<int32_t>(Dt(dst)), static_cast<int32_t>(rdt), FBits(s0), FBits(s1), FBits(gg),
         static_cast<int32_t>(res + 1), static_cast<int32_t>(out0 + 1), static_cast<int32_t>(dt0), static_cast<int32_t>(out1 + 1), static_cast<int32_t>(dt1)};
   return true;

@@ -31,3 +31,21 @@ def viewed_product(M, K, N, dtype, dims, strides, off, elems):
 # a of 16 x 64 out of 1024 elements, as (2, 8, 64): blocks of eight rows, each block's rows last to first / first to last
 REVERSED = (16, 64, 24, "f32", (2, 8, 64), (512, -64, 1), 448, 1024)
 BLOCKED = (16, 64, 24, "f32", (8, 2, 64), (64, 512, 1), 0, 1024)
+
+
+def widened_product(M, K, N, dtype, what):
+    """A 16-bit product whose last value is converted to f32: of the product itself, or of what follows it in 16 bits."""
+    p = cases._Assembler(148)
+    a, w, x = p.input((M, K), dtype), p.input((K, N), dtype), p.input((M, N), dtype)
+    y = p.matmul(a, w, M, N, K, dtype)
+    p.phase()
+    if what == "residual":
+        y = p.chain((cases._ADD, (x, y), dtype))
+    elif what == "gelu":
+        y = p.chain((cases._GELU, (y,), dtype))
+    elif what == "both":
+        y = p.chain((cases._ADD, (x, y), dtype), (cases._GELU, (-1,), dtype))
+    if what != "product":
+        p.phase()
+    p.output(p.chain((cases._CONVERT, (y,), "f32")), (M, N))
+    return p

@@ -166,3 +166,25 @@ def test_product_through_an_operand_view(spec):
     ref = a.double()[idx.reshape(M, K).cuda()]
     # K products and sums of f32: K x 2^-24 of the sum of magnitudes
     assert bool(((out.double() - ref @ w.double()).abs() <= K * 2.0 ** -24 * (ref.abs() @ w.double().abs())).all())
+
+
+@pytest.mark.parametrize("what", ["product", "residual", "gelu", "both"])
+@pytest.mark.parametrize("mnk", [(300, 264, 64), (16, 72, 64), (40, 33, 45)], ids=["gemm", "skinny", "sgemm"])
+def test_product_converted_after_a_16_bit_value(what, mnk):
+    """What the program holds in bf16 has bf16's values after the convert to f32. Small integers: products and sums are exact in
+    f32, so the roundings to bf16 are all there is and the bits are known (but for GELU, whose result has to be a bf16 number)."""
+    M, N, K = mnk
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    a, w, x = (torch.randint(-8, 9, s, generator=gen, device="cuda").to(torch.bfloat16) for s in ((M, K), (K, N), (M, N)))
+    lp, (out,) = _execute(progs.widened_product(M, K, N, "bf16", what), [a, w, x])
+    assert lp.stat("replanned") == 1
+    y = (a.double() @ w.double()).to(torch.bfloat16)
+    assert float(y.abs().max()) > 256                  # beyond 8 bits: it had to be rounded
+    if what in ("residual", "both"):
+        y = (x.double() + y.double()).to(torch.bfloat16)
+    assert torch.equal(out, out.to(torch.bfloat16).float())
+    if what in ("gelu", "both"):
+        want = _gelu(y.double())
+        assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())      # half a step of bf16, and gelu_tanh's own error
+    else:
+        assert torch.equal(out, y.float())

@@ -13,6 +13,7 @@ import plan_programs as progs
 CSRC = os.path.join(ROOT, "pjrt-ocl_b200", "csrc")
 FUSE_ROWS, GEMM, SGEMM, SKINNY, MMA = 33, 35, 37, 38, 1
 RES, LN, MUL, ADD = 2, 4, 16, 32           # row pipeline stages (plan_format.h)
+F32, BF16, QUANT0, EPI_GELU, EPI_RES = 0, 7, 1, 2, 16
 
 
 @pytest.fixture(scope="session")
@@ -48,3 +49,14 @@ def test_reversed_operand_views_stay_off_the_cuda_core_product(plan):
     # reversed along k, beside a plain second axis; and a plain reversed k
     for dims, strides, off in (((2, 8, 64), (512, 64, -1), 63), ((2, 8, 2, 32), (512, 64, -32, 1), 32), ((16, 64), (64, -1), 63)):
         assert not [t for t in plan(progs.viewed_product(16, 64, 24, "f32", dims, strides, off, 1024).blob())["tasks"] if t["op"] in (SGEMM, SKINNY)]
+
+
+@pytest.mark.parametrize("what, flags, dt1", [("product", QUANT0, F32), ("residual", QUANT0 | EPI_RES, BF16), ("gelu", QUANT0 | EPI_GELU, BF16),
+                                              ("both", QUANT0 | EPI_RES, BF16)])
+@pytest.mark.parametrize("mnk", [(256, 256, 64), (16, 64, 64), (40, 33, 45)])
+def test_products_keep_the_roundings_of_what_they_hand_on(plan, what, flags, dt1, mnk):
+    """A value that the program holds in 16 bits leaves a store epilogue in 16 bits, or rounded."""
+    M, N, K = mnk
+    tasks = plan(progs.widened_product(M, K, N, "bf16", what).blob())["tasks"]
+    got = [(q["epi"], q["dt1"]) for t in tasks for q in t.get("prob", [t]) if "epi" in q]
+    assert got == [(flags, dt1)]
