@@ -1624,8 +1624,8 @@ bool Planner::Run(VmProgram *q, ReplanStats *st) {
 
 bool Replan(const VmProgram &p, uint32_t device_lanes, VmProgram *q, ReplanStats *st) {
   *st = ReplanStats{};
-  // A schedule for less than half the device leaves the rest to somebody else: it keeps its lanes and its cut.
-  if (std::getenv("B2VM_NO_REPLAN") || device_lanes < 4 || p.n_lanes * 2 < device_lanes || p.lane_tab.size() != p.n_lanes) return false;
+  // A schedule for half the device or less leaves room for another beside it: it keeps its lanes and its cut.
+  if (std::getenv("B2VM_NO_REPLAN") || device_lanes < 4 || p.n_lanes * 2 <= device_lanes || p.lane_tab.size() != p.n_lanes) return false;
   Planner pl(p, device_lanes);
   return pl.Run(q, st);
 }

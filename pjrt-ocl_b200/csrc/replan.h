@@ -9,7 +9,7 @@
 // hands on in a narrower type; sums may be taken in another order.
 //
 // It leaves a program alone (returns false) when nothing in it fuses, when it uses control flow other than one counted
-// loop at the top, or when it was scheduled for a small part of the device.
+// loop at the top, or when it was scheduled for half of the device or less.
 #ifndef B2VM_REPLAN_H_
 #define B2VM_REPLAN_H_
 

@@ -477,7 +477,7 @@ b2_status b2_program_load(b2_runtime *rt, b2_program *prog, b2_loaded **out, cha
   // Re-planned for this device where that fuses anything (replan.h). The program is checked as it came first: the
   // re-planner relies on every index the tables' builder refuses to be in range.
   b2::VmProgram planned;
-  if (p.n_lanes * 2 >= static_cast<uint32_t>(rt->prop.multiProcessorCount)) {
+  if (p.n_lanes * 2 > static_cast<uint32_t>(rt->max_lanes)) {
     b2::DeviceTables check;
     if (!b2::BuildDeviceTables(p, 0, &check, &m, &unimpl)) {
       SetErr(err, err_cap, "load: " + m);

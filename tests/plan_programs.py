@@ -4,9 +4,9 @@ from __future__ import annotations
 import perf.cases as cases
 
 
-def residual_norm(rows, cols, dtype):
+def residual_norm(rows, cols, dtype, lanes=148):
     """LayerNorm(x + y) gamma + beta: the norm of a post-norm transformer layer."""
-    p = cases._Assembler(148)
+    p = cases._Assembler(lanes)
     x, y = p.input((rows, cols), dtype), p.input((rows, cols), dtype)
     gamma, beta = p.input((cols,), dtype), p.input((cols,), dtype)
     out = p.chain((cases._ADD, (x, y), dtype))

@@ -60,3 +60,8 @@ def test_products_keep_the_roundings_of_what_they_hand_on(plan, what, flags, dt1
     tasks = plan(progs.widened_product(M, K, N, "bf16", what).blob())["tasks"]
     got = [(q["epi"], q["dt1"]) for t in tasks for q in t.get("prob", [t]) if "epi" in q]
     assert got == [(flags, dt1)]
+
+
+@pytest.mark.parametrize("lanes, device, planned", [(74, 148, False), (75, 148, True), (66, 132, False), (66, 131, True), (148, 148, True)])
+def test_schedules_for_half_the_device_stay_side_by_side(plan, lanes, device, planned):
+    assert plan(progs.residual_norm(600, 256, "f32", lanes).blob(), device)["planned"] == planned
