@@ -42,6 +42,13 @@ __device__ __forceinline__ float fast_rsqrt(float a) {
   return r;
 }
 
+// The smaller of two, a NaN if either is one.
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 template <int NI, bool UNIT>
 static __device__ __noinline__ void pairs_run(const Lane &L, const DPairs &p, const float *pos, const float *mass, uint32_t lo, uint32_t hi,
                                               uint32_t groups) {
@@ -95,7 +102,8 @@ static __device__ __noinline__ void pairs_run(const Lane &L, const DPairs &p, co
 #pragma unroll
       for (int k = 0; k < NI; ++k) {
         const float dx = q.x - px[k], dy = q.y - py[k], dz = q.z - pz[k];
-        const float a = UNIT ? fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, at))) : fmaf(fmaf(dz, dz, fmaf(dy, dy, dx * dx)), as, at);
+        // (a squared distance beyond f32 weighs nothing: infinity times the root's zero would be a NaN)
+        const float a = min_nan(UNIT ? fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, at))) : fmaf(fmaf(dz, dz, fmaf(dy, dy, dx * dx)), as, at), 3.402823466e38f);
         const float r = fast_rsqrt(a), r2 = r * r;
         // a^-1.5 = r^3 (1 + 1.5 (1 - a r^2) + ...): first-order correction of the approximate root
         const float wj = (r2 * r) * fmaf(fmaf(-a, r2, 1.0f), m15, q.w);

@@ -188,3 +188,32 @@ def test_product_converted_after_a_16_bit_value(what, mnk):
         assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())      # half a step of bf16, and gelu_tanh's own error
     else:
         assert torch.equal(out, y.float())
+
+
+@pytest.mark.parametrize("bodies", [258, 400])
+def test_bodies_whose_squared_distance_overflows(bodies):
+    """Two clusters 1e20 apart: between them the squared distance is infinite in f32 and the weight 0, as pow(inf, -1.5) is;
+    inside each the accelerations are those of the cluster alone."""
+    import perf.cases as cases
+    c = {"kind": "nbody", "bodies": bodies, "steps": 1}
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    pos = torch.rand((bodies, 3), generator=gen, device="cuda") * 2 - 1
+    vel, mass = torch.zeros((bodies, 3), device="cuda"), torch.rand(bodies, generator=gen, device="cuda") + 0.5
+    half = bodies // 2
+    pos[half:, 0] = 1e20                               # (their own x distances are 0: 1e20 swallows the rest)
+    lp, (p1, v1) = _execute(cases._BUILD["nbody"](c), [pos, vel, mass])
+    assert lp.stat("pairs") == 4
+    for s in (slice(0, half), slice(half, bodies)):
+        near = pos[s].clone()
+        if s.start:
+            near[:, 0] = 0.0
+        want = _reference(c, [near, vel[s], mass[s]])
+        got = p1[s].clone()
+        if s.start:
+            got[:, 0] -= 1e20
+        for g, w in ((got, want[0]), (v1[s], want[1])):
+            assert torch.isfinite(g).all() and float((g.double() - w).norm()) <= 1e-5 * float(w.norm())
+    # a NaN is no infinite distance: it reaches everyone
+    pos[3, 1] = float("nan")
+    _, (p1, v1) = _execute(cases._BUILD["nbody"](c), [pos, vel, mass])
+    assert bool(torch.isnan(v1[:half]).any(1).all())
