@@ -331,7 +331,7 @@ static __device__ __noinline__ void flash_decode_ring(const Lane &L, const DTask
 // of 64 that the lane loads once for all of them: K as [d][key], V as [key][d], f32 in shared memory. A thread owns two
 // keys of the chunk for the scores and DJ columns for the output; q and p are read as fours along d and the keys.
 // Bound: shared-memory reads (2.5 per 4 FMAs). A warp per row with every element of K and V fetched through its view by each
-// row's warp took 606 us where this takes 25 (f32, 32 heads x 128 x 128 x 64).
+// row's warp took 606 us where this takes 60 (f32, 32 heads x 128 x 128 x 64).
 template <int DJ>
 static __device__ __noinline__ void flash_rows_tiles(const Lane &L, const DTask &t, const DFlash &df, const int32_t *x, uint32_t tile_lo, int64_t hi) {
   constexpr int HDP = DJ * 32, KC = 64, KP = KC + 1;
@@ -412,8 +412,13 @@ static __device__ __noinline__ void flash_rows_tiles(const Lane &L, const DTask 
         for (int j = 0; j < DJ; ++j) o[r][j] *= alpha;
       }
       __syncwarp();
+      // Keys that both rows see, by fours; then those that one of them may not: p is 0 there, but 0 times what an unwritten
+      // cache row holds (NaN, infinity) would not be. (A second row that is not there goes along with the first.)
+      const int n0 = static_cast<int>(min(static_cast<int64_t>(KC), c_end[0] - c0));
+      const int n1 = c_end[1] == 0 ? n0 : static_cast<int>(min(static_cast<int64_t>(KC), c_end[1] - c0));
+      const int both = max(min(n0, n1), 0) & ~3, most = max(n0, n1);
 #pragma unroll 2
-      for (int c = 0; c < KC; c += 4) {
+      for (int c = 0; c < both; c += 4) {
         const float4 pa = *reinterpret_cast<const float4 *>(ps + c), pb = *reinterpret_cast<const float4 *>(ps + KC + c);
         const float a4[4] = {pa.x, pa.y, pa.z, pa.w}, b4[4] = {pb.x, pb.y, pb.z, pb.w};
 #pragma unroll
@@ -424,6 +429,16 @@ static __device__ __noinline__ void flash_rows_tiles(const Lane &L, const DTask 
             o[0][j] = fmaf(a4[e], v, o[0][j]);
             o[1][j] = fmaf(b4[e], v, o[1][j]);
           }
+      }
+#pragma unroll 1
+      for (int c = both; c < most; ++c) {
+        const float pa = ps[c], pb = ps[KC + c];
+#pragma unroll
+        for (int j = 0; j < DJ; ++j) {
+          const float v = vs[c * HDP + l + 32 * j];
+          if (c < n0) o[0][j] = fmaf(pa, v, o[0][j]);
+          if (c < n1) o[1][j] = fmaf(pb, v, o[1][j]);
+        }
       }
       __syncwarp();
     }

@@ -49,3 +49,14 @@ def widened_product(M, K, N, dtype, what):
         p.phase()
     p.output(p.chain((cases._CONVERT, (y,), "f32")), (M, N))
     return p
+
+
+def attention_of_sums(H, T, C, hd, dtype, causal):
+    """(q + q0) K^T, softmax, V: a program with an attention task that something around it lets the re-planner take."""
+    p = cases._Assembler(148)
+    q, q0 = p.input((H, T, hd), dtype), p.input((H, T, hd), dtype)
+    k, v = p.input((H, hd, C), dtype), p.input((H, C, hd), dtype)
+    s = p.chain((cases._ADD, (q, q0), dtype))
+    p.phase()
+    p.output(p.attention(s, k, v, H, T, C, hd, causal), (H, T, hd))
+    return p

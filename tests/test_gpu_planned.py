@@ -217,3 +217,22 @@ def test_bodies_whose_squared_distance_overflows(bodies):
     pos[3, 1] = float("nan")
     _, (p1, v1) = _execute(cases._BUILD["nbody"](c), [pos, vel, mass])
     assert bool(torch.isnan(v1[:half]).any(1).all())
+
+
+@pytest.mark.parametrize("H, T, C, hd", [(40, 64, 64, 64), (12, 129, 129, 64), (41, 33, 100, 64), (20, 70, 131, 40), (22, 64, 67, 128), (6, 300, 301, 200), (3, 33, 70, 64)])
+def test_masked_values_do_not_reach_the_rows_that_mask_them(H, T, C, hd):
+    """Causal attention on the CUDA cores: a NaN, or an infinity, in the V row of key c shows in the query rows that see c and
+    in no other, wherever c lies in its chunk of 64. f32 in another order than torch's: C x 2^-24, and the exponentials."""
+    q, q0, k, v = (_normal(s, torch.float32, i) for i, s in enumerate(((H, T, hd), (H, T, hd), (H, hd, C), (H, C, hd))))
+    seen = torch.arange(C, device="cuda")[None, :] <= torch.arange(T, device="cuda")[:, None] + C - T
+    s = ((q + q0).double() @ k.double() / hd ** 0.5).masked_fill(~seen, float("-inf"))
+    want = torch.softmax(s, -1) @ v.double()
+    for c in sorted({C - T, C - T + 1, C - T + 2, C - 1, C - 2, min(C - 1, 63), min(C - 1, 64)}):
+        bad = v.clone()
+        bad[:, c] = float("nan")
+        bad[0, c] = float("inf")
+        lp, (out,) = _execute(progs.attention_of_sums(H, T, C, hd, "f32", True), [q, q0, k, bad])
+        assert lp.stat("replanned") == 1
+        clean = ~seen[:, c]
+        assert bool((~torch.isfinite(out[:, ~clean])).all())
+        assert bool(((out[:, clean].double() - want[:, clean]).abs() <= 1e-5 * (1.0 + want[:, clean].abs())).all())
