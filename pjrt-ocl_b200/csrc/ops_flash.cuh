@@ -215,6 +215,7 @@ static __device__ __noinline__ void flash_decode_ring(const Lane &L, const DTask
     bulk_g2s(ring + b * 2u * stage_b + stage_b, V + (g * df.dv_g + k0 * HD) * 2, bytes, &full[2u * b + 1u]);
     ++p_stage; ++p_seq;
   };
+  fence_proxy_async_smem();   // what the entry before wrote here by ordinary stores, before asynchronous copies overwrite it
   __syncthreads();
   if (L.tid == 0) {
     for (uint32_t i = 0; i < kDepth; ++i) { mbar_init(&full[2u * i], 1); mbar_init(&full[2u * i + 1u], 1); mbar_init(&empty[i], nw); }

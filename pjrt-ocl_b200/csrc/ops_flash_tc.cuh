@@ -98,6 +98,7 @@ static __device__ __noinline__ bool flash_tc_tiles(const Lane &L, const DTask &t
     __syncwarp();
     tmem_alloc(&S->tmem_base, kFaCols);
   }
+  fence_proxy_async_smem();   // what the entry before wrote here by ordinary stores, before asynchronous copies overwrite it
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();

@@ -211,6 +211,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
     fence_mbar_init();
   }
   if (w == 2u) tmem_alloc(&S->tmem_base, 512u);
+  fence_proxy_async_smem();   // what the entry before wrote here by ordinary stores, before asynchronous copies overwrite it
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();

@@ -191,6 +191,7 @@ static __device__ __noinline__ bool mma_tc_tiles(const Lane &L, const DTask &t, 
     __syncwarp();
     tmem_alloc(&S->tmem_base, tcols);
   }
+  fence_proxy_async_smem();   // what the entry before wrote here by ordinary stores, before asynchronous copies overwrite it
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();

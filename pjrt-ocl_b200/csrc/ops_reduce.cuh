@@ -300,6 +300,7 @@ __device__ __forceinline__ bool red_part_stream(const Lane &L, const DTask &t, u
     const uint64_t left = total - static_cast<uint64_t>(c) * kStreamChunk;
     return left < kStreamChunk ? static_cast<uint32_t>(left) : kStreamChunk;
   };
+  fence_proxy_async_smem();   // what the entry before wrote here by ordinary stores, before asynchronous copies overwrite it
   __syncthreads();
   if (L.tid == 0) {
     for (uint32_t i = 0; i < kStreamBufs; ++i) mbar_init(&bar[i], 1);
@@ -377,6 +378,7 @@ __device__ __forceinline__ uint32_t red_words_lane(const Lane &L, const uint8_t 
       mbar_arrive_expect_tx(&full[bb], bytes_of(c));
       bulk_g2s(bufs + bb * kStreamChunk, src + static_cast<size_t>(c) * kStreamChunk, bytes_of(c), &full[bb]);
     };
+    fence_proxy_async_smem();   // what the entry before wrote here by ordinary stores, before asynchronous copies overwrite it
     __syncthreads();
     if (L.tid == 0) {
       for (uint32_t i = 0; i < kStreamBufs; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], nwarps); }

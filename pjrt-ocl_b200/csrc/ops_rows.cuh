@@ -82,6 +82,7 @@ __device__ __forceinline__ void rows_staged(const Lane &L, const DTask &t, uint3
                             (L.smem_bytes - kSmemSys - kRowHdr) / (ngroups * buf_stride));
   uint8_t *bufs = L.smem + kSmemSys + kRowHdr + static_cast<size_t>(gi) * nbuf * buf_stride;
 
+  fence_proxy_async_smem();   // what the entry before wrote here by ordinary stores, before asynchronous copies overwrite it
   __syncthreads();
   if (L.tid == 0) {
     for (uint32_t i = 0; i < ngroups * kRowMaxBufs; ++i) mbar_init(&bars[i], 1);

@@ -1,8 +1,10 @@
 """What the re-planner makes of a program, on the host: the planner and the table builder alone, without a device."""
 from __future__ import annotations
 
+import glob
 import json
 import os
+import re
 import subprocess
 
 import pytest
@@ -65,3 +67,20 @@ def test_products_keep_the_roundings_of_what_they_hand_on(plan, what, flags, dt1
 @pytest.mark.parametrize("lanes, device, planned", [(74, 148, False), (75, 148, True), (66, 132, False), (66, 131, True), (148, 148, True)])
 def test_schedules_for_half_the_device_stay_side_by_side(plan, lanes, device, planned):
     assert plan(progs.residual_norm(600, 256, "f32", lanes).blob(), device)["planned"] == planned
+
+
+def test_asynchronous_copies_follow_a_fence_over_the_workspace():
+    """Every function that sets up barriers for copies into shared memory first fences the asynchronous proxy against what the
+    lane's entry before wrote there by ordinary stores (no run shows a missing fence for certain: the source does)."""
+    n = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "ops_*.cuh"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"fence_mbar_init\(\)", text):
+            n += 1
+            # a fence by all threads, then the barrier that the thread which issues the copies passes
+            before, after = text[:m.start()], text[m.start():]
+            fenced = before.rfind("fence_proxy_async_smem()")
+            first = after.index("__syncthreads()")
+            near = fenced >= 0 and "__global__" not in before[fenced:] and "static __device__" not in before[fenced:] and "__syncthreads()" in before[fenced:]
+            assert near or "fence_proxy_async_smem()" in after[:first], (os.path.basename(path), before.count("\n"))
+    assert n >= 6
