@@ -164,7 +164,8 @@ uint32_t FlatOps(const DFuStep *st, uint32_t n) {
 }
 
 // Is a fused step list one of the row pipelines of ops_rowpipe.cuh? Every tensor in one storage type; between the stages
-// of 16-bit rows either every value is rounded or none.
+// of 16-bit rows either every value is rounded or only the last. A norm is not needed: x gamma + beta, GELU over 8192 x 4096 f32
+// takes 133 us in the step interpreter, 70 as a pipeline (77 as the program's own tile ops).
 void MatchPipe(const DFuStep *st, uint32_t n, bool whole_rows, bool one_row, DPipe *out) {
   std::memset(out, 0, sizeof(*out));
   uint32_t i = 0;
@@ -176,10 +177,12 @@ void MatchPipe(const DFuStep *st, uint32_t n, bool whole_rows, bool one_row, DPi
   p.x = st[0].ptr;
   const bool half = p.dt != kF32;
   int rounded = 0, plain = 0;              // stages followed / not followed by a rounding
+  bool last = true;                        // ... the last stage is
   i = 1;
   auto quant = [&] {
     if (!half) return;
-    if (i < n && st[i].code == kFuQuant && st[i].dt == p.dt) { ++i; ++rounded; } else { ++plain; }
+    last = i < n && st[i].code == kFuQuant && st[i].dt == p.dt;
+    if (last) { ++i; ++rounded; } else { ++plain; }
   };
   auto at = [&](uint32_t k, uint32_t code) { return k < n && st[k].code == code; };
   if (at(i, kFuLoadY) && st[i].dt == p.dt && at(i + 1, kFuAdd)) {
@@ -208,11 +211,11 @@ void MatchPipe(const DFuStep *st, uint32_t n, bool whole_rows, bool one_row, DPi
   if (at(i, kFuCarrySum)) { p.flags |= kRpCarry; ++i; }
   if (at(i, kFuStore) && st[i].dt == p.dt) p.out = st[i++].ptr;
   if (at(i, kFuCarrySum) && !(p.flags & kRpCarry)) { p.flags |= kRpCarry; ++i; }
-  if (i != n || (p.flags & (kRpLn | kRpRms | kRpSoftmax)) == 0u) return;
+  if (i != n || p.flags == kRpOn) return;
   if (half) {
     // rounded after every stage, or (the RMS norm on f32 intermediates) only at the end
     if (plain == 0) p.flags |= kRpQ;
-    else if (!(rounded == 1 && plain >= 1 && (p.flags & (kRpLn | kRpSoftmax)) == 0u)) return;
+    else if (!(rounded == 1 && last && (p.flags & (kRpLn | kRpSoftmax)) == 0u)) return;
   }
   *out = p;
 }

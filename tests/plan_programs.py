@@ -60,3 +60,29 @@ def attention_of_sums(H, T, C, hd, dtype, causal):
     p.phase()
     p.output(p.attention(s, k, v, H, T, C, hd, causal), (H, T, hd))
     return p
+
+
+def stages(rows, cols, dtype, what, total=False):
+    """x (+ y) (x gamma) (+ beta) (GELU), each as a task that rounds to `dtype`, and the sum of the result."""
+    p = cases._Assembler(148)
+    x = p.input((rows, cols), dtype)
+    ops, by_col, cur = [], p.view((rows, cols), (0, 1)), x
+    for w in what:
+        if w == "res":
+            ops.append((cases._ADD, (cur, p.input((rows, cols), dtype)), dtype))
+        elif w == "gelu":
+            ops.append((cases._GELU, (cur,), dtype))
+        else:
+            ops.append(({"mul": cases._MUL, "add": cases._ADD}[w], (cur, p.input((cols,), dtype)), dtype, 0, by_col))
+        cur = -1
+    out = x
+    if ops:
+        out = p.chain(*ops)
+        p.output(out, (rows, cols))
+        p.phase()
+    if total:
+        if dtype != "f32":
+            out = p.chain((cases._CONVERT, (out,), "f32"))
+            p.phase()
+        p.output(p.full_sum(out), ())
+    return p

@@ -236,3 +236,33 @@ def test_masked_values_do_not_reach_the_rows_that_mask_them(H, T, C, hd):
         clean = ~seen[:, c]
         assert bool((~torch.isfinite(out[:, ~clean])).all())
         assert bool(((out[:, clean].double() - want[:, clean]).abs() <= 1e-5 * (1.0 + want[:, clean].abs())).all())
+
+
+@pytest.mark.parametrize("what, total", [
+    (("mul", "add", "gelu"), False), (("mul", "add", "gelu"), True), (("add",), False), (("mul",), True), (("gelu",), False), (("mul", "gelu"), False), (("res", "gelu"), True),
+    (("res", "mul", "add"), False), (("res",), True), ((), True)], ids=lambda v: "-".join(v) if isinstance(v, tuple) else "sum" if v else "")
+@pytest.mark.parametrize("rows, cols, dtype", [(1, 640, "f32"), (700, 1024, "f32"), (333, 130, "f32"), (150, 4096, "bf16"), (64, 1023, "f16"), (2048, 512, "bf16"), (77, 8192, "f32")])
+def test_pipelines_without_a_norm(what, total, rows, cols, dtype):
+    """Every stage on its own and together, in rows and in pieces of a flat list: a value differs from the same stages rounded one
+    by one in float64 by a step of its type at most (GELU's approximation may turn a rounding), f32 by a few 2^-23; the sum
+    by the f32 additions of a lane's chain and the tree over them."""
+    dt = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dtype]
+    x = _normal((rows, cols), dt, 1)
+    args, cur = [x], x.double()
+    for i, w in enumerate(what):
+        if w == "gelu":
+            cur = _gelu(cur)
+        else:
+            args.append(_normal((rows, cols) if w == "res" else (cols,), dt, 2 + i, *((0.1, 1.0) if w == "mul" else (1.0,))))
+            cur = cur * args[-1].double() if w == "mul" else cur + args[-1].double()
+        cur = cur.to(dt).double()
+    lp, outs = _execute(progs.stages(rows, cols, dtype, what, total), args)
+    step = {"f32": 2.0 ** -21, "bf16": 2.0 ** -7, "f16": 2.0 ** -10}[dtype]
+    if what:
+        got = outs[0].double()
+        assert bool(((got - cur).abs() <= step * cur.abs() + (2e-6 if "gelu" in what else 2.0 ** -24)).all())
+    if total:
+        # of what was stored (bit for bit), in f32: chains of at most rows x cols / (148 x 512) + 8, then trees of 9 and 8
+        kept = (outs[0] if what else x).double()
+        bound = (rows * cols / (148 * 512) + 64) * 2.0 ** -24 * float(kept.abs().sum())
+        assert abs(float(outs[-1]) - float(kept.sum())) <= bound

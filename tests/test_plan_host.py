@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import glob
+import gzip
 import json
 import os
 import re
@@ -14,7 +15,7 @@ import plan_programs as progs
 
 CSRC = os.path.join(ROOT, "pjrt-ocl_b200", "csrc")
 FUSE_ROWS, GEMM, SGEMM, SKINNY, MMA = 33, 35, 37, 38, 1
-RES, LN, MUL, ADD = 2, 4, 16, 32           # row pipeline stages (plan_format.h)
+ON, RES, LN, MUL, ADD, GELU, CARRY = 1, 2, 4, 16, 32, 64, 256           # row pipeline stages (plan_format.h)
 F32, BF16, QUANT0, EPI_GELU, EPI_RES = 0, 7, 1, 2, 16
 
 
@@ -84,3 +85,14 @@ def test_asynchronous_copies_follow_a_fence_over_the_workspace():
             near = fenced >= 0 and "__global__" not in before[fenced:] and "static __device__" not in before[fenced:] and "__syncthreads()" in before[fenced:]
             assert near or "fence_proxy_async_smem()" in after[:first], (os.path.basename(path), before.count("\n"))
     assert n >= 6
+
+
+def committed(name):
+    return gzip.open(os.path.join(ROOT, "pjrt-ocl_b200", "programs", name + ".vmprog.gz")).read()
+
+
+def test_chains_without_a_norm_are_row_pipelines(plan):
+    (t,) = plan(committed("c2_stage_affine_gelu_f32"))["tasks"]
+    assert t["pipe"] == ON | MUL | ADD | GELU
+    (t,) = plan(committed("c2_stage_sum_f32"))["tasks"]
+    assert t["pipe"] == ON | CARRY
