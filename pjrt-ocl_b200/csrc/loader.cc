@@ -1314,7 +1314,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         DFuStep *fs = reinterpret_cast<DFuStep *>(f + 1);
         bool vec = x[4] != 0;
         for (int32_t k = 0; k < x[2]; ++k) {
-          const int32_t *w = x + 7 + 6 * k;
+          const int32_t *w = x + kFuseWords + 6 * k;
           DFuStep &st = fs[k];
           st.code = static_cast<uint32_t>(w[0]);
           st.dt = static_cast<uint32_t>(w[1]);
@@ -1333,6 +1333,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         if (f->pipe.flags && 2u * pipe_shape(f->pipe.flags, static_cast<uint32_t>(DtypeSize(f->pipe.dt)), vec, f->cols, 512u, 512u).buf_bytes > kPlanStageBytes)
           std::memset(&f->pipe, 0, sizeof(f->pipe));
         f->flat = f->vec && f->cols % 4u == 0u && f->cols <= 4096u ? FlatOps(fs, static_cast<uint32_t>(x[2])) : 0u;
+        (f->pipe.flags || f->flat || x[7] > 1 ? out->planned_gain : out->planned_loss) += f->n_elems;
         if (f->total) out->needs_scratch = true;
         d.desc = static_cast<uint32_t>(out->desc.size());
         if (d.desc % 2) { out->desc.push_back(0); ++d.desc; }              // 16-byte copies
@@ -1392,6 +1393,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
           ++out->n_mma;
           ++out->n_mma_tc;
           out->mma_flops += 2ull * q.M * q.N * q.K;
+          out->planned_gain += static_cast<uint64_t>(q.M) * q.N;
         }
         const size_t bytes = (offsetof(DGemm, prob) + g->n_prob * sizeof(DGemmProb) + 15) / 16 * 16;
         if (out->desc.size() % 2) out->desc.push_back(0);
@@ -1433,6 +1435,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         ++out->n_mma;
         if (d.op == kTopSkinny) ++out->n_mma_tc;
         out->mma_flops += 2ull * g.M * g.N * g.K;
+        out->planned_gain += static_cast<uint64_t>(g.M) * g.N;
         if (out->desc.size() % 2) out->desc.push_back(0);
         d.desc = c.PushDesc(g);
         if (out->desc.size() % 2) out->desc.push_back(0);
@@ -1453,6 +1456,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         pr.mass = c.Ref(static_cast<uint32_t>(x[4]));
         pr.out = c.Ref(static_cast<uint32_t>(x[5]));
         pr.n_tail = static_cast<uint32_t>(x[6]);
+        out->planned_gain += static_cast<uint64_t>(pr.n) * pr.n;
         for (uint32_t k = 0; k < pr.n_tail; ++k) {
           const int32_t *w = x + 7 + 8 * k;
           DPairTail &tl = pr.tail[k];

@@ -65,6 +65,7 @@ struct DeviceTables {
   uint32_t n_spread = 0;                // reduction phases re-cut over all lanes
   uint32_t n_fused_reduce = 0;          // ... of which full reductions (RED_PART + RED_COMB in one phase)
   bool needs_scratch = false;           // a re-cut full reduction leaves lane totals in the program's scratch
+  uint64_t planned_gain = 0, planned_loss = 0;   // elements that planned ops make faster / slower than the schedule (PlanGains)
   uint32_t families = kFamEw;           // tile-op families the program's tasks use (picks the megakernel build)
 };
 
@@ -76,6 +77,14 @@ bool BuildDeviceTables(const VmProgram &p, uint64_t arena_base, DeviceTables *ou
 
 // The same for a program the re-planner made (replan.h): its own ops are known, its cut and its phases stand.
 bool BuildPlannedTables(const VmProgram &p, uint64_t arena_base, DeviceTables *out, std::string *err, bool *unimplemented);
+
+// Is a planned program worth having? Its products, all-pairs ops and straight-line chains are faster than the tile ops they
+// replace, and so is a chain in the step interpreter that merges several phases of the schedule. One that merges none saves the
+// wire kernel's longer way to its first load (6 us of 18) and pays for it with every element: max((a + b) ^ c, d) over
+// 33.55 M + 1 i32 195 us planned, 145 as scheduled, a bf16 sum of two 164 and 86; even at about 3 M elements (4 M + 1: 33.7
+// and 34.3, 26.9 and 24.9).
+constexpr uint64_t kPlanLossFree = 3u << 20;
+inline bool PlanGains(const DeviceTables &t) { return t.planned_loss <= t.planned_gain + kPlanLossFree; }
 
 // How a 16-bit matmul task's operands lie, for the tensor cores (batch of one): unit stride along k, or along the rows /
 // columns (`mn`), leading dimension and offset in elements. False where they cannot be fed directly.

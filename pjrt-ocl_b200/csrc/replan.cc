@@ -40,6 +40,7 @@ struct Node {
   VmTask t{};
   uint32_t op = 0, dt = 0, adt = 0;
   int region = 0;            // 0 root before the loop, 1 its body, 2 root after it
+  int phase = 0;             // the schedule's
   int order = 0;             // program order inside the whole walk
   uint32_t tiles = 0;
   double cost = 1.0;         // of one tile, relative
@@ -59,6 +60,7 @@ class Planner {
   bool Run(VmProgram *q, ReplanStats *st);
 
  private:
+  struct Chain;
   const VmProgram &p_;
   const uint32_t L_;
   std::vector<Node> n_;                      // original tasks in program order, then planned ops
@@ -72,6 +74,7 @@ class Planner {
 
   bool Extract();
   bool TaskTiles(const VmTask &t, uint32_t *tiles) const;
+  int PhasesMerged(const Chain &c) const;
   void Lists(const VmTask &t, std::vector<uint32_t> *rd, std::vector<uint32_t> *wr) const;
   void Dependences();
   bool Acyclic() const;
@@ -97,7 +100,6 @@ class Planner {
   }
   int AddPlanned(Node nd, const std::vector<int> &members);
 
-  struct Chain;
   bool FusePairs(int seed);
   bool FuseGemm(int seed);
   void SgShape(uint32_t op, uint64_t M, uint64_t N, uint64_t K, uint32_t lanes, int *shape, uint32_t *tiles, double *cost) const;
@@ -263,6 +265,7 @@ bool Planner::Extract() {
       nd.dt = (nd.t.tile_op >> 8) & 0xFFu;
       nd.adt = (nd.t.tile_op >> 16) & 0xFFu;
       nd.region = kv.first.first;
+      nd.phase = kv.first.second;
       nd.order = seq++;
       if (!TaskTiles(nd.t, &nd.tiles)) return false;
       auto &r = at[ti].ranges;
@@ -1240,6 +1243,19 @@ bool Planner::FuseRows(int seed) {
   return false;
 }
 
+// Phases of the schedule that a chain's tasks are from: how many passes over memory it is instead of. A full sum is one, with
+// its combine and a convert that only feeds it (the wire programs' tables fold those too).
+int Planner::PhasesMerged(const Chain &c) const {
+  std::set<int> ph;
+  for (int m : c.members) {
+    const Node &nd = n_[m];
+    if (nd.op == kTopRedComb) continue;
+    if (nd.op == kTopEw && nd.t.p0 == kConvert && Uses(nd.t.dst).size() == 1 && n_[Uses(nd.t.dst)[0]].op == kTopRedPart) continue;
+    ph.insert(nd.phase);
+  }
+  return static_cast<int>(ph.size());
+}
+
 Node Planner::RowsNode(const Chain &c, uint32_t start, const std::vector<uint32_t> &writes, uint64_t R, uint64_t C, uint64_t n) const {
   Node nd;
   nd.op = kTopFuseRows;
@@ -1252,7 +1268,7 @@ Node Planner::RowsNode(const Chain &c, uint32_t start, const std::vector<uint32_
   nd.tiles = static_cast<uint32_t>(R);
   nd.cost = std::max(0.02, static_cast<double>(C) / 4096.0);
   nd.payload = {static_cast<int32_t>(R), static_cast<int32_t>(C), static_cast<int32_t>(c.steps.size()), c.total + 1,
-                C % 4 == 0 && n % 4 == 0 ? 1 : 0, 0, static_cast<int32_t>(n)};
+                C % 4 == 0 && n % 4 == 0 ? 1 : 0, 0, static_cast<int32_t>(n), PhasesMerged(c)};
   nd.owner_word = 5;
   nd.carry_slot = c.total >= 0 ? 0 : -1;
   for (const Step &s : c.steps)
@@ -1309,7 +1325,7 @@ void Planner::NormIntoProducts(std::vector<int> *live, std::vector<std::set<int>
     const Node &nd = n_[r];
     ++k;
     if (!nd.planned || nd.op != kTopFuseRows || nd.wr.size() != 1 || nd.payload[0] > 32 || nd.payload[1] > 1024 || nd.payload[1] % 32 != 0 || nd.payload[2] != 9) continue;
-    const int32_t *st = &nd.payload[7];
+    const int32_t *st = &nd.payload[kFuseWords];
     auto code = [&](int i) { return static_cast<uint32_t>(st[6 * i]); };
     const uint32_t dt = static_cast<uint32_t>(st[1]), h = nd.wr[0];
     if (!Half(dt) || code(0) != kFuLoadX || code(1) != kFuRedSumSq || code(2) != kFuSAffine || code(3) != kFuSRsqrt || code(4) != kFuMulS ||

@@ -8,7 +8,8 @@
 // remaining buffers anew. Results keep the roundings of every value that the program stores or
 // hands on in a narrower type; sums may be taken in another order.
 //
-// It leaves a program alone (returns false) when nothing in it fuses, when it uses control flow other than one counted
+// A program keeps its schedule (loader.h: PlanGains) where the plan would make the same passes over memory, on the step
+// interpreter. The re-planner leaves it alone (returns false) when nothing in it fuses, when it uses control flow other than one counted
 // loop at the top, or when it was scheduled for half of the device or less.
 #ifndef B2VM_REPLAN_H_
 #define B2VM_REPLAN_H_
@@ -33,6 +34,10 @@ bool Replan(const VmProgram &p, uint32_t device_lanes, VmProgram *q, ReplanStats
 bool IsPlannedOp(uint32_t tile_op);
 void PlannedLists(const VmProgram &p, const VmTask &t, const int32_t **reads, int *n_reads, const int32_t **writes, int *n_writes,
                   const int32_t **payload);
+
+// Words before the steps in a kTopFuseRows payload: rows cols steps total+1 vec owners elements, and the phases of the schedule that
+// it takes the place of.
+constexpr int kFuseWords = 8;
 
 // Words per product in a kTopGemm payload {n, total + 1, owner lanes, products}: M N K halves bn amn bmn adt a b a_ld b_ld a_off b_off
 // epi qdt rdt s0 s1 gg res+1 out0+1 dt0 out1+1 dt1.

@@ -485,7 +485,7 @@ b2_status b2_program_load(b2_runtime *rt, b2_program *prog, b2_loaded **out, cha
     }
     b2::DeviceTables fits;
     lp->is_planned = b2::Replan(p, static_cast<uint32_t>(rt->max_lanes), &planned, &lp->plan) &&
-                     b2::BuildPlannedTables(planned, 0, &fits, &m, &unimpl) && build_for(fits) >= 0;
+                     b2::BuildPlannedTables(planned, 0, &fits, &m, &unimpl) && build_for(fits) >= 0 && b2::PlanGains(fits);
   }
   const b2::VmProgram &use = lp->is_planned ? planned : p;
   cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&lp->arena), std::max<uint64_t>(use.arena_bytes, 256));

@@ -29,7 +29,7 @@ int main(int argc, char **argv) {
     std::fprintf(stderr, "planned: %s\n", err.c_str());
     return 1;
   }
-  std::printf("{\"planned\": true, \"families\": %u, \"phases\": %u, \"tasks\": [", t.families, st.phases);
+  std::printf("{\"planned\": true, \"gains\": %s, \"families\": %u, \"phases\": %u, \"tasks\": [", b2::PlanGains(t) ? "true" : "false", t.families, st.phases);
   for (uint32_t i = 0; i < t.tasks.size(); ++i) {
     const b2::DTask &d = t.tasks[i];
     const uint64_t *w = &t.desc[d.desc];

@@ -86,3 +86,14 @@ def stages(rows, cols, dtype, what, total=False):
             p.phase()
         p.output(p.full_sum(out), ())
     return p
+
+
+def flat(n, dtype, ops):
+    """A chain of elementwise ops over n elements (subops of perf/cases.py; the binary ones take a second argument each)."""
+    p = cases._Assembler(148)
+    cur, chain = p.input((n,), dtype), []
+    for k in ops:
+        chain.append((k, (cur,) if k in (cases._GELU, cases._TANH) else (cur, p.input((n,), dtype)), dtype))
+        cur = -1
+    p.output(p.chain(*chain), (n,))
+    return p

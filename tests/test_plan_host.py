@@ -11,6 +11,7 @@ import subprocess
 import pytest
 
 from conftest import ROOT
+import perf.cases as cases
 import plan_programs as progs
 
 CSRC = os.path.join(ROOT, "pjrt-ocl_b200", "csrc")
@@ -96,3 +97,22 @@ def test_chains_without_a_norm_are_row_pipelines(plan):
     assert t["pipe"] == ON | MUL | ADD | GELU
     (t,) = plan(committed("c2_stage_sum_f32"))["tasks"]
     assert t["pipe"] == ON | CARRY
+
+
+@pytest.mark.parametrize("n, dtype, ops, kept", [
+    (131, "i32", (cases._ADD, cases._XOR, cases._MAX), True), (33550001, "i32", (cases._ADD, cases._XOR, cases._MAX), False),
+    (33550000, "i32", (cases._ADD, cases._XOR, cases._MAX), True), (400001, "bf16", (cases._ADD,), True), (4000001, "bf16", (cases._ADD,), False),
+    (33550000, "bf16", (cases._ADD, cases._MUL), False), (8192 * 4096, "bf16", (cases._GELU,), True), (33550001, "f32", (cases._TANH, cases._MUL), False)])
+def test_long_chains_that_only_the_step_interpreter_runs_keep_their_schedule(plan, n, dtype, ops, kept):
+    p = plan(progs.flat(n, dtype, ops).blob())
+    assert p["planned"] and p["gains"] == kept
+
+
+def test_norm_chains_and_products_keep_their_plans(plan):
+    for c in cases.listed():
+        if c["kind"] != "nbody":
+            assert plan(cases._BUILD[c["kind"]](c).blob())["gains"], c["name"]
+    # an odd width: the interpreter, but instead of four passes
+    assert plan(cases._BUILD["norm_chain"]({"rows": 8192, "cols": 4095, "dtype": "f32"}).blob())["gains"]
+    # a lone sum of a length that no piece divides: the tile op streams it faster
+    assert not plan(progs.stages(8191, 4095, "f32", (), True).blob())["gains"]
