@@ -75,6 +75,7 @@ class Planner {
   bool Extract();
   bool TaskTiles(const VmTask &t, uint32_t *tiles) const;
   int PhasesMerged(const Chain &c) const;
+  double MoveCost(const Node &nd) const;
   void Lists(const VmTask &t, std::vector<uint32_t> *rd, std::vector<uint32_t> *wr) const;
   void Dependences();
   bool Acyclic() const;
@@ -125,6 +126,19 @@ bool Planner::TaskTiles(const VmTask &t, uint32_t *tiles) const {
     case kTopFlashAttn: *tiles = t.p1 * t.p2; return *tiles > 0;
     default: return false;      // window / index / convolution ops: programs with them keep their schedule
   }
+}
+
+// A tile of a move by its bytes: 23 per cycle is a lane's share of the copy rate; runs that are not contiguous at the far side
+// come at about a quarter of it. (A contiguous 16-bit tile is 0.12 of the unit; taken for 1.5, the copies of a decode step's
+// caches left all 96 tiles of the products beside them to one lane: 2.18 ms, 1.22 ms now.)
+double Planner::MoveCost(const Node &nd) const {
+  const double cycles = 2.0 * kEwTs * static_cast<double>(DtypeSize(nd.dt)) / 23.0;
+  bool runs = true;
+  if (nd.op == kTopGather) {
+    const View v = ViewAt(nd.t.p0 + 1);
+    runs = v.ok && v.v.rank > 0 && v.v.stride[v.v.rank - 1] == 1;
+  }
+  return cycles * (runs ? 1.0 : 4.0) / 6000.0;
 }
 
 void Planner::Lists(const VmTask &t, std::vector<uint32_t> *rd, std::vector<uint32_t> *wr) const {
@@ -276,7 +290,7 @@ bool Planner::Extract() {
       Lists(nd.t, &nd.rd, &nd.wr);
       switch (nd.op) {
         case kTopMma: nd.cost = 20.0; break;
-        case kTopGather: case kTopScatter: case kTopDynGather: case kTopDynScatter: nd.cost = 1.5; break;
+        case kTopGather: case kTopScatter: case kTopDynGather: case kTopDynScatter: nd.cost = MoveCost(nd); break;
         case kTopRedSeg: case kTopSoftmaxSeg: case kTopLayernormSeg: nd.cost = std::max(0.02, nd.t.p1 / 4096.0); break;
         case kTopRedPart: nd.cost = nd.t.p1 / 4096.0; break;
         case kTopFlashAttn: nd.cost = 0.5; break;
@@ -1494,13 +1508,22 @@ bool Planner::Assemble(VmProgram *q, ReplanStats *st) {
     if (region == 1 && !for_placed) { prev_region = seen_in_region[0] ? 0 : -1; place_for(); prev_region = 1; }
     const auto &us = kv.second;
     std::vector<std::vector<std::pair<uint32_t, uint32_t>>> cut(us.size(), std::vector<std::pair<uint32_t, uint32_t>>(L_, {0u, 0u}));
-    bool plenty = true;
+    // Units of many tiles are cut evenly over all lanes, whatever they cost. Products with few tiles are dear: beside such units they
+    // share all lanes among themselves, as they would without them (`mixed`); else units lie side by side by cost.
+    bool plenty = true, mixed = false;
+    size_t n_slot = 0;
+    for (int u : us) { plenty = plenty && n_[u].tiles >= 2 * L_; n_slot += n_[u].by_slot ? 1 : 0; }
+    if (!plenty && n_slot && n_slot < us.size()) {
+      mixed = true;
+      for (int u : us) mixed = mixed && (n_[u].by_slot || n_[u].tiles >= 2 * L_);
+    }
+    auto even = [&](int u) { return us.size() == 1 || plenty || (mixed && !n_[u].by_slot); };
     double total = 0;
-    for (int u : us) { plenty = plenty && n_[u].tiles >= 2 * L_; total += n_[u].cost * n_[u].tiles * static_cast<double>(of[u].size()); }
+    for (int u : us) if (!even(u)) total += n_[u].cost * n_[u].tiles * static_cast<double>(of[u].size());
     double at = 0;
     for (size_t k = 0; k < us.size(); ++k) {
       const uint64_t T = n_[us[k]].tiles;
-      if (us.size() == 1 || plenty) {
+      if (even(us[k])) {
         for (uint64_t l = 0; l < L_; ++l) cut[k][l] = {static_cast<uint32_t>(T * l / L_), static_cast<uint32_t>(T * (l + 1) / L_)};
       } else {
         // units side by side: lane l takes the tiles whose middle falls in its share of the phase's cost
@@ -1522,7 +1545,7 @@ bool Planner::Assemble(VmProgram *q, ReplanStats *st) {
         // a share of the lanes, each with a slot number (alone in the phase: all of them, as many as there are tiles)
         std::vector<uint32_t> mine;
         for (uint32_t l = 0; l < L_; ++l)
-          if (us.size() == 1 ? l < T : cut[k][l].second > cut[k][l].first) mine.push_back(l);
+          if (us.size() == 1 || (mixed && n_slot == 1) ? l < T : cut[k][l].second > cut[k][l].first) mine.push_back(l);
         owners = static_cast<uint32_t>(mine.size());
         for (uint32_t i = 0; i < owners; ++i) {
           VmEntry e = blank;

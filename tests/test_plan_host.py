@@ -116,3 +116,19 @@ def test_norm_chains_and_products_keep_their_plans(plan):
     assert plan(cases._BUILD["norm_chain"]({"rows": 8192, "cols": 4095, "dtype": "f32"}).blob())["gains"]
     # a lone sum of a length that no piece divides: the tile op streams it faster
     assert not plan(progs.stages(8191, 4095, "f32", (), True).blob())["gains"]
+
+
+def test_products_beside_large_moves_get_their_lanes(plan):
+    """The decode step that copies its caches: three products share a phase with the copies. They share the lanes among
+    themselves as they would alone, and the copies are cut evenly over all."""
+    tasks = plan(committed("c5_decode_bf16"))["tasks"]
+    qkv = [t for t in tasks if t["op"] == SKINNY and t["mnk"] == [32, 1024, 1024]][:3]
+    for t in qkv:
+        assert len({lane for lane, _, _ in t["cut"]}) >= 32                 # 32 tiles of 32 columns each
+    lanes = [lane for t in qkv for lane, _, _ in t["cut"]]
+    assert len(lanes) == len(set(lanes))
+    moves = [t for t in tasks if t["op"] in (2, 6) and max(hi for _, _, hi in t["cut"]) >= 2 * 148]
+    assert len(moves) == 3
+    for t in moves:
+        per = [hi - lo for _, lo, hi in t["cut"]]
+        assert len(per) == 148 and max(per) - min(per) <= 1
