@@ -80,3 +80,36 @@ class Builder:
             for e in stream:
                 out += struct.pack("<8I", *e)
         return bytes(out)
+
+
+def widen(blob: bytes, n_lanes: int) -> bytes:
+    """The same program scheduled for `n_lanes` lanes: the added ones walk lane 0's control flow and barriers and do no work."""
+    _, _, n_buf, n_instr, n_const, _, n_in, n_out, n_aux, _, _ = struct.unpack_from("<IIIIIIIIIIQ", blob)
+    at = 48 + 24 * n_buf
+
+    def pad8(x):
+        return (x + 7) // 8 * 8
+    at = pad8(at + 4 * n_in)
+    at = pad8(at + 4 * n_out)
+    for _ in range(n_in + n_out):
+        at += 8 + 8 * struct.unpack_from("<I", blob, at)[0]
+    at = pad8(at + 4 * n_aux)
+    for _ in range(n_const):
+        at = pad8(at + 8 + struct.unpack_from("<I", blob, at + 4)[0])
+    at += 32 * n_instr
+    n_tasks, n_entries, n_flags, had = struct.unpack_from("<IIII", blob, at)
+    tasks = blob[at + 16:at + 16 + 48 * n_tasks]
+    lane_at = at + 16 + 48 * n_tasks
+    lanes = [struct.unpack_from("<IIII", blob, lane_at + 16 * i) for i in range(had)]
+    ent_at = lane_at + 16 * had
+    entries = blob[ent_at:ent_at + 32 * n_entries]
+    assert ent_at + 32 * n_entries == len(blob) and n_lanes >= had
+    off, count, root, _ = lanes[0]
+    idle = b""
+    for i in range(off, off + count):
+        e = entries[32 * i:32 * i + 32]
+        idle += e if struct.unpack_from("<I", e)[0] >= FOR else struct.pack("<8I", NOP, 0, 0, FLAG_NONE, 0, FLAG_NONE, 0, 0)
+    for k in range(n_lanes - had):
+        lanes.append((n_entries + k * count, count, root, 0))
+    return (blob[:at] + struct.pack("<IIII", n_tasks, n_entries + (n_lanes - had) * count, n_flags, n_lanes) + tasks +
+            b"".join(struct.pack("<IIII", *x) for x in lanes) + entries + idle * (n_lanes - had))

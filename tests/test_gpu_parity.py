@@ -40,6 +40,29 @@ def test_execute_matches_reference_validators(rt, name):
         np.testing.assert_array_equal(a, b)
 
 
+REPLANNED = {"c1_relu_matmul", "c2_chain_decomposed_small", "c2_chain_f32_small", "c2_int_chain_small", "c3_dp2_grads_f32_small",
+             "c3_mlp_bf16_small", "c3_mlp_f32_small", "c4_nbody_mid", "c4_nbody_small", "c5_block_bf16_small", "c5_block_f32_small",
+             "c5_decode_in_place_bf16_small", "c5_decode_in_place_f32_small", "dot_bf16", "dot_bf16_f32out", "dot_f16", "dot_f32",
+             "dot_kat_2x2", "for_loop_cross_lane", "norms_recognized", "rmsnorm_rows_bf16", "rows_then_full_sum_bf16",
+             "rows_then_full_sum_f32", "rows_then_full_sum_ragged", "ew_views_aligned_f32_bf16", "for_loop_carries",
+             "golden_layout_kat", "reduce_full_16bit_source"}
+
+
+@pytest.mark.parametrize("name", golden_names())
+def test_widened_to_the_whole_device_matches_reference_validators(rt, name):
+    """The same blobs scheduled for every lane of the device (they come for 2 to 8): what the re-planner can take of them runs
+    re-planned, against the same expectations at the same tolerances."""
+    from blobs import widen
+    vm = package()
+    g = Golden(name)
+    lp = vm.LoadedProgram.Load(rt, vm.VmProgram.Parse(widen(g.blob, rt.lanes)))
+    assert lp.prog.n_lanes == rt.lanes
+    assert (lp.stat("replanned") == 1) == (name in REPLANNED)
+    for _ in range(2):
+        check_outputs(g, _raw(lp.Execute(g.args)), "cuda-widened")
+    assert lp.Status()["code"] == 0
+
+
 @pytest.mark.parametrize("name", ["c2_int_chain_small", "c2_chain_f32_small", "c3_mlp_bf16_small",
                                   "c4_nbody_small", "c5_block_bf16_small", "dynslice",
                                   "while_loop_data_dependent", "c5_decode_in_place_bf16_small"])
