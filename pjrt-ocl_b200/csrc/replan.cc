@@ -47,6 +47,7 @@ struct Node {
   bool planned = false;      // one of this file's own ops
   std::vector<uint32_t> rd, wr;
   std::vector<int32_t> payload;
+  std::vector<int> members;  // of a planned op: the tasks it is made of
   int carry_slot = -1;       // full sum counter it uses
   bool by_slot = false;      // entries name {lane slot, slots} instead of a tile range (matmuls)
   size_t owner_word = 0;     // payload word that takes the number of owner lanes (carry_slot >= 0)
@@ -64,7 +65,8 @@ class Planner {
   const VmProgram &p_;
   const uint32_t L_;
   std::vector<Node> n_;                      // original tasks in program order, then planned ops
-  std::vector<std::set<int>> pred_;          // original data dependences
+  std::vector<std::set<int>> pred_;          // original data dependences,
+  std::vector<std::vector<int>> succ_;       // ... the other way
   std::vector<int> rep_;                     // node -> the node it is now part of
   int n_orig_ = 0;
   int loop_trip_ = -1;
@@ -78,7 +80,7 @@ class Planner {
   double MoveCost(const Node &nd) const;
   void Lists(const VmTask &t, std::vector<uint32_t> *rd, std::vector<uint32_t> *wr) const;
   void Dependences();
-  bool Acyclic() const;
+  bool Cyclic(int id) const;
   uint64_t Count(uint32_t id) const { return p_.buffers[id].bytes / DtypeSize(p_.buffers[id].dtype); }
   uint32_t Dt(uint32_t id) const { return p_.buffers[id].dtype; }
   bool Pinned(uint32_t id) const { return in_.count(id) || out_.count(id) || const_.count(id); }
@@ -188,10 +190,15 @@ bool Planner::Extract() {
   struct Place { int region = -1, phase = -1; std::vector<std::pair<uint32_t, uint32_t>> ranges; };
   std::vector<Place> at(p_.tasks.size());
   std::map<std::pair<int, int>, std::vector<uint32_t>> order;         // (region, phase) -> tasks
-  std::map<std::pair<int, int>, std::set<std::pair<uint32_t, uint32_t>>> before;   // ... and which ran before which on some lane
+  std::map<std::pair<int, int>, std::set<std::vector<uint32_t>>> seqs;  // ... and the orders that lanes run several of them in
   for (uint32_t l = 0; l < lanes; ++l) {
     const VmLane &ln = p_.lane_tab[l];
-    std::map<std::pair<int, int>, std::vector<uint32_t>> mine;
+    std::vector<uint32_t> seq;                                          // this lane's tasks of the phase
+    std::pair<int, int> seq_at{0, 0};
+    auto close = [&] {
+      if (seq.size() > 1) seqs[seq_at].insert(seq);
+      seq.clear();
+    };
     auto tile = [&](const VmEntry &e, int region, int phase) {
       if (e.task >= p_.tasks.size()) return false;
       if ((e.wait_flag != 0xFFFFFFFFu && e.wait_flag) || e.wait_count || (e.signal_flag != 0xFFFFFFFFu && e.signal_flag)) return false;
@@ -201,11 +208,8 @@ bool Planner::Extract() {
         order[{region, phase}].push_back(e.task);
       }
       if (pl.region != region || pl.phase != phase) return false;
-      auto &seq = mine[{region, phase}];
-      if (std::find(seq.begin(), seq.end(), e.task) == seq.end()) {       // (a lane may hold several pieces of a task)
-        for (uint32_t t : seq) before[{region, phase}].insert({t, e.task});
-        seq.push_back(e.task);
-      }
+      if (seq_at != std::make_pair(region, phase)) { close(); seq_at = {region, phase}; }
+      if (std::find(seq.begin(), seq.end(), e.task) == seq.end()) seq.push_back(e.task);       // (a lane may hold several pieces of a task)
       if (e.tile_hi > e.tile_lo) pl.ranges.push_back({e.tile_lo, e.tile_hi});
       return true;
     };
@@ -234,6 +238,7 @@ bool Planner::Extract() {
       if (!tile(e, region, phase)) return false;
     }
     if (covered != ln.count) return false;
+    close();
     if (l == 0) { loop_trip_ = trip; has_loop_ = trip >= 0; }
     else if (trip != loop_trip_) return false;
   }
@@ -241,8 +246,13 @@ bool Planner::Extract() {
   // Inside a phase only tasks of one lane's chain may touch the same buffer: those keep the lane's order.
   for (auto &kv : order) {
     auto &ts = kv.second;
-    const auto &bf = before[kv.first];
     std::sort(ts.begin(), ts.end());
+    std::set<std::pair<uint32_t, uint32_t>> bf;          // which ran before which on some lane
+    const auto sq = seqs.find(kv.first);
+    if (sq != seqs.end())
+      for (const auto &v : sq->second)
+        for (size_t i = 0; i < v.size(); ++i)
+          for (size_t j = i + 1; j < v.size(); ++j) bf.insert({v[i], v[j]});
     std::vector<std::vector<uint32_t>> rd(ts.size()), wr(ts.size());
     for (size_t i = 0; i < ts.size(); ++i) Lists(p_.tasks[ts[i]], &rd[i], &wr[i]);
     auto meet = [](const std::vector<uint32_t> &a, const std::vector<uint32_t> &b) {
@@ -327,27 +337,26 @@ void Planner::Dependences() {
     for (uint32_t b : n_[i].wr) writers[b].push_back(i);
     for (uint32_t b : n_[i].rd) readers[b].push_back(i);
   }
+  succ_.assign(n_orig_, {});
+  for (int i = 0; i < n_orig_; ++i) for (int j : pred_[i]) succ_[j].push_back(i);
 }
 
-bool Planner::Acyclic() const {
-  const int N = static_cast<int>(n_.size());
-  std::vector<std::set<int>> succ(N);
-  std::vector<int> deg(N, 0);
-  for (int i = 0; i < n_orig_; ++i)
-    for (int j : pred_[i]) {
-      const int a = rep_[j], b = rep_[i];
-      if (a != b && succ[a].insert(b).second) ++deg[b];
-    }
-  std::vector<int> todo;
-  int seen = 0, all = 0;
-  for (int i = 0; i < N; ++i) if (rep_[i] == i) { ++all; if (!deg[i]) todo.push_back(i); }
+// Does anything that node `id` is made of need something that needs the node? (Without it the graph had no cycle.)
+bool Planner::Cyclic(int id) const {
+  std::vector<char> seen(n_.size(), 0);
+  std::vector<int> todo{id};
   while (!todo.empty()) {
-    const int i = todo.back();
+    const int g = todo.back();
     todo.pop_back();
-    ++seen;
-    for (int j : succ[i]) if (--deg[j] == 0) todo.push_back(j);
+    const std::vector<int> own{g};
+    for (int m : n_[g].planned ? n_[g].members : own)
+      for (int k : succ_[m]) {
+        const int r = rep_[k];
+        if (r == id && g != id) return true;
+        if (r != id && !seen[r]) { seen[r] = 1; todo.push_back(r); }
+      }
   }
-  return seen == all;
+  return false;
 }
 
 // Members become part of the new node, unless that would need something that needs the node itself.
@@ -356,13 +365,14 @@ int Planner::AddPlanned(Node nd, const std::vector<int> &members) {
   nd.region = n_[members[0]].region;
   nd.order = n_[members[0]].order;
   for (int m : members) { if (n_[m].region != nd.region) return -1; nd.order = std::max(nd.order, n_[m].order); }
-  const std::vector<int> before = rep_;
   const int id = static_cast<int>(n_.size());
+  nd.members = members;
   n_.push_back(nd);
   rep_.push_back(id);
   for (int m : members) rep_[m] = id;
-  if (Acyclic()) return id;
-  rep_ = before;
+  if (!Cyclic(id)) return id;
+  for (int m : members) rep_[m] = m;
+  rep_.pop_back();
   n_.pop_back();
   return -1;
 }
@@ -1175,25 +1185,30 @@ void Planner::GroupGemms(std::vector<int> *live, std::map<std::pair<int, int>, s
         const int32_t *w = &nd.payload[3 + kGemmWords * p];
         return static_cast<double>((w[0] + 128 * shapes[s][0] - 1) / (128 * shapes[s][0])) * ((w[1] + shapes[s][1] - 1) / shapes[s][1]);
       };
-      std::vector<int> best(np, 0);
-      double best_t = 1e300;
+      std::vector<int> best(np, 0), sh(np);
+      double best_t = 1e300, cost[kGemmMaxProbs][6], n_tiles[kGemmMaxProbs][6];
+      for (int p = 0; p < np; ++p)
+        for (int i = 0; i < 6; ++i) { cost[p][i] = tile_cost(p, i); n_tiles[p][i] = tiles(p, i); }
+      std::vector<double> load(L_);
       const int combos = np == 1 ? 6 : np == 2 ? 36 : np == 3 ? 216 : 6;
       for (int k = 0; k < combos; ++k) {
-        std::vector<int> sh(np);
-        for (int p = 0, q = k; p < np; ++p) { sh[p] = np <= 3 ? q % 6 : k; if (np <= 3) q /= 6; }
-        // the lanes' loads when tiles are dealt out in order
-        double load_max = 0, at = 0;
-        std::vector<double> load(L_, 0.0);
-        uint64_t next = 0;
-        for (int p = 0; p < np; ++p) {
-          const double T = tiles(p, sh[p]), c = tile_cost(p, sh[p]);
-          const uint64_t n = static_cast<uint64_t>(T), whole = n / L_, left = n % L_;
-          for (uint32_t l = 0; l < L_; ++l) load[l] += c * static_cast<double>(whole);
-          for (uint64_t i = 0; i < left; ++i) load[(next + i) % L_] += c;
-          next += n;
-          at += c;
+        double all = 0;
+        for (int p = 0, q = k; p < np; ++p) {
+          sh[p] = np <= 3 ? q % 6 : k;
+          if (np <= 3) q /= 6;
+          all += cost[p][sh[p]] * n_tiles[p][sh[p]];
         }
-        for (double x : load) load_max = std::max(load_max, x);
+        if (all >= best_t * L_) continue;              // even cut perfectly no sooner done
+        // the lanes' loads when tiles are dealt out in order
+        std::fill(load.begin(), load.end(), 0.0);
+        uint32_t next = 0;
+        for (int p = 0; p < np; ++p) {
+          const double c = cost[p][sh[p]];
+          const uint64_t n = static_cast<uint64_t>(n_tiles[p][sh[p]]), whole = n / L_;
+          for (double &x : load) x += c * static_cast<double>(whole);
+          for (uint64_t i = n - whole * L_; i; --i) { load[next] += c; if (++next == L_) next = 0; }
+        }
+        const double load_max = *std::max_element(load.begin(), load.end());
         if (load_max < best_t) { best_t = load_max; best = sh; }
       }
       uint64_t total = 0;
@@ -1440,9 +1455,15 @@ bool Planner::Assemble(VmProgram *q, ReplanStats *st) {
   GroupGemms(&live, &phases, &of);
 
   // ---- the program ----
-  *q = p_;
-  q->tasks.clear();
-  q->entries.clear();
+  *q = VmProgram{};
+  q->buffers = p_.buffers;
+  q->args = p_.args;
+  q->results = p_.results;
+  q->aux = p_.aux;
+  q->consts = p_.consts;
+  q->n_instrs = p_.n_instrs;
+  q->root_instrs = p_.root_instrs;
+  q->n_flags = p_.n_flags;
   std::vector<uint32_t> task_of(N, 0);
   std::map<int, size_t> payload_at;
   // one full-sum counter per op of a phase

@@ -474,6 +474,12 @@ b2_status b2_program_load(b2_runtime *rt, b2_program *prog, b2_loaded **out, cha
       if ((t.families & ~b2::kVariants[v].families) == 0u) return v;
     return -1;
   };
+  cudaError_t e = cudaSuccess;
+  auto make_arena = [&](const b2::VmProgram &of) {
+    e = cudaMalloc(reinterpret_cast<void **>(&lp->arena), std::max<uint64_t>(of.arena_bytes, 256));
+    if (e != cudaSuccess) { lp->arena = nullptr; cudaGetLastError(); }
+    return e == cudaSuccess;
+  };
   // Re-planned for this device where that fuses anything (replan.h). The program is checked as it came first: the
   // re-planner relies on every index the tables' builder refuses to be in range.
   b2::VmProgram planned;
@@ -483,20 +489,26 @@ b2_status b2_program_load(b2_runtime *rt, b2_program *prog, b2_loaded **out, cha
       SetErr(err, err_cap, "load: " + m);
       return unimpl ? B2_UNIMPLEMENTED : B2_INVALID_ARGUMENT;
     }
-    b2::DeviceTables fits;
-    lp->is_planned = b2::Replan(p, static_cast<uint32_t>(rt->max_lanes), &planned, &lp->plan) &&
-                     b2::BuildPlannedTables(planned, 0, &fits, &m, &unimpl) && build_for(fits) >= 0 && b2::PlanGains(fits);
+    // (its tables are built where its arena is, once; the arena goes back if the plan is not kept)
+    if (b2::Replan(p, static_cast<uint32_t>(rt->max_lanes), &planned, &lp->plan) && make_arena(planned)) {
+      lp->is_planned = b2::BuildPlannedTables(planned, reinterpret_cast<uint64_t>(lp->arena), &lp->tab, &m, &unimpl) && build_for(lp->tab) >= 0 && b2::PlanGains(lp->tab);
+      if (!lp->is_planned) {
+        cudaFree(lp->arena);
+        lp->arena = nullptr;
+        lp->tab = b2::DeviceTables();
+      }
+    }
   }
   const b2::VmProgram &use = lp->is_planned ? planned : p;
-  cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&lp->arena), std::max<uint64_t>(use.arena_bytes, 256));
-  if (e != cudaSuccess) {
-    SetErr(err, err_cap, CudaMsg("arena allocation", e) + " for " + std::to_string(use.arena_bytes) + " bytes");
-    cudaGetLastError();
-    return B2_RESOURCE_EXHAUSTED;
-  }
-  if (!(lp->is_planned ? b2::BuildPlannedTables : b2::BuildDeviceTables)(use, reinterpret_cast<uint64_t>(lp->arena), &lp->tab, &m, &unimpl)) {
-    SetErr(err, err_cap, "load: " + m);
-    return unimpl ? B2_UNIMPLEMENTED : B2_INVALID_ARGUMENT;
+  if (!lp->is_planned) {
+    if (!make_arena(p)) {
+      SetErr(err, err_cap, CudaMsg("arena allocation", e) + " for " + std::to_string(p.arena_bytes) + " bytes");
+      return B2_RESOURCE_EXHAUSTED;
+    }
+    if (!b2::BuildDeviceTables(p, reinterpret_cast<uint64_t>(lp->arena), &lp->tab, &m, &unimpl)) {
+      SetErr(err, err_cap, "load: " + m);
+      return unimpl ? B2_UNIMPLEMENTED : B2_INVALID_ARGUMENT;
+    }
   }
   lp->variant = std::max(0, build_for(lp->tab));
   if (const char *force = std::getenv("B2VM_VARIANT")) {   // measurement aid: run on a named (larger) build
