@@ -97,3 +97,22 @@ def flat(n, dtype, ops):
         cur = -1
     p.output(p.chain(*chain), (n,))
     return p
+
+
+def rms_norm(p, x, gain, rows, cols, dtype, eps):
+    """x rsqrt(mean of squares + eps) gain, in the tile ops that a decoder block's norm arrives in."""
+    half = dtype != "f32"
+    xf = p.buf(rows * cols, "f32") if half else x
+    p_sq = p.chain(*([(cases._CONVERT, (x,), xf)] if half else []), (cases._MUL, (xf, xf), "f32"))
+    p.phase()
+    ss = p.row_sums(p_sq, rows, cols)
+    p.phase()
+    r = p.region((ss,), rows, ((cases._AFFINE, 1, 0, 0, 1.0 / cols, eps), (cases._RSQRT, 0, 1, 1)))
+    p.phase()
+    by_row, by_col = p.view((rows, cols), (1, 0)), p.view((rows, cols), (0, 1))
+    if not half:
+        return p.chain((cases._MUL, (xf, r), "f32", 0, by_row), (cases._MUL, (-1, gain), "f32", 0, by_col))
+    t = p.chain((cases._MUL, (xf, r), "f32", 0, by_row))
+    gf = p.chain((cases._CONVERT, (gain,), "f32"))
+    p.phase()
+    return p.chain((cases._MUL, (t, gf), "f32", 0, by_col), (cases._CONVERT, (-1,), dtype))

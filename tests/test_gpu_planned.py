@@ -109,6 +109,10 @@ def test_planned_program(c):
             continue
         got, want = got.double(), want.double()
         assert torch.isfinite(got).all() and float((got - want).norm()) <= tol["rel"] * float(want.norm()) + 1e-30
+        # ... and row by row, against the row and a typical one: a wrong row of many is lost in the whole
+        if want.dim():
+            rows, err = want.reshape(want.shape[0], -1).norm(dim=1), (got - want).reshape(want.shape[0], -1).norm(dim=1)
+            assert bool((err <= 4 * tol["rel"] * (rows + rows.square().mean().sqrt())).all())
 
 
 def _load(asm):
@@ -266,3 +270,32 @@ def test_pipelines_without_a_norm(what, total, rows, cols, dtype):
         kept = (outs[0] if what else x).double()
         bound = (rows * cols / (148 * 512) + 64) * 2.0 ** -24 * float(kept.abs().sum())
         assert abs(float(outs[-1]) - float(kept.sum())) <= bound
+
+
+@pytest.mark.parametrize("cols, dtype", [(64, "f32"), (100, "f32"), (640, "bf16")])
+def test_reciprocal_roots_and_reciprocals_against_the_exact_ones(cols, dtype):
+    """Rows v, 0, 0, ... normed without an epsilon come out as sqrt(cols), rows of equal elements through a softmax as 1 / cols,
+    whatever v's magnitude: 1 / sqrt(x) and 1 / x by one Newton step on the approximations. Bound for f32: 2 units for the step
+    (CUDA documents 2 ulp and 1 ulp for the approximations alone), and the products' own."""
+    import perf.cases as cases
+    dt = {"f32": torch.float32, "bf16": torch.bfloat16}[dtype]
+    rows = 4096
+    lo, hi = (-17.0, 17.0) if dtype == "f32" else (-15.0, 15.0)
+    v = (10.0 ** torch.linspace(lo, hi, rows, device="cuda", dtype=torch.float64)).to(dt)
+    x = torch.zeros((rows, cols), dtype=dt, device="cuda")
+    x[:, 3] = v
+    ones = torch.ones(cols, dtype=dt, device="cuda")
+    p = cases._Assembler(148)
+    xi, g = p.input((rows, cols), dtype), p.input((cols,), dtype)
+    p.output(progs.rms_norm(p, xi, g, rows, cols, dtype, eps=0.0), (rows, cols))
+    lp, (out,) = _execute(p, [x, ones])
+    assert lp.stat("replanned") == 1
+    want = cols ** 0.5
+    step = 6 * 2.0 ** -24 if dtype == "f32" else 2.0 ** -8
+    assert bool(((out[:, 3].double() - want).abs() <= step * want).all()) and int((out != 0).sum()) == rows
+    if dtype == "f32":
+        x = (v / v.max() * 80.0)[:, None].expand(rows, cols).contiguous()
+        p = cases._Assembler(148)
+        p.output(p.rows(cases._SOFTMAX, p.input((rows, cols), dtype), rows, cols), (rows, cols))
+        lp, (out,) = _execute(p, [x])
+        assert lp.stat("replanned") == 1 and bool(((out.double() * cols - 1).abs() <= 4 * 2.0 ** -24).all())
