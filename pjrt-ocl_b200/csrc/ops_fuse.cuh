@@ -48,6 +48,14 @@ __device__ __forceinline__ float rsqrt_nr(float x) {
   return x > 1.0e-37f && x < 1.0e37f ? fmaf(0.5f * r, e, r) : r;
 }
 
+// The same for a mean square that may be denormal (a norm without an epsilon): scaled, where the approximation would flush it.
+// (Layer norms, whose variance is a difference that loses such numbers, keep the shorter form: 98 us for 101 at 8192 x 4096 f32.)
+__device__ __forceinline__ float rsqrt_nr_tiny(float x) {
+  const bool tiny = x < 1.0e-37f;
+  const float r = rsqrt_nr(x * (tiny ? 0x1p+64f : 1.0f));
+  return tiny ? r * 0x1p+32f : r;
+}
+
 // d/dz of tanh-GELU, 0.5 (1 + t) + 0.5 z (1 - t^2) u' with t = tanh(u), u = k (z + 0.044715 z^3), u' = k + c z^2: with
 // e = exp(2u) and r = 1 / (1 + e) that is 0.5 (1 + t) = e r and 1 - t^2 = 4 e r^2, so e r (1 + 2 z r u'): one exponential
 // and one reciprocal, no cancellation. c = 3 x 0.7978845608 x 0.044715 as the program rounds it.
@@ -334,7 +342,7 @@ static __device__ __noinline__ float fuse_rows_run(uint32_t tid, uint32_t nthr, 
           break;
         }
         case kFuSAffine: { const float v = affine2(st.reg ? S[1] : S[0], st.s, st.t); if (st.reg) S[1] = v; else S[0] = v; break; }
-        case kFuSRsqrt: { const float v = rsqrt_nr(st.reg ? S[1] : S[0]); if (st.reg) S[1] = v; else S[0] = v; break; }
+        case kFuSRsqrt: { const float v = rsqrt_nr_tiny(st.reg ? S[1] : S[0]); if (st.reg) S[1] = v; else S[0] = v; break; }
         case kFuLayerNorm: {
           float a[4] = {0.0f, 0.0f, 0.0f, 0.0f}, b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
           B2_FU_IN(a[e] += X[g][e]; b[e] = fmaf(X[g][e], X[g][e], b[e]))

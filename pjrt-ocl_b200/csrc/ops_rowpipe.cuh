@@ -181,7 +181,7 @@ static __device__ __noinline__ float row_pipe_run(uint32_t tid, uint32_t nthr, u
       float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
       B2_RP_G B2_RP_E a[e] = __fadd_rn(a[e], __fmul_rn(X[g][e], X[g][e]));
       const float ss = fuse_group_reduce((a[0] + a[1]) + (a[2] + a[3]), add_f, slot, T, gi, gl, turn);
-      const float r = rsqrt_nr(affine2(ss, A.s, A.t));
+      const float r = rsqrt_nr_tiny(affine2(ss, A.s, A.t));
       B2_RP_G { B2_RP_E X[g][e] = __fmul_rn(X[g][e], r); if (fl & kRpQ) pipe_q4<DT>(X[g]); }
     }
     if (fl & kRpMul) {
@@ -272,7 +272,7 @@ static __device__ __noinline__ void rms_rows(const Lane &L, const DPipe &p, uint
 #pragma unroll
       for (int e = 0; e < 8; ++e) ss[e & 1] = fmaf(f[e], f[e], ss[e & 1]);
     }
-    const float r = rsqrt_nr(affine2(warp_reduce(ss[0] + ss[1], [](float a, float c) { return a + c; }), p.s, p.t));
+    const float r = rsqrt_nr_tiny(affine2(warp_reduce(ss[0] + ss[1], [](float a, float c) { return a + c; }), p.s, p.t));
 #pragma unroll
     for (uint32_t k = 0; k < 4u; ++k) {
       if (l + 32u * k < words) {

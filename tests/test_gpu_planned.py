@@ -299,3 +299,17 @@ def test_reciprocal_roots_and_reciprocals_against_the_exact_ones(cols, dtype):
         p.output(p.rows(cases._SOFTMAX, p.input((rows, cols), dtype), rows, cols), (rows, cols))
         lp, (out,) = _execute(p, [x])
         assert lp.stat("replanned") == 1 and bool(((out.double() * cols - 1).abs() <= 4 * 2.0 ** -24).all())
+
+
+def test_norm_of_rows_whose_mean_square_is_denormal():
+    """Powers of two down to 2^-70, no epsilon: the mean square is exact down to 2^-146 and its root finite."""
+    import perf.cases as cases
+    rows, cols = 148 * 4, 64
+    x = torch.zeros((rows, cols), device="cuda")
+    x[:, 5] = 2.0 ** -(60 + torch.arange(rows, device="cuda") % 11)
+    p = cases._Assembler(148)
+    xi, g = p.input((rows, cols), "f32"), p.input((cols,), "f32")
+    p.output(progs.rms_norm(p, xi, g, rows, cols, "f32", eps=0.0), (rows, cols))
+    lp, (out,) = _execute(p, [x, torch.ones(cols, device="cuda")])
+    assert lp.stat("replanned") == 1
+    assert bool(((out[:, 5].double() - 8).abs() <= 8 * 4 * 2.0 ** -23).all())      # 2 ulp of the approximation, and the product
