@@ -491,6 +491,8 @@ def main():
             e2e = {"seconds": dt, "h2d": h2d, "d2h": d2h, "steps": n_e2e}
         if lp2 is not None:
             lp2.close()
+        build = importlib.import_module("pjrt-ocl_b200.build").variants()[lp.stat("kernel_build")][0]
+        st["kernel"] = f"b2_{build}" if build.startswith("plan") else f"b2_vm_{build}<512>"
         st["tensor_core_matmuls"] = [lp.stat("tensor_core_matmuls"), lp.stat("matmuls")]
         lp.close()
         st["phase_ns"] = phases
@@ -567,7 +569,7 @@ def main():
                     roofline={"bound": w["bound"], "achieved": achieved, "peak": peak,
                               "unit": "GB/s" if w["bound"] == "hbm" else "TFLOP/s",
                               "frac": achieved / peak, "traffic": w["traffic"], "peak_source": peak_src,
-                              "kernel": "b2_vm<512> (one launch per step)"},
+                              "kernel": f"{st['kernel']} (one launch per step)"},
                     cpu_baseline=cpu, device_ns_per_step=st["device_ns"], grid_barriers=st["barriers"],
                     phase_end_ns=st["phase_ns"], tensor_core_matmuls=st["tensor_core_matmuls"],
                     verified=verified, verified_what=st["verified_what"], stages_ms=st["stages"],
