@@ -161,7 +161,9 @@ uint64_t b2_loaded_launch_count(const b2_loaded *lp);
  * 17 full sums taken from the row op (softmax / layer norm) that wrote their input,
  * 18 grid barriers between such a row op and its sum that were dropped (they ordered nothing any more),
  * 19 decomposed RMS norms over bf16 rows (convert, square, row sum, scalar region, two broadcast multiplies,
- * convert) run as one row op, 20 barriers dropped because the phase they closed holds nothing after that.
+ * convert) run as one row op, 20 barriers dropped because the phase they closed holds nothing after that,
+ * 21 whether the program runs re-planned, and of the plan: 22 fused chains and row pipelines, 23 all-pairs ops, 24 tasks of
+ * the program that became part of a fused op, 25 phases.
  * Unknown `which` returns 0. */
 uint64_t b2_loaded_stat(const b2_loaded *lp, int which);
 /* Per-wait budget of device-side bounded waits, in nanoseconds (default 2e9). */

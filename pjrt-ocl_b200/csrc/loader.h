@@ -29,11 +29,11 @@ struct TmapSpec {
   int64_t strides[3];     // elements, of dims[1..]; must be positive multiples of 8
   uint32_t box[4];
   uint32_t desc_word;     // where the owning DMma / DFlash sits in the descriptor pool (to clear its tmap on failure)
-  uint32_t owner_is_flash;   // 0: two maps of a matmul; 1: three of an attention task; kTmapPlanned*: of a planned op
+  uint32_t owner_is_flash;   // 0: two maps of a matmul; 1: three of an attention task; kTmapPlanned2: two of a planned op
   bool valid;             // false: known at load to be indescribable (e.g. a batch-broadcast operand)
 };
 
-constexpr uint32_t kTmapPlanned2 = 2, kTmapPlanned3 = 3;   // ... in groups of two / three
+constexpr uint32_t kTmapPlanned2 = 2;   // ... two of a planned product
 
 struct DeviceTables {
   std::vector<DTask> tasks;

@@ -33,6 +33,16 @@ static_assert(kFuseData + 128u <= kLaneSmemBytes - kPlanStageBytes, "what the lo
 struct FuStep { uint32_t code, dt; float s, t; uint8_t *ptr; uint32_t reg, slot; };
 static_assert(sizeof(FuStep) == 32, "same size as on the wire");
 
+// Eight 16-bit values out of a 16-byte word.
+__device__ __forceinline__ void unpack8(const uint4 &u, uint32_t dt, float (&f)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = dt == kBF16 ? __uint_as_float(w[i] << 16) : f16_bits_to_f32(w[i] & 0xffffu);
+    f[2 * i + 1] = dt == kBF16 ? __uint_as_float(w[i] & 0xffff0000u) : f16_bits_to_f32(w[i] >> 16);
+  }
+}
+
 // 1 / x and 1 / sqrt(x) to about one unit in the last place, for normal x: the special-function unit's approximation and
 // one Newton step. Used where the correctly rounded forms would put a subroutine call (their slow path) into the step
 // loop, which makes the compiler keep a thread's elements where the call wants them and move them around every step.
@@ -315,7 +325,6 @@ static __device__ __noinline__ float fuse_rows_run(uint32_t tid, uint32_t nthr, 
         case kFuSubS: { const float v = st.reg ? S[1] : S[0]; B2_FU_ALL(X[g][e] = __fsub_rn(X[g][e], v)) break; }
         case kFuDivS: if constexpr (RARE) { const float v = st.reg ? S[1] : S[0]; B2_FU_ALL(X[g][e] = __fdiv_rn(X[g][e], v)) } break;
         case kFuAffine: { const float s = st.s, t = st.t; B2_FU_ALL(X[g][e] = affine2(X[g][e], s, t)) break; }
-        case kFuAffineY: { const float s = st.s, t = st.t; B2_FU_ALL(Y[g][e] = affine2(Y[g][e], s, t)) break; }
         case kFuGelu: B2_FU_ALL(X[g][e] = gelu_tanh(X[g][e])) break;
         case kFuGeluGrad: B2_FU_ALL(X[g][e] = gelu_grad(X[g][e], st.s)) break;
         case kFuGeluGradY: B2_FU_ALL(Y[g][e] = gelu_grad(Y[g][e], st.s)) break;

@@ -75,21 +75,11 @@ __device__ __forceinline__ void gemm_quant(float (&v)[32], uint32_t dt) {
     for (int j = 0; j < 32; ++j) v[j] = f16_bits_to_f32(f32_to_f16_bits(v[j]));
   }
 }
-// eight residual elements from memory (ragged edge, or f32) ...
+// Eight residual elements from memory (ragged edge, or f32); else they come out of a prefetched 16-byte word.
 __device__ __forceinline__ void gemm_res8(const uint8_t *row, uint32_t dt, uint32_t c, uint32_t left, float (&y)[8]) {
 #pragma unroll
   for (uint32_t k = 0; k < 8u; ++k) y[k] = k < left ? loadf(row, dt, static_cast<int64_t>(c) + k) : 0.0f;
 }
-// ... or out of a prefetched 16-byte word
-__device__ __forceinline__ void gemm_unpack8(const uint4 u, uint32_t dt, float (&y)[8]) {
-  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (dt == kBF16) { y[2 * k] = __uint_as_float(w[k] << 16); y[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u); }
-    else { y[2 * k] = f16_bits_to_f32(w[k] & 0xffffu); y[2 * k + 1] = f16_bits_to_f32(w[k] >> 16); }
-  }
-}
-
 __device__ __forceinline__ void gemm_epilogue(const GemmEpi &E, float (&v)[32], const uint8_t *res_row, const uint4 (&pre)[4], bool have_pre, uint32_t c,
                                               uint32_t left, bool row_ok, float &csum) {
   if (E.flags & kGeGelu) {
@@ -109,7 +99,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmEpi &E, float (&v)[32], 
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       float y[8];
-      if (have_pre) gemm_unpack8(pre[b], E.rdt, y);
+      if (have_pre) unpack8(pre[b], E.rdt, y);
       else if (row_ok) gemm_res8(res_row, E.rdt, c + 8u * b, left > 8u * b ? left - 8u * b : 0u, y);
       else {
 #pragma unroll

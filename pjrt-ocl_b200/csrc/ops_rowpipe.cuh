@@ -245,14 +245,6 @@ static __device__ __noinline__ void rms_rows(const Lane &L, const DPipe &p, uint
   uint4 *gs = reinterpret_cast<uint4 *>(L.smem + kFuseData);
   for (uint32_t i = L.tid; i < words; i += L.nthr) gs[i] = ldg_v4(gam + 16u * i);
   __syncthreads();
-  auto unpack = [](const uint4 &u, float (&f)[8]) {
-    const uint32_t q[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      f[2 * i] = DT == kBF16 ? __uint_as_float(q[i] << 16) : f16_bits_to_f32(q[i] & 0xffffu);
-      f[2 * i + 1] = DT == kBF16 ? __uint_as_float(q[i] & 0xffff0000u) : f16_bits_to_f32(q[i] >> 16);
-    }
-  };
   uint4 v[4], n[4];
   auto load = [&](uint32_t row) {
 #pragma unroll
@@ -268,7 +260,7 @@ static __device__ __noinline__ void rms_rows(const Lane &L, const DPipe &p, uint
     float ss[2] = {0.0f, 0.0f}, f[8], g[8];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      unpack(v[k], f);
+      unpack8(v[k], DT, f);
 #pragma unroll
       for (int e = 0; e < 8; ++e) ss[e & 1] = fmaf(f[e], f[e], ss[e & 1]);
     }
@@ -276,8 +268,8 @@ static __device__ __noinline__ void rms_rows(const Lane &L, const DPipe &p, uint
 #pragma unroll
     for (uint32_t k = 0; k < 4u; ++k) {
       if (l + 32u * k < words) {
-        unpack(v[k], f);
-        unpack(gs[l + 32u * k], g);
+        unpack8(v[k], DT, f);
+        unpack8(gs[l + 32u * k], DT, g);
         uint32_t o[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {

@@ -23,14 +23,6 @@ namespace b2 {
 constexpr uint32_t kSkWarps = 16, kSkRing = 12800;        // bytes of a warp's ring
 constexpr uint32_t kSkNormRing = 8192, kSkNormRows = 65536;   // with the normed rows kept whole beside the rings: 32 rows x 1024
 
-__device__ __forceinline__ void sk_unpack8(const uint4 &v, uint32_t dt, float (&f)[8]) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    f[2 * i] = dt == kBF16 ? __uint_as_float(w[i] << 16) : f16_bits_to_f32(w[i] & 0xffffu);
-    f[2 * i + 1] = dt == kBF16 ? __uint_as_float(w[i] & 0xffff0000u) : f16_bits_to_f32(w[i] >> 16);
-  }
-}
 // The lane's copy of the normed rows: blocks of 32 k, each rows of 64 bytes like a ring block's. A warp takes every 16th row, 32 lanes
 // x 8 elements at a time. Rows past M are zero.
 static __device__ __noinline__ void skinny_norm(const Lane &L, const DSgemm &g, uint32_t rows) {
@@ -49,7 +41,7 @@ static __device__ __noinline__ void skinny_norm(const Lane &L, const DSgemm &g, 
     }
 #pragma unroll
     for (uint32_t q = 0; q < 4u; ++q) {
-      sk_unpack8(v[q], dt, f);
+      unpack8(v[q], dt, f);
 #pragma unroll
       for (int e = 0; e < 8; ++e) ss = fmaf(f[e], f[e], ss);
     }
@@ -61,8 +53,8 @@ static __device__ __noinline__ void skinny_norm(const Lane &L, const DSgemm &g, 
       if (k >= K) break;
       float y[8];
       uint32_t o[4];
-      sk_unpack8(v[q], dt, f);
-      sk_unpack8(ldg_v4(gam + k * 2u), dt, y);
+      unpack8(v[q], dt, f);
+      unpack8(ldg_v4(gam + k * 2u), dt, y);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float lo = __fmul_rn(__fmul_rn(f[2 * e], rs), y[2 * e]), hi = __fmul_rn(__fmul_rn(f[2 * e + 1], rs), y[2 * e + 1]);

@@ -22,7 +22,7 @@ enum FuCode : uint32_t {
   kFuAdd, kFuMul, kFuSub, kFuRSub, kFuDiv, kFuRDiv, kFuMax, kFuMin,   // X = X op Y (R: Y op X)
   kFuAddS, kFuMulS, kFuSubS, kFuDivS,                                 // X = X op the row scalar `reg`
   kFuAffine, kFuGelu, kFuGeluGrad, kFuExp, kFuTanh, kFuNeg, kFuSqrt, kFuRsqrt, kFuLog, kFuAbs,   // on X
-  kFuAffineY, kFuGeluGradY,        // on Y
+  kFuGeluGradY,                    // on Y
   kFuRedSum, kFuRedSumSq, kFuRedMax,   // row reduction of X into row scalar `reg`
   kFuSAffine, kFuSRsqrt,           // on row scalar `reg`
   kFuLayerNorm, kFuSoftmax,        // whole-row normalisations of X (s = eps)

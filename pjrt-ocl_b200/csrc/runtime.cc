@@ -523,7 +523,7 @@ b2_status b2_program_load(b2_runtime *rt, b2_program *prog, b2_loaded **out, cha
   lp->tmap_off.assign(lp->tab.tmaps.size(), 0);
   for (size_t i = 0; i < lp->tab.tmaps.size();) {
     const uint32_t owner = lp->tab.tmaps[i].owner_is_flash;
-    const size_t group = owner == 1 || owner == b2::kTmapPlanned3 ? 3 : 2;   // Q K V, or A B
+    const size_t group = owner == 1 ? 3 : 2;   // Q K V, or A B
     bool ok = i + group <= lp->tab.tmaps.size();
     for (size_t j = i; ok && j < i + group; ++j) {
       const b2::TmapSpec &sp = lp->tab.tmaps[j];
