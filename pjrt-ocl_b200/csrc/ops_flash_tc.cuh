@@ -413,6 +413,7 @@ static __device__ __noinline__ bool flash_tc_tiles(const Lane &L, const DTask &t
   }
 
   // ---------------- teardown ----------------
+  if (w == 0 && lane == 0 && !*failed) tc_drain(S->kv_empty, kFaStages, kvpos, failed, budget);
   tc_fence_before_sync();
   __syncthreads();
   const bool gave_up = S->failed != 0u;

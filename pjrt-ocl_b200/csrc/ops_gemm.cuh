@@ -239,6 +239,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
           fetch(sa + kGemmBOff, tb, pr.bmn, pr.bn, c0, k0, &S->full[s]);
         }
       }
+      if (ok) tc_drain(S->empty, kGemmStages, it, failed, budget);
     }
   } else if (w == 1u) {
     // ---------------- issuer: the whole warp in step, one elected lane issuing ----------------

@@ -269,6 +269,7 @@ static __device__ __noinline__ bool mma_tc_tiles(const Lane &L, const DTask &t, 
           mbar_arrive_tx(&S->full[s], static_cast<uint32_t>(kTcABytes + 16384 * nt));
         }
       }
+      if (ok) tc_drain(S->empty, kTcStages, it, failed, budget);
     }
   } else if (w < 8) {
     // ---------------- producers: per-thread asynchronous copies ----------------
@@ -307,6 +308,7 @@ static __device__ __noinline__ bool mma_tc_tiles(const Lane &L, const DTask &t, 
       }
     }
     cp_async_wait_all();                          // nothing of this thread is still in flight
+    if (ok && L.tid == 0) tc_drain(S->empty, kTcStages, it, failed, budget);
   }
   // ---------------- MMA issue ----------------
   // With TMA producers (one thread) warp 1 is free to issue, so the accumulator is

@@ -40,5 +40,13 @@ __device__ __forceinline__ bool tc_wait_warp(uint64_t *bar, uint32_t parity, vol
   return __shfl_sync(0xffffffffu, ok, 0) != 0u;
 }
 
+// The thread that fills a ring of stages, at its end: waits until the products have read what it filled last (`it` stages so
+// far). Their commits arrive on the stages' empty barriers, which nobody else waits for: one still under way when the barriers
+// are invalidated, or when the CTA is gone, is a fault.
+__device__ __forceinline__ void tc_drain(uint64_t *empty, uint32_t stages, uint32_t it, volatile uint32_t *failed, unsigned long long budget_ns) {
+  for (uint32_t k = 0; k < stages; ++k, ++it)
+    if (!tc_wait(&empty[it % stages], ((it / stages) & 1u) ^ 1u, failed, budget_ns)) return;
+}
+
 }  // namespace b2
 #endif

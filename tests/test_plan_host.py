@@ -132,3 +132,16 @@ def test_products_beside_large_moves_get_their_lanes(plan):
     for t in moves:
         per = [hi - lo for _, lo, hi in t["cut"]]
         assert len(per) == 148 and max(per) - min(per) <= 1
+
+
+def test_tensor_core_ops_end_with_no_commit_under_way():
+    """Every op whose products free its stages by a commit waits for the last of them before its barriers go: an arrival on an
+    invalidated barrier, or in a CTA that has left, is a fault that a run shows once in many."""
+    n = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "ops_*.cuh"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        if "tc_commit(" not in text:
+            continue
+        n += 1
+        assert text.rindex("tc_drain(") < text.rindex("mbar_inval("), os.path.basename(path)
+    assert n == 3
