@@ -189,7 +189,7 @@ static __device__ __noinline__ bool flash_tc_tiles(const Lane &L, const DTask &t
         // S: A = Q (K-major), B = K block; O: A = P (K-major), B = V (d is the unit-stride "MN" dimension)
         const uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((k_mn ? 1u : 0u) << 16) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
         const uint32_t idesc_o = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 16) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
-        bool ok = tc_wait_warp(&S->q_full, qn & 1u, failed, budget);
+        bool ok = tc_wait_uniform(&S->q_full, qn & 1u, failed, budget);
         tc_fence_after_sync();
         // Descriptors of stage 0 / slot 0; the others differ in the 16-byte-unit address field only.
         const uint64_t dq0 = tc_desc(q_s, 16u, 1024u), dp0 = tc_desc(p_s, 16u, 1024u);
@@ -266,14 +266,10 @@ static __device__ __noinline__ bool flash_tc_tiles(const Lane &L, const DTask &t
           }
           nanosleep_ns(32);      // leave the issue slots to the softmax warps of this scheduler
           if ((++idle & 1023u) == 0u) {
-            uint32_t give_up = 0u;
-            if (lane == 0) {
-              if (*failed) give_up = 1u;
-              const unsigned long long now = globaltimer_ns();
-              if (idle == 1024u) t_idle = now;
-              else if (now - t_idle > budget) { *failed = 1u; give_up = 1u; }
-            }
-            if (__shfl_sync(0xffffffffu, give_up, 0)) { ok = false; break; }
+            // (every lane looks: the warp stays in step, see tc_wait_uniform)
+            const unsigned long long now = globaltimer_ns();
+            if (idle == 1024u) t_idle = now;
+            if (__any_sync(0xffffffffu, *failed != 0u || now - t_idle > budget)) { *failed = 1u; ok = false; break; }
           }
         }
       }

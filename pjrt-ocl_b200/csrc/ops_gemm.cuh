@@ -8,7 +8,8 @@
 //
 // Roles: warp 0 feeds the stages (3 x 64 KB: A 256 x 64 k, B 256 x 64 k, each as 64 x 64 TMA boxes of 8 KB in the
 // 128-byte swizzle, either operand k-contiguous or row / column-contiguous); warp 1 issues tcgen05.mma, the whole warp in
-// step and one elected lane issuing, so that descriptors stay in uniform registers; warps 4-15 drain and store.
+// step (its waits too: tc_wait_uniform) and one elected lane issuing, so that descriptors stay in uniform registers; warps
+// 4-15 drain and store.
 // Accumulator slots: a half tile takes slot (running number) % 2. A tile of one half thus runs under the previous one's
 // epilogue; a tile of two halves starts its first half's k blocks as soon as that slot is drained, as far ahead as
 // the stages reach, while the second slot drains.
@@ -192,7 +193,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
   GemmShared *S = reinterpret_cast<GemmShared *>(sm + kSmemRed);
   volatile uint32_t *failed = &S->failed;
   const uint32_t stage0 = (smem_addr(sm + kSmemSys) + 1023u) & ~1023u;
-  const uint32_t w = L.tid / kWarp, lane = L.tid % kWarp;
+  const uint32_t w = __shfl_sync(0xffffffffu, L.tid / kWarp, 0), lane = L.tid % kWarp;   // the warp index, provably uniform
   const unsigned long long budget = P.wait_budget_ns;
   if (L.tid == 0) {
     for (int s = 0; s < kGemmStages; ++s) { mbar_init(&S->full[s], 1u); mbar_init(&S->empty[s], 1u); }
@@ -200,6 +201,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
     S->failed = 0u;
     fence_mbar_init();
   }
+  __syncwarp();
   if (w == 2u) tmem_alloc(&S->tmem_base, 512u);
   fence_proxy_async_smem();   // what the entry before wrote here by ordinary stores, before asynchronous copies overwrite it
   tc_fence_before_sync();
@@ -246,6 +248,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
     uint32_t it = 0, n = 0;                         // stages consumed; accumulator slots taken
     bool ok = true;
     GemmTile q;
+    __syncwarp();
     const bool leader = elect_one_sync();
     for (uint32_t tile = slot; ok && gemm_tile(G, tile, q); tile += n_slots) {
       const DGemmProb &pr = G.prob[q.prob];
@@ -265,7 +268,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
         }
       };
       auto drained = [&](uint32_t num) {            // accumulator slot of running number `num` is free
-        const bool f = tc_wait_warp(&S->acc_empty[num & 1u], ((num >> 1) & 1u) ^ 1u, failed, budget);
+        const bool f = tc_wait_uniform(&S->acc_empty[num & 1u], ((num >> 1) & 1u) ^ 1u, failed, budget);
         tc_fence_after_sync();
         return f;
       };
@@ -276,7 +279,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
         const uint32_t ahead = min(nkb, static_cast<uint32_t>(kGemmStages));
         for (uint32_t i = 0; ok && i < ahead; ++i) {
           const uint32_t s = (it + i) % kGemmStages;
-          ok = tc_wait_warp(&S->full[s], ((it + i) / kGemmStages) & 1u, failed, budget);
+          ok = tc_wait_uniform(&S->full[s], ((it + i) / kGemmStages) & 1u, failed, budget);
           tc_fence_after_sync();
           if (ok) mma(s, 0u, i);
         }
@@ -292,7 +295,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
       }
       for (; ok && kb < nkb; ++kb, ++it) {
         const uint32_t s = it % kGemmStages;
-        ok = tc_wait_warp(&S->full[s], (it / kGemmStages) & 1u, failed, budget);
+        ok = tc_wait_uniform(&S->full[s], (it / kGemmStages) & 1u, failed, budget);
         tc_fence_after_sync();
         if (!ok) break;
         mma(s, 0u, kb);
@@ -373,6 +376,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
     while (globaltimer_ns() - t0 < 50000ull) nanosleep_ns(1000);
   }
   if (w == 2u) {
+    __syncwarp();
     tc_fence_after_sync();
     tmem_dealloc(tmem, 512u);
   }

@@ -40,6 +40,23 @@ __device__ __forceinline__ bool tc_wait_warp(uint64_t *bar, uint32_t parity, vol
   return __shfl_sync(0xffffffffu, ok, 0) != 0u;
 }
 
+// The same with every lane polling and the warp in step throughout: for a warp whose elected lane issues products and commits.
+// With lane 0 polling for the others a long wait (operands and code out of L2) now and then cost the warp a commit of its
+// elected lane, and the lane's stages stood still until the wait ran out: 33 x 4096 by 4096 x 16000 within 40 launches.
+__device__ __forceinline__ bool tc_wait_uniform(uint64_t *bar, uint32_t parity, volatile uint32_t *failed, unsigned long long budget_ns) {
+  if (__all_sync(0xffffffffu, mbar_try_wait_parity(bar, parity))) return true;
+  const unsigned long long t0 = globaltimer_ns();
+  for (;;) {
+    for (int i = 0; i < 32; ++i)
+      if (__all_sync(0xffffffffu, mbar_try_wait_parity(bar, parity))) return true;
+    const bool stop = *failed != 0u, late = globaltimer_ns() - t0 > budget_ns;
+    if (__any_sync(0xffffffffu, stop || late)) {
+      *failed = 1u;
+      return false;
+    }
+  }
+}
+
 // The thread that fills a ring of stages, at its end: waits until the products have read what it filled last (`it` stages so
 // far). Their commits arrive on the stages' empty barriers, which nobody else waits for: one still under way when the barriers
 // are invalidated, or when the CTA is gone, is a fault.

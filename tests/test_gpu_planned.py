@@ -313,3 +313,20 @@ def test_norm_of_rows_whose_mean_square_is_denormal():
     lp, (out,) = _execute(p, [x, torch.ones(cols, device="cuda")])
     assert lp.stat("replanned") == 1
     assert bool(((out[:, 5].double() - 8).abs() <= 8 * 4 * 2.0 ** -23).all())      # 2 ulp of the approximation, and the product
+
+
+@pytest.mark.parametrize("m, k, n, transposed", [(33, 4096, 16000, True), (33, 512, 11008, True), (100, 1024, 16000, False), (33, 64, 8192, True)])
+def test_products_of_one_tile_per_lane_with_cold_caches(m, k, n, transposed):
+    """A lane's last product ends the launch, and nothing of it may still be under way: many launches, code and operands out of L2."""
+    import perf.cases as cases
+    st = cases.prepare(dict(kind="dot", m=m, k=k, n=n, dtype="bf16", transposed=transposed), 3)
+    assert st["lp"].stat("replanned") == 1 and st["lp"].stat("tensor_core_matmuls") == 1
+    flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
+    a, w = (x.double() for x in st["args"])
+    want = a @ (w.T if transposed else w)
+    for i in range(40):
+        flush.fill_(i)
+        torch.cuda.synchronize()
+        (out,) = cases.run(st)
+        assert st["lp"].Status()["code"] == 0
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + k * 2.0 ** -24 * (a.abs() @ (w.T if transposed else w).abs())).all())
