@@ -220,6 +220,19 @@ void MatchPipe(const DFuStep *st, uint32_t n, bool whole_rows, bool one_row, DPi
   *out = p;
 }
 
+// Is a fused chain one tile op that is faster as it stood? A row norm alone whose rows the tile op stages by bulk copies, 4 groups of
+// two (ops_rows.cuh), past 2048 columns: softmax over 8192 x 4096 f32 64 us planned and 58 as scheduled, bf16 65 and 50, 4096 x 8192
+// bf16 71 and 44 (2048 columns: 38 and 42; rows it does not stage take it 750). A full sum alone, which it streams through a ring:
+// 8192 x 4096 bf16 42 and 34, f32 46 and 46, 3001 x 128 f32 16 and 13.
+bool TileOpFaster(const DFuse &f, const DFuStep *st, int phases) {
+  if (phases != 1) return false;
+  const uint64_t row = static_cast<uint64_t>(f.cols) * DtypeSize(st[0].dt);
+  const uint32_t only = f.pipe.flags & ~static_cast<uint32_t>(kRpQ);
+  if (only == (kRpOn | kRpLn) || only == (kRpOn | kRpSoftmax))
+    return f.cols > 2048 && f.cols % 4 == 0 && row % 16 == 0 && 9216 + 8 * ((row + 127) & ~127ull) <= kLaneSmemBytes;
+  return f.n_steps == 2 && st[1].code == kFuCarrySum && f.n_elems >= 65536;
+}
+
 // Is the view, read over the row-major flat index of a [n0, n1, n2] tensor, affine
 // in the three coordinates? The view's (collapsed) dims and [n0, n1, n2] are two
 // factorisations of the same index space; walk their common refinement from the
@@ -1333,7 +1346,9 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
         if (f->pipe.flags && 2u * pipe_shape(f->pipe.flags, static_cast<uint32_t>(DtypeSize(f->pipe.dt)), vec, f->cols, 512u, 512u).buf_bytes > kPlanStageBytes)
           std::memset(&f->pipe, 0, sizeof(f->pipe));
         f->flat = f->vec && f->cols % 4u == 0u && f->cols <= 4096u ? FlatOps(fs, static_cast<uint32_t>(x[2])) : 0u;
-        (f->pipe.flags || f->flat || x[7] > 1 ? out->planned_gain : out->planned_loss) += f->n_elems;
+        const bool slower = TileOpFaster(*f, fs, x[7]);
+        ((f->pipe.flags || f->flat || x[7] > 1) && !slower ? out->planned_gain : out->planned_loss) += f->n_elems;
+        if (slower && f->total) out->planned_loss += kPlanLossFree;        // (at every length)
         if (f->total) out->needs_scratch = true;
         d.desc = static_cast<uint32_t>(out->desc.size());
         if (d.desc % 2) { out->desc.push_back(0); ++d.desc; }              // 16-byte copies

@@ -82,7 +82,7 @@ bool BuildPlannedTables(const VmProgram &p, uint64_t arena_base, DeviceTables *o
 // replace, and so is a chain in the step interpreter that merges several phases of the schedule. One that merges none saves the
 // wire kernel's longer way to its first load (6 us of 18) and pays for it with every element: max((a + b) ^ c, d) over
 // 33.55 M + 1 i32 195 us planned, 145 as scheduled, a bf16 sum of two 164 and 86; even at about 3 M elements (4 M + 1: 33.7
-// and 34.3, 26.9 and 24.9).
+// and 34.3, 26.9 and 24.9). One that is a single tile op which is faster by itself counts the same (TileOpFaster in loader.cc).
 constexpr uint64_t kPlanLossFree = 3u << 20;
 inline bool PlanGains(const DeviceTables &t) { return t.planned_loss <= t.planned_gain + kPlanLossFree; }
 

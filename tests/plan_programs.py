@@ -116,3 +116,10 @@ def rms_norm(p, x, gain, rows, cols, dtype, eps):
     gf = p.chain((cases._CONVERT, (gain,), "f32"))
     p.phase()
     return p.chain((cases._MUL, (t, gf), "f32", 0, by_col), (cases._CONVERT, (-1,), dtype))
+
+
+def lone_norm(rows, cols, dtype, softmax):
+    p = cases._Assembler(148)
+    x = p.input((rows, cols), dtype)
+    p.output(p.rows(cases._SOFTMAX, x, rows, cols) if softmax else p.rows(cases._LAYERNORM, x, rows, cols, cases._bits(1e-5)), (rows, cols))
+    return p

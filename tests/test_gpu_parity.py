@@ -45,7 +45,7 @@ REPLANNED = {"c1_relu_matmul", "c2_chain_decomposed_small", "c2_chain_f32_small"
              "c5_decode_in_place_bf16_small", "c5_decode_in_place_f32_small", "dot_bf16", "dot_bf16_f32out", "dot_f16", "dot_f32",
              "dot_kat_2x2", "for_loop_cross_lane", "norms_recognized", "rmsnorm_rows_bf16", "rows_then_full_sum_bf16",
              "rows_then_full_sum_f32", "rows_then_full_sum_ragged", "ew_views_aligned_f32_bf16", "for_loop_carries",
-             "golden_layout_kat", "reduce_full_16bit_source"}
+             "golden_layout_kat"}
 
 
 @pytest.mark.parametrize("name", golden_names())

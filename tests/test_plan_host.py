@@ -145,3 +145,17 @@ def test_tensor_core_ops_end_with_no_commit_under_way():
         n += 1
         assert text.rindex("tc_drain(") < text.rindex("mbar_inval("), os.path.basename(path)
     assert n == 3
+
+
+@pytest.mark.parametrize("rows, cols, dtype, kept", [
+    (8192, 2048, "f32", True), (8192, 2052, "f32", False), (8192, 4096, "bf16", False), (8192, 4094, "f32", True), (4096, 6912, "f32", False),
+    (4096, 8192, "f32", True), (4096, 8192, "bf16", False), (2048, 13824, "bf16", False), (2048, 16384, "bf16", True), (64, 4096, "f32", True)])
+def test_lone_norms_and_sums_stay_where_the_tile_op_is_faster(plan, rows, cols, dtype, kept):
+    for softmax in (False, True):
+        assert plan(progs.lone_norm(rows, cols, dtype, softmax).blob())["gains"] == kept
+    assert plan(progs.stages(rows, cols, dtype, (), True).blob())["gains"] is False
+    assert plan(progs.stages(rows, cols, dtype, ("gelu",), True).blob())["gains"]
+
+
+def test_short_lone_sums_keep_their_plan(plan):
+    assert plan(progs.stages(64, 128, "f32", (), True).blob())["gains"]
