@@ -1030,8 +1030,14 @@ bool Planner::FuseGemm(int seed) {
   for (int64_t v : {lay.a_ld, lay.b_ld, lay.a_off, lay.b_off}) tensor = tensor && v <= 0x7fffffff;
   if (!tensor && !SgOperandsFit(p_, t)) return false;
   // Up to 32 rows: every lane a few columns (ops_skinny.cuh). Above that re-reading the rows for every lane's columns costs more
-  // than 128-row tiles leave idle (a 64-row training step: 132 us against 111).
-  const bool skinny = tensor && t.p0 <= 32 && !lay.amn && t.p2 % 8 == 0 && t.p1 >= 8 && (!lay.bmn || t.p1 % 8 == 0) &&
+  // than 128-row tiles leave idle (a 64-row training step: 132 us against 111). So does a second round of columns, where
+  // nothing of it is fetched under the first one's sums: 32 x 1024 by 1024 x 8192 33 us against 23 on the tensor-core tiles (29 as
+  // scheduled), 1 x 4096 by 4096 x 32000 147 against 82 (88). Few rows and a long K keep it a little further, with k contiguous to
+  // four rounds (1 x 4096, 16000 columns 61 against 70, 32000 94 and 82), else to two of up to 4 rows (8192 columns 53 and 59; a
+  // batch 1 step of width 2048 147 and 153).
+  const uint64_t rounds = (t.p1 + 32ull * L_ - 1) / (32ull * L_);
+  const bool few = rounds <= 1 || (lay.bmn ? rounds <= 2 && t.p0 <= 4 && t.p2 >= 2048 : rounds <= 4 && t.p0 <= 16 && t.p2 >= 4096);
+  const bool skinny = tensor && few && t.p0 <= 32 && !lay.amn && t.p2 % 8 == 0 && t.p1 >= 8 && (!lay.bmn || t.p1 % 8 == 0) &&
                       static_cast<uint64_t>(t.p1) * t.p2 < (1ull << 31) && SgOperandsFit(p_, t);
   // as many of the tasks that follow as the epilogue has room for: all that the chain takes, then ever fewer
   for (int limit = 1 << 30; limit >= 0;) {

@@ -83,6 +83,9 @@ def _case(kind, **kw):
     # few rows: one and two row blocks, column blocks of every width, K of less than a group per warp
     *(_case("dot", m=m, k=k, n=n, dtype=dt, transposed=t) for m, k, n, dt, t in
       [(1, 8, 8, "bf16", False), (16, 40, 72, "f16", True), (17, 1032, 1000, "bf16", False), (32, 512, 4096, "bf16", True), (32, 2048, 2408, "f16", False)]),
+    # ... by more columns than the lanes take in one round
+    *(_case("dot", m=m, k=k, n=n, dtype=dt, transposed=t) for m, k, n, dt, t in
+      [(1, 64, 4744, "bf16", False), (31, 72, 9480, "f16", True), (2, 4096, 9472, "bf16", False), (16, 4096, 9480, "bf16", True)]),
     # row pipelines and flat chains
     *(_case("norm_chain", rows=r, cols=n, dtype=dt) for r, n, dt in
       [(1, 128, "f32"), (149, 130, "bf16"), (64, 1023, "f16"), (300, 2048, "bf16"), (33, 4096, "f32")]),

@@ -159,3 +159,11 @@ def test_lone_norms_and_sums_stay_where_the_tile_op_is_faster(plan, rows, cols, 
 
 def test_short_lone_sums_keep_their_plan(plan):
     assert plan(progs.stages(64, 128, "f32", (), True).blob())["gains"]
+
+
+@pytest.mark.parametrize("m, k, n, transposed, op", [
+    (32, 1024, 4736, False, SKINNY), (32, 1024, 4744, False, GEMM), (32, 1024, 4744, True, GEMM), (1, 4096, 9472, False, SKINNY), (5, 4096, 9472, False, GEMM),
+    (1, 4096, 9480, False, GEMM), (16, 4096, 18944, True, SKINNY), (17, 4096, 9472, True, GEMM), (16, 4096, 18952, True, GEMM), (1, 2048, 9472, True, GEMM), (1, 2048, 9472, False, SKINNY), (1, 2040, 9472, False, GEMM)])
+def test_few_rows_by_many_columns(plan, m, k, n, transposed, op):
+    (t,) = plan(cases._BUILD["dot"](dict(m=m, k=k, n=n, dtype="bf16", transposed=transposed)).blob())["tasks"]
+    assert t["op"] == op
