@@ -66,7 +66,7 @@ WORKLOADS = {
     "c2_f32": _wl("c2_chain_f32", "eltwise HBM GB/s", "GB/s", 7 * N_C2 * 4 + 2 * 4096 * 4, 1e9, "hbm", "f32",
                   "config 2: LayerNorm -> tanh-GELU -> softmax -> full sum on f32 (8192,4096); "
                   "bytes = LayerNorm r+w, GELU r+w, softmax r+w, sum r, + gamma/beta",
-                  sample="c2_chain_f32_cpu_sample", sample_frac=512 / 8192, traffic=778.3e6,
+                  sample="c2_chain_f32_cpu_sample", sample_frac=512 / 8192, traffic=232.6e6,
                   sample_what="512 of the 8192 rows"),
     "c2_bf16": _wl("c2_chain_bf16", "eltwise HBM GB/s", "GB/s", 7 * N_C2 * 2 + 2 * 4096 * 2, 1e9, "hbm", "bf16",
                    "config 2 on bf16-storage copies of the same values",
@@ -77,7 +77,7 @@ WORKLOADS = {
     "dot_bf16_8192": _wl("dot_bf16_8192", "dot_general TFLOP/s", "TFLOP/s", 2 * 8192 ** 3, 1e12, "tensor", "bf16",
                          "one dot_general bf16 8192 x 8192 x 8192, f32 accumulate, bf16 result"),
     "dot_bf16_4096": _wl("dot_bf16_4096", "dot_general TFLOP/s", "TFLOP/s", 2 * 4096 ** 3, 1e12, "tensor", "bf16",
-                         "one dot_general bf16 4096 x 4096 x 4096", secondary=True, traffic=163.1e6),
+                         "one dot_general bf16 4096 x 4096 x 4096", secondary=True, traffic=99.8e6),
     "flash_bf16": _wl("flash_bf16_c5", "flash-attention TFLOP/s", "TFLOP/s", _C5_ATT_FLOPS, 1e12, "tensor", "bf16",
                       "config 5's attention alone: 128 heads x 2048 x 2048, head_dim 64, causal (flops count the "
                       "causal half)", secondary=True, traffic=150.6e6),
@@ -87,7 +87,7 @@ WORKLOADS = {
     "c5_block": _wl("c5_block_bf16", "transformer-block tokens/s per B200", "tokens/s", _C5_TOK, 1.0, "tensor", "bf16",
                     "config 5: pre-norm decoder block forward, batch 8 x seq 2048, d_model 1024, 16 x 64 heads, "
                     "causal flash attention, GELU FFN 4096, bf16",
-                    roof_alg=_C5_MM_FLOPS + _C5_ATT_FLOPS, plan="c5_block", traffic=1139.5e6,
+                    roof_alg=_C5_MM_FLOPS + _C5_ATT_FLOPS, plan="c5_block", traffic=902.6e6,
                     sample="c5_block_bf16_cpu_sample", sample_frac=512 / _C5_TOK,
                     sample_what="one sequence of 512 tokens through the same block (8 x 2048 in the workload)"),
     "c4_nbody": _wl("c4_nbody", "n-body pair interactions/s", "G interactions/s", 4096 * 4096 * 4 * 200, 1e9, "hbm",
@@ -111,7 +111,7 @@ WORKLOADS = {
                               "config 5 decode step, batch 32, KV cache 2048 + the new position: K/V written in place "
                               "(in/out buffers), K read through its view; bytes = weights + KV cache read once",
                               roof_alg=2 * (4 * 1024 * 1024 + 2 * 1024 * 4096) + 2 * 32 * 16 * 2049 * 64 * 2,
-                              plan="c5_decode_in_place", traffic=310.5e6),
+                              plan="c5_decode_in_place", traffic=317.2e6),
     "c5_decode": _wl("c5_decode_bf16", "transformer-block tokens/s per B200", "tokens/s", 32, 1.0, "hbm", "bf16",
                      "config 5 decode step: batch 32, KV cache 2048; bytes = weights + KV cache read once",
                      roof_alg=2 * (4 * 1024 * 1024 + 2 * 1024 * 4096) + 2 * 32 * 16 * 2048 * 64 * 2, plan="c5_decode"),
