@@ -91,15 +91,13 @@ WORKLOADS = {
                     sample="c5_block_bf16_cpu_sample", sample_frac=512 / _C5_TOK,
                     sample_what="one sequence of 512 tokens through the same block (8 x 2048 in the workload)"),
     "c4_nbody": _wl("c4_nbody", "n-body pair interactions/s", "G interactions/s", 4096 * 4096 * 4 * 200, 1e9, "hbm",
-                    "f32", "config 4: 4096 bodies, RK4, 200 steps in one FOR loop (one system per GPU), executed as "
-                    "the decomposed bytecode, whose (N,N,3) intermediates make it HBM-bound; bytes per step = the "
-                    "tile ops' inputs + outputs over the four acceleration evaluations, A = 201 MB (N,N,3) and "
-                    "B = 67 MB (N,N) tensors: 28 A + 16 B",
-                    roof_alg=(28 * 4096 * 4096 * 3 * 4 + 16 * 4096 * 4096 * 4) * 200, secondary=True, plan="c4",
+                    "f32", "config 4: 4096 bodies, RK4, 200 steps in one FOR loop (one system per GPU); bytes per "
+                    "step = arguments and results once (the all-pairs op makes no (N,N,3) tensors; it is bound by issue)",
+                    roof_alg=4 * 13 * 4096, secondary=True, plan="c4",
                     max_steps=3),
     "c4_nbody_2steps": _wl("c4_nbody_2steps", "n-body pair interactions/s", "G interactions/s", 4096 * 4096 * 4 * 2, 1e9, "hbm",
-                           "f32", "config 4 cut to 2 RK4 steps (46 grid barriers): the same phases as the 200-step launch, "
-                           "short enough to profile", roof_alg=(28 * 4096 * 4096 * 3 * 4 + 16 * 4096 * 4096 * 4) * 2,
+                           "f32", "config 4 cut to 2 RK4 steps: the same phases as the 200-step launch, "
+                           "short enough to profile", roof_alg=4 * 13 * 4096,
                            secondary=True),
     "c3_stage_gelu_grad": _wl("c3_stage_gelu_grad_f32", "eltwise HBM GB/s", "GB/s", 2 * N_C2 * 4, 1e9, "hbm", "f32",
                               "config 3 stage: the GELU-derivative MAP_REGION (14 micro-ops) over 8192 x 4096 f32",

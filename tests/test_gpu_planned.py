@@ -333,3 +333,28 @@ def test_products_of_one_tile_per_lane_with_cold_caches(m, k, n, transposed):
         (out,) = cases.run(st)
         assert st["lp"].Status()["code"] == 0
     assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + k * 2.0 ** -24 * (a.abs() @ (w.T if transposed else w).abs())).all())
+
+
+@pytest.mark.parametrize("m, heads", [(300, 0), (0, 4)])
+def test_arguments_and_results_at_other_addresses_every_call(m, heads):
+    """Operands that are arguments are fetched through tensor maps made anew when an address changes: calls that alternate between
+    two sets of buffers, with nothing in between, each see their own."""
+    import perf.cases as cases
+    c = dict(kind="dot", m=m, k=264, n=520, dtype="bf16", transposed=False) if m else dict(kind="block", batch=1, seq=130, heads=heads, dtype="bf16")
+    a, b = cases.prepare(c, 1), cases.prepare(c, 2)
+    want = []
+    for st in (a, b):
+        cases.run(st)
+        assert st["lp"].Status()["code"] == 0
+        want.append([o.clone() for o in st["outs"]])
+    lp, stream = a["lp"], a["stream"]
+    for _ in range(20):
+        for st in (a, b):
+            for o in st["outs"]:
+                o.zero_()
+        torch.cuda.synchronize()
+        for st in (a, b, a, b):
+            lp.ExecuteDeviceAsync(st["in_ptr"], st["out_ptr"], stream)
+        assert lp.Status()["code"] == 0
+        for st, w in zip((a, b), want):
+            assert all(torch.equal(o, x) for o, x in zip(st["outs"], w))
