@@ -1373,6 +1373,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
           DGemmProb &q = g->prob[k];
           q.M = w[0]; q.N = w[1]; q.K = w[2]; q.halves = w[3]; q.bn = w[4];
           q.amn = w[5]; q.bmn = w[6]; q.adt = w[7];
+          g->stage_bytes = std::max(g->stage_bytes, (128u * q.halves + q.bn) * 128u);
           q.first = g->tiles;
           q.tm = (q.M + 128u * q.halves - 1u) / (128u * q.halves);
           q.tn = (q.N + q.bn - 1u) / q.bn;
@@ -1382,6 +1383,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
           q.res = w[20] ? c.Ref(static_cast<uint32_t>(w[20] - 1)) : 0;
           q.out0 = w[21] ? c.Ref(static_cast<uint32_t>(w[21] - 1)) : 0; q.dt0 = w[22];
           q.out1 = w[23] ? c.Ref(static_cast<uint32_t>(w[23] - 1)) : 0; q.dt1 = w[24];
+          q.form = gemm_form_of(q.epi, q.N, q.out0 != 0, q.out1 != 0, q.dt0, q.dt1, q.qdt, q.rdt);
           q.tmap = static_cast<int32_t>(out->tmaps.size());
           for (int side = 0; side < 2; ++side) {
             TmapSpec sp;
@@ -1410,6 +1412,7 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
           out->mma_flops += 2ull * q.M * q.N * q.K;
           out->planned_gain += static_cast<uint64_t>(q.M) * q.N;
         }
+        g->stages = std::min(kGemmStagesMax, kGemmRing / g->stage_bytes);
         const size_t bytes = (offsetof(DGemm, prob) + g->n_prob * sizeof(DGemmProb) + 15) / 16 * 16;
         if (out->desc.size() % 2) out->desc.push_back(0);
         d.desc = static_cast<uint32_t>(out->desc.size());

@@ -6,8 +6,9 @@
 // a 128 x 256 tile took up to six per 512 tensor cycles. Here a stage is two boxes (32 KB each at most) and feeds 1024.
 // A 256 x 256 tile is two 128-row halves that share the B block and fill all of tensor memory.
 //
-// Roles: warp 0 feeds the stages (3 x 64 KB: A 256 x 64 k, B 256 x 64 k, each as 64 x 64 TMA boxes of 8 KB in the
-// 128-byte swizzle, either operand k-contiguous or row / column-contiguous); warp 1 issues tcgen05.mma, the whole warp in
+// Roles: warp 0 feeds the stages (64 k of A's rows and of B's columns, as 64 x 64 TMA boxes of 8 KB in the 128-byte swizzle, either
+// operand k-contiguous or row / column-contiguous; as many stages of the task's largest tile as the ring's 192 KB hold, 3 of 256 x
+// 256, 4 of 128 x 256, 8 of 128 x 64); warp 1 issues tcgen05.mma, the whole warp in
 // step (its waits too: tc_wait_uniform) and one elected lane issuing, so that descriptors stay in uniform registers; warps
 // 4-15 drain and store.
 // Accumulator slots: a half tile takes slot (running number) % 2. A tile of one half thus runs under the previous one's
@@ -26,14 +27,13 @@
 
 namespace b2 {
 
-constexpr int kGemmStages = 3;
-constexpr uint32_t kGemmStageBytes = 65536, kGemmBOff = 32768, kGemmBox = 8192;
+constexpr uint32_t kGemmBox = 8192;
 constexpr uint32_t kGemmEpiWarps = 12, kGemmEpiFirst = 4;
 constexpr uint32_t kGemmSlab = 32u * 64u;                  // staging of one epilogue warp: 32 rows x 64 bytes, 64-byte swizzle
 constexpr uint32_t kGemmGroup = 8;
 
 struct GemmShared {
-  uint64_t full[kGemmStages], empty[kGemmStages];
+  uint64_t full[kGemmStagesMax], empty[kGemmStagesMax];
   uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base, failed;
 };
@@ -186,17 +186,332 @@ __device__ __forceinline__ void gemm_store(uint8_t *dst, uint32_t dt, uint32_t N
     if (static_cast<uint32_t>(j) < left) storef(dst, dt, static_cast<int64_t>(rr) * N + c + j, v[j]);
 }
 
+// ---- the epilogue warps: warp w reads tensor-memory lanes 32 (w % 4) .. + 31; three warps share a quarter's 32-column chunks ----
+// Where a warp stands: its next tile, half tiles done, its share of the full sum.
+struct GemmAt { uint32_t tile, n; float csum; bool ok; };
+// What the warp works with.
+struct GemmWarp {
+  const KParams *P;
+  uint32_t tmem, n_slots, stg, quarter, third, lane;
+};
+// The task's descriptor and barriers, at fixed places of the lane's shared memory.
+__device__ __forceinline__ const DGemm &gemm_desc() { B2_DYN_SMEM(sm); return *reinterpret_cast<const DGemm *>(sm + kSmemDesc); }
+__device__ __forceinline__ GemmShared *gemm_shared() { B2_DYN_SMEM(sm); return reinterpret_cast<GemmShared *>(sm + kSmemRed); }
+// The accumulator slot of half tile `n` is full; the warp is done with it.
+__device__ __forceinline__ bool gemm_slot_full(const GemmWarp &W, uint32_t n) {
+  const bool f = tc_wait_warp(&gemm_shared()->acc_full[n & 1u], (n >> 1) & 1u, &gemm_shared()->failed, W.P->wait_budget_ns, 32u);
+  tc_fence_after_sync();
+  return f;
+}
+__device__ __forceinline__ void gemm_slot_done(const GemmWarp &W, uint32_t n) {
+  tc_fence_before_sync();
+  __syncwarp();
+  if (W.lane == 0u) mbar_arrive(&gemm_shared()->acc_empty[n & 1u]);
+}
+
+// Any epilogue, its steps looked at chunk by chunk; the warp's tiles from `at` on as long as they want this.
+static __device__ __noinline__ GemmAt gemm_form_any(GemmWarp W, GemmAt at) {
+  const DGemm &G = gemm_desc();
+  const KParams &P = *W.P;
+  const uint32_t lane = W.lane;
+  GemmTile q;
+  for (; at.ok && gemm_tile(G, at.tile, q) && G.prob[q.prob].form == kGfAny; at.tile += W.n_slots) {
+    const DGemmProb &pr = G.prob[q.prob];
+    GemmEpi E;
+    E.flags = pr.epi; E.qdt = pr.qdt; E.rdt = pr.rdt; E.s0 = pr.s0; E.s1 = pr.s1; E.gg = pr.gg;
+    E.res = (pr.epi & kGeRes) ? resolve(P, pr.res) : nullptr;
+    uint8_t *out0 = pr.out0 ? resolve(P, pr.out0) : nullptr, *out1 = pr.out1 ? resolve(P, pr.out1) : nullptr;
+    const uint32_t M = pr.M, N = pr.N;
+    const bool vec = (N & 7u) == 0u;                                    // 16-byte pieces of a row start on 16-byte boundaries
+    const bool pre_ok = E.res && E.rdt != kF32 && vec;       // residual by 16-byte words, a chunk ahead
+    for (uint32_t h = 0; h < q.halves; ++h, ++at.n) {
+      const uint32_t rf = q.r0 + 128u * h + 32u * W.quarter, r = rf + lane, acc = W.tmem + ((32u * W.quarter) << 16) + (at.n & 1u) * 256u;
+      const bool row_ok = r < M;
+      const uint8_t *res_row = E.res ? E.res + static_cast<size_t>(min(r, M - 1u)) * N * (E.rdt == kF32 ? 4u : 2u) : nullptr;
+      uint4 nxt[4];
+      auto prefetch = [&](uint32_t col) {
+        const uint32_t c = q.c0 + col;
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k)
+          nxt[k] = row_ok && c + 8u * k < N ? ldg_v4(res_row + static_cast<size_t>(c + 8u * k) * 2u) : make_uint4(0u, 0u, 0u, 0u);
+      };
+      if (pre_ok && 32u * W.third < q.n_inst) prefetch(32u * W.third);
+      if (!gemm_slot_full(W, at.n)) { at.ok = false; return at; }
+#pragma unroll 1
+      for (uint32_t col = 32u * W.third; col < q.n_inst; col += 96u) {
+        uint32_t raw[32];
+        __syncwarp();
+        tc_ld32(acc + col, raw);
+        uint4 cur[4];
+        if (pre_ok) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) cur[k] = nxt[k];
+          if (col + 96u < q.n_inst) prefetch(col + 96u);
+        }
+        tc_wait_ld();
+        const uint32_t c = q.c0 + col, left = c < N ? min(32u, N - c) : 0u;
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
+        if (E.flags & kGeQuant0) gemm_quant(v, E.qdt);
+        if (out0) gemm_store(out0, pr.dt0, N, rf, M, c, left, vec, W.stg, lane, v);
+        gemm_epilogue(E, v, res_row, cur, pre_ok, c, left, row_ok, at.csum);
+        if (out1) gemm_store(out1, pr.dt1, N, rf, M, c, left, vec, W.stg, lane, v);
+      }
+      gemm_slot_done(W, at.n);
+    }
+  }
+  return at;
+}
+
+// An epilogue whose steps are known when this is compiled: FL = its flags but for kGeQuant0, every value that is stored or
+// read 16-bit of one type (BF: bf16), rows whole 16-byte words. Such a form is a function of its own, entered once for all of the
+// warp's tiles in a row that want it, so that what a chunk needs stays in registers: the lane's shared memory leaves hardly any
+// L1, every use of a spilled value is a trip to L2, and the general form has its steps as branches and predicates. A 256 x 256
+// tile that only leaves as bf16 takes 7000 cycles here, 22000 in the general form (2 tiles of K = 64: 31 us, now 15.5); what is left
+// is mostly the SM's way to L2, 32 bytes a cycle. Rows of the residual come as the result goes: whole 64-byte row pieces through the
+// warp's slab, a chunk ahead. Tried: all of a tile's chunks held in registers first and stored when the slots are given back
+// (more code and registers, slower: 110 us against 107 for 16384 x 4096 by K = 1024); 32-byte stores from the rows as they come
+// (an SM then sends 17 bytes a cycle).
+template <bool BF>
+__device__ __forceinline__ uint32_t gemm_pack(float lo, float hi) { return BF ? cvt_bf16x2(hi, lo) : cvt_f16x2(hi, lo); }
+template <uint32_t FORM, uint32_t FL, bool BF>
+static __device__ __noinline__ GemmAt gemm_form(GemmWarp W, GemmAt at) {
+  constexpr uint32_t dt = BF ? static_cast<uint32_t>(kBF16) : static_cast<uint32_t>(kF16);
+  constexpr bool kRes = (FL & kGeRes) != 0u;
+  const DGemm &G = gemm_desc();
+  const uint32_t lane = W.lane, sw = (lane >> 1) & 3u, row = W.stg + lane * 64u, r8 = lane >> 2, ch = lane & 3u;
+  const uint32_t piece = W.stg + r8 * 64u + ((ch ^ ((r8 >> 1) & 3u)) << 4);          // + 512 p: row 8 p + r8
+  GemmTile q;
+  for (; gemm_tile(G, at.tile, q) && G.prob[q.prob].form == FORM; at.tile += W.n_slots) {
+    const DGemmProb &pr = G.prob[q.prob];
+    const uint32_t M = pr.M, N = pr.N;
+    const bool quant = (pr.epi & kGeQuant0) != 0u;
+    const float s0 = pr.s0, s1 = pr.s1, gg = pr.gg;
+    const uint8_t *res = kRes ? resolve(*W.P, pr.res) : nullptr;
+    uint8_t *out0 = FL == kGeGelu && pr.out0 ? resolve(*W.P, pr.out0) : nullptr, *out1 = resolve(*W.P, pr.out1);
+    for (uint32_t h = 0; h < q.halves; ++h, ++at.n) {
+      const uint32_t rf = q.r0 + 128u * h + 32u * W.quarter, acc = W.tmem + ((32u * W.quarter) << 16) + (at.n & 1u) * 256u;
+      const uint32_t rows = M > rf + r8 ? (M - rf - r8 + 7u) / 8u : 0u;               // of this thread's four row pieces
+      const size_t first = (static_cast<size_t>(rf + r8) * N + q.c0 + 8u * ch) * 2u, step = static_cast<size_t>(N) * 16u;
+      uint4 nxt[4] = {};
+      auto prefetch = [&](uint32_t col) {
+        const uint8_t *src = res + first + col * 2u;
+#pragma unroll
+        for (uint32_t p = 0; p < 4u; ++p)
+          nxt[p] = p < rows && q.c0 + col + 8u * ch < N ? ldg_v4(src + p * step) : make_uint4(0u, 0u, 0u, 0u);
+      };
+      auto leave = [&](uint8_t *out, uint32_t col) {             // the slab to memory
+        __syncwarp();
+        uint8_t *dst = out + first + col * 2u;
+        const uint32_t live = q.c0 + col + 8u * ch < N ? rows : 0u;
+#pragma unroll
+        for (uint32_t p = 0; p < 4u; ++p) {
+          const uint4 x = lds_v4(piece + 512u * p);
+          if (p < live) stg_v4(dst + p * step, x);
+        }
+        __syncwarp();
+      };
+      if (kRes && 32u * W.third < q.n_inst) prefetch(32u * W.third);
+      if (!gemm_slot_full(W, at.n)) { at.ok = false; return at; }
+      if (32u * W.third >= q.n_inst) gemm_slot_done(W, at.n);
+#pragma unroll 1
+      for (uint32_t col = 32u * W.third; col < q.n_inst; col += 96u) {
+        uint32_t raw[32];
+        __syncwarp();
+        tc_ld32(acc + col, raw);
+        if (kRes) {
+#pragma unroll
+          for (uint32_t p = 0; p < 4u; ++p) sts_v4(piece + 512u * p, nxt[p]);
+          if (col + 96u < q.n_inst) prefetch(col + 96u);
+          __syncwarp();
+        }
+        tc_wait_ld();
+        if (col + 96u >= q.n_inst) gemm_slot_done(W, at.n);      // its last columns are in registers
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
+        if (FL != 0u && quant) {                                 // (alone, the store rounds)
+          uint32_t w[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            w[j] = gemm_pack<BF>(v[2 * j], v[2 * j + 1]);
+            if (BF) { v[2 * j] = __uint_as_float(w[j] << 16); v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u); }
+            else { v[2 * j] = f16_bits_to_f32(w[j] & 0xffffu); v[2 * j + 1] = f16_bits_to_f32(w[j] >> 16); }
+          }
+          if constexpr (FL == kGeGelu) {
+            if (out0) {
+#pragma unroll
+              for (uint32_t k = 0; k < 4u; ++k) sts_v4(row + ((k ^ sw) << 4), make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]));
+              leave(out0, col);
+            }
+          }
+        }
+        float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k) {
+          float *x = &v[8 * k];
+          if constexpr ((FL & kGeGelu) != 0u) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] = gelu_tanh(x[e]);
+          }
+          if constexpr ((FL & kGeScale0) != 0u) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] = __fmul_rn(x[e], s0);
+          }
+          if constexpr (kRes) {
+            constexpr uint32_t op = FL & kGeResMask;
+            float y[8];
+            unpack8(lds_v4(row + ((k ^ sw) << 4)), dt, y);
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              x[e] = op == kGeResAdd ? __fadd_rn(x[e], y[e]) : op == kGeResSub ? __fsub_rn(x[e], y[e]) : op == kGeResRSub ? __fsub_rn(y[e], x[e])
+                   : __fmul_rn(x[e], gelu_grad(y[e], gg));
+          }
+          if constexpr ((FL & kGeCarrySq) != 0u) {
+            if (rf + lane < M && q.c0 + col + 8u * k < N) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) part[e & 3] = __fadd_rn(part[e & 3], __fmul_rn(x[e], x[e]));
+            }
+          }
+          if constexpr ((FL & kGeScale1) != 0u) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] = __fmul_rn(x[e], s1);
+          }
+          sts_v4(row + ((k ^ sw) << 4), make_uint4(gemm_pack<BF>(x[0], x[1]), gemm_pack<BF>(x[2], x[3]), gemm_pack<BF>(x[4], x[5]), gemm_pack<BF>(x[6], x[7])));
+        }
+        if constexpr ((FL & kGeCarrySq) != 0u) at.csum += (part[0] + part[1]) + (part[2] + part[3]);
+        leave(out1, col);
+      }
+    }
+  }
+  return at;
+}
+
+// ---- the warps that feed the tensor cores, each a function of its own: what they need per stage stays in registers ----
+struct GemmLane { const KParams *P; uint32_t stage0, tmem, slot, n_slots; };
+// One thread: fills the stages.
+static __device__ __noinline__ void gemm_produce(GemmLane X) {
+  const DGemm &G = gemm_desc();
+  GemmShared *S = gemm_shared();
+  volatile uint32_t *failed = &S->failed;
+  const unsigned long long budget = X.P->wait_budget_ns;
+  const uint32_t n_stages = G.stages, stage_bytes = G.stage_bytes;
+  fence_proxy_async_global();        // operands written by the previous phase's ordinary stores
+  uint32_t it = 0, s = 0, turn = 1u;         // stages filled; the next one, and the parity that it is empty with
+  bool ok = true;
+  GemmTile q;
+  for (uint32_t tile = X.slot; ok && gemm_tile(G, tile, q); tile += X.n_slots) {
+    const DGemmProb &pr = G.prob[q.prob];
+    const DTmap *ta = X.P->tmaps + pr.tmap, *tb = ta + 1;
+    const uint32_t nkb = (pr.K + 63u) / 64u, a_rows = 128u * pr.halves;
+    const uint32_t bytes = (a_rows + pr.bn) * 128u;
+    const int32_t r0 = static_cast<int32_t>(q.r0), c0 = static_cast<int32_t>(q.c0);
+    // An operand's part of a stage is one box; one whose rows are the unit-stride axis comes as 64-row blocks (a box over
+    // the blocks), or block by block where they do not divide the axis.
+    auto fetch = [&](uint32_t dst, const DTmap *tm, uint32_t mode, uint32_t rows, int32_t r, int32_t k0, uint64_t *bar) {
+      if (mode == kGmK) tma_load_3d(dst, tm, k0, r, 0, bar);
+      else if (mode == kGmMnBlocks) tma_load_3d(dst, tm, 0, k0, r / 64, bar);
+      else
+        for (uint32_t i = 0; i < rows / 64u; ++i) tma_load_3d(dst + i * kGemmBox, tm, r + static_cast<int32_t>(64u * i), k0, 0, bar);
+    };
+    for (uint32_t kb = 0; kb < nkb; ++kb, ++it) {
+      if (!tc_wait(&S->empty[s], turn, failed, budget)) { ok = false; break; }
+      mbar_arrive_tx(&S->full[s], bytes);
+      const uint32_t sa = X.stage0 + s * stage_bytes;
+      const int32_t k0 = static_cast<int32_t>(kb * 64u);
+      fetch(sa, ta, pr.amn, a_rows, r0, k0, &S->full[s]);
+      fetch(sa + a_rows * 128u, tb, pr.bmn, pr.bn, c0, k0, &S->full[s]);
+      if (++s == n_stages) { s = 0u; turn ^= 1u; }
+    }
+  }
+  if (ok) tc_drain(S->empty, n_stages, it, failed, budget);
+}
+// A whole warp in step, one elected lane issuing.
+static __device__ __noinline__ void gemm_issue(GemmLane X) {
+  const DGemm &G = gemm_desc();
+  GemmShared *S = gemm_shared();
+  volatile uint32_t *failed = &S->failed;
+  const unsigned long long budget = X.P->wait_budget_ns;
+  const uint32_t n_stages = G.stages, stage_bytes = G.stage_bytes, stage0 = X.stage0, tmem = X.tmem;
+  uint32_t s = 0, turn = 0, n = 0;                // the next stage, and the parity that it is full with; accumulator slots taken
+  bool ok = true;
+  GemmTile q;
+  __syncwarp();
+  const bool leader = elect_one_sync();
+  for (uint32_t tile = X.slot; ok && gemm_tile(G, tile, q); tile += X.n_slots) {
+    const DGemmProb &pr = G.prob[q.prob];
+    const uint32_t nkb = (pr.K + 63u) / 64u, fmt = pr.adt == kBF16 ? 1u : 0u;
+    const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((pr.amn ? 1u : 0u) << 15) | ((pr.bmn ? 1u : 0u) << 16) |
+                           ((q.n_inst >> 3) << 17) | ((128u >> 4) << 24);
+    const uint64_t a_base = pr.amn ? tc_desc(stage0, 8192u, 1024u) : tc_desc(stage0, 16u, 1024u);
+    const uint32_t b0 = stage0 + 16384u * pr.halves;
+    const uint64_t b_base = pr.bmn ? tc_desc(b0, 8192u, 1024u) : tc_desc(b0, 16u, 1024u);
+    const uint64_t adv_a = pr.amn ? (2048u >> 4) : (32u >> 4), adv_b = pr.bmn ? (2048u >> 4) : (32u >> 4);
+    const uint32_t slot0 = n & 1u, slot1 = (n + 1u) & 1u;
+    auto mma = [&](uint32_t s, uint32_t h, uint32_t kb) {
+      const uint64_t da = a_base + static_cast<uint64_t>((s * stage_bytes + h * 16384u) >> 4), db = b_base + static_cast<uint64_t>((s * stage_bytes) >> 4);
+      const uint32_t d = tmem + (h ? slot1 : slot0) * 256u;
+      if (leader) {
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; ++j) tc_mma_f16(d, da + j * adv_a, db + j * adv_b, idesc, (kb > 0u || j > 0u) ? 1u : 0u);
+      }
+    };
+    auto drained = [&](uint32_t num) {            // accumulator slot of running number `num` is free
+      const bool f = tc_wait_uniform(&S->acc_empty[num & 1u], ((num >> 1) & 1u) ^ 1u, failed, budget);
+      tc_fence_after_sync();
+      return f;
+    };
+    ok = drained(n);
+    auto landed = [&](uint32_t st, uint32_t parity) {
+      const bool f = tc_wait_uniform(&S->full[st], parity, failed, budget);
+      tc_fence_after_sync();
+      return f;
+    };
+    uint32_t kb = 0;
+    if (ok && q.halves == 2u) {
+      // the first half runs ahead over the stages that are there while the second slot drains
+      const uint32_t ahead = min(nkb, n_stages);
+      uint32_t s1 = s, turn1 = turn;
+      for (uint32_t i = 0; ok && i < ahead; ++i) {
+        ok = landed(s1, turn1);
+        if (ok) mma(s1, 0u, i);
+        if (++s1 == n_stages) { s1 = 0u; turn1 ^= 1u; }
+      }
+      if (ok && ahead == nkb && leader) tc_commit(&S->acc_full[slot0]);
+      ok = ok && drained(n + 1u);
+      for (uint32_t i = 0; ok && i < ahead; ++i) {
+        mma(s, 1u, i);
+        if (leader) tc_commit(&S->empty[s]);
+        if (++s == n_stages) { s = 0u; turn ^= 1u; }
+      }
+      kb = ahead;
+    }
+    for (; ok && kb < nkb; ++kb) {
+      ok = landed(s, turn);
+      if (!ok) break;
+      mma(s, 0u, kb);
+      if (kb + 1u == nkb && leader) tc_commit(&S->acc_full[slot0]);
+      if (q.halves == 2u) mma(s, 1u, kb);
+      if (leader) tc_commit(&S->empty[s]);
+      if (++s == n_stages) { s = 0u; turn ^= 1u; }
+    }
+    if (ok && q.halves == 2u && leader) tc_commit(&S->acc_full[slot1]);
+    n += q.halves;
+  }
+}
+
 static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, uint32_t slot, uint32_t n_slots) {
   const KParams &P = *L.P;
-  const DGemm &G = *reinterpret_cast<const DGemm *>(planned_desc(L, t));
+  planned_desc(L, t);
   B2_DYN_SMEM(sm);
-  GemmShared *S = reinterpret_cast<GemmShared *>(sm + kSmemRed);
-  volatile uint32_t *failed = &S->failed;
+  const DGemm &G = gemm_desc();
+  GemmShared *S = gemm_shared();
   const uint32_t stage0 = (smem_addr(sm + kSmemSys) + 1023u) & ~1023u;
   const uint32_t w = __shfl_sync(0xffffffffu, L.tid / kWarp, 0), lane = L.tid % kWarp;   // the warp index, provably uniform
-  const unsigned long long budget = P.wait_budget_ns;
+  const uint32_t n_stages = G.stages;
   if (L.tid == 0) {
-    for (int s = 0; s < kGemmStages; ++s) { mbar_init(&S->full[s], 1u); mbar_init(&S->empty[s], 1u); }
+    for (uint32_t s = 0; s < n_stages; ++s) { mbar_init(&S->full[s], 1u); mbar_init(&S->empty[s], 1u); }
     for (int b = 0; b < 2; ++b) { mbar_init(&S->acc_full[b], 1u); mbar_init(&S->acc_empty[b], kGemmEpiWarps); }
     S->failed = 0u;
     fence_mbar_init();
@@ -211,158 +526,30 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
   float csum = 0.0f;
 
   if (w == 0u) {
-    // ---------------- producer ----------------
-    if (lane == 0u) {
-      fence_proxy_async_global();        // operands written by the previous phase's ordinary stores
-      uint32_t it = 0;
-      bool ok = true;
-      GemmTile q;
-      for (uint32_t tile = slot; ok && gemm_tile(G, tile, q); tile += n_slots) {
-        const DGemmProb &pr = G.prob[q.prob];
-        const DTmap *ta = P.tmaps + pr.tmap, *tb = ta + 1;
-        const uint32_t nkb = (pr.K + 63u) / 64u, a_rows = 128u * pr.halves;
-        const uint32_t bytes = (a_rows + pr.bn) * 128u;
-        const int32_t r0 = static_cast<int32_t>(q.r0), c0 = static_cast<int32_t>(q.c0);
-        // An operand's part of a stage is one box; one whose rows are the unit-stride axis comes as 64-row blocks (a box over
-        // the blocks), or block by block where they do not divide the axis.
-        auto fetch = [&](uint32_t dst, const DTmap *tm, uint32_t mode, uint32_t rows, int32_t r, int32_t k0, uint64_t *bar) {
-          if (mode == kGmK) tma_load_3d(dst, tm, k0, r, 0, bar);
-          else if (mode == kGmMnBlocks) tma_load_3d(dst, tm, 0, k0, r / 64, bar);
-          else
-            for (uint32_t i = 0; i < rows / 64u; ++i) tma_load_3d(dst + i * kGemmBox, tm, r + static_cast<int32_t>(64u * i), k0, 0, bar);
-        };
-        for (uint32_t kb = 0; kb < nkb; ++kb, ++it) {
-          const uint32_t s = it % kGemmStages;
-          if (!tc_wait(&S->empty[s], ((it / kGemmStages) & 1u) ^ 1u, failed, budget)) { ok = false; break; }
-          mbar_arrive_tx(&S->full[s], bytes);
-          const uint32_t sa = stage0 + s * kGemmStageBytes;
-          const int32_t k0 = static_cast<int32_t>(kb * 64u);
-          fetch(sa, ta, pr.amn, a_rows, r0, k0, &S->full[s]);
-          fetch(sa + kGemmBOff, tb, pr.bmn, pr.bn, c0, k0, &S->full[s]);
-        }
-      }
-      if (ok) tc_drain(S->empty, kGemmStages, it, failed, budget);
-    }
+    if (lane == 0u) gemm_produce(GemmLane{&P, stage0, tmem, slot, n_slots});
   } else if (w == 1u) {
-    // ---------------- issuer: the whole warp in step, one elected lane issuing ----------------
-    uint32_t it = 0, n = 0;                         // stages consumed; accumulator slots taken
-    bool ok = true;
-    GemmTile q;
-    __syncwarp();
-    const bool leader = elect_one_sync();
-    for (uint32_t tile = slot; ok && gemm_tile(G, tile, q); tile += n_slots) {
-      const DGemmProb &pr = G.prob[q.prob];
-      const uint32_t nkb = (pr.K + 63u) / 64u, fmt = pr.adt == kBF16 ? 1u : 0u;
-      const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((pr.amn ? 1u : 0u) << 15) | ((pr.bmn ? 1u : 0u) << 16) |
-                             ((q.n_inst >> 3) << 17) | ((128u >> 4) << 24);
-      const uint64_t a_base = pr.amn ? tc_desc(stage0, 8192u, 1024u) : tc_desc(stage0, 16u, 1024u);
-      const uint64_t b_base = pr.bmn ? tc_desc(stage0 + kGemmBOff, 8192u, 1024u) : tc_desc(stage0 + kGemmBOff, 16u, 1024u);
-      const uint64_t adv_a = pr.amn ? (2048u >> 4) : (32u >> 4), adv_b = pr.bmn ? (2048u >> 4) : (32u >> 4);
-      const uint32_t slot0 = n & 1u, slot1 = (n + 1u) & 1u;
-      auto mma = [&](uint32_t s, uint32_t h, uint32_t kb) {
-        const uint64_t da = a_base + static_cast<uint64_t>((s * kGemmStageBytes + h * 16384u) >> 4), db = b_base + static_cast<uint64_t>((s * kGemmStageBytes) >> 4);
-        const uint32_t d = tmem + (h ? slot1 : slot0) * 256u;
-        if (leader) {
-#pragma unroll
-          for (uint32_t j = 0; j < 4u; ++j) tc_mma_f16(d, da + j * adv_a, db + j * adv_b, idesc, (kb > 0u || j > 0u) ? 1u : 0u);
-        }
-      };
-      auto drained = [&](uint32_t num) {            // accumulator slot of running number `num` is free
-        const bool f = tc_wait_uniform(&S->acc_empty[num & 1u], ((num >> 1) & 1u) ^ 1u, failed, budget);
-        tc_fence_after_sync();
-        return f;
-      };
-      ok = drained(n);
-      uint32_t kb = 0;
-      if (ok && q.halves == 2u) {
-        // the first half runs ahead over the stages that are there while the second slot drains
-        const uint32_t ahead = min(nkb, static_cast<uint32_t>(kGemmStages));
-        for (uint32_t i = 0; ok && i < ahead; ++i) {
-          const uint32_t s = (it + i) % kGemmStages;
-          ok = tc_wait_uniform(&S->full[s], ((it + i) / kGemmStages) & 1u, failed, budget);
-          tc_fence_after_sync();
-          if (ok) mma(s, 0u, i);
-        }
-        if (ok && ahead == nkb && leader) tc_commit(&S->acc_full[slot0]);
-        ok = ok && drained(n + 1u);
-        for (uint32_t i = 0; ok && i < ahead; ++i) {
-          const uint32_t s = (it + i) % kGemmStages;
-          mma(s, 1u, i);
-          if (leader) tc_commit(&S->empty[s]);
-        }
-        kb = ahead;
-        it += ahead;
-      }
-      for (; ok && kb < nkb; ++kb, ++it) {
-        const uint32_t s = it % kGemmStages;
-        ok = tc_wait_uniform(&S->full[s], (it / kGemmStages) & 1u, failed, budget);
-        tc_fence_after_sync();
-        if (!ok) break;
-        mma(s, 0u, kb);
-        if (kb + 1u == nkb && leader) tc_commit(&S->acc_full[slot0]);
-        if (q.halves == 2u) mma(s, 1u, kb);
-        if (leader) tc_commit(&S->empty[s]);
-      }
-      if (ok && q.halves == 2u && leader) tc_commit(&S->acc_full[slot1]);
-      n += q.halves;
-    }
+    gemm_issue(GemmLane{&P, stage0, tmem, slot, n_slots});
   } else if (w >= kGemmEpiFirst) {
-    // ---------------- epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. + 31; three warps share a quarter's column chunks ----------------
-    const uint32_t ew = w - kGemmEpiFirst, quarter = w & 3u, third = ew >> 2;
-    const uint32_t stg = stage0 + kGemmStages * kGemmStageBytes + ew * kGemmSlab;
-    uint32_t n = 0;
-    bool ok = true;
+    const uint32_t ew = w - kGemmEpiFirst;
+    const GemmWarp W = {&P, tmem, n_slots, stage0 + kGemmRing + ew * kGemmSlab, w & 3u, ew >> 2, lane};
+    GemmAt at = {slot, 0u, 0.0f, true};
     GemmTile q;
-    for (uint32_t tile = slot; ok && gemm_tile(G, tile, q); tile += n_slots) {
-      const DGemmProb &pr = G.prob[q.prob];
-      GemmEpi E;
-      E.flags = pr.epi; E.qdt = pr.qdt; E.rdt = pr.rdt; E.s0 = pr.s0; E.s1 = pr.s1; E.gg = pr.gg;
-      E.res = (pr.epi & kGeRes) ? resolve(P, pr.res) : nullptr;
-      uint8_t *out0 = pr.out0 ? resolve(P, pr.out0) : nullptr, *out1 = pr.out1 ? resolve(P, pr.out1) : nullptr;
-      const uint32_t M = pr.M, N = pr.N;
-      const bool vec = (N & 7u) == 0u;                                    // 16-byte pieces of a row start on 16-byte boundaries
-      const bool pre_ok = E.res && E.rdt != kF32 && vec;       // residual by 16-byte words, a chunk ahead
-      for (uint32_t h = 0; ok && h < q.halves; ++h, ++n) {
-        const uint32_t sl = n & 1u;
-        const uint32_t rf = q.r0 + 128u * h + 32u * quarter, r = rf + lane;
-        const bool row_ok = r < M;
-        const uint8_t *res_row = E.res ? E.res + static_cast<size_t>(min(r, M - 1u)) * N * (E.rdt == kF32 ? 4u : 2u) : nullptr;
-        uint4 nxt[4];
-        auto prefetch = [&](uint32_t col) {
-          const uint32_t c = q.c0 + col;
-#pragma unroll
-          for (uint32_t k = 0; k < 4u; ++k)
-            nxt[k] = row_ok && c + 8u * k < N ? ldg_v4(res_row + static_cast<size_t>(c + 8u * k) * 2u) : make_uint4(0u, 0u, 0u, 0u);
-        };
-        if (pre_ok && 32u * third < q.n_inst) prefetch(32u * third);
-        if (!tc_wait_warp(&S->acc_full[sl], (n >> 1) & 1u, failed, budget, 32u)) { ok = false; break; }
-        tc_fence_after_sync();
-#pragma unroll 1
-        for (uint32_t col = 32u * third; col < q.n_inst; col += 96u) {
-          uint32_t raw[32];
-          __syncwarp();
-          tc_ld32(tmem + ((32u * quarter) << 16) + sl * 256u + col, raw);
-          uint4 cur[4];
-          if (pre_ok) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) cur[k] = nxt[k];
-            if (col + 96u < q.n_inst) prefetch(col + 96u);
-          }
-          tc_wait_ld();
-          const uint32_t c = q.c0 + col, left = c < N ? min(32u, N - c) : 0u;
-          float v[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
-          if (E.flags & kGeQuant0) gemm_quant(v, E.qdt);
-          if (out0) gemm_store(out0, pr.dt0, N, rf, M, c, left, vec, stg, lane, v);
-          gemm_epilogue(E, v, res_row, cur, pre_ok, c, left, row_ok, csum);
-          if (out1) gemm_store(out1, pr.dt1, N, rf, M, c, left, vec, stg, lane, v);
-        }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0u) mbar_arrive(&S->acc_empty[sl]);          // the warp is done with the slot
+    while (at.ok && gemm_tile(G, at.tile, q)) {
+      switch (G.prob[q.prob].form) {
+#define B2_GEMM_FORM(f, flags)                                          \
+        case f: at = gemm_form<f, flags, true>(W, at); break;           \
+        case f + kGfF16: at = gemm_form<f + kGfF16, flags, false>(W, at); break;
+        B2_GEMM_FORM(kGfPlain, 0u)
+        B2_GEMM_FORM(kGfGelu, kGeGelu)
+        B2_GEMM_FORM(kGfAdd, kGeRes | kGeResAdd)
+        B2_GEMM_FORM(kGfGrad, kGeRes | kGeResGeluGrad)
+        B2_GEMM_FORM(kGfStep, kGeScale0 | kGeRes | kGeResRSub)
+        B2_GEMM_FORM(kGfLoss, kGeRes | kGeResSub | kGeCarrySq | kGeScale1)
+#undef B2_GEMM_FORM
+        default: at = gemm_form_any(W, at); break;
       }
     }
+    csum = at.csum;
   }
 
   // ---------------- teardown ----------------
@@ -383,7 +570,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
   if (L.tid == 0) {
     if (gave_up) set_status(P, kStTensorTimeout, L.lane, slot, kTopGemm);
     else {
-      for (int s = 0; s < kGemmStages; ++s) { mbar_inval(&S->full[s]); mbar_inval(&S->empty[s]); }
+      for (uint32_t s = 0; s < n_stages; ++s) { mbar_inval(&S->full[s]); mbar_inval(&S->empty[s]); }
       for (int b = 0; b < 2; ++b) { mbar_inval(&S->acc_full[b]); mbar_inval(&S->acc_empty[b]); }
     }
   }

@@ -104,6 +104,25 @@ enum GemmEpi_ : uint32_t {
   kGeCarrySq = 32u,        // add its square to the task's full sum
   kGeScale1 = 64u          // times s1
 };
+// Epilogues that have a form of their own on the device (ops_gemm.cuh): what the programs of the benchmark configurations leave
+// after a product. kGfF16 is added for f16.
+enum GemmForm : uint32_t { kGfAny = 0, kGfPlain, kGfGelu, kGfAdd, kGfGrad, kGfStep, kGfLoss, kGfF16 = 16 };
+// One 16-bit type throughout, whole 16-byte words, and a second result only where a form stores it.
+inline uint32_t gemm_form_of(uint32_t epi, uint32_t N, bool out0, bool out1, uint32_t dt0, uint32_t dt1, uint32_t qdt, uint32_t rdt) {
+  if (!out1 || (dt1 != kBF16 && dt1 != kF16) || N % 8u || ((epi & kGeQuant0) && qdt != dt1) || ((epi & kGeRes) && rdt != dt1)) return kGfAny;
+  uint32_t form;
+  switch (epi & ~kGeQuant0) {
+    case 0u: form = kGfPlain; break;                               // (the store rounds)
+    case kGeGelu: form = kGfGelu; break;
+    case kGeRes | kGeResAdd: form = kGfAdd; break;
+    case kGeRes | kGeResGeluGrad: form = kGfGrad; break;
+    case kGeScale0 | kGeRes | kGeResRSub: form = kGfStep; break;
+    case kGeRes | kGeResSub | kGeCarrySq | kGeScale1: form = kGfLoss; break;
+    default: return kGfAny;
+  }
+  if (out0 && !(form == kGfGelu && (epi & kGeQuant0) && dt0 == dt1)) return kGfAny;
+  return form + (dt1 == kF16 ? kGfF16 : 0u);
+}
 // unit stride along k; along the rows / columns (MN), fetched as a box of 64-row blocks or block by block
 enum GemmOperand : uint32_t { kGmK = 0, kGmMnBlocks = 1, kGmMnSingle = 2 };
 struct DGemmProb {
@@ -115,13 +134,17 @@ struct DGemmProb {
   int32_t tmap;
   uint32_t epi, qdt, rdt;
   float s0, s1, gg;                // gg: the GELU derivative's free constant
+  uint32_t form, pad;              // GemmForm
   BufRef res, out0, out1;
 };
 constexpr int kGemmMaxProbs = 6;
+constexpr uint32_t kGemmRing = 196608, kGemmStagesMax = 8;
 struct DGemm {
   uint32_t n_prob, tiles;
   BufRef total;
-  uint32_t n_owner_lanes, pad;
+  uint32_t n_owner_lanes;
+  uint32_t stages, stage_bytes;    // of the ring: one holds 64 k of the task's largest tile
+  uint32_t pad;
   DGemmProb prob[kGemmMaxProbs];
 };
 

@@ -69,6 +69,20 @@ __device__ __forceinline__ uint32_t cvt_bf16x2(float hi, float lo) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
+// Two f32 -> packed f16 (round to nearest even).
+__device__ __forceinline__ uint32_t cvt_f16x2(float hi, float lo) {
+  uint32_t r;
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ void sts_v4(uint32_t addr, uint4 w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
+}
+__device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
+  uint4 w;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(addr) : "memory");
+  return w;
+}
 // Accesses known to be in the global space (a pointer read back from a table is
 // generic to the compiler; these skip the address-space resolution).
 __device__ __forceinline__ uint4 ldg_v4(const void *p) {

@@ -51,6 +51,20 @@ def widened_product(M, K, N, dtype, what):
     return p
 
 
+def product_then(M, K, N, dtype, what, transposed=False):
+    """A 16-bit product and what follows it in its own type: nothing, a residual, GELU (with the product kept: "kept")."""
+    p = cases._Assembler(148)
+    a, w, x = p.input((M, K), dtype), p.input((N, K) if transposed else (K, N), dtype), p.input((M, N), dtype)
+    y = p.matmul(a, w, M, N, K, dtype, vb=p.view((K, N), (1, K)) if transposed else 0)
+    if what == "kept":
+        p.output(y, (M, N))
+    if what != "product":
+        p.phase()
+        y = p.chain((cases._ADD, (x, y), dtype)) if what == "residual" else p.chain((cases._GELU, (y,), dtype))
+    p.output(y, (M, N))
+    return p
+
+
 def attention_of_sums(H, T, C, hd, dtype, causal):
     """(q + q0) K^T, softmax, V: a program with an attention task that something around it lets the re-planner take."""
     p = cases._Assembler(148)

@@ -91,7 +91,7 @@ def _case(kind, **kw):
       [(1, 128, "f32"), (149, 130, "bf16"), (64, 1023, "f16"), (300, 2048, "bf16"), (33, 4096, "f32")]),
     _case("int_chain", rows=1, cols=131), _case("int_chain", rows=601, cols=1025), _case("int_chain", rows=2048, cols=512),
     # store epilogues: GELU, its derivative, the update step, the loss sum
-    _case("mlp", batch=72, d0=64, d1=136, d2=264, d3=72, dtype="bf16"), _case("mlp", batch=67, d0=33, d1=50, d2=21, d3=40, dtype="f32"),
+    _case("mlp", batch=72, d0=64, d1=136, d2=264, d3=72, dtype="bf16"), _case("mlp", batch=300, d0=64, d1=264, d2=520, d3=72, dtype="f16"), _case("mlp", batch=67, d0=33, d1=50, d2=21, d3=40, dtype="f32"),
     # attention between products; a decode step with its cache rows stored by the products
     _case("block", batch=2, seq=65, heads=4, dtype="bf16"), _case("block", batch=1, seq=77, heads=4, dtype="f32"), _case("block", batch=1, seq=300, heads=2, dtype="f32"),
     _case("decode", batch=1, cache=64, heads=4, dtype="bf16"), _case("decode", batch=17, cache=301, heads=8, dtype="f16"), _case("decode", batch=3, cache=70, heads=4, dtype="f32"),
@@ -195,6 +195,29 @@ def test_product_converted_after_a_16_bit_value(what, mnk):
         assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())      # half a step of bf16, and gelu_tanh's own error
     else:
         assert torch.equal(out, y.float())
+
+
+@pytest.mark.parametrize("what", ["product", "residual", "gelu", "kept"])
+@pytest.mark.parametrize("M, K, N, dtype, transposed", [
+    (33, 64, 8, "bf16", False), (128, 72, 104, "f16", False), (129, 200, 264, "bf16", False), (300, 1096, 520, "f16", True), (200, 64, 99, "bf16", True),
+    (2100, 136, 1032, "bf16", False), (9600, 64, 4104, "f16", False)])
+def test_store_epilogues_at_the_edges_of_tiles(what, M, K, N, dtype, transposed):
+    """One and two halves of 128 rows, column chunks that end inside a tile, rows that are no whole 16-byte words (the general
+    form), rings of 3 to 8 stages that wrap. Small integers: products and sums are exact in f32, so the roundings to the 16-bit type
+    are all there is and the bits are known (but for GELU: a step of the type, and gelu_tanh's own error)."""
+    dt = {"bf16": torch.bfloat16, "f16": torch.float16}[dtype]
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    a, w, x = (torch.randint(-3, 4, s, generator=gen, device="cuda").to(dt) for s in ((M, K), (N, K) if transposed else (K, N), (M, N)))
+    lp, outs = _execute(progs.product_then(M, K, N, dtype, what, transposed), [a, w, x])
+    assert lp.stat("tensor_core_matmuls") == 1
+    y = (a.float() @ (w.T if transposed else w).float()).to(dt)
+    if what in ("product", "kept"):
+        assert torch.equal(outs[0], y)
+    if what == "residual":
+        assert torch.equal(outs[0], (x.float() + y.float()).to(dt))
+    if what in ("gelu", "kept"):
+        want = _gelu(y.double())
+        assert bool(((outs[-1].double() - want).abs() <= (2.0 ** -8 if dtype == "bf16" else 2.0 ** -11) * want.abs() + 1e-6).all())
 
 
 @pytest.mark.parametrize("bodies", [258, 400])
