@@ -10,6 +10,9 @@
 // (smallest first; `all` holds every family a wire program can name; the ones after
 // it hold the re-planner's own ops and run on plan_kernel.cu). The build script
 // reads the same list to compile one object per entry.
+//
+// The builds for decode steps, f32 blocks and 16-bit blocks have the attention with only the products such a program runs: in the
+// one build with all of them a batch 32 decode step takes 158 us (148 in its own), an f32 block of width 512 320 us (291).
 #ifndef B2VM_VARIANTS_H_
 #define B2VM_VARIANTS_H_
 
@@ -26,6 +29,9 @@
   X(plan_pairs, b2::kFamFuse | b2::kFamPairs)            \
   X(plan_gemm, b2::kFamFuse | b2::kFamGemm | b2::kFamSkinny) \
   X(plan_sgemm, b2::kFamFuse | b2::kFamSgemm)            \
+  X(plan_decode, b2::kFamFuse | b2::kFamSkinny | b2::kFamFlash | b2::kFamMove) \
+  X(plan_f32, b2::kFamFuse | b2::kFamSgemm | b2::kFamFlash | b2::kFamMove) \
+  X(plan_block, b2::kFamFuse | b2::kFamGemm | b2::kFamFlash | b2::kFamMove) \
   X(plan_attn, b2::kFamFuse | b2::kFamGemm | b2::kFamSgemm | b2::kFamSkinny | b2::kFamFlash | b2::kFamMove)
 
 #endif
