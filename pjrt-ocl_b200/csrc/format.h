@@ -272,7 +272,7 @@ struct DFlash {        // loader-built
   uint32_t h0_size;
   uint32_t k_mn;                  // K: keys are the unit-stride dimension (the plain [H, hd, C] operand), else d is
   // Dynamic work distribution: when every lane that owns a share of the task enters it
-  // exactly once per phase, the lanes draw 256-row units from one counter pair in the
+  // exactly once per phase, the lanes draw 128-row tiles from one counter pair in the
   // program's scratch (heaviest first) instead of keeping their static ranges.
   uint32_t work_slot;             // index of the {next, done} pair in the scratch, or kNoWorkSlot
   uint32_t n_owner_lanes;

@@ -1171,9 +1171,9 @@ static bool BuildDeviceTablesFor(const VmProgram &p, uint64_t arena_base, Device
             f.k_mn = k_dmajor ? 0u : 1u;
             f.tmap = static_cast<int32_t>(out->tmaps.size());
             out->tmaps.push_back(fa_spec(d.ptr[1], oq, 64, static_cast<uint64_t>(T), sq[2], sq[1], sq[0], 128u));
-            if (k_dmajor) out->tmaps.push_back(fa_spec(d.ptr[2], ok_, 64, static_cast<uint64_t>(C), sk[3], sk[1], sk[0], 128u));
+            if (k_dmajor) out->tmaps.push_back(fa_spec(d.ptr[2], ok_, 64, static_cast<uint64_t>(C), sk[3], sk[1], sk[0], 64u));
             else out->tmaps.push_back(fa_spec(d.ptr[2], ok_, static_cast<uint64_t>(C), 64, sk[2], sk[1], sk[0], 64u));
-            out->tmaps.push_back(fa_spec(d.ptr[3], ov, 64, static_cast<uint64_t>(C), sv[2], sv[1], sv[0], 128u));
+            out->tmaps.push_back(fa_spec(d.ptr[3], ov, 64, static_cast<uint64_t>(C), sv[2], sv[1], sv[0], 64u));
             ++out->n_flash_tc;
           }
         }
