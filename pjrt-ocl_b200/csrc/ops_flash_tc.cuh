@@ -121,47 +121,56 @@ static __device__ __noinline__ void fa_feed(uint32_t s) {
       if (fa_tile(F, u).blocks > 0) return u;
     }
   };
-  uint32_t n = 0, b = 0;               // tiles and key blocks so far
-  bool ok = true;
-  uint32_t u = next();
-  for (;; ++n) {
+  struct Place { int32_t m0, h0, h1, blocks; };
+  auto place = [&](uint32_t u) {
+    const FaTile t = fa_tile(F, u);
+    const int32_t h1 = t.g / static_cast<int32_t>(F.h0_size);
+    return Place{t.m0, t.g - h1 * static_cast<int32_t>(F.h0_size), h1, t.blocks};
+  };
+  auto load_q = [&](const Place &t) {
+    if (leader) {
+      mbar_arrive_tx(&S->q_full[s], kFaQ);
+      tma_load_4d(q_s, tm, 0, t.m0, t.h0, t.h1, &S->q_full[s]);                        // rows past T arrive as zeros
+    }
+  };
+  // block j of the tile, number blk of all
+  auto load_k = [&](const Place &t, int32_t j, uint32_t blk) {
+    const uint32_t st = blk % kFaStages, dst = k_s + st * kFaKv;
+    if (leader && j < t.blocks) {
+      mbar_arrive_tx(&S->k_full[s][st], kFaKv);
+      if (k_mn) tma_load_4d(dst, tm + 1, j * 64, 0, t.h0, t.h1, &S->k_full[s][st]);    // K as [d][keys]
+      else tma_load_4d(dst, tm + 1, 0, j * 64, t.h0, t.h1, &S->k_full[s][st]);
+    }
+  };
+  auto load_v = [&](const Place &t, int32_t j, uint32_t blk) {
+    const uint32_t st = blk % kFaStages;
+    if (leader && j < t.blocks) {
+      mbar_arrive_tx(&S->v_full[s][st], kFaKv);
+      tma_load_4d(v_s + st * kFaKv, tm + 2, 0, j * 64, t.h0, t.h1, &S->v_full[s][st]);
+    }
+  };
+  auto post = [&](uint32_t u, uint32_t n) {
     if (leader) {
       S->tile[s][n & 1u] = u;
       mbar_arrive(&S->t_full[s]);
     }
     __syncwarp();
-    if (u == kFaNone) break;
-    const FaTile t = fa_tile(F, u);
-    const int32_t h1 = t.g / static_cast<int32_t>(F.h0_size), h0 = t.g - h1 * static_cast<int32_t>(F.h0_size);
-    auto load_k = [&](int32_t j, uint32_t blk) {
-      const uint32_t st = blk % kFaStages, dst = k_s + st * kFaKv;
-      if (leader) {
-        mbar_arrive_tx(&S->k_full[s][st], kFaKv);
-        if (k_mn) tma_load_4d(dst, tm + 1, j * 64, 0, h0, h1, &S->k_full[s][st]);      // K as [d][keys]
-        else tma_load_4d(dst, tm + 1, 0, j * 64, h0, h1, &S->k_full[s][st]);
-      }
-    };
-    auto load_v = [&](int32_t j, uint32_t blk) {
-      const uint32_t st = blk % kFaStages;
-      if (leader) {
-        mbar_arrive_tx(&S->v_full[s][st], kFaKv);
-        tma_load_4d(v_s + st * kFaKv, tm + 2, 0, j * 64, h0, h1, &S->v_full[s][st]);
-      }
-    };
-    // The tile before is through: its last P was seen full, so all its scores and all but its last product are done (Q and three
-    // stages of K are free, two of V).
-    if (leader) {
-      mbar_arrive_tx(&S->q_full[s], kFaQ);
-      tma_load_4d(q_s, tm, 0, t.m0, h0, h1, &S->q_full[s]);                            // rows past T arrive as zeros
-    }
-    for (int32_t j = 0; j < min(3, t.blocks); ++j) load_k(j, b + static_cast<uint32_t>(j));
-    for (int32_t j = 0; j < min(2, t.blocks); ++j) load_v(j, b + static_cast<uint32_t>(j));
+  };
+  uint32_t n = 0, b = 0;               // tiles and key blocks so far
+  bool ok = true;
+  uint32_t u = next();
+  post(u, n);
+  if (u == kFaNone) return;
+  Place t = place(u);
+  load_q(t);
+  for (uint32_t j = 0; j < kFaStages; ++j) { load_k(t, static_cast<int32_t>(j), j); if (j < 2u) load_v(t, static_cast<int32_t>(j), j); }
+  for (;;) {
     u = next();                        // (its atomic under the loads' flight)
     ok = tc_wait_uniform(&S->q_full[s], n & 1u, failed, budget);
     // O (+)= P V of block `blk`, number j of the tile
     auto product = [&](int32_t j, uint32_t blk) {
       const uint32_t st = blk % kFaStages;
-      ok = tc_wait_uniform(&S->v_full[s][st], (blk / kFaStages) & 1u, failed, budget) && tc_wait_uniform(&S->p_full[s], blk & 1u, failed, budget);
+      ok = ok && tc_wait_uniform(&S->v_full[s][st], (blk / kFaStages) & 1u, failed, budget) && tc_wait_uniform(&S->p_full[s], blk & 1u, failed, budget);
       if (!ok) return;
       tc_fence_after_sync();
       const uint64_t db = dv + ((st * kFaKv) >> 4);
@@ -172,7 +181,7 @@ static __device__ __noinline__ void fa_feed(uint32_t s) {
       }
       __syncwarp();
       // P(j) is full: the softmax saw the product before this one done
-      if (j + 2 < t.blocks) load_v(j + 2, blk + 2u);
+      load_v(t, j + 2, blk + 2u);
     };
     for (int32_t j = 0; ok && j < t.blocks; ++j, ++b) {
       const uint32_t st = b % kFaStages;
@@ -187,13 +196,25 @@ static __device__ __noinline__ void fa_feed(uint32_t s) {
       }
       __syncwarp();
       if (j > 0) {
-        // the scores before have been read, so their product is done
-        if (j + 2 < t.blocks) load_k(j + 2, b + 2u);
+        load_k(t, j + 2, b + 2u);      // the scores before have been read, so their product is done
         product(j - 1, b - 1u);
       }
     }
-    if (ok) product(t.blocks - 1, b - 1u);
-    if (!ok) break;
+    // The last scores are read: Q and all stages of K are free for the next tile, V's but for the last two blocks'.
+    ok = ok && tc_wait_uniform(&S->s_free[s], (b - 1u) & 1u, failed, budget);
+    if (!ok) return;
+    post(u, ++n);
+    Place t2 = t;
+    if (u != kFaNone) {
+      t2 = place(u);
+      load_q(t2);
+      for (uint32_t j = 0; j < kFaStages; ++j) load_k(t2, static_cast<int32_t>(j), b + j);
+      load_v(t2, 0, b);
+    }
+    product(t.blocks - 1, b - 1u);
+    if (!ok || u == kFaNone) return;
+    load_v(t2, 1, b + 1u);
+    t = t2;
   }
 }
 
@@ -210,7 +231,7 @@ static __device__ __noinline__ void fa_rows(uint32_t s, uint32_t q4) {
   const unsigned long long sl2_2 = pack_f32x2(sl2, sl2);
   uint32_t n = 0, b = 0;
   for (;; ++n) {
-    if (!tc_wait_warp(&S->t_full[s], n & 1u, failed, budget)) return;
+    if (!tc_wait_uniform(&S->t_full[s], n & 1u, failed, budget)) return;
     const uint32_t u = *reinterpret_cast<volatile uint32_t *>(&S->tile[s][n & 1u]);
     if (u == kFaNone) return;
     const FaTile t = fa_tile(F, u);
@@ -219,7 +240,7 @@ static __device__ __noinline__ void fa_rows(uint32_t s, uint32_t q4) {
     float m_used = -INFINITY, l_run = 0.0f;
 #pragma unroll 1
     for (int32_t j = 0; j < t.blocks; ++j, ++b) {
-      if (!tc_wait_warp(&S->s_full[s], b & 1u, failed, budget)) return;
+      if (!tc_wait_uniform(&S->s_full[s], b & 1u, failed, budget)) return;
       tc_fence_after_sync();
       uint32_t lo[32], hi[32];
       __syncwarp();
@@ -239,16 +260,17 @@ static __device__ __noinline__ void fa_rows(uint32_t s, uint32_t q4) {
       }
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};     // four independent chains
 #pragma unroll
-      for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(fmaxf(mx4[i & 3], __uint_as_float(lo[i])), __uint_as_float(hi[i]));
+      for (int i = 0; i < 32; ++i) mx4[i & 3] = max3(mx4[i & 3], __uint_as_float(lo[i]), __uint_as_float(hi[i]));
       // sl2 > 0 for every softmax scale in use; a non-positive scale takes the CUDA-core path
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sl2;
       // the maximum in use moves only when the row's true maximum outgrew it by 2^8
       const bool grow = mx > m_used + kFaRescale;
-      bool waited = j == 0;                                // (at a tile's start the product before was waited for, for the result)
+      // Is P free, the product before done? (At a tile's start it was waited for, for the result.) Looked at before the exponentials.
+      bool waited = j == 0 || __all_sync(0xffffffffu, mbar_test_wait_parity(&S->pv_done[s], (b - 1u) & 1u));
       if (__any_sync(0xffffffffu, grow)) {
         const float alpha = !grow ? 1.0f : (m_used == -INFINITY ? 0.0f : fast_ex2(m_used - mx));
         if (j > 0) {
-          if (!tc_wait_warp(&S->pv_done[s], (b - 1u) & 1u, failed, budget)) return;
+          if (!waited && !tc_wait_uniform(&S->pv_done[s], (b - 1u) & 1u, failed, budget)) return;
           tc_fence_after_sync();
           waited = true;
 #pragma unroll 1
@@ -284,7 +306,7 @@ static __device__ __noinline__ void fa_rows(uint32_t s, uint32_t q4) {
       unpack_f32x2(add_f32x2(sum[0], sum[1]), a0, a1);
       l_run += a0 + a1;
       // P's columns are free when the product before has read them
-      if (!waited && !tc_wait_warp(&S->pv_done[s], (b - 1u) & 1u, failed, budget)) return;
+      if (!waited && !tc_wait_uniform(&S->pv_done[s], (b - 1u) & 1u, failed, budget)) return;
       tc_fence_after_sync();
       __syncwarp();
       tc_st32(p_addr, pk);
@@ -294,7 +316,7 @@ static __device__ __noinline__ void fa_rows(uint32_t s, uint32_t q4) {
       if (lane == 0u) mbar_arrive(&S->p_full[s]);
     }
     // ---- output: O / l ----
-    if (!tc_wait_warp(&S->pv_done[s], (b - 1u) & 1u, failed, budget)) return;
+    if (!tc_wait_uniform(&S->pv_done[s], (b - 1u) & 1u, failed, budget)) return;
     tc_fence_after_sync();
     const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
 #pragma unroll 1

@@ -63,6 +63,12 @@ __device__ __forceinline__ float fast_rcp(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// The largest of three (a NaN loses).
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 // Two f32 -> packed bf16 (round to nearest even; NaN becomes the canonical 0x7fff).
 __device__ __forceinline__ uint32_t cvt_bf16x2(float hi, float lo) {
   uint32_t r;
