@@ -61,7 +61,7 @@ struct FaTask {
   uint8_t *out;
   unsigned long long budget;
   int32_t H, T, C, per_head;                   // tiles of 128 rows per head
-  uint32_t first, stop;                        // static: the lane's tiles
+  uint32_t first, stop;                        // static: the lane's tiles. dynamic: the lane, tiles that slots take first (or 0)
   uint32_t h0_size, causal, k_mn, adt, dt, base;
   float sl2;
 };
@@ -101,14 +101,20 @@ static __device__ __noinline__ void fa_feed(uint32_t s) {
   fence_proxy_async_global();          // operands written by the previous phase's ordinary stores
   __syncwarp();
   const bool leader = elect_one_sync();
-  uint32_t u_next = F.first + s;
+  uint32_t u_next = F.first + s;                                        // static
+  uint32_t first_draw = F.stop ? F.first + s * (F.stop / kFaSlots) : kFaNone;      // dynamic
   auto next = [&]() -> uint32_t {      // tiles that see no key have no result
     for (;;) {
       uint32_t u;
       if (F.work) {
-        uint32_t tk = 0;
-        if (lane == 0u) tk = atomicAdd(F.work, 1u);
-        tk = __shfl_sync(0xffffffffu, tk, 0);
+        // A slot's first tile is its own, so that few tiles go to one slot of each lane (all three of the lanes that come first drew
+        // them: 252 tiles of up to 777 keys 32 us, 25 so); the counter gives out what is left.
+        uint32_t tk = first_draw;
+        if (tk == kFaNone) {
+          if (lane == 0u) tk = atomicAdd(F.work, 1u);
+          tk = __shfl_sync(0xffffffffu, tk, 0) + F.stop;
+        }
+        first_draw = kFaNone;
         if (tk >= static_cast<uint32_t>(F.H) * static_cast<uint32_t>(F.per_head)) return kFaNone;
         // heaviest first: with a causal mask the last rows of a head see the most keys
         const uint32_t lvl = tk / static_cast<uint32_t>(F.H), g = tk - lvl * static_cast<uint32_t>(F.H);
@@ -212,7 +218,12 @@ static __device__ __noinline__ void fa_feed(uint32_t s) {
       load_v(t2, 0, b);
     }
     product(t.blocks - 1, b - 1u);
-    if (!ok || u == kFaNone) return;
+    if (!ok) return;
+    if (u == kFaNone) {
+      if (lane == 0u) tc_drain(&S->pv_done[s], 1u, b, failed, budget);
+      __syncwarp();
+      return;
+    }
     load_v(t2, 1, b + 1u);
     t = t2;
   }
@@ -265,12 +276,11 @@ static __device__ __noinline__ void fa_rows(uint32_t s, uint32_t q4) {
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sl2;
       // the maximum in use moves only when the row's true maximum outgrew it by 2^8
       const bool grow = mx > m_used + kFaRescale;
-      // Is P free, the product before done? (At a tile's start it was waited for, for the result.) Looked at before the exponentials.
-      bool waited = j == 0 || __all_sync(0xffffffffu, mbar_test_wait_parity(&S->pv_done[s], (b - 1u) & 1u));
+      bool waited = j == 0;                                // (at a tile's start the product before was waited for, for the result)
       if (__any_sync(0xffffffffu, grow)) {
         const float alpha = !grow ? 1.0f : (m_used == -INFINITY ? 0.0f : fast_ex2(m_used - mx));
         if (j > 0) {
-          if (!waited && !tc_wait_uniform(&S->pv_done[s], (b - 1u) & 1u, failed, budget)) return;
+          if (!tc_wait_uniform(&S->pv_done[s], (b - 1u) & 1u, failed, budget)) return;
           tc_fence_after_sync();
           waited = true;
 #pragma unroll 1
@@ -371,8 +381,9 @@ static __device__ __noinline__ bool flash_tc_tiles(const Lane &L, const DTask &t
     F->out = out;
     F->budget = P.wait_budget_ns;
     F->H = x[0]; F->T = x[1]; F->C = x[2]; F->per_head = static_cast<int32_t>(per_head);
-    F->first = dynamic ? 0u : tile_at_or_after(static_cast<int64_t>(tile_lo));
-    F->stop = dynamic ? 0u : tile_at_or_after(rows_end);
+    const bool all_lanes = df.n_owner_lanes == P.n_lanes;             // (a lane's number is its number among the owners)
+    F->first = dynamic ? L.lane : tile_at_or_after(static_cast<int64_t>(tile_lo));
+    F->stop = dynamic ? (all_lanes ? kFaSlots * P.n_lanes : 0u) : tile_at_or_after(rows_end);
     F->h0_size = df.h0_size; F->causal = x[5] != 0 ? 1u : 0u; F->k_mn = df.k_mn; F->adt = t.adt; F->dt = t.dt;
     F->base = (smem_addr(sm + kSmemSys) + 1023u) & ~1023u;
     F->sl2 = __int_as_float(x[4]) * 1.4426950408889634f;   // scores in the log2 domain
@@ -393,7 +404,7 @@ static __device__ __noinline__ bool flash_tc_tiles(const Lane &L, const DTask &t
   }
 
   // ---------------- teardown ----------------
-  // (no copy or product is under way: the softmax waited for every product, the products for every copy)
+  // (no copy or product is under way: the feeding warps waited for the last products, the products for every copy)
   __syncwarp();
   tc_fence_before_sync();
   __syncthreads();
