@@ -85,13 +85,13 @@ static __device__ __noinline__ void pairs_run(const Lane &L, const DPairs &p, co
       const float *q = pos + 3u * static_cast<size_t>(c0 + j);
       sj[j] = make_float4(q[0], q[1], q[2], mass[c0 + j]);
     }
-    if (c0 == 0u) {                                             // the tail's operands from memory, under the pair loop
-      for (uint32_t k = L.tid; k < n_tail * 2u * elems; k += L.nthr) {
-        const uint32_t op = k / (2u * elems), rem = k % (2u * elems), ab = rem / elems, e = rem % elems;
-        const DPairTail &tl = p.tail[op];
-        const BufRef r = ab ? tl.b : tl.a;
-        if ((ab ? tl.b_src : tl.a_src) == 0u && r)
-          ext[(op * 2u + ab) * (kPairsRows * 3u) + e] = reinterpret_cast<const float *>(resolve(P, r))[3u * static_cast<size_t>(lo) + e];
+    if (c0 == 0u) {                                             // the tail's operands from memory, a warp each, under the pair loop
+      for (uint32_t oa = w; oa < 2u * n_tail; oa += nw) {
+        const DPairTail &tl = p.tail[oa >> 1];
+        const BufRef r = (oa & 1u) ? tl.b : tl.a;
+        if (((oa & 1u) ? tl.b_src : tl.a_src) != 0u || !r) continue;
+        const float *src = reinterpret_cast<const float *>(resolve(P, r)) + 3u * static_cast<size_t>(lo);
+        for (uint32_t e = lane; e < elems; e += kWarp) cp_async_4_zfill(smem_addr(ext + oa * (kPairsRows * 3u) + e), src + e, 4u);
       }
     }
     __syncthreads();
@@ -114,16 +114,35 @@ static __device__ __noinline__ void pairs_run(const Lane &L, const DPairs &p, co
       }
     }
   }
-  const auto add = [](float a, float b) { return a + b; };
+  // The warp's sums: of 24 values (eight bodies) a lane hands on half, then half of that, then half again; two whole steps are left,
+  // and lanes 4 k .. 4 k + 3 hold body k. (One value at a time the 21 of seven bodies took 1900 cycles.)
   const uint32_t cover = groups * NI;
+  {
+    float v[24] = {};
 #pragma unroll
-  for (int k = 0; k < NI; ++k) {
-    const float sx = warp_reduce(ax[k], add), sy = warp_reduce(ay[k], add), sz = warp_reduce(az[k], add);
-    if (lane == 0) {
+    for (int k = 0; k < NI; ++k) { v[3 * k] = ax[k]; v[3 * k + 1] = ay[k]; v[3 * k + 2] = az[k]; }
+#pragma unroll
+    for (int h = 12, o = 16; h >= 3; h /= 2, o /= 2) {
+      const bool up = (lane & static_cast<uint32_t>(o)) != 0u;
+#pragma unroll
+      for (int k = 0; k < 12; ++k)
+        if (k < h) {
+          const float send = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k];
+          v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    const uint32_t k = lane >> 2;                 // 4 b4 + 2 b3 + b2
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      v[e] += __shfl_xor_sync(0xffffffffu, v[e], 2);
+      v[e] += __shfl_xor_sync(0xffffffffu, v[e], 1);
+    }
+    if ((lane & 3u) == 0u && k < static_cast<uint32_t>(NI)) {
       float *o = part + (static_cast<size_t>(slice) * cover + grp * NI + k) * 3u;
-      o[0] = sx; o[1] = sy; o[2] = sz;
+      o[0] = v[0]; o[1] = v[1]; o[2] = v[2];
     }
   }
+  cp_async_wait_all();
   __syncthreads();
   float *out = reinterpret_cast<float *>(resolve(P, p.out));
   for (uint32_t e = L.tid; e < elems; e += L.nthr) {

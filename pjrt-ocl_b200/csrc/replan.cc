@@ -499,13 +499,38 @@ bool Planner::FusePairs(int seed) {
     for (int j : pred_[i]) depth[i] = std::max(depth[i], depth[j]);
     if (n_[i].op == kTopRedStrided) depth[i] = i + 1;
   }
-  for (int i = 0; i < n_orig_ && n_tail < kPairTailMax; ++i) {
+  auto tail_op = [&](int i) {
     const Node &e = n_[i];
-    if (e.region != sum.region || !Free(i) || e.op != kTopEw || e.dt != kF32 || e.adt != kF32 || e.t.p1 != 3 * n) continue;
+    if (e.region != sum.region || !Free(i) || e.op != kTopEw || e.dt != kF32 || e.adt != kF32 || e.t.p1 != 3 * n) return false;
     const uint32_t sub = e.t.p0;
     const bool bin = sub == kAdd || sub == kSubt || sub == kMul;
-    if (!(bin || sub == kAffine || sub == kCopy)) continue;
-    if (sub != kAffine && (e.t.p2 || e.t.p3)) continue;
+    return (bin || sub == kAffine || sub == kCopy) && (sub == kAffine || !(e.t.p2 || e.t.p3));
+  };
+  // Tasks that need no evaluation and that only other evaluations want, where they read their positions: side by side with this
+  // one they would be an op of their own on a few lanes, for which the others wait (8 us of the 88 of a Runge-Kutta step).
+  // Only for an evaluation that needs no other: what it takes along is done when any later one starts.
+  std::set<int> early;
+  bool first = true;
+  for (int m : members) for (int j : pred_[m]) first = first && (in_group.count(j) || depth[j] == 0);
+  for (int i = 0; first && i < n_orig_; ++i)
+    if (tail_op(i) && depth[i] == 0 && Def(n_[i].t.dst) == i && !out_.count(n_[i].t.dst) && n_[i].t.dst != pos && n_[i].t.dst != mass && !Uses(n_[i].t.dst).empty()) early.insert(i);
+  for (bool changed = true; changed;) {
+    changed = false;
+    for (auto it = early.begin(); it != early.end();) {
+      bool keep = true;
+      for (int u : Uses(n_[*it].t.dst))
+        keep = keep && !in_group.count(u) && (early.count(u) || (n_[u].region == sum.region && (n_[u].op == kTopEw || n_[u].op == kTopGather) && n_[u].t.p1 == 3 * n * n));
+      for (int j : pred_[*it]) keep = keep && (early.count(j) || n_[j].region != sum.region);
+      for (int u : succ_[*it]) keep = keep && !in_group.count(u);
+      if (keep) ++it;
+      else { it = early.erase(it); changed = true; }
+    }
+  }
+  for (int i = 0; i < n_orig_ && n_tail < kPairTailMax; ++i) {
+    const Node &e = n_[i];
+    if (!tail_op(i)) continue;
+    const uint32_t sub = e.t.p0;
+    const bool bin = sub == kAdd || sub == kSubt || sub == kMul;
     bool mine = false, foreign = false;
     for (int j : pred_[i]) {
       if (in_group.count(j)) mine = true;
@@ -515,6 +540,7 @@ bool Planner::FusePairs(int seed) {
       mine = !Uses(e.t.dst).empty();
       for (int u : Uses(e.t.dst)) if (!in_group.count(u) && depth[u] <= depth[seed]) mine = false;
     }
+    if (early.count(i)) { mine = true; foreign = false; }
     if (!mine || foreign || e.t.dst == pos || e.t.dst == mass) continue;     // other lanes may still read those
     // rows of the operands are this lane's own only when they come from the group or from before it
     auto src = [&](uint32_t b) { auto it = made.find(b); return it == made.end() ? 0 : it->second; };
