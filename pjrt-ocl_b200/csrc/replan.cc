@@ -1570,6 +1570,24 @@ bool Planner::Assemble(VmProgram *q, ReplanStats *st) {
       mixed = true;
       for (int u : us) mixed = mixed && (n_[u].by_slot || n_[u].tiles >= 2 * L_);
     }
+    // Only products: each has lanes of its own, by cost. (Cut like tiles, the lane where one product ends and the next begins had a slot
+    // in both, and a slot is a whole share of a product: three f32 products of 512 cubed 84 us, where most lanes had done after 50.)
+    std::vector<std::pair<uint32_t, uint32_t>> own_lanes(us.size(), {0u, 0u});
+    const bool apart = us.size() > 1 && n_slot == us.size() && us.size() <= L_;
+    if (apart) {
+      std::vector<uint32_t> n(us.size(), 1u);
+      for (uint32_t left = L_ - static_cast<uint32_t>(us.size()); left; --left) {
+        size_t most = 0;
+        auto load = [&](size_t k) { return n_[us[k]].cost * n_[us[k]].tiles / n[k]; };
+        for (size_t k = 1; k < us.size(); ++k) if (load(k) > load(most)) most = k;
+        ++n[most];
+      }
+      uint32_t lane = 0;
+      for (size_t k = 0; k < us.size(); ++k) {
+        own_lanes[k] = {lane, lane + std::min(n[k], n_[us[k]].tiles)};
+        lane += n[k];
+      }
+    }
     auto even = [&](int u) { return us.size() == 1 || plenty || (mixed && !n_[u].by_slot); };
     double total = 0;
     for (int u : us) if (!even(u)) total += n_[u].cost * n_[u].tiles * static_cast<double>(of[u].size());
@@ -1598,7 +1616,7 @@ bool Planner::Assemble(VmProgram *q, ReplanStats *st) {
         // a share of the lanes, each with a slot number (alone in the phase: all of them, as many as there are tiles)
         std::vector<uint32_t> mine;
         for (uint32_t l = 0; l < L_; ++l)
-          if (us.size() == 1 || (mixed && n_slot == 1) ? l < T : cut[k][l].second > cut[k][l].first) mine.push_back(l);
+          if (apart ? l >= own_lanes[k].first && l < own_lanes[k].second : us.size() == 1 || (mixed && n_slot == 1) ? l < T : cut[k][l].second > cut[k][l].first) mine.push_back(l);
         owners = static_cast<uint32_t>(mine.size());
         for (uint32_t i = 0; i < owners; ++i) {
           VmEntry e = blank;
