@@ -183,8 +183,8 @@ static __device__ __noinline__ void flash_decode_ring(const Lane &L, const DTask
   const uint32_t part = l % LPK, sub = l / LPK;
   const uint32_t kps = nw * 4u * KPL;      // keys per stage: every warp gets 4 load positions of KPL keys
   const uint32_t stage_b = kps * kRowB;    // bytes of K (and of V) per stage
-  float *ml = reinterpret_cast<float *>(L.smem + kSmemSys);                          // [nw][2]
-  float *os = ml + 2 * 32;                                                           // [nw][HD]
+  float *ml = reinterpret_cast<float *>(L.smem + kSmemSys);                          // [2][16 warps]{maximum, scaled sum}
+  float *os = ml + 2 * 32;                                                           // [2][16 warps][HD]
   uint64_t *full = reinterpret_cast<uint64_t *>(L.smem + kSmemSys + 256 + 4u * 32u * HD);   // after ml / os
   uint64_t *empty = full + 2u * kDepth;           // full[2 b] : K of buffer b has landed, full[2 b + 1] : V
   uint8_t *ring = L.smem + ((kSmemSys + 256 + 4u * 32u * HD + 96 + 127) & ~127u);
@@ -197,15 +197,18 @@ static __device__ __noinline__ void flash_decode_ring(const Lane &L, const DTask
     }
   };
   // the lane's stages, in order: tile by tile, kps keys each (the last of a tile ragged)
-  auto c_end_of = [&](int64_t tile) { const int64_t m = tile % T; return causal ? min(C, m + (C - T) + 1) : C; };
-  auto stages_of = [&](int64_t tile) { return static_cast<uint32_t>((c_end_of(tile) + kps - 1) / kps); };
+  // (One query row per head sees every key, and needs no 64-bit division per stage and request.)
+  const bool one = T == 1;
+  const uint32_t n_all = (static_cast<uint32_t>(C) + kps - 1u) / kps;
+  auto c_end_of = [&](int64_t tile) { return one || !causal ? C : min(C, tile % T + (C - T) + 1); };
+  auto stages_of = [&](int64_t tile) { return one || !causal ? n_all : static_cast<uint32_t>((c_end_of(tile) + kps - 1) / kps); };
   // producer state (thread 0): the next stage to request
   int64_t p_tile = tile_lo;
   uint32_t p_stage = 0, p_seq = 0;
   auto request = [&]() {          // thread 0: issue the copies of the next stage, if any is left
     while (p_tile < hi && p_stage >= stages_of(p_tile)) { ++p_tile; p_stage = 0; }
     if (p_tile >= hi) return;
-    const int64_t g = p_tile / T, c_end = c_end_of(p_tile);
+    const int64_t g = one ? p_tile : p_tile / T, c_end = c_end_of(p_tile);
     const int64_t k0 = static_cast<int64_t>(p_stage) * kps;
     const uint32_t bytes = static_cast<uint32_t>(min(static_cast<int64_t>(kps), c_end - k0)) * kRowB;
     const uint32_t b = p_seq % kDepth;
@@ -224,15 +227,18 @@ static __device__ __noinline__ void flash_decode_ring(const Lane &L, const DTask
   }
   __syncthreads();
   const float sl2 = scale * 1.4426950408889634f;
+  uint4 q_next = tile_lo < hi ? ldg_v4(Q + static_cast<int64_t>(tile_lo) * HD + part * 8) : make_uint4(0u, 0u, 0u, 0u);
+  uint32_t turn = 0;               // which half of the merge's workspace
   uint32_t seq = 0;                // stages consumed so far by this lane (all threads count alike)
   bool ok = true;
   for (int64_t tile = tile_lo; tile < hi && ok; ++tile) {
-    const int64_t g = tile / T, m = tile % T;
+    const int64_t g = one ? tile : tile / T, m = one ? 0 : tile % T;
     const int64_t c_end = c_end_of(tile);
     float q[8];
-    unpack8(ldg_v4(Q + (g * T + m) * HD + part * 8), q);
+    unpack8(q_next, q);
 #pragma unroll
     for (int i = 0; i < 8; ++i) q[i] *= sl2;
+    if (tile + 1 < hi) q_next = ldg_v4(Q + (tile + 1) * HD + part * 8);          // under this head's stages
     float m_run = -INFINITY, l_run = 0.0f, o[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) o[i] = 0.0f;
@@ -303,21 +309,28 @@ static __device__ __noinline__ void flash_decode_ring(const Lane &L, const DTask
 #pragma unroll
       for (int i = 0; i < 8; ++i) o[i] += __shfl_xor_sync(0xffffffffu, o[i], d);
     }
-    __syncthreads();            // the previous tile's merge has read the workspace
-    if (l == 0) { ml[2 * w] = m_run; ml[2 * w + 1] = l_run; }
+    // Every warp scales its own part to the common maximum, so that what is left per value are plain sums. The workspace's halves
+    // are used in turn: a half's readers are two barriers before its next writers.
+    float *ml_t = ml + 32u * turn, *os_t = os + 16u * HD * turn;
+    turn ^= 1u;
+    if (l == 0) ml_t[2 * w] = m_run;
+    __syncthreads();
+    float M = -INFINITY;
+#pragma unroll
+    for (uint32_t ww = 0; ww < 16u; ++ww) M = fmaxf(M, ml_t[2 * ww]);
+    const float mine = m_run == -INFINITY ? 0.0f : fast_ex2(m_run - M);
+    if (l == 0) ml_t[2 * w + 1] = l_run * mine;
     if (sub == 0) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) os[w * HD + part * 8 + i] = o[i];
+      for (int i = 0; i < 8; ++i) os_t[w * HD + part * 8 + i] = o[i] * mine;
     }
     __syncthreads();
     for (int64_t d = L.tid; d < HD; d += L.nthr) {
-      float M = -INFINITY;
-      for (uint32_t ww = 0; ww < nw; ++ww) M = fmaxf(M, ml[2 * ww]);
       float num = 0.0f, den = 0.0f;
-      for (uint32_t ww = 0; ww < nw; ++ww) {
-        const float e = ml[2 * ww] == -INFINITY ? 0.0f : fast_ex2(ml[2 * ww] - M);
-        num = fmaf(os[ww * HD + d], e, num);
-        den = fmaf(ml[2 * ww + 1], e, den);
+#pragma unroll
+      for (uint32_t ww = 0; ww < 16u; ++ww) {
+        num += os_t[ww * HD + d];
+        den += ml_t[2 * ww + 1];
       }
       storef(out, t.dt, (g * T + m) * HD + d, __fdiv_rn(num, den));
     }
