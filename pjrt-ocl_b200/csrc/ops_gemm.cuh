@@ -510,11 +510,13 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
   const uint32_t stage0 = (smem_addr(sm + kSmemSys) + 1023u) & ~1023u;
   const uint32_t w = __shfl_sync(0xffffffffu, L.tid / kWarp, 0), lane = L.tid % kWarp;   // the warp index, provably uniform
   const uint32_t n_stages = G.stages;
-  if (L.tid == 0) {
-    for (uint32_t s = 0; s < n_stages; ++s) { mbar_init(&S->full[s], 1u); mbar_init(&S->empty[s], 1u); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&S->acc_full[b], 1u); mbar_init(&S->acc_empty[b], kGemmEpiWarps); }
-    S->failed = 0u;
+  if (w == 0u) {
+    if (lane < n_stages) { mbar_init(&S->full[lane], 1u); mbar_init(&S->empty[lane], 1u); }
+    else if (lane < n_stages + 2u) { mbar_init(&S->acc_full[lane - n_stages], 1u); mbar_init(&S->acc_empty[lane - n_stages], kGemmEpiWarps); }
+    else if (lane == 31u) S->failed = 0u;
     fence_mbar_init();
+  } else if (w == 1u && lane < 2u * G.n_prob) {
+    prefetch_tmap(P.tmaps + G.prob[lane >> 1].tmap + (lane & 1u));       // the first copy would wait for it
   }
   __syncwarp();
   if (w == 2u) tmem_alloc(&S->tmem_base, 512u);
@@ -567,12 +569,11 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
     tc_fence_after_sync();
     tmem_dealloc(tmem, 512u);
   }
-  if (L.tid == 0) {
-    if (gave_up) set_status(P, kStTensorTimeout, L.lane, slot, kTopGemm);
-    else {
-      for (uint32_t s = 0; s < n_stages; ++s) { mbar_inval(&S->full[s]); mbar_inval(&S->empty[s]); }
-      for (int b = 0; b < 2; ++b) { mbar_inval(&S->acc_full[b]); mbar_inval(&S->acc_empty[b]); }
-    }
+  if (gave_up) {
+    if (L.tid == 0) set_status(P, kStTensorTimeout, L.lane, slot, kTopGemm);
+  } else if (w == 0u) {
+    if (lane < n_stages) { mbar_inval(&S->full[lane]); mbar_inval(&S->empty[lane]); }
+    else if (lane < n_stages + 2u) { mbar_inval(&S->acc_full[lane - n_stages]); mbar_inval(&S->acc_empty[lane - n_stages]); }
   }
   __syncthreads();
   if (G.total) fuse_full_sum(L, csum, reinterpret_cast<float *>(resolve(P, G.total)), t.p[3], G.n_owner_lanes);

@@ -200,6 +200,8 @@ __device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const void *tmap,
       ::"r"(smem_dst), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_addr(bar))
       : "memory");
 }
+// Brings a tensor map towards the copy unit ahead of its first use.
+__device__ __forceinline__ void prefetch_tmap(const void *tmap) { asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory"); }
 // Generic-proxy writes to global memory made visible here are ordered before this thread's later asynchronous-proxy reads.
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 // One arrival that also announces `bytes` of transactions (issued before or after it).

@@ -93,7 +93,10 @@ def _case(kind, **kw):
     # store epilogues: GELU, its derivative, the update step, the loss sum
     _case("mlp", batch=72, d0=64, d1=136, d2=264, d3=72, dtype="bf16"), _case("mlp", batch=300, d0=64, d1=264, d2=520, d3=72, dtype="f16"), _case("mlp", batch=67, d0=33, d1=50, d2=21, d3=40, dtype="f32"),
     # attention between products; a decode step with its cache rows stored by the products
-    _case("block", batch=2, seq=65, heads=4, dtype="bf16"), _case("block", batch=1, seq=77, heads=4, dtype="f32"), _case("block", batch=1, seq=300, heads=2, dtype="f32"),
+    _case("block", batch=3, seq=1100, heads=12, dtype="f16"), _case("block", batch=2, seq=65, heads=4, dtype="bf16"), _case("block", batch=1, seq=77, heads=4, dtype="f32"), _case("block", batch=1, seq=300, heads=2, dtype="f32"),
+    # decode attention: fewer heads than lanes and more, whole stages of keys and one key past them, several heads per lane
+    _case("decode", batch=1, cache=2047, heads=4, dtype="bf16"), _case("decode", batch=10, cache=600, heads=16, dtype="f16"), _case("decode", batch=32, cache=256, heads=5, dtype="bf16"),
+    _case("decode", batch=1, cache=9000, heads=16, dtype="bf16"),
     _case("decode", batch=1, cache=64, heads=4, dtype="bf16"), _case("decode", batch=17, cache=301, heads=8, dtype="f16"), _case("decode", batch=3, cache=70, heads=4, dtype="f32"),
     _case("nbody", bodies=257, steps=2),
 ])
