@@ -390,8 +390,9 @@ static __device__ __noinline__ GemmAt gemm_form(GemmWarp W, GemmAt at) {
 
 // ---- the warps that feed the tensor cores, each a function of its own: what they need per stage stays in registers ----
 struct GemmLane { const KParams *P; uint32_t stage0, tmem, slot, n_slots; };
-// One thread: fills the stages.
-static __device__ __noinline__ void gemm_produce(GemmLane X) {
+// Two threads, one for each operand: fill the stages. (A box takes its thread ~270 cycles to start; with both operands' boxes from one
+// thread a stage of a small tile took 640-780, more than its products.)
+static __device__ __noinline__ void gemm_produce(GemmLane X, uint32_t side) {
   const DGemm &G = gemm_desc();
   GemmShared *S = gemm_shared();
   volatile uint32_t *failed = &S->failed;
@@ -403,25 +404,23 @@ static __device__ __noinline__ void gemm_produce(GemmLane X) {
   GemmTile q;
   for (uint32_t tile = X.slot; ok && gemm_tile(G, tile, q); tile += X.n_slots) {
     const DGemmProb &pr = G.prob[q.prob];
-    const DTmap *ta = X.P->tmaps + pr.tmap, *tb = ta + 1;
-    const uint32_t nkb = (pr.K + 63u) / 64u, a_rows = 128u * pr.halves;
-    const uint32_t bytes = (a_rows + pr.bn) * 128u;
-    const int32_t r0 = static_cast<int32_t>(q.r0), c0 = static_cast<int32_t>(q.c0);
+    const DTmap *tm = X.P->tmaps + pr.tmap + side;
+    const uint32_t nkb = (pr.K + 63u) / 64u, mode = side ? pr.bmn : pr.amn, rows = side ? pr.bn : 128u * pr.halves;
+    const uint32_t bytes = rows * 128u, at = X.stage0 + (side ? 16384u * pr.halves : 0u);
     // An operand's part of a stage is one box; one whose rows are the unit-stride axis comes as 64-row blocks (a box over
     // the blocks), or block by block where they do not divide the axis.
-    auto fetch = [&](uint32_t dst, const DTmap *tm, uint32_t mode, uint32_t rows, int32_t r, int32_t k0, uint64_t *bar) {
-      if (mode == kGmK) tma_load_3d(dst, tm, k0, r, 0, bar);
-      else if (mode == kGmMnBlocks) tma_load_3d(dst, tm, 0, k0, r / 64, bar);
-      else
-        for (uint32_t i = 0; i < rows / 64u; ++i) tma_load_3d(dst + i * kGemmBox, tm, r + static_cast<int32_t>(64u * i), k0, 0, bar);
-    };
+    const int32_t r = static_cast<int32_t>(side ? q.c0 : q.r0);
+    const int32_t dx = mode == kGmK ? 64 : 0, dy = mode == kGmK ? 0 : 64, z = mode == kGmMnBlocks ? r / 64 : 0;
+    int32_t x = mode == kGmMnSingle ? r : 0, y = mode == kGmK ? r : 0;
     for (uint32_t kb = 0; kb < nkb; ++kb, ++it) {
       if (!tc_wait(&S->empty[s], turn, failed, budget)) { ok = false; break; }
       mbar_arrive_tx(&S->full[s], bytes);
-      const uint32_t sa = X.stage0 + s * stage_bytes;
-      const int32_t k0 = static_cast<int32_t>(kb * 64u);
-      fetch(sa, ta, pr.amn, a_rows, r0, k0, &S->full[s]);
-      fetch(sa + a_rows * 128u, tb, pr.bmn, pr.bn, c0, k0, &S->full[s]);
+      const uint32_t dst = at + s * stage_bytes;
+      tma_load_3d(dst, tm, x, y, z, &S->full[s]);
+      if (mode == kGmMnSingle)
+        for (uint32_t i = 1; i < rows / 64u; ++i) tma_load_3d(dst + i * kGemmBox, tm, x + static_cast<int32_t>(64u * i), y, 0, &S->full[s]);
+      x += dx;
+      y += dy;
       if (++s == n_stages) { s = 0u; turn ^= 1u; }
     }
   }
@@ -511,7 +510,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
   const uint32_t w = __shfl_sync(0xffffffffu, L.tid / kWarp, 0), lane = L.tid % kWarp;   // the warp index, provably uniform
   const uint32_t n_stages = G.stages;
   if (w == 0u) {
-    if (lane < n_stages) { mbar_init(&S->full[lane], 1u); mbar_init(&S->empty[lane], 1u); }
+    if (lane < n_stages) { mbar_init(&S->full[lane], 2u); mbar_init(&S->empty[lane], 1u); }
     else if (lane < n_stages + 2u) { mbar_init(&S->acc_full[lane - n_stages], 1u); mbar_init(&S->acc_empty[lane - n_stages], kGemmEpiWarps); }
     else if (lane == 31u) S->failed = 0u;
     fence_mbar_init();
@@ -528,7 +527,7 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
   float csum = 0.0f;
 
   if (w == 0u) {
-    if (lane == 0u) gemm_produce(GemmLane{&P, stage0, tmem, slot, n_slots});
+    if (lane < 2u) gemm_produce(GemmLane{&P, stage0, tmem, slot, n_slots}, lane);
   } else if (w == 1u) {
     gemm_issue(GemmLane{&P, stage0, tmem, slot, n_slots});
   } else if (w >= kGemmEpiFirst) {
