@@ -6,11 +6,10 @@
 // a 128 x 256 tile took up to six per 512 tensor cycles. Here a stage is two boxes (32 KB each at most) and feeds 1024.
 // A 256 x 256 tile is two 128-row halves that share the B block and fill all of tensor memory.
 //
-// Roles: warp 0 feeds the stages (64 k of A's rows and of B's columns, as 64 x 64 TMA boxes of 8 KB in the 128-byte swizzle, either
-// operand k-contiguous or row / column-contiguous; as many stages of the task's largest tile as the ring's 192 KB hold, 3 of 256 x
-// 256, 4 of 128 x 256, 8 of 128 x 64); warp 1 issues tcgen05.mma, the whole warp in
-// step (its waits too: tc_wait_uniform) and one elected lane issuing, so that descriptors stay in uniform registers; warps
-// 4-15 drain and store.
+// Roles: two threads of warp 0 feed the stages, one for each operand (64 k of A's rows and of B's columns, as 64 x 64 TMA boxes of 8 KB
+// in the 128-byte swizzle, either operand k-contiguous or row / column-contiguous; as many stages of the task's largest tile as the
+// ring's 192 KB hold, 3 of 256 x 256, 4 of 128 x 256, 8 of 128 x 64); warp 1 issues tcgen05.mma, the whole warp in step (its waits
+// too: tc_wait_uniform) and one elected lane issuing, so that descriptors stay in uniform registers; warps 4-15 drain and store.
 // Accumulator slots: a half tile takes slot (running number) % 2. A tile of one half thus runs under the previous one's
 // epilogue; a tile of two halves starts its first half's k blocks as soon as that slot is drained, as far ahead as
 // the stages reach, while the second slot drains.
