@@ -381,7 +381,7 @@ int Planner::AddPlanned(Node nd, const std::vector<int> &members) {
 //   out = RED_STRIDED(d * w[., ., broadcast]); d = x[j] - x[i] (views, or gathers of carried positions);
 //   w = POW(AFFINE(RED_SEG(d * d)), -1.5) * m[j]
 bool Planner::FusePairs(int seed) {
-  const Node &sum = n_[seed];
+  const Node sum = n_[seed];
   const int64_t n = sum.t.p1;
   if (sum.dt != kF32 || sum.adt != kF32 || sum.t.p2 != 3 || sum.t.p3 != kSum || n < 2 || sum.t.p0 != 3 * n || n > (1 << 14)) return false;
   std::vector<int> members{seed};
@@ -469,15 +469,10 @@ bool Planner::FusePairs(int seed) {
   nd.op = kTopPairs; nd.dt = nd.adt = kF32;
   nd.t = VmTask{};
   nd.t.dst = sum.t.dst; nd.t.a = pos;
-  nd.rd = {pos, mass};
-  nd.wr = {sum.t.dst};
   nd.tiles = static_cast<uint32_t>(n);
   nd.cost = 0.33 * static_cast<double>(n) / 4096.0;
-  // The elementwise tasks on the n x 3 result that need nothing from elsewhere after this evaluation.
-  std::vector<int32_t> tail;
-  int n_tail = 0;
-  std::set<int> in_group(members.begin(), members.end());
-  std::map<uint32_t, int32_t> made{{sum.t.dst, 1}};      // buffer -> where the tail finds its value (format.h: DPairTail)
+  const std::set<int> core(members.begin(), members.end());
+  std::set<int> in_group = core;
   auto depends = [&](int i) {        // does i need anything of the group (through tasks outside it too)?
     std::vector<int> todo{i};
     std::set<int> seen;
@@ -508,10 +503,11 @@ bool Planner::FusePairs(int seed) {
   };
   // Tasks that need no evaluation and that only other evaluations want, where they read their positions: side by side with this
   // one they would be an op of their own on a few lanes, for which the others wait (8 us of the 88 of a Runge-Kutta step).
-  // Only for an evaluation that needs no other: what it takes along is done when any later one starts.
+  // Only for an evaluation that has nothing to wait for, and so runs in the phase that these would run in: another's positions
+  // stand in a phase before it, together, and evaluations that are independent of each other stay so.
   std::set<int> early;
   bool first = true;
-  for (int m : members) for (int j : pred_[m]) first = first && (in_group.count(j) || depth[j] == 0);
+  for (int m : core) for (int j : pred_[m]) first = first && core.count(j);
   for (int i = 0; first && i < n_orig_; ++i)
     if (tail_op(i) && depth[i] == 0 && Def(n_[i].t.dst) == i && !out_.count(n_[i].t.dst) && n_[i].t.dst != pos && n_[i].t.dst != mass && !Uses(n_[i].t.dst).empty()) early.insert(i);
   for (bool changed = true; changed;) {
@@ -519,45 +515,60 @@ bool Planner::FusePairs(int seed) {
     for (auto it = early.begin(); it != early.end();) {
       bool keep = true;
       for (int u : Uses(n_[*it].t.dst))
-        keep = keep && !in_group.count(u) && (early.count(u) || (n_[u].region == sum.region && (n_[u].op == kTopEw || n_[u].op == kTopGather) && n_[u].t.p1 == 3 * n * n));
-      for (int j : pred_[*it]) keep = keep && (early.count(j) || n_[j].region != sum.region);
-      for (int u : succ_[*it]) keep = keep && !in_group.count(u);
+        keep = keep && !core.count(u) && (early.count(u) || (n_[u].region == sum.region && (n_[u].op == kTopEw || n_[u].op == kTopGather) && n_[u].t.p1 == 3 * n * n));
+      for (int j : pred_[*it]) keep = keep && early.count(j);
+      for (int u : succ_[*it]) keep = keep && !core.count(u);
       if (keep) ++it;
       else { it = early.erase(it); changed = true; }
     }
   }
-  for (int i = 0; i < n_orig_ && n_tail < kPairTailMax; ++i) {
-    const Node &e = n_[i];
-    if (!tail_op(i)) continue;
-    const uint32_t sub = e.t.p0;
-    const bool bin = sub == kAdd || sub == kSubt || sub == kMul;
-    bool mine = false, foreign = false;
-    for (int j : pred_[i]) {
-      if (in_group.count(j)) mine = true;
-      else if (depends(j) || depth[j] >= depth[seed]) foreign = true;
+  // With the early tasks, if the tail has room for them beside its own and nothing of the group then waits for the group.
+  for (int with_early = early.empty() ? 0 : 1; with_early >= 0; --with_early) {
+    // The elementwise tasks on the n x 3 result that need nothing from elsewhere after this evaluation.
+    members.assign(core.begin(), core.end());
+    in_group = core;
+    std::vector<int32_t> tail;
+    int n_tail = 0;
+    bool room = true;
+    std::map<uint32_t, int32_t> made{{sum.t.dst, 1}};      // buffer -> where the tail finds its value (plan_format.h: DPairTail)
+    nd.rd = {pos, mass};
+    nd.wr = {sum.t.dst};
+    for (int i = 0; i < n_orig_; ++i) {
+      const Node &e = n_[i];
+      if (!tail_op(i)) continue;
+      const uint32_t sub = e.t.p0;
+      const bool bin = sub == kAdd || sub == kSubt || sub == kMul;
+      bool mine = false, foreign = false;
+      for (int j : pred_[i]) {
+        if (in_group.count(j)) mine = true;
+        else if (depends(j) || depth[j] >= depth[seed]) foreign = true;
+      }
+      if (!mine && !foreign && depth[i] >= 1 && depth[i] < depth[seed]) {
+        mine = !Uses(e.t.dst).empty();
+        for (int u : Uses(e.t.dst)) if (!in_group.count(u) && depth[u] <= depth[seed]) mine = false;
+      }
+      if (with_early && early.count(i)) { mine = true; foreign = false; }
+      if (!mine || foreign || e.t.dst == pos || e.t.dst == mass) continue;     // other lanes may still read those
+      if (n_tail == kPairTailMax) { room = false; break; }
+      // rows of the operands are this lane's own only when they come from the group or from before it
+      auto src = [&](uint32_t b) { auto it = made.find(b); return it == made.end() ? 0 : it->second; };
+      tail.insert(tail.end(), {static_cast<int32_t>(sub), src(e.t.a), bin ? src(e.t.b) : 0, static_cast<int32_t>(sub == kAffine ? e.t.p2 : 0u),
+                               static_cast<int32_t>(sub == kAffine ? e.t.p3 : 0u), static_cast<int32_t>(e.t.dst), static_cast<int32_t>(e.t.a),
+                               static_cast<int32_t>(bin ? e.t.b : e.t.a)});
+      ++n_tail;
+      for (uint32_t b : e.rd) if (!made.count(b)) nd.rd.push_back(b);
+      nd.wr.push_back(e.t.dst);
+      made[e.t.dst] = 1 + n_tail;
+      members.push_back(i);
+      in_group.insert(i);
     }
-    if (!mine && !foreign && depth[i] >= 1 && depth[i] < depth[seed]) {
-      mine = !Uses(e.t.dst).empty();
-      for (int u : Uses(e.t.dst)) if (!in_group.count(u) && depth[u] <= depth[seed]) mine = false;
-    }
-    if (early.count(i)) { mine = true; foreign = false; }
-    if (!mine || foreign || e.t.dst == pos || e.t.dst == mass) continue;     // other lanes may still read those
-    // rows of the operands are this lane's own only when they come from the group or from before it
-    auto src = [&](uint32_t b) { auto it = made.find(b); return it == made.end() ? 0 : it->second; };
-    tail.insert(tail.end(), {static_cast<int32_t>(sub), src(e.t.a), bin ? src(e.t.b) : 0, static_cast<int32_t>(sub == kAffine ? e.t.p2 : 0u),
-                             static_cast<int32_t>(sub == kAffine ? e.t.p3 : 0u), static_cast<int32_t>(e.t.dst), static_cast<int32_t>(e.t.a),
-                             static_cast<int32_t>(bin ? e.t.b : e.t.a)});
-    ++n_tail;
-    for (uint32_t b : e.rd) if (!made.count(b)) nd.rd.push_back(b);
-    nd.wr.push_back(e.t.dst);
-    made[e.t.dst] = 1 + n_tail;
-    members.push_back(i);
-    in_group.insert(i);
+    if (with_early && !room) continue;
+    nd.payload = {static_cast<int32_t>(n), FBits(s), FBits(t), static_cast<int32_t>(pos), static_cast<int32_t>(mass),
+                  static_cast<int32_t>(sum.t.dst), n_tail};
+    nd.payload.insert(nd.payload.end(), tail.begin(), tail.end());
+    if (AddPlanned(nd, members) >= 0) return true;
   }
-  nd.payload = {static_cast<int32_t>(n), FBits(s), FBits(t), static_cast<int32_t>(pos), static_cast<int32_t>(mass),
-                static_cast<int32_t>(sum.t.dst), n_tail};
-  nd.payload.insert(nd.payload.end(), tail.begin(), tail.end());
-  return AddPlanned(nd, members) >= 0;
+  return false;
 }
 
 // A value carried through a list of steps. The builder starts from a value in X and follows it forward: reductions of

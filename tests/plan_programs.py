@@ -137,3 +137,41 @@ def lone_norm(rows, cols, dtype, softmax):
     x = p.input((rows, cols), dtype)
     p.output(p.rows(cases._SOFTMAX, x, rows, cols) if softmax else p.rows(cases._LAYERNORM, x, rows, cols, cases._bits(1e-5)), (rows, cols))
     return p
+
+
+def accelerations(p, at, mass, n):
+    """sum_j m_j (|x_j - x_i|^2 + eps)^-1.5 (x_j - x_i), as a body of perf/cases.py's N-body loop."""
+    d = p.buf(3 * n * n, "f32")
+    sq = p.chain((cases._SUB, (at, at), d, p.view((n, n, 3), (0, 3, 1)), p.view((n, n, 3), (3, 0, 1))), (cases._MUL, (-1, -1), "f32"))
+    p.phase()
+    r2 = p.row_sums(sq, n * n, 3)
+    p.phase()
+    w = p.chain((cases._AFFINE, (r2,), "f32", cases._bits(1.0), cases._bits(1e-4)),
+                (cases._POW, (-1, p.scalar(-1.5)), "f32", 0, p.view((n, n), (0, 0))), (cases._MUL, (-1, mass), "f32", 0, p.view((n, n), (0, 1))))
+    p.phase()
+    f = p.chain((cases._MUL, (d, w), "f32", 0, p.view((n, n, 3), (n, 1, 0))))
+    p.phase()
+    return p.strided_sum(f, 3 * n, n, 3)
+
+
+def evaluations(n, steps, after=0):
+    """Accelerations at x + s v for every s (0: at x itself), none of which needs another's. `after`: that many ops on the first
+    one, plus x and then its sign turned, and what they make are the positions of one more."""
+    p = cases._Assembler(148)
+    x, v, mass = p.input((n, 3), "f32"), p.input((n, 3), "f32"), p.input((n,), "f32")
+    at = [p.chain((cases._AFFINE, (v,), "f32", cases._bits(s), 0), (cases._ADD, (x, -1), "f32")) if s else x for s in steps]
+    if any(steps):
+        p.phase()
+    outs = []
+    for k, a in enumerate(at):
+        if k:
+            p.phase()
+        outs.append(accelerations(p, a, mass, n))
+    if after:
+        p.phase()
+        outs.append(p.chain((cases._ADD, (outs[0], x), "f32"), *[(cases._AFFINE, (-1,), "f32", cases._bits(-1.0), 0)] * (after - 1)))
+        p.phase()
+        outs.append(accelerations(p, outs[-1], mass, n))
+    for a in outs:
+        p.output(a, (n, 3))
+    return p

@@ -252,6 +252,27 @@ def test_bodies_whose_squared_distance_overflows(bodies):
     assert bool(torch.isnan(v1[:half]).any(1).all())
 
 
+@pytest.mark.parametrize("n, steps, after", [(64, (0.5, 0.25), 0), (301, (0.5, 0.25, 0.125), 0), (1000, (0.0, 0.5, 0.25), 20), (257, (0.5, 0.0), 24)])
+def test_independent_evaluations(n, steps, after):
+    """Evaluations that share phases, and positions made in another one's tail. f32 from the same positions: a difference, a few
+    products and the root per pair (2^-20), sums of n terms as chains of at most n / 32 and a tree."""
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x, v = (torch.rand((n, 3), generator=gen, device="cuda") * 2 - 1 for _ in range(2))
+    mass = torch.rand(n, generator=gen, device="cuda") + 0.5
+    lp, outs = _execute(progs.evaluations(n, steps, after), [x, v, mass])
+    at, acc = [v * s + x for s in steps], outs[:len(steps)]
+    if after:
+        moved, last = outs[-2:]
+        assert torch.equal(moved, (acc[0] + x) * (-1.0) ** (after - 1))
+        at, acc = at + [moved], acc + [last]
+    assert lp.stat("replanned") == 1 and lp.stat("pairs") == len(at) == len(acc)
+    for out, p in zip(acc, at):
+        p = p.double()
+        d = p[None] - p[:, None]
+        f = d * ((d * d).sum(2) + 1e-4).pow(-1.5).mul(mass.double()[None])[..., None]
+        assert bool(((out.double() - f.sum(1)).abs() <= (n / 32 + 64) * 2.0 ** -24 * f.abs().sum(1)).all())
+
+
 @pytest.mark.parametrize("H, T, C, hd", [(40, 64, 64, 64), (12, 129, 129, 64), (41, 33, 100, 64), (20, 70, 131, 40), (22, 64, 67, 128), (6, 300, 301, 200), (3, 33, 70, 64)])
 def test_masked_values_do_not_reach_the_rows_that_mask_them(H, T, C, hd):
     """Causal attention on the CUDA cores: a NaN, or an infinity, in the V row of key c shows in the query rows that see c and

@@ -15,7 +15,7 @@ import perf.cases as cases
 import plan_programs as progs
 
 CSRC = os.path.join(ROOT, "pjrt-ocl_b200", "csrc")
-FUSE_ROWS, GEMM, SGEMM, SKINNY, MMA = 33, 35, 37, 38, 1
+FUSE_ROWS, PAIRS, GEMM, SGEMM, SKINNY, MMA = 33, 34, 35, 37, 38, 1
 ON, RES, LN, MUL, ADD, GELU, CARRY = 1, 2, 4, 16, 32, 64, 256           # row pipeline stages (plan_format.h)
 F32, BF16, QUANT0, EPI_GELU, EPI_RES = 0, 7, 1, 2, 16
 
@@ -167,3 +167,28 @@ def test_short_lone_sums_keep_their_plan(plan):
 def test_few_rows_by_many_columns(plan, m, k, n, transposed, op):
     (t,) = plan(cases._BUILD["dot"](dict(m=m, k=k, n=n, dtype="bf16", transposed=transposed)).blob())["tasks"]
     assert t["op"] == op
+
+
+@pytest.mark.parametrize("n", [64, 4096])
+@pytest.mark.parametrize("steps, phases, others", [
+    ((0.5, 0.25), 2, 2), ((0.5, 0.25, 0.125), 2, 3),                 # all positions side by side, then all evaluations
+    ((0.0, 0.5), 2, 0), ((0.5, 0.0), 2, 0), ((0.0, 0.5, 0.25), 2, 0)])       # positions in the tail of the one that waits for none
+def test_independent_evaluations_are_all_fused(plan, n, steps, phases, others):
+    p = plan(progs.evaluations(n, steps).blob())
+    run = [t["op"] for t in p["tasks"] if t["cut"]]
+    assert p["gains"] and p["phases"] == phases and run.count(PAIRS) == len(steps) and run.count(FUSE_ROWS) == len(run) - len(steps) == others
+
+
+@pytest.mark.parametrize("after, others", [(22, 0), (23, 1), (24, 1)])
+def test_an_evaluations_own_tail_comes_before_other_evaluations_positions(plan, after, others):
+    """A tail holds 24 ops: its own, and if they fit the two that make the other evaluation's positions. One of its own left out
+    would be a phase of its own, for the evaluation that waits for it."""
+    p = plan(progs.evaluations(64, (0.0, 0.5), after).blob())
+    run = [t["op"] for t in p["tasks"] if t["cut"]]
+    assert run.count(PAIRS) == 3 and len(run) == 3 + others and p["phases"] == 2
+
+
+def test_an_rk4_step_is_four_evaluations(plan):
+    p = plan(cases._BUILD["nbody"]({"bodies": 4096, "steps": 10}).blob())
+    run = [t["op"] for t in p["tasks"] if t["cut"]]
+    assert p["phases"] == 5 and run == [FUSE_ROWS, FUSE_ROWS] + [PAIRS] * 4
