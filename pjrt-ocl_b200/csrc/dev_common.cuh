@@ -21,7 +21,7 @@ namespace b2 {
 
 // Shared-memory map of one lane (CTA). The first kSmemSys bytes are reserved for
 // the interpreter and CTA-wide reductions; tile ops carve the rest.
-constexpr int kSmemRed = 0;          // 64 x 16 B reduction scratch
+constexpr int kSmemRed = 0;          // 64 x 8 B reduction scratch
 constexpr int kSmemPtrs = 512;       // 8 resolved pointers (MAP_REGION inputs)
 constexpr int kSmemFlag = 576;       // grid-barrier outcome, broadcast from thread 0
 // (plan_kernel.cu, which has no elementwise chain cache)

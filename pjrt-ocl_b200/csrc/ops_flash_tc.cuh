@@ -65,9 +65,11 @@ struct FaTask {
   uint32_t h0_size, causal, k_mn, adt, dt, base;
   float sl2;
 };
-static_assert(sizeof(FaShared) <= 512 && sizeof(FaTask) <= 256, "fit the scratch slot");
+// Both lie in the reduction scratch, which nothing else uses while the op runs: past it is the interpreter's (the task itself).
+constexpr uint32_t kFaTaskAt = kSmemRed + (sizeof(FaShared) + 15u) / 16u * 16u;
+static_assert(kFaTaskAt + sizeof(FaTask) <= static_cast<uint32_t>(kSmemPtrs), "fit the reduction scratch");
 __device__ __forceinline__ FaShared *fa_shared() { B2_DYN_SMEM(sm); return reinterpret_cast<FaShared *>(sm + kSmemRed); }
-__device__ __forceinline__ FaTask *fa_task() { B2_DYN_SMEM(sm); return reinterpret_cast<FaTask *>(sm + kSmemRed + 512); }
+__device__ __forceinline__ FaTask *fa_task() { B2_DYN_SMEM(sm); return reinterpret_cast<FaTask *>(sm + kFaTaskAt); }
 
 // A tile: head, first row, blocks of keys that its rows may see.
 struct FaTile { int32_t g, m0, blocks; };
