@@ -1581,21 +1581,30 @@ bool Planner::Assemble(VmProgram *q, ReplanStats *st) {
       mixed = true;
       for (int u : us) mixed = mixed && (n_[u].by_slot || n_[u].tiles >= 2 * L_);
     }
-    // Only products: each has lanes of its own, by cost. (Cut like tiles, the lane where one product ends and the next begins had a slot
-    // in both, and a slot is a whole share of a product: three f32 products of 512 cubed 84 us, where most lanes had done after 50.)
+    // Only products, not all of them with tiles for everybody: each has lanes of its own. (Cut like tiles, the lane where one product ends
+    // and the next begins had a slot in both, and a slot is a whole share of a product: three f32 products of 512 cubed 84 us, where
+    // most lanes had done after 50.) A lane works in whole tiles, so one lane after another goes to the product whose busiest lane is
+    // done last (of equal ones the one with more work to a lane), as long as it has a tile for it. (By tiles / lanes, not capped, 777 x
+    // 100 by K = 512 beside 1024 x 256 by 64 took 31 us, 19 so, 64 x 640 by 64, 400 x 512 by 1024 and 256 x 640 by 2048 together 88, 51
+    // so; 4096 x 4096 by 256 beside 2048 x 2048 by 1024, tiles for everybody, 643 apart and 605 side by side.)
     std::vector<std::pair<uint32_t, uint32_t>> own_lanes(us.size(), {0u, 0u});
-    const bool apart = us.size() > 1 && n_slot == us.size() && us.size() <= L_;
+    const bool apart = us.size() > 1 && n_slot == us.size() && us.size() <= L_ && !plenty;
     if (apart) {
       std::vector<uint32_t> n(us.size(), 1u);
+      auto load = [&](size_t k) -> std::pair<double, double> {
+        const uint32_t T = n_[us[k]].tiles;
+        if (n[k] >= T) return {0.0, 0.0};
+        return {n_[us[k]].cost * ((T + n[k] - 1) / n[k]), n_[us[k]].cost * T / n[k]};
+      };
       for (uint32_t left = L_ - static_cast<uint32_t>(us.size()); left; --left) {
         size_t most = 0;
-        auto load = [&](size_t k) { return n_[us[k]].cost * n_[us[k]].tiles / n[k]; };
         for (size_t k = 1; k < us.size(); ++k) if (load(k) > load(most)) most = k;
+        if (load(most).first == 0.0) break;
         ++n[most];
       }
       uint32_t lane = 0;
       for (size_t k = 0; k < us.size(); ++k) {
-        own_lanes[k] = {lane, lane + std::min(n[k], n_[us[k]].tiles)};
+        own_lanes[k] = {lane, lane + n[k]};
         lane += n[k];
       }
     }

@@ -45,7 +45,7 @@ int main(int argc, char **argv) {
       std::printf(", \"rows\": %u, \"cols\": %u, \"pipe\": %u, \"flat\": %u, \"steps\": %u, \"stage\": %u, \"room\": %u", u.rows, u.cols, u.pipe.flags, u.flat, u.n_steps, stage, b2::kPlanStageBytes);
     } else if (d.op == b2::kTopSgemm || d.op == b2::kTopSkinny) {
       const b2::DSgemm &g = *reinterpret_cast<const b2::DSgemm *>(w);
-      std::printf(", \"mnk\": [%u, %u, %u], \"viewed\": [%u, %u], \"epi\": %u, \"dt1\": %u", g.M, g.N, g.K, g.a.viewed, g.b.viewed, g.epi, g.dt1);
+      std::printf(", \"mnk\": [%u, %u, %u], \"viewed\": [%u, %u], \"epi\": %u, \"dt1\": %u, \"shape\": %u", g.M, g.N, g.K, g.a.viewed, g.b.viewed, g.epi, g.dt1, g.shape);
     } else if (d.op == b2::kTopGemm) {
       const b2::DGemm &g = *reinterpret_cast<const b2::DGemm *>(w);
       std::printf(", \"prob\": [");

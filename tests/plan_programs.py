@@ -28,6 +28,14 @@ def viewed_product(M, K, N, dtype, dims, strides, off, elems):
     return p
 
 
+def products(dtype, *mkn):
+    """Products that need nothing of each other, one phase."""
+    p = cases._Assembler(148)
+    for M, K, N in mkn:
+        p.output(p.matmul(p.input((M, K), dtype), p.input((K, N), dtype), M, N, K, dtype), (M, N))
+    return p
+
+
 # a of 16 x 64 out of 1024 elements, as (2, 8, 64): blocks of eight rows, each block's rows last to first / first to last
 REVERSED = (16, 64, 24, "f32", (2, 8, 64), (512, -64, 1), 448, 1024)
 BLOCKED = (16, 64, 24, "f32", (8, 2, 64), (64, 512, 1), 0, 1024)

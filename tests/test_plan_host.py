@@ -3,7 +3,9 @@ from __future__ import annotations
 
 import glob
 import gzip
+import itertools
 import json
+import math
 import os
 import re
 import subprocess
@@ -192,3 +194,36 @@ def test_an_rk4_step_is_four_evaluations(plan):
     p = plan(cases._BUILD["nbody"]({"bodies": 4096, "steps": 10}).blob())
     run = [t["op"] for t in p["tasks"] if t["cut"]]
     assert p["phases"] == 5 and run == [FUSE_ROWS, FUSE_ROWS] + [PAIRS] * 4
+
+
+# a tile's rows and columns, slices of K and share of the issue rate, by shape, and its time, as Planner::SgShape has them
+SGEMM_SHAPES = [(128, 64, 4, 0.75), (64, 64, 8, 0.75), (64, 32, 8, 0.6), (32, 32, 8, 0.45), (16, 16, 8, 0.2)]
+
+
+def _sgemm_tiles(t):
+    (m, n, k), (tm, tn, slices, rate) = t["mnk"], SGEMM_SHAPES[t["shape"]]
+    return -(-m // tm) * -(-n // tn), max(k * tm * tn / (128 * rate), math.ceil(-(-k // 16) / slices) * 700.0) + 1500.0 + tm * tn * 0.15
+
+
+@pytest.mark.parametrize("mkn", [
+    ((512, 512, 512),) * 3, ((64, 8192, 64), (1024, 512, 1024)), ((777, 512, 100), (1024, 64, 256)), ((100, 512, 256), (400, 128, 100)),
+    ((777, 2048, 100), (100, 256, 1024), (400, 64, 64)), ((400, 256, 1024), (777, 512, 1024), (512, 128, 256))], ids=str)
+def test_products_side_by_side_share_the_lanes_by_whole_tiles(plan, mkn):
+    """Lanes of their own, none without a tile, and no split of the lanes whose busiest one is done sooner."""
+    tasks = [t for t in plan(progs.products("f32", *mkn).blob())["tasks"] if t["op"] == SGEMM]
+    lanes = [lane for t in tasks for lane, _, _ in t["cut"]]
+    tiles, cost = zip(*map(_sgemm_tiles, tasks))
+    own = [len(t["cut"]) for t in tasks]
+    assert len(tasks) == len(mkn) and len(lanes) == len(set(lanes)) and len(lanes) == min(148, sum(tiles))
+    assert all(sorted(c[1:] for c in t["cut"]) == [[i, n] for i in range(n)] and n <= k for t, n, k in zip(tasks, own, tiles))
+
+    def last(split):
+        return max(c * -(-k // n) for c, k, n in zip(cost, tiles, split))
+    splits = ((*s, 148 - sum(s)) for s in itertools.product(range(1, 148), repeat=len(mkn) - 1) if sum(s) < 148)
+    assert last(own) <= min(map(last, splits)) * (1 + 1e-12)
+
+
+def test_products_with_tiles_for_everybody_are_spread_over_all_lanes(plan):
+    """Whatever the cost model makes of them."""
+    for t in plan(progs.products("f32", (4096, 256, 4096), (2048, 1024, 2048)).blob())["tasks"]:
+        assert sorted(lane for lane, _, _ in t["cut"]) == list(range(148))
