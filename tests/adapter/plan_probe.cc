@@ -25,7 +25,8 @@ int main(int argc, char **argv) {
   }
   const bool planned = b2::Replan(p, static_cast<uint32_t>(std::atoi(argv[2])), &q, &st);
   if (!planned) { std::printf("{\"planned\": false, \"tasks\": []}\n"); return 0; }
-  if (!b2::BuildPlannedTables(q, 0, &t, &err, &unimpl)) {
+  // (an arena that does not start at address 0, which stands for no buffer)
+  if (!b2::BuildPlannedTables(q, 1u << 20, &t, &err, &unimpl)) {
     std::fprintf(stderr, "planned: %s\n", err.c_str());
     return 1;
   }
@@ -50,7 +51,7 @@ int main(int argc, char **argv) {
       const b2::DGemm &g = *reinterpret_cast<const b2::DGemm *>(w);
       std::printf(", \"prob\": [");
       for (uint32_t k = 0; k < g.n_prob; ++k)
-        std::printf("%s{\"mnk\": [%u, %u, %u], \"epi\": %u, \"dt1\": %u}", k ? ", " : "", g.prob[k].M, g.prob[k].N, g.prob[k].K, g.prob[k].epi, g.prob[k].dt1);
+        std::printf("%s{\"mnk\": [%u, %u, %u], \"epi\": %u, \"dt1\": %u, \"form\": %u}", k ? ", " : "", g.prob[k].M, g.prob[k].N, g.prob[k].K, g.prob[k].epi, g.prob[k].dt1, g.prob[k].form);
       std::printf("]");
     }
     std::printf(", \"cut\": [");

@@ -60,27 +60,53 @@ def widened_product(M, K, N, dtype, what):
 
 
 def product_then(M, K, N, dtype, what, transposed=False):
-    """A 16-bit product and what follows it in its own type: nothing, a residual, GELU (with the product kept: "kept")."""
+    """A 16-bit product and what follows it in its own type: nothing, a residual, GELU (with the product kept: "kept"); or as in a
+    training step: times GELU's derivative at x ("grad"), x less a thousandth of it ("step"), its difference to x scaled, and the sum
+    of the difference's squares ("loss")."""
     p = cases._Assembler(148)
     a, w, x = p.input((M, K), dtype), p.input((N, K) if transposed else (K, N), dtype), p.input((M, N), dtype)
-    y = p.matmul(a, w, M, N, K, dtype, vb=p.view((K, N), (1, K)) if transposed else 0)
+    y = p.matmul(a, w, M, N, K, "f32" if what == "step" else dtype, vb=p.view((K, N), (1, K)) if transposed else 0)
     if what == "kept":
         p.output(y, (M, N))
+    if what in ("grad", "step"):
+        xf = p.chain((cases._CONVERT, (x,), "f32"))
     if what != "product":
         p.phase()
-        y = p.chain((cases._ADD, (x, y), dtype)) if what == "residual" else p.chain((cases._GELU, (y,), dtype))
+    if what == "residual":
+        y = p.chain((cases._ADD, (x, y), dtype))
+    elif what in ("gelu", "kept"):
+        y = p.chain((cases._GELU, (y,), dtype))
+    elif what == "grad":
+        g, yf = p.region((xf,), M * N, cases._GELU_GRAD), p.chain((cases._CONVERT, (y,), "f32"))
+        p.phase()
+        y = p.chain((cases._MUL, (g, yf), "f32"), (cases._CONVERT, (-1,), dtype))
+    elif what == "step":
+        u = p.region((y, xf), M * N, ((cases._AFFINE, 2, 0, 0, 1e-3, 0.0), (cases._SUB, 0, 1, 2)))
+        p.phase()
+        y = p.chain((cases._CONVERT, (u,), dtype))
+    elif what == "loss":
+        yf, xf, diff = (p.buf(M * N, "f32") for _ in range(3))
+        sq = p.chain((cases._CONVERT, (y,), yf), (cases._CONVERT, (x,), xf), (cases._SUB, (yf, xf), diff), (cases._MUL, (-1, -1), "f32"))
+        p.phase()
+        total = p.full_sum(sq)
+        p.phase()
+        y = p.chain((cases._AFFINE, (diff,), "f32", cases._bits(2.0 / (M * N)), 0), (cases._CONVERT, (-1,), dtype))
+        p.output(total, ())
     p.output(y, (M, N))
     return p
 
 
-def attention_of_sums(H, T, C, hd, dtype, causal):
-    """(q + q0) K^T, softmax, V: a program with an attention task that something around it lets the re-planner take."""
+def attention_of_sums(H, T, C, hd, dtype, causal, trips=0, by_key=False):
+    """(q + q0) K^T, softmax, V: a program with an attention task that something around it lets the re-planner take. `trips`: the
+    attention is the body of a loop; `by_key`: K as [H, C, hd], seen through its transpose."""
     p = cases._Assembler(148)
     q, q0 = p.input((H, T, hd), dtype), p.input((H, T, hd), dtype)
-    k, v = p.input((H, hd, C), dtype), p.input((H, C, hd), dtype)
+    k, v = p.input((H, C, hd) if by_key else (H, hd, C), dtype), p.input((H, C, hd), dtype)
     s = p.chain((cases._ADD, (q, q0), dtype))
     p.phase()
-    p.output(p.attention(s, k, v, H, T, C, hd, causal), (H, T, hd))
+    if trips:
+        p.loop = (len(p.phases) - 1, trips)
+    p.output(p.attention(s, k, v, H, T, C, hd, causal, 0, p.view((H, hd, C), (C * hd, 1, hd)) if by_key else 0), (H, T, hd))
     return p
 
 

@@ -200,20 +200,35 @@ def test_product_converted_after_a_16_bit_value(what, mnk):
         assert torch.equal(out, y.float())
 
 
-@pytest.mark.parametrize("what", ["product", "residual", "gelu", "kept"])
+@pytest.mark.parametrize("what", ["product", "residual", "gelu", "kept", "grad", "step", "loss"])
 @pytest.mark.parametrize("M, K, N, dtype, transposed", [
     (33, 64, 8, "bf16", False), (128, 72, 104, "f16", False), (129, 200, 264, "bf16", False), (300, 1096, 520, "f16", True), (200, 64, 99, "bf16", True),
     (2100, 136, 1032, "bf16", False), (9600, 64, 4104, "f16", False)])
 def test_store_epilogues_at_the_edges_of_tiles(what, M, K, N, dtype, transposed):
     """One and two halves of 128 rows, column chunks that end inside a tile, rows that are no whole 16-byte words (the general
     form), rings of 3 to 8 stages that wrap. Small integers: products and sums are exact in f32, so the roundings to the 16-bit type
-    are all there is and the bits are known (but for GELU: a step of the type, and gelu_tanh's own error)."""
+    are all there is and the bits are known (but for GELU: a step of the type, and gelu_tanh's own error; its derivative alike, of which
+    the product takes a multiple; and the sum of squares, added in f32 by chains of at most 64 terms, 256 chunks and a tree)."""
     dt = {"bf16": torch.bfloat16, "f16": torch.float16}[dtype]
     gen = torch.Generator(device="cuda").manual_seed(1)
     a, w, x = (torch.randint(-3, 4, s, generator=gen, device="cuda").to(dt) for s in ((M, K), (N, K) if transposed else (K, N), (M, N)))
     lp, outs = _execute(progs.product_then(M, K, N, dtype, what, transposed), [a, w, x])
     assert lp.stat("tensor_core_matmuls") == 1
-    y = (a.float() @ (w.T if transposed else w).float()).to(dt)
+    y = (a.double() @ (w.T if transposed else w).double()).float()
+    if what == "step":
+        assert torch.equal(outs[0], (x.float() - y * torch.tensor(1e-3, device="cuda")).to(dt))
+    y = y.to(dt)
+    if what == "loss":
+        d = y.float() - x.float()
+        total, scaled = outs
+        assert torch.equal(scaled, (d * torch.tensor(2.0 / (M * N), device="cuda")).to(dt))
+        want = float((d.double() ** 2).sum())
+        assert abs(float(total) - want) <= 384 * 2.0 ** -24 * want
+    if what == "grad":
+        z = x.double().requires_grad_()
+        slope, = torch.autograd.grad(_gelu(z).sum(), z)
+        want = y.double() * slope
+        assert bool(((outs[0].double() - want).abs() <= (2.0 ** -8 if dtype == "bf16" else 2.0 ** -11) * want.abs() + 2e-6 * y.double().abs()).all())
     if what in ("product", "kept"):
         assert torch.equal(outs[0], y)
     if what == "residual":
@@ -290,6 +305,95 @@ def test_masked_values_do_not_reach_the_rows_that_mask_them(H, T, C, hd):
         clean = ~seen[:, c]
         assert bool((~torch.isfinite(out[:, ~clean])).all())
         assert bool(((out[:, clean].double() - want[:, clean]).abs() <= 1e-5 * (1.0 + want[:, clean].abs())).all())
+
+
+@pytest.mark.parametrize("mkn", [((64, 8192, 64), (1024, 512, 1024)), ((100, 512, 256), (400, 128, 100)), ((64, 64, 640), (400, 1024, 512), (256, 2048, 640)),
+                                 ((2000, 64, 2000), (1500, 100, 3000))], ids=str)
+def test_products_side_by_side(mkn):
+    """f32: K products and sums, K x 2^-24 of the sum of magnitudes."""
+    args = [_normal(s, torch.float32, i) for M, K, N in mkn for i, s in enumerate(((M, K), (K, N)))]
+    lp, outs = _execute(progs.products("f32", *mkn), args)
+    assert lp.stat("replanned") == 1 and lp.stat("planned_phases") == 1
+    for out, a, w in zip(outs, args[::2], args[1::2]):
+        a, w = a.double(), w.double()
+        assert bool(((out.double() - a @ w).abs() <= a.shape[1] * 2.0 ** -24 * (a.abs() @ w.abs())).all())
+
+
+def _attention(q, k, v, causal):
+    """Attention in float64, sum p |v|, and which keys a row sees."""
+    T, C = q.shape[1], v.shape[1]
+    seen = torch.arange(C, device="cuda")[None, :] <= torch.arange(T, device="cuda")[:, None] + (C - T if causal else C)
+    p = torch.softmax((q.double() @ k.double() / q.shape[2] ** 0.5).masked_fill(~seen, float("-inf")), -1)
+    return p @ v.double(), p @ v.double().abs(), seen
+
+
+# What the roundings allow: P and the result to half a step each, 2^-8 of a bf16 value and 2^-11 of an f16 one; a score's f32 sum of 64
+# products (4 x: the tensor cores' own order and truncation); f16: the denormal steps of P, whose largest value in a row is at least 1.
+def _attention_bound(q, k, v, mag):
+    score = 64 * 2.0 ** -22 * float((q.double().abs() @ k.double().abs()).max()) / 8
+    return ((2.0 ** -7 if q.dtype == torch.bfloat16 else 2.0 ** -10) + 2 * score) * mag + v.shape[1] * 2.0 ** -25 * float(v.abs().max()) + 1e-6
+
+
+@pytest.mark.parametrize("trips", [0, 2], ids=["drawn", "split"])
+@pytest.mark.parametrize("H, T, C, dtype, causal", [
+    (4, 320, 320, "bf16", True), (5, 130, 1104, "f16", False), (3, 300, 1111, "bf16", True), (230, 129, 300, "bf16", True), (75, 129, 129, "f16", True), (1, 16, 64, "bf16", False)])
+def test_attention_whose_row_maxima_grow(H, T, C, dtype, causal, trips, monkeypatch):
+    """Scores that grow by up to 2^12 from one block of 64 keys to the next (rows by turns: none, 2^6, 2^12, and shrinking), so that
+    the accumulators are rescaled at every block of some rows, at every other of others, in no row of a warp or in some. Tiles
+    drawn from a counter (an attention that runs once) and split by rows (the body of a loop); re-planned and as scheduled."""
+    dt = {"bf16": torch.bfloat16, "f16": torch.float16}[dtype]
+    u = torch.full((64,), 0.125, device="cuda")
+    row, key = torch.arange(T, device="cuda"), torch.arange(C, device="cuda")
+    lean = torch.tensor([0.0, 2.0, 4.0, -4.0], device="cuda")[torch.where(row % 96 < 32, row % 4, row // 32 % 4)]
+    q = (_normal((H, T, 64), torch.float32, 1) + lean[None, :, None] * u).to(dt)
+    k = (_normal((H, 64, C), torch.float32, 2, 0.5) + 16.6 * (key // 64)[None, None, :] * u[:, None]).to(dt)
+    v, zero = _normal((H, C, 64), dt, 3), torch.zeros_like(q)
+    want, mag, _ = _attention(q, k, v, causal)
+    bound = _attention_bound(q, k, v, mag)
+    for replanned in (1, 0):
+        if not replanned:
+            monkeypatch.setenv("B2VM_NO_REPLAN", "1")
+        by_key = C % 8 != 0                # (rows of [64, C] start on 16-byte boundaries, or the tensor cores are not used)
+        lp, (out,) = _execute(progs.attention_of_sums(H, T, C, 64, dtype, causal, trips, by_key), [q, zero, k.mT.contiguous() if by_key else k, v])
+        assert lp.stat("replanned") == replanned and lp.stat("tensor_core_flash") == 1
+        assert bool(((out.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("C, causal", [(333, True), (336, False), (200, True)])
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+def test_attention_with_nan_and_infinite_scores(dtype, C, causal):
+    """A NaN in a query row shows in that row alone; a NaN or an infinite score of a key in the rows that see the key and no other;
+    a score of minus infinity takes the key out."""
+    H, T = 3, 200
+    dt = {"bf16": torch.bfloat16, "f16": torch.float16}[dtype]
+    q, k, v = _normal((H, T, 64), dt, 1), _normal((H, 64, C), dt, 2), _normal((H, C, 64), dt, 3)
+    q[:, :, 7] = q[:, :, 7].abs() + 0.5
+    zero = torch.zeros_like(q)
+    want, mag, seen = _attention(q, k, v, causal)
+    bound = _attention_bound(q, k, v, mag)
+
+    def run(q, k):
+        by_key = C % 8 != 0
+        lp, (out,) = _execute(progs.attention_of_sums(H, T, C, 64, dtype, causal, 0, by_key), [q, zero, k.mT.contiguous() if by_key else k, v])
+        assert lp.stat("tensor_core_flash") == 1
+        return out
+    bad = q.clone()
+    bad[1, 131, 9] = float("nan")
+    out, hit = run(bad, k), torch.zeros((H, T), dtype=torch.bool, device="cuda")
+    hit[1, 131] = True
+    assert bool(torch.isnan(out[hit]).all()) and bool(((out.double() - want).abs() <= bound)[~hit].all())
+    for c in (0, 63, 64, 150, C - 1):
+        for x in (float("nan"), float("inf")):
+            bad = k.clone()
+            bad[2, 7, c] = x
+            out, hit = run(q, bad), torch.zeros((H, T), dtype=torch.bool, device="cuda")
+            hit[2] = seen[:, c]
+            assert bool(torch.isnan(out[hit]).all()) and bool(((out.double() - want).abs() <= bound)[~hit].all())
+        if c:                      # (every row sees key 0 at least)
+            bad = k.clone()
+            bad[:, 7, c] = float("-inf")
+            want_c, mag_c, _ = _attention(q, bad, v, causal)
+            assert bool(((run(q, bad).double() - want_c).abs() <= _attention_bound(q, k, v, mag_c)).all())
 
 
 @pytest.mark.parametrize("what, total", [

@@ -227,3 +227,24 @@ def test_products_with_tiles_for_everybody_are_spread_over_all_lanes(plan):
     """Whatever the cost model makes of them."""
     for t in plan(progs.products("f32", (4096, 256, 4096), (2048, 1024, 2048)).blob())["tasks"]:
         assert sorted(lane for lane, _, _ in t["cut"]) == list(range(148))
+
+
+# ops_gemm.cuh: an epilogue that is compiled for its steps (+ 16: of f16), 0 the general one
+FORMS = {"product": 1, "gelu": 2, "kept": 2, "residual": 3, "grad": 4, "step": 5, "loss": 6}
+
+
+@pytest.mark.parametrize("what", FORMS)
+@pytest.mark.parametrize("M, K, N, dtype, transposed, general", [
+    (33, 64, 8, "bf16", False, False), (129, 200, 264, "f16", False, False), (200, 64, 99, "bf16", True, True), (9600, 64, 4104, "bf16", False, False)])
+def test_epilogues_run_in_the_form_for_their_steps(plan, what, M, K, N, dtype, transposed, general):
+    p = plan(progs.product_then(M, K, N, dtype, what, transposed).blob())
+    (t,) = [t for t in p["tasks"] if t["op"] == GEMM]
+    assert [q["form"] for q in t["prob"]] == [0 if general else FORMS[what] + (16 if dtype == "f16" else 0)]
+    assert not [t for t in p["tasks"] if t["op"] not in (GEMM, FUSE_ROWS) and t["cut"]]
+
+
+def test_epilogues_without_a_form_of_their_own(plan):
+    """A 16-bit value that leaves as f32; 16-bit ones that are widened later do not."""
+    for what, form in (("product", 0), ("residual", 3), ("gelu", 2), ("both", 3)):
+        (t,) = [t for t in plan(progs.widened_product(256, 64, 256, "bf16", what).blob())["tasks"] if t["op"] == GEMM]
+        assert [q["form"] for q in t["prob"]] == [form]
