@@ -13,6 +13,8 @@
 //
 // The builds for decode steps, f32 blocks and 16-bit blocks have the attention with only the products such a program runs: in the
 // one build with all of them a batch 32 decode step takes 158 us (148 in its own), an f32 block of width 512 320 us (291).
+// The decode build comes before plan_gemm: lone skinny products run on it, where their code keeps more of its values in registers (spilled
+// bytes 56 for 244; three of 32 x 1024 by 1024 16.2 us for 17.9, 1 x 4096 by 4096 22.0 for 25.0).
 #ifndef B2VM_VARIANTS_H_
 #define B2VM_VARIANTS_H_
 
@@ -27,9 +29,9 @@
   X(all, b2::kFamWire)                                   \
   X(plan_rows, b2::kFamFuse)                             \
   X(plan_pairs, b2::kFamFuse | b2::kFamPairs)            \
+  X(plan_decode, b2::kFamFuse | b2::kFamSkinny | b2::kFamFlash | b2::kFamMove) \
   X(plan_gemm, b2::kFamFuse | b2::kFamGemm | b2::kFamSkinny) \
   X(plan_sgemm, b2::kFamFuse | b2::kFamSgemm)            \
-  X(plan_decode, b2::kFamFuse | b2::kFamSkinny | b2::kFamFlash | b2::kFamMove) \
   X(plan_f32, b2::kFamFuse | b2::kFamSgemm | b2::kFamFlash | b2::kFamMove) \
   X(plan_block, b2::kFamFuse | b2::kFamGemm | b2::kFamFlash | b2::kFamMove) \
   X(plan_attn, b2::kFamFuse | b2::kFamGemm | b2::kFamSgemm | b2::kFamSkinny | b2::kFamFlash | b2::kFamMove)

@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import glob
 import gzip
+import importlib
 import itertools
 import json
 import math
@@ -248,3 +249,15 @@ def test_epilogues_without_a_form_of_their_own(plan):
     for what, form in (("product", 0), ("residual", 3), ("gelu", 2), ("both", 3)):
         (t,) = [t for t in plan(progs.widened_product(256, 64, 256, "bf16", what).blob())["tasks"] if t["op"] == GEMM]
         assert [q["form"] for q in t["prob"]] == [form]
+
+
+def test_few_rows_side_by_side_lie_spread_over_the_device(plan):
+    """Tiles for 96 lanes of 148, two of three in use everywhere; on a kernel build that has the skinny products without the tiles of the
+    tensor-core ones, which cost them registers."""
+    p = plan(progs.products("bf16", *((16, 1024, 1024),) * 3).blob())
+    lanes = sorted(lane for t in p["tasks"] for lane, _, _ in t["cut"])
+    assert len(lanes) == len(set(lanes)) == 96 and all(0 < b - a <= 2 for a, b in zip(lanes, lanes[1:])) and lanes[0] == 0 and lanes[-1] >= 146
+    builds = importlib.import_module("pjrt-ocl_b200.build").variants()
+    gemm = int(re.search(r"kFamGemm = 1u << (\d+)", open(os.path.join(CSRC, "format.h")).read()).group(1))
+    name, families = next((n, m) for n, m in builds if m & p["families"] == p["families"])
+    assert name.startswith("plan") and not families >> gemm & 1
