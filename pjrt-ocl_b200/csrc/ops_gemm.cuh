@@ -56,12 +56,15 @@ __device__ __forceinline__ bool gemm_tile(const DGemm &g, uint32_t tile, GemmTil
   return true;
 }
 
+// How the general epilogue gets its residual: not at all, by prefetched 16-byte words, or element by element (f32, ragged rows). Each is
+// a function of its own: the words' registers would be missing in the others (a 16-bit product that leaves as f32, 4096 x 4096 by K =
+// 1024: 60 us with all in one, 50 so; 52 when the epilogue was part of gemm_tiles).
+enum GemmRes : uint32_t { kGrNone, kGrWords, kGrElems };
+struct GemmEpi { uint32_t epi, qdt, rdt; float s0, s1, gg; };
+__device__ __forceinline__ GemmRes gemm_res_of(const DGemmProb &pr) {
+  return !(pr.epi & kGeRes) ? kGrNone : pr.rdt != kF32 && (pr.N & 7u) == 0u ? kGrWords : kGrElems;
+}
 // The store epilogue on 32 consecutive columns of one row (plan_format.h: GemmEpi), in place.
-struct GemmEpi {
-  uint32_t flags, qdt, rdt;
-  float s0, s1, gg;
-  const uint8_t *res;
-};
 __device__ __forceinline__ void gemm_quant(float (&v)[32], uint32_t dt) {
   if (dt == kBF16) {
 #pragma unroll
@@ -77,29 +80,40 @@ __device__ __forceinline__ void gemm_quant(float (&v)[32], uint32_t dt) {
 }
 // Eight residual elements from memory (ragged edge, or f32); else they come out of a prefetched 16-byte word.
 __device__ __forceinline__ void gemm_res8(const uint8_t *row, uint32_t dt, uint32_t c, uint32_t left, float (&y)[8]) {
+  if (dt == kF32) {
+    const float *p = reinterpret_cast<const float *>(row) + c;
 #pragma unroll
-  for (uint32_t k = 0; k < 8u; ++k) y[k] = k < left ? loadf(row, dt, static_cast<int64_t>(c) + k) : 0.0f;
+    for (uint32_t k = 0; k < 8u; ++k) y[k] = k < left ? p[k] : 0.0f;
+  } else {
+    const uint16_t *p = reinterpret_cast<const uint16_t *>(row) + c;
+#pragma unroll
+    for (uint32_t k = 0; k < 8u; ++k) {
+      const uint32_t x = k < left ? p[k] : 0u;
+      y[k] = dt == kBF16 ? bf16_bits_to_f32(x) : f16_bits_to_f32(x);
+    }
+  }
 }
-__device__ __forceinline__ void gemm_epilogue(const GemmEpi &E, float (&v)[32], const uint8_t *res_row, const uint4 (&pre)[4], bool have_pre, uint32_t c,
-                                              uint32_t left, bool row_ok, float &csum) {
-  if (E.flags & kGeGelu) {
+template <GemmRes RES, typename Epi>
+__device__ __forceinline__ void gemm_epilogue(const Epi &E, float (&v)[32], const uint8_t *res_row, uint32_t stg, uint32_t lane, uint32_t c, uint32_t left,
+                                              bool row_ok, float &csum) {
+  if (E.epi & kGeGelu) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = gelu_tanh(v[j]);
   }
-  if (E.flags & kGeScale0) {
+  if (E.epi & kGeScale0) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = __fmul_rn(v[j], E.s0);
   }
-  if (E.flags & kGeMaxS) {
+  if (E.epi & kGeMaxS) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = np_max(v[j], E.s1);
   }
-  if (E.flags & kGeRes) {
-    const uint32_t op = E.flags & kGeResMask;
+  if constexpr (RES != kGrNone) {
+    const uint32_t op = E.epi & kGeResMask;
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       float y[8];
-      if (have_pre) unpack8(pre[b], E.rdt, y);
+      if (RES == kGrWords) unpack8(lds_v4(stg + lane * 64u + ((static_cast<uint32_t>(b) ^ ((lane >> 1) & 3u)) << 4)), E.rdt, y);
       else if (row_ok) gemm_res8(res_row, E.rdt, c + 8u * b, left > 8u * b ? left - 8u * b : 0u, y);
       else {
 #pragma unroll
@@ -124,13 +138,13 @@ __device__ __forceinline__ void gemm_epilogue(const GemmEpi &E, float (&v)[32], 
       }
     }
   }
-  if (E.flags & kGeCarrySq) {
+  if (E.epi & kGeCarrySq) {
     float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int j = 0; j < 32; ++j) if (row_ok && static_cast<uint32_t>(j) < left) a[j & 3] = __fadd_rn(a[j & 3], __fmul_rn(v[j], v[j]));
     csum += (a[0] + a[1]) + (a[2] + a[3]);
   }
-  if (E.flags & kGeScale1) {
+  if (E.epi & kGeScale1) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = __fmul_rn(v[j], E.s1);
   }
@@ -144,7 +158,7 @@ __device__ __forceinline__ void gemm_store(uint8_t *dst, uint32_t dt, uint32_t N
                                            uint32_t stg, uint32_t lane, const float (&v)[32]) {
   if (left == 0u) return;
   const uint32_t esz = dt == kF32 ? 4u : 2u;
-  if (vec && left == 32u) {
+  if (vec) {                                               // (and then whole 16-byte pieces are all there is)
     const uint32_t row = stg + lane * 64u, sw = (lane >> 1) & 3u, r8 = lane >> 2, ch = lane & 3u;
 #pragma unroll
     for (uint32_t h = 0; h < 2u; ++h) {                    // 16 columns of f32 fill the 64 bytes
@@ -173,7 +187,7 @@ __device__ __forceinline__ void gemm_store(uint8_t *dst, uint32_t dt, uint32_t N
         const uint32_t rr = 8u * p + r8;
         uint4 w;
         asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(stg + rr * 64u + ((ch ^ ((rr >> 1) & 3u)) << 4)) : "memory");
-        if (r_first + rr < M) stg_v4(out + p * step, w);
+        if (r_first + rr < M && h * 16u + ch * (16u / esz) < left) stg_v4(out + p * step, w);
       }
     }
     return;
@@ -209,52 +223,57 @@ __device__ __forceinline__ void gemm_slot_done(const GemmWarp &W, uint32_t n) {
 }
 
 // Any epilogue, its steps looked at chunk by chunk; the warp's tiles from `at` on as long as they want this.
+template <GemmRes RES>
 static __device__ __noinline__ GemmAt gemm_form_any(GemmWarp W, GemmAt at) {
   const DGemm &G = gemm_desc();
   const KParams &P = *W.P;
-  const uint32_t lane = W.lane;
+  const uint32_t lane = W.lane, r8 = lane >> 2, ch = lane & 3u, piece = W.stg + r8 * 64u + ((ch ^ ((r8 >> 1) & 3u)) << 4);
   GemmTile q;
-  for (; at.ok && gemm_tile(G, at.tile, q) && G.prob[q.prob].form == kGfAny; at.tile += W.n_slots) {
+  for (; at.ok && gemm_tile(G, at.tile, q) && G.prob[q.prob].form == kGfAny && gemm_res_of(G.prob[q.prob]) == RES; at.tile += W.n_slots) {
     const DGemmProb &pr = G.prob[q.prob];
-    GemmEpi E;
-    E.flags = pr.epi; E.qdt = pr.qdt; E.rdt = pr.rdt; E.s0 = pr.s0; E.s1 = pr.s1; E.gg = pr.gg;
-    E.res = (pr.epi & kGeRes) ? resolve(P, pr.res) : nullptr;
+    const GemmEpi own = {pr.epi, pr.qdt, pr.rdt, pr.s0, pr.s1, pr.gg};
+    // With the words' registers there are none to keep these in: they are read where they are wanted (78 us for 72, 8192 x 1024 by K = 4096
+    // times a 16-bit array; without the words 199 us for 205, 4096 x 4100 by K = 1024).
+    const auto &E = [&]() -> const auto & { if constexpr (RES == kGrWords) return pr; else return own; }();
+    const uint8_t *res = RES != kGrNone ? resolve(P, pr.res) : nullptr;
     uint8_t *out0 = pr.out0 ? resolve(P, pr.out0) : nullptr, *out1 = pr.out1 ? resolve(P, pr.out1) : nullptr;
     const uint32_t M = pr.M, N = pr.N;
-    const bool vec = (N & 7u) == 0u;                                    // 16-byte pieces of a row start on 16-byte boundaries
-    const bool pre_ok = E.res && E.rdt != kF32 && vec;       // residual by 16-byte words, a chunk ahead
+    const bool vec = RES == kGrWords || (N & 7u) == 0u;                 // 16-byte pieces of a row start on 16-byte boundaries
     for (uint32_t h = 0; h < q.halves; ++h, ++at.n) {
       const uint32_t rf = q.r0 + 128u * h + 32u * W.quarter, r = rf + lane, acc = W.tmem + ((32u * W.quarter) << 16) + (at.n & 1u) * 256u;
       const bool row_ok = r < M;
-      const uint8_t *res_row = E.res ? E.res + static_cast<size_t>(min(r, M - 1u)) * N * (E.rdt == kF32 ? 4u : 2u) : nullptr;
-      uint4 nxt[4];
+      const uint8_t *res_row = RES == kGrElems ? res + static_cast<size_t>(min(r, M - 1u)) * N * (E.rdt == kF32 ? 4u : 2u) : nullptr;
+      const uint32_t rows = M > rf + r8 ? (M - rf - r8 + 7u) / 8u : 0u;               // of this thread's four row pieces
+      uint4 nxt[4];                                          // the residual's words, a chunk ahead: 64-byte pieces of four rows
       auto prefetch = [&](uint32_t col) {
-        const uint32_t c = q.c0 + col;
+        const uint8_t *src = res + (static_cast<size_t>(rf + r8) * N + q.c0 + col + 8u * ch) * 2u;
 #pragma unroll
-        for (uint32_t k = 0; k < 4u; ++k)
-          nxt[k] = row_ok && c + 8u * k < N ? ldg_v4(res_row + static_cast<size_t>(c + 8u * k) * 2u) : make_uint4(0u, 0u, 0u, 0u);
+        for (uint32_t p = 0; p < 4u; ++p)
+          nxt[p] = p < rows && q.c0 + col + 8u * ch < N ? ldg_v4(src + static_cast<size_t>(p) * N * 16u) : make_uint4(0u, 0u, 0u, 0u);
       };
-      if (pre_ok && 32u * W.third < q.n_inst) prefetch(32u * W.third);
+      if (RES == kGrWords && 32u * W.third < q.n_inst) prefetch(32u * W.third);
       if (!gemm_slot_full(W, at.n)) { at.ok = false; return at; }
 #pragma unroll 1
       for (uint32_t col = 32u * W.third; col < q.n_inst; col += 96u) {
         uint32_t raw[32];
         __syncwarp();
         tc_ld32(acc + col, raw);
-        uint4 cur[4];
-        if (pre_ok) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) cur[k] = nxt[k];
-          if (col + 96u < q.n_inst) prefetch(col + 96u);
-        }
         tc_wait_ld();
         const uint32_t c = q.c0 + col, left = c < N ? min(32u, N - c) : 0u;
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
-        if (E.flags & kGeQuant0) gemm_quant(v, E.qdt);
+        if (E.epi & kGeQuant0) gemm_quant(v, E.qdt);
         if (out0) gemm_store(out0, pr.dt0, N, rf, M, c, left, vec, W.stg, lane, v);
-        gemm_epilogue(E, v, res_row, cur, pre_ok, c, left, row_ok, at.csum);
+        if (RES == kGrWords) {
+          __syncwarp();
+#pragma unroll
+          for (uint32_t p = 0; p < 4u; ++p) sts_v4(piece + 512u * p, nxt[p]);
+          if (col + 96u < q.n_inst) prefetch(col + 96u);
+          __syncwarp();
+        }
+        gemm_epilogue<RES>(E, v, res_row, W.stg, lane, c, left, row_ok, at.csum);
+        if (RES == kGrWords) __syncwarp();
         if (out1) gemm_store(out1, pr.dt1, N, rf, M, c, left, vec, W.stg, lane, v);
       }
       gemm_slot_done(W, at.n);
@@ -546,7 +565,13 @@ static __device__ __noinline__ void gemm_tiles(const Lane &L, const DTask &t, ui
         B2_GEMM_FORM(kGfStep, kGeScale0 | kGeRes | kGeResRSub)
         B2_GEMM_FORM(kGfLoss, kGeRes | kGeResSub | kGeCarrySq | kGeScale1)
 #undef B2_GEMM_FORM
-        default: at = gemm_form_any(W, at); break;
+        default:
+          switch (gemm_res_of(G.prob[q.prob])) {
+            case kGrNone: at = gemm_form_any<kGrNone>(W, at); break;
+            case kGrWords: at = gemm_form_any<kGrWords>(W, at); break;
+            default: at = gemm_form_any<kGrElems>(W, at); break;
+          }
+          break;
       }
     }
     csum = at.csum;

@@ -60,11 +60,11 @@ def widened_product(M, K, N, dtype, what):
 
 
 def product_then(M, K, N, dtype, what, transposed=False):
-    """A 16-bit product and what follows it in its own type: nothing, a residual, GELU (with the product kept: "kept"); or as in a
-    training step: times GELU's derivative at x ("grad"), x less a thousandth of it ("step"), its difference to x scaled, and the sum
+    """A 16-bit product and what follows it in its own type: nothing, a residual, a product with x ("times"), GELU (with the product
+    kept: "kept"); the f32 sum with an f32 x ("wide"); or as in a training step: times GELU's derivative at x ("grad"), x less a thousandth of it ("step"), its difference to x scaled, and the sum
     of the difference's squares ("loss")."""
     p = cases._Assembler(148)
-    a, w, x = p.input((M, K), dtype), p.input((N, K) if transposed else (K, N), dtype), p.input((M, N), dtype)
+    a, w, x = p.input((M, K), dtype), p.input((N, K) if transposed else (K, N), dtype), p.input((M, N), "f32" if what == "wide" else dtype)
     y = p.matmul(a, w, M, N, K, "f32" if what == "step" else dtype, vb=p.view((K, N), (1, K)) if transposed else 0)
     if what == "kept":
         p.output(y, (M, N))
@@ -74,6 +74,10 @@ def product_then(M, K, N, dtype, what, transposed=False):
         p.phase()
     if what == "residual":
         y = p.chain((cases._ADD, (x, y), dtype))
+    elif what == "times":
+        y = p.chain((cases._MUL, (y, x), dtype))
+    elif what == "wide":
+        y = p.chain((cases._CONVERT, (y,), "f32"), (cases._ADD, (-1, x), "f32"))
     elif what in ("gelu", "kept"):
         y = p.chain((cases._GELU, (y,), dtype))
     elif what == "grad":

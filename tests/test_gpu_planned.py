@@ -200,7 +200,7 @@ def test_product_converted_after_a_16_bit_value(what, mnk):
         assert torch.equal(out, y.float())
 
 
-@pytest.mark.parametrize("what", ["product", "residual", "gelu", "kept", "grad", "step", "loss"])
+@pytest.mark.parametrize("what", ["product", "residual", "gelu", "kept", "grad", "step", "loss", "times", "wide"])
 @pytest.mark.parametrize("M, K, N, dtype, transposed", [
     (33, 64, 8, "bf16", False), (128, 72, 104, "f16", False), (129, 200, 264, "bf16", False), (300, 1096, 520, "f16", True), (200, 64, 99, "bf16", True),
     (2100, 136, 1032, "bf16", False), (9600, 64, 4104, "f16", False)])
@@ -212,12 +212,14 @@ def test_store_epilogues_at_the_edges_of_tiles(what, M, K, N, dtype, transposed)
     dt = {"bf16": torch.bfloat16, "f16": torch.float16}[dtype]
     gen = torch.Generator(device="cuda").manual_seed(1)
     a, w, x = (torch.randint(-3, 4, s, generator=gen, device="cuda").to(dt) for s in ((M, K), (N, K) if transposed else (K, N), (M, N)))
-    lp, outs = _execute(progs.product_then(M, K, N, dtype, what, transposed), [a, w, x])
+    lp, outs = _execute(progs.product_then(M, K, N, dtype, what, transposed), [a, w, x.float() if what == "wide" else x])
     assert lp.stat("tensor_core_matmuls") == 1
     y = (a.double() @ (w.T if transposed else w).double()).float()
     if what == "step":
         assert torch.equal(outs[0], (x.float() - y * torch.tensor(1e-3, device="cuda")).to(dt))
     y = y.to(dt)
+    if what in ("times", "wide"):
+        assert torch.equal(outs[0], y * x if what == "times" else y.float() + x.float())
     if what == "loss":
         d = y.float() - x.float()
         total, scaled = outs

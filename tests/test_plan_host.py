@@ -231,7 +231,7 @@ def test_products_with_tiles_for_everybody_are_spread_over_all_lanes(plan):
 
 
 # ops_gemm.cuh: an epilogue that is compiled for its steps (+ 16: of f16), 0 the general one
-FORMS = {"product": 1, "gelu": 2, "kept": 2, "residual": 3, "grad": 4, "step": 5, "loss": 6}
+FORMS = {"product": 1, "gelu": 2, "kept": 2, "residual": 3, "grad": 4, "step": 5, "loss": 6, "times": 0, "wide": 0}
 
 
 @pytest.mark.parametrize("what", FORMS)
@@ -240,7 +240,7 @@ FORMS = {"product": 1, "gelu": 2, "kept": 2, "residual": 3, "grad": 4, "step": 5
 def test_epilogues_run_in_the_form_for_their_steps(plan, what, M, K, N, dtype, transposed, general):
     p = plan(progs.product_then(M, K, N, dtype, what, transposed).blob())
     (t,) = [t for t in p["tasks"] if t["op"] == GEMM]
-    assert [q["form"] for q in t["prob"]] == [0 if general else FORMS[what] + (16 if dtype == "f16" else 0)]
+    assert [q["form"] for q in t["prob"]] == [0 if general or not FORMS[what] else FORMS[what] + (16 if dtype == "f16" else 0)]
     assert not [t for t in p["tasks"] if t["op"] not in (GEMM, FUSE_ROWS) and t["cut"]]
 
 
