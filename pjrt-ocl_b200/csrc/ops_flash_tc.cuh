@@ -9,8 +9,9 @@
 // (viewed) layouts three rank-4 TMA tensor maps can describe (DFlash::tc_mode; the
 // loader decides), so a [batch, seq, heads, hd] projection is attended in place.
 //
-// Bound: the exponentials. The special-function units take 16 a cycle and SM, 512 cycles for 128 rows x 64 keys, where the two
-// products take ~330. To keep them fed a lane works on three query tiles of 128 rows at a time ("slots"), independent of
+// Bound: latency. Of the units the exponentials' is the busiest: 16 a cycle and SM, 512 cycles for 128 rows x 64 keys, where the two
+// products take ~330; it is 47 % busy (8 x 2048 causal, 16 heads: 141 us, 66 of them exponentials). A block takes a slot alone 1870
+// cycles, three slots together 2750 for 1536 of exponentials. To fill them a lane works on three query tiles of 128 rows at a time ("slots"), independent of
 // each other: each has its own softmax warps (one of each on every scheduler), its own feeding warp, its own Q, K and V in shared
 // memory and its own columns of tensor memory, draws its own tiles, and waits for nobody else. (Two slots that shared one
 // stream of 128-key blocks, one issuing warp looking after both and P in shared memory: 6300 cycles per block and slot, of which

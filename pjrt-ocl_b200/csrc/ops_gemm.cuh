@@ -286,7 +286,7 @@ static __device__ __noinline__ GemmAt gemm_form_any(GemmWarp W, GemmAt at) {
 // read 16-bit of one type (BF: bf16), rows whole 16-byte words. Such a form is a function of its own, entered once for all of the
 // warp's tiles in a row that want it, so that what a chunk needs stays in registers: the lane's shared memory leaves hardly any
 // L1, every use of a spilled value is a trip to L2, and the general form has its steps as branches and predicates. A 256 x 256
-// tile that only leaves as bf16 takes 7000 cycles here, 22000 in the general form (2 tiles of K = 64: 31 us, now 15.5); what is left
+// tile that only leaves as bf16 takes 7000 cycles here, 22000 with all steps in one function (2 tiles of K = 64: 31 us, now 15.5); what is left
 // is mostly the SM's way to L2, 32 bytes a cycle. Rows of the residual come as the result goes: whole 64-byte row pieces through the
 // warp's slab, a chunk ahead. Tried: all of a tile's chunks held in registers first and stored when the slots are given back
 // (more code and registers, slower: 110 us against 107 for 16384 x 4096 by K = 1024); 32-byte stores from the rows as they come

@@ -5,9 +5,9 @@
 // shared memory as float4, a thread keeps NI bodies i and their sums in registers and walks the
 // j's of its slice.
 //
-// Bound: 22 us per evaluation of 4096 bodies in a loop of them (40 evaluations 898 us). By count the pairs are 7-8 us of FP32
-// issue (16.8 M of ~16 instructions on 148 SMs) and 3.6 us of square roots, the barrier 1.2; what the rest waits for has not
-// been measured.
+// Bound: 18.8 us per evaluation of 4096 bodies in a loop of them (40 evaluations 763 us): 10.4 the pair loop - 7-8 of FP32 issue by count
+// (16.8 M pairs of ~16 instructions on 148 SMs) beside 3.6 of square roots -, 3 the staging of all bodies, 1.2 the grid barrier, the
+// rest sums, tail and set-up. Issue is 45 % active; barriers, of the lane and of the grid, are the top stall.
 //
 // Split: a lane owns bodies [lo, hi). Its 16 warps form `groups` i-groups (NI bodies each, all 32
 // lanes of a warp the same ones) x 16 / groups j-slices; groups x NI is the smallest cover of the

@@ -104,8 +104,10 @@ enum GemmEpi_ : uint32_t {
   kGeCarrySq = 32u,        // add its square to the task's full sum
   kGeScale1 = 64u          // times s1
 };
-// Epilogues that have a form of their own on the device (ops_gemm.cuh): what the programs of the benchmark configurations leave
-// after a product. kGfF16 is added for f16.
+// Epilogues that have a form of their own on the device (ops_gemm.cuh): what a layer leaves after a product going forward (itself, GELU,
+// a sum with a residual) and in a training step (GELU's derivative, the update, the loss). Every form is code in each build with
+// products; the rest, and what leaves as f32 or in rows that are no whole 16-byte words, takes the general epilogue (4096 x 4096 by
+// K = 1024 times an array 62 us, plus one by its form 47; as f32 50, as bf16 by its form 37). kGfF16 is added for f16.
 enum GemmForm : uint32_t { kGfAny = 0, kGfPlain, kGfGelu, kGfAdd, kGfGrad, kGfStep, kGfLoss, kGfF16 = 16 };
 // One 16-bit type throughout, whole 16-byte words, and a second result only where a form stores it.
 inline uint32_t gemm_form_of(uint32_t epi, uint32_t N, bool out0, bool out1, uint32_t dt0, uint32_t dt1, uint32_t qdt, uint32_t rdt) {

@@ -1179,8 +1179,9 @@ void Planner::SgShape(uint32_t op, uint64_t M, uint64_t N, uint64_t K, uint32_t 
 }
 
 // Matmuls of one phase become one task (deepest first), and every product gets its tile shape. A lane's time for a tile is
-// the larger of its tensor cycles (2 per column and half, per 64 k) and what it pulls through L2 (~36 bytes per cycle and SM: what
-// 128 x 256 tiles were measured to get), plus the part of the epilogue that nothing hides.
+// the larger of its tensor cycles (2 per column and half, per 64 k) and what it pulls through L2 (~36 bytes per cycle and SM), plus
+// the part of the epilogue that nothing hides. The constants were measured with one copying thread and the general epilogue: absolute times
+// come out too long (8192 cubed at least 830 us at the top clock, measured 694 at a lower one); they only rank the shapes.
 void Planner::GroupGemms(std::vector<int> *live, std::map<std::pair<int, int>, std::vector<int>> *phases, std::vector<std::vector<int>> *of) {
   for (auto &kv : *phases) {
     std::vector<int> gs, rest;

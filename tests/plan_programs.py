@@ -61,18 +61,18 @@ def widened_product(M, K, N, dtype, what):
 
 def product_then(M, K, N, dtype, what, transposed=False):
     """A 16-bit product and what follows it in its own type: nothing, a residual, a product with x ("times"), GELU (with the product
-    kept: "kept"); the f32 sum with an f32 x ("wide"); or as in a training step: times GELU's derivative at x ("grad"), x less a thousandth of it ("step"), its difference to x scaled, and the sum
+    kept: "kept"), a residual with the product kept ("both"); the f32 sum with an f32 x ("wide"); or as in a training step: times GELU's derivative at x ("grad"), x less a thousandth of it ("step"), its difference to x scaled, and the sum
     of the difference's squares ("loss")."""
     p = cases._Assembler(148)
     a, w, x = p.input((M, K), dtype), p.input((N, K) if transposed else (K, N), dtype), p.input((M, N), "f32" if what == "wide" else dtype)
     y = p.matmul(a, w, M, N, K, "f32" if what == "step" else dtype, vb=p.view((K, N), (1, K)) if transposed else 0)
-    if what == "kept":
+    if what in ("kept", "both"):
         p.output(y, (M, N))
     if what in ("grad", "step"):
         xf = p.chain((cases._CONVERT, (x,), "f32"))
     if what != "product":
         p.phase()
-    if what == "residual":
+    if what in ("residual", "both"):
         y = p.chain((cases._ADD, (x, y), dtype))
     elif what == "times":
         y = p.chain((cases._MUL, (y, x), dtype))

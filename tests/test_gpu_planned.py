@@ -200,7 +200,7 @@ def test_product_converted_after_a_16_bit_value(what, mnk):
         assert torch.equal(out, y.float())
 
 
-@pytest.mark.parametrize("what", ["product", "residual", "gelu", "kept", "grad", "step", "loss", "times", "wide"])
+@pytest.mark.parametrize("what", ["product", "residual", "gelu", "kept", "grad", "step", "loss", "times", "wide", "both"])
 @pytest.mark.parametrize("M, K, N, dtype, transposed", [
     (33, 64, 8, "bf16", False), (128, 72, 104, "f16", False), (129, 200, 264, "bf16", False), (300, 1096, 520, "f16", True), (200, 64, 99, "bf16", True),
     (2100, 136, 1032, "bf16", False), (9600, 64, 4104, "f16", False)])
@@ -231,10 +231,10 @@ def test_store_epilogues_at_the_edges_of_tiles(what, M, K, N, dtype, transposed)
         slope, = torch.autograd.grad(_gelu(z).sum(), z)
         want = y.double() * slope
         assert bool(((outs[0].double() - want).abs() <= (2.0 ** -8 if dtype == "bf16" else 2.0 ** -11) * want.abs() + 2e-6 * y.double().abs()).all())
-    if what in ("product", "kept"):
+    if what in ("product", "kept", "both"):
         assert torch.equal(outs[0], y)
-    if what == "residual":
-        assert torch.equal(outs[0], (x.float() + y.float()).to(dt))
+    if what in ("residual", "both"):
+        assert torch.equal(outs[-1], (x.float() + y.float()).to(dt))
     if what in ("gelu", "kept"):
         want = _gelu(y.double())
         assert bool(((outs[-1].double() - want).abs() <= (2.0 ** -8 if dtype == "bf16" else 2.0 ** -11) * want.abs() + 1e-6).all())

@@ -231,7 +231,7 @@ def test_products_with_tiles_for_everybody_are_spread_over_all_lanes(plan):
 
 
 # ops_gemm.cuh: an epilogue that is compiled for its steps (+ 16: of f16), 0 the general one
-FORMS = {"product": 1, "gelu": 2, "kept": 2, "residual": 3, "grad": 4, "step": 5, "loss": 6, "times": 0, "wide": 0}
+FORMS = {"product": 1, "gelu": 2, "kept": 2, "residual": 3, "grad": 4, "step": 5, "loss": 6, "times": 0, "wide": 0, "both": 0}
 
 
 @pytest.mark.parametrize("what", FORMS)
